@@ -284,6 +284,7 @@ static int launch_p(pgld_context* h, const BandArgs& a, cudaStream_t st) {
 
 int launch_band_plain(pgld_context* h, const BandArgs& a, int mode, cudaStream_t st) {
   if (band_fast_applies(a, mode)) return launch_band_fast(h, a, mode, st);
+  if (band_multi_applies(a, mode)) return launch_band_multi(h, a, st);
   if (mode == kModePairs) return launch_p<1, kModePairs>(h, a, st);
   switch (a.n_pops) {
     case 1: return launch_p<1, kModeBinned>(h, a, st);

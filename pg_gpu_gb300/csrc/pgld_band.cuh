@@ -63,5 +63,8 @@ int launch_band_plain(pgld_context* h, const BandArgs& a, int mode, cudaStream_t
 // the one/two-population kernel with the float32 epilogue (pgld_band_fast.cu)
 bool band_fast_applies(const BandArgs& a, int mode);
 int launch_band_fast(pgld_context* h, const BandArgs& a, int mode, cudaStream_t st);
+// binned sums of three or four populations in float32 (pgld_band_multi.cu)
+bool band_multi_applies(const BandArgs& a, int mode);
+int launch_band_multi(pgld_context* h, const BandArgs& a, cudaStream_t st);
 
 }  // namespace pgld
