@@ -37,6 +37,7 @@
 #include "pgld_geno_mom.cuh"
 #include "pgld_internal.cuh"
 #include "pgld_geno.cuh"
+#include "pgld_multi_sum.cuh"
 #include "pgld_scan.cuh"
 #include "pgld_tc_common.cuh"
 #include "pgld_tcgen05.cuh"
@@ -508,12 +509,14 @@ __global__ void __launch_bounds__(256) pack_gtc_kernel(const uint32_t* __restric
 // (the operand rows of population p start at row p * n_blocks * 96), each
 // into its own 96 TMEM columns of the tile's accumulator stage.  One
 // population: DD, Dz and pi2 in float32 straight from the moments
-// (gmom::stats_f32).  Several: the epilogue turns each population's moments
-// into 9-way counts and evaluates the term table of the statistics (the
-// exact 64-bit integer forms of the popcount kernel, pgld_geno.cuh) per pair,
-// which costs far more than the counting (the form is then as fast as the
-// popcount one).  Sums per distance bin in float64 slots of the CTA.  G epilogue groups take alternate tiles: G = 2 for at most two
-// populations (two accumulator stages of 256 columns), G = 1 for three or
+// (gmom::stats_f32).  Several: the group orders the tile's pairs by distance
+// bin and its warps take them in steps of 32 pairs of one bin, the statistics
+// unrolled in float32 from the moments (pgld_multi.cuh); the rare pair with
+// fewer than four valid individuals in a population, where the reference's
+// thresholds and zero denominators differ from statistic to statistic, goes
+// through the exact term table by itself.  Sums per distance bin in float64
+// slots of the CTA.  G epilogue groups take alternate tiles: G = 2 for at most
+// two populations (two accumulator stages of 256 columns), G = 1 for three or
 // four (one stage of 384 columns).
 // ---------------------------------------------------------------------------
 struct BParams {
@@ -525,9 +528,12 @@ struct BParams {
   int pop_rows;             // operand rows per population (n_blocks * 96)
   const double* pos;
   const double* bcoord;     // distances for binning (NULL: positions)
+  const int* ipos;          // integer positions (valid when *ipos_bad == 0)
+  const int* ipos_bad;
   double max_dist;
   const double* bins;
   int n_bins;
+  int exact;                // every pair through the term table (samples above multi::kMaxN)
   const pgld_term* terms;
   int n_terms, n_stats;
   double* sums;             // [n_bins][n_stats]
@@ -536,25 +542,50 @@ struct BParams {
   int stages;
 };
 
-template <int G>
+// the statistics of one pair through the exact term table, added to slots
+template <int P>
+__device__ __noinline__ void term_table_pair(const gmom::Mom* mo, const BParams& a, double* slots) {
+  int cc[P][9];
+  geno::GPop gp[P];
+  const int* cp[P];
+  for (int p = 0; p < P; ++p) {
+    gmom::to_counts(mo[p], cc[p]);
+    gp[p] = geno::make_gpop(cc[p], -1);
+    cp[p] = cc[p];
+  }
+  int t = 0;
+  for (int s = 0; s < a.n_stats; ++s) {
+    float v = 0.f;
+    for (; t < a.n_terms && a.terms[t].stat == s; ++t) {
+      const pgld_term tm = a.terms[t];
+      v += (float)tm.weight * geno::term_value<float>(tm, gp, cp);
+    }
+    atomicAdd(slots + s, (double)v);
+  }
+}
+
+template <int P>
 __global__ void __launch_bounds__(kThreads, 1)
-    gtc_binned_kernel(const __grid_constant__ CUtensorMap map, BParams a) {
+    gtc_binned_kernel(const __grid_constant__ CUtensorMap map, const __grid_constant__ BParams a,
+                      const __grid_constant__ multi::Places pl) {
+  constexpr int G = P <= 2 ? 2 : 1;
   constexpr int kGW = kEpiWarps / G;   // warps per epilogue group
-  constexpr int kPMax = G == 2 ? 2 : 4;
+  constexpr int kRows = 32 / kGW;      // rows of a tile per warp
   constexpr uint32_t kStageCols = G == 2 ? 256u : 0u;
   extern __shared__ unsigned char smem_dyn[];
   unsigned char* base = smem_dyn + ((1024 - (smem_u32(smem_dyn) & 1023)) & 1023);
   const int stages = a.stages;
   unsigned char* ring = base;
   GCtrl* ctrl = reinterpret_cast<GCtrl*>(ring + (size_t)stages * kGStageBytes);
-  int16_t* cnt = reinterpret_cast<int16_t*>(ctrl + 1);  // [G][kPMax][96][kCntPitch]
-  double* sbins = reinterpret_cast<double*>(cnt + (size_t)G * kPMax * 96 * kCntPitch);
+  int16_t* cnt = reinterpret_cast<int16_t*>(ctrl + 1);  // [G][P][96][kCntPitch]
+  double* sbins = reinterpret_cast<double*>(cnt + (size_t)G * P * 96 * kCntPitch);
   double* acc = sbins + (kMaxBins + 1);                 // [n_bins][n_stats]
   unsigned long long* bcnt =
       reinterpret_cast<unsigned long long*>(acc + (size_t)a.n_bins * a.n_stats);
+  int* thr = reinterpret_cast<int*>(bcnt + a.n_bins);   // ceil(bins[k]), integer distances
+  multi::Groups<kGW>* groups = reinterpret_cast<multi::Groups<kGW>*>(thr + kMaxBins + 2);  // [G]
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   volatile int* abort_flag = &ctrl->abort_flag;
-  const int P = a.n_pops;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < stages; ++s) {
@@ -584,7 +615,11 @@ __global__ void __launch_bounds__(kThreads, 1)
   }
   for (int x = threadIdx.x; x < a.n_bins * a.n_stats; x += blockDim.x) acc[x] = 0.0;
   for (int x = threadIdx.x; x < a.n_bins; x += blockDim.x) bcnt[x] = 0ull;
-  for (int x = threadIdx.x; x <= a.n_bins; x += blockDim.x) sbins[x] = a.bins[x];
+  for (int x = threadIdx.x; x <= a.n_bins; x += blockDim.x) {
+    const double b = a.bins[x], cb = ceil(b);
+    sbins[x] = b;
+    thr[x] = cb > 2147483647.0 ? 2147483647 : (cb < -2147483647.0 ? -2147483647 : (int)cb);
+  }
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   tc_fence_before();
   __syncthreads();
@@ -696,7 +731,9 @@ __global__ void __launch_bounds__(kThreads, 1)
     const int wq = warp & 3;               // TMEM lane quarter: plane wq of the SNPs i
     const uint32_t lane_base = (uint32_t)(wq * 32) << 16;
     const uint32_t bar_id = 1u + (uint32_t)grp;
-    int16_t* gbuf = cnt + (size_t)grp * kPMax * 96 * kCntPitch;
+    int16_t* gbuf = cnt + (size_t)grp * P * 96 * kCntPitch;
+    const bool use_int = a.bcoord == nullptr && *a.ipos_bad == 0;
+    const int maxd_int = a.max_dist >= 2147483647.0 ? 2147483647 : (int)floor(a.max_dist);
     long long lo = 0;
     for (int t = grp, u = 0;; t += G, ++u) {
       const long long item = (long long)blockIdx.x + (long long)t * gridDim.x;
@@ -749,6 +786,75 @@ __global__ void __launch_bounds__(kThreads, 1)
       const long long i0 = lo * kTileSnp, j0 = (lo + (item - a.item_off[lo])) * kTileSnp;
       const long long j = j0 + lane;
       const bool j_ok = j < a.n_snp;
+      if constexpr (P > 1) {
+        // bins of the warp's rows, then the tile's pairs grouped by bin
+        int bin[kRows];
+        if (use_int) {
+          const int pj = j_ok ? a.ipos[j] : 0;
+          const int pi = i0 + lane < a.n_snp ? a.ipos[i0 + lane] : 0;
+#pragma unroll
+          for (int q = 0; q < kRows; ++q) {
+            const int il = gi * kRows + q;
+            const int d = pj - __shfl_sync(0xffffffffu, pi, il);
+            bin[q] = i0 + il < j && j_ok && d <= maxd_int ? bin_of_int(thr, a.n_bins, d) : -1;
+          }
+        } else {
+          const double pj = j_ok ? a.pos[j] : 0.0;
+          const double cj = (j_ok && a.bcoord) ? a.bcoord[j] : 0.0;
+#pragma unroll
+          for (int q = 0; q < kRows; ++q) {
+            const long long i = i0 + gi * kRows + q;
+            bin[q] = -1;
+            if (i < j && j_ok) {
+              const double dpos = pj - a.pos[i];
+              if (dpos <= a.max_dist)
+                bin[q] = bin_of_f64(sbins, a.n_bins, a.bcoord ? fabs(cj - a.bcoord[i]) : dpos);
+            }
+          }
+        }
+        multi::Groups<kGW>& g = groups[grp];
+        multi::group_pairs<kGW, kRows>(g, bin, gi * kRows, gi, a.n_bins, bcnt, [&] {
+          asm volatile("bar.sync %0, %1;" ::"r"(bar_id), "r"(kGW * 32) : "memory");
+        });
+        // with two passes over the steps the first takes the term-table pairs
+        auto load = [&](int pair, int b, multi::Geno(&f)[P], bool first) {
+          gmom::Mom mo[P];
+          const int il = (pair >> 5) & 31, jl = pair & 31;
+          int n_least = 1 << 20;
+#pragma unroll
+          for (int p = 0; p < P; ++p) {
+            const int16_t* bp = gbuf + (size_t)p * 96 * kCntPitch;
+#pragma unroll
+            for (int x = 0; x < 3; ++x)
+#pragma unroll
+              for (int y = 0; y < 3; ++y)
+                mo[p].m[3 * x + y] = bp[(x * 32 + il) * kCntPitch + y * 32 + jl];
+            n_least = min(n_least, mo[p].m[0]);
+          }
+          const bool live = pair < multi::kGroupPairs;
+          const bool table = live && (n_least < 4 || a.exact);
+          if (table && first) term_table_pair<P>(mo, a, acc + b * a.n_stats);
+          if (!live || table) {
+#pragma unroll
+            for (int p = 0; p < P; ++p)
+#pragma unroll
+              for (int x = 0; x < 9; ++x) mo[p].m[x] = 0;
+          }
+#pragma unroll
+          for (int p = 0; p < P; ++p) f[p] = multi::make_geno(mo[p]);
+        };
+        const int s0 = g.n_steps * gi / kGW, s1 = g.n_steps * (gi + 1) / kGW;
+        multi::sum_steps<P, 0, multi::Geno>(
+            g, s0, s1, acc, a.n_stats, pl,
+            [&](int pair, int b, multi::Geno(&f)[P]) { load(pair, b, f, true); });
+        if constexpr (P == 4)
+          multi::sum_steps<P, 1, multi::Geno>(
+              g, s0, s1, acc, a.n_stats, pl,
+              [&](int pair, int b, multi::Geno(&f)[P]) { load(pair, b, f, false); });
+        continue;
+      }
+      // one population: DD, Dz, pi2 in float32 from the moments
+      // (gmom::stats_f32, within 1e-6 relative of each exact value)
       const double pj = j_ok ? a.pos[j] : 0.0;
       const double cj = (j_ok && a.bcoord) ? a.bcoord[j] : 0.0;
 #pragma unroll 1
@@ -768,68 +874,28 @@ __global__ void __launch_bounds__(kThreads, 1)
         }
         unsigned pending = __ballot_sync(0xffffffffu, b >= 0);
         if (!pending) continue;
-        if (P == 1) {
-          // one population: DD, Dz, pi2 in float32 from the moments
-          // (gmom::stats_f32, within 1e-6 relative of each exact value)
-          gmom::Mom mo;
+        gmom::Mom mo;
 #pragma unroll
-          for (int x = 0; x < 3; ++x)
+        for (int x = 0; x < 3; ++x)
 #pragma unroll
-            for (int y = 0; y < 3; ++y)
-              mo.m[3 * x + y] = gbuf[(x * 32 + il) * kCntPitch + y * 32 + lane];
-          const float4 o4 = gmom::stats_f32<14>(mo, 14);
-          while (pending) {
-            const int bb = __shfl_sync(0xffffffffu, b, __ffs(pending) - 1);
-            const bool mine = (b == bb);
-            const unsigned grpm = __ballot_sync(0xffffffffu, mine);
-            float v[3] = {mine ? o4.y : 0.f, mine ? o4.z : 0.f, mine ? o4.w : 0.f};
-#pragma unroll
-            for (int q = 0; q < 3; ++q) {
-#pragma unroll
-              for (int o = 16; o > 0; o >>= 1) v[q] += __shfl_xor_sync(0xffffffffu, v[q], o);
-            }
-            if (lane == 0) {
-#pragma unroll
-              for (int q = 0; q < 3; ++q) atomicAdd(&acc[bb * 3 + q], (double)v[q]);
-              atomicAdd(&bcnt[bb], (unsigned long long)__popc(grpm));
-            }
-            pending &= ~grpm;
-          }
-          continue;
-        }
-        int cc[kPMax][9];
-        geno::GPop gp[kPMax];
-        const int* cp[kPMax];
-#pragma unroll
-        for (int p = 0; p < kPMax; ++p) {
-          if (p < P) {
-            gmom::Mom mo;
-            const int16_t* bp = gbuf + (size_t)p * 96 * kCntPitch;
-#pragma unroll
-            for (int x = 0; x < 3; ++x)
-#pragma unroll
-              for (int y = 0; y < 3; ++y) mo.m[3 * x + y] = bp[(x * 32 + il) * kCntPitch + y * 32 + lane];
-            gmom::to_counts(mo, cc[p]);
-            gp[p] = geno::make_gpop(cc[p], -1);
-          }
-          cp[p] = cc[p];
-        }
+          for (int y = 0; y < 3; ++y)
+            mo.m[3 * x + y] = gbuf[(x * 32 + il) * kCntPitch + y * 32 + lane];
+        const float4 o4 = gmom::stats_f32<14>(mo, 14);
         while (pending) {
           const int bb = __shfl_sync(0xffffffffu, b, __ffs(pending) - 1);
           const bool mine = (b == bb);
           const unsigned grpm = __ballot_sync(0xffffffffu, mine);
-          int tt = 0;
-          for (int s = 0; s < a.n_stats; ++s) {
-            float v = 0.f;
-            for (; tt < a.n_terms && a.terms[tt].stat == s; ++tt) {
-              const pgld_term tm = a.terms[tt];
-              if (mine) v += (float)tm.weight * geno::term_value<float>(tm, gp, cp);
-            }
+          float v[3] = {mine ? o4.y : 0.f, mine ? o4.z : 0.f, mine ? o4.w : 0.f};
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-            if (lane == 0) atomicAdd(&acc[bb * a.n_stats + s], (double)v);
+          for (int q = 0; q < 3; ++q) {
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) v[q] += __shfl_xor_sync(0xffffffffu, v[q], o);
           }
-          if (lane == 0) atomicAdd(&bcnt[bb], (unsigned long long)__popc(grpm));
+          if (lane == 0) {
+#pragma unroll
+            for (int q = 0; q < 3; ++q) atomicAdd(&acc[bb * 3 + q], (double)v[q]);
+            atomicAdd(&bcnt[bb], (unsigned long long)__popc(grpm));
+          }
           pending &= ~grpm;
         }
       }
@@ -945,6 +1011,9 @@ int pgld_geno_tc_pairs(pgld_context* h, const pgld_geno_panel* panel, const doub
   return PGLD_OK;
 }
 
+int pgld_tc_int_positions(pgld_context* h, const double* pos, long long n, int* ipos, int* bad,
+                          cudaStream_t st);
+
 // Genotype distance-binned sums on the tensor cores: 1-4 populations of
 // dosages 0/1/2 (missing allowed, no values above 2), at most kMaxGenoN
 // individuals each; ba carries the bins, term table and outputs (sums and
@@ -966,7 +1035,8 @@ int pgld_geno_tc_binned(pgld_context* h, const pgld_geno_panel* panel, const pgl
   const size_t sb = pgld::scan_scratch_bytes(nb);
   auto al = [](size_t x) { return (x + 1023) & ~size_t(1023); };
   const size_t off_items = 0, off_scan = al((nb + 1) * 8), off_op = off_scan + al(sb),
-               total = off_op + al(op_pop * P);
+               off_ipos = off_op + al(op_pop * P), off_bad = off_ipos + al((size_t)n * 4),
+               total = off_bad + 1024;
   void* ws = nullptr;
   rc = pgld_workspace(h, total, &ws);
   if (rc) return rc;
@@ -982,6 +1052,10 @@ int pgld_geno_tc_binned(pgld_context* h, const pgld_geno_panel* panel, const pgl
   }
   rc = pgld::band_schedule(h, ba.pos, n, ba.max_dist, items, w + off_scan, sb, st, kTileSnp);
   if (rc) return rc;
+  int* ipos = (int*)(w + off_ipos);
+  int* ipos_bad = (int*)(w + off_bad);
+  rc = pgld_tc_int_positions(h, ba.pos, n, ipos, ipos_bad, st);
+  if (rc) return rc;
   CUtensorMap map;
   rc = pgld::tchost::make_map(h, &map, op, (long long)P * nb * kBlkRows, k_pad, kBlkRows);
   if (rc) return rc;
@@ -994,9 +1068,12 @@ int pgld_geno_tc_binned(pgld_context* h, const pgld_geno_panel* panel, const pgl
   prm.pop_rows = (int)(nb * kBlkRows);
   prm.pos = ba.pos;
   prm.bcoord = ba.bcoord;
+  prm.ipos = ipos;
+  prm.ipos_bad = ipos_bad;
   prm.max_dist = ba.max_dist;
   prm.bins = ba.bins;
   prm.n_bins = ba.n_bins;
+  prm.exact = 32 * W > pgld::multi::kMaxN;
   prm.terms = ba.terms;
   prm.n_terms = ba.n_terms;
   prm.n_stats = ba.n_stats;
@@ -1004,10 +1081,11 @@ int pgld_geno_tc_binned(pgld_context* h, const pgld_geno_panel* panel, const pgl
   prm.pair_counts = reinterpret_cast<unsigned long long*>(ba.pair_counts);
   prm.status = h->dev_status;
   const int G = P <= 2 ? 2 : 1;
-  const int pmax = G == 2 ? 2 : 4;
-  const size_t fixed = sizeof(GCtrl) + (size_t)G * pmax * 96 * kCntPitch * 2 +
+  const size_t group_bytes = G == 2 ? 2 * sizeof(pgld::multi::Groups<kEpiWarps / 2>)
+                                    : sizeof(pgld::multi::Groups<kEpiWarps>);
+  const size_t fixed = sizeof(GCtrl) + (size_t)G * P * 96 * kCntPitch * 2 +
                        (size_t)(pgld::kMaxBins + 1) * 8 + (size_t)ba.n_bins * ba.n_stats * 8 +
-                       (size_t)ba.n_bins * 8 + 1024;
+                       (size_t)ba.n_bins * 8 + (size_t)(pgld::kMaxBins + 2) * 4 + group_bytes + 1024;
   int max_smem = 0;
   cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, h->device);
   const int stages =
@@ -1016,11 +1094,14 @@ int pgld_geno_tc_binned(pgld_context* h, const pgld_geno_panel* panel, const pgl
     return pgld_fail(h, PGLD_ERR_TOO_LARGE, "genotype tensor-core binned form: shared memory");
   prm.stages = stages;
   const size_t smem = (size_t)stages * kGStageBytes + fixed;
-  void (*kern)(CUtensorMap, BParams) = G == 2 ? gtc_binned_kernel<2> : gtc_binned_kernel<1>;
+  void (*kern)(CUtensorMap, BParams, pgld::multi::Places) =
+      P == 1 ? gtc_binned_kernel<1> : P == 2 ? gtc_binned_kernel<2>
+      : P == 3 ? gtc_binned_kernel<3> : gtc_binned_kernel<4>;
+  const pgld::multi::Places pl = P > 1 ? pgld::multi::places(P, true) : pgld::multi::Places{};
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return pgld_cuda_fail(h, e, "gtc binned smem attribute");
   pgld_time_begin(h, st);
-  kern<<<(unsigned)h->n_sm, kThreads, smem, st>>>(map, prm);
+  kern<<<(unsigned)h->n_sm, kThreads, smem, st>>>(map, prm, pl);
   pgld_time_end(h, st);
   e = cudaGetLastError();
   if (e != cudaSuccess) return pgld_cuda_fail(h, e, "gtc_binned_kernel");

@@ -937,6 +937,17 @@ static int check_launch_regs(pgld_context* h, const void* kern) {
   return PGLD_OK;
 }
 
+// int32 copies of integer positions; *bad != 0 where one is no such integer
+int pgld_tc_int_positions(pgld_context* h, const double* pos, long long n, int* ipos, int* bad,
+                          cudaStream_t st) {
+  PGLD_CHECK_CUDA(h, cudaMemsetAsync(bad, 0, 4, st));
+  const unsigned blocks =
+      (unsigned)std::max<long long>(1, std::min<long long>((n + 255) / 256, h->n_sm * 8));
+  pgld::tc::pos_to_int_kernel<<<blocks, 256, 0, st>>>(pos, n, ipos, bad);
+  PGLD_CHECK_CUDA(h, cudaGetLastError());
+  return PGLD_OK;
+}
+
 int pgld_tc_supported(pgld_context* h, const pgld_hap_panel* panel) {
   if (panel->n_pops < 1 || panel->n_pops > 2) return 0;
   for (int p = 0; p < panel->n_pops; ++p) {
@@ -1005,14 +1016,8 @@ static int tc_launch(pgld_context* h, const pgld_hap_panel* panel, pgld::BandArg
   if (rc) return rc;
   int* ipos = (int*)(w + off_ipos);
   int* ipos_bad = (int*)(w + off_bad);
-  {
-    cudaError_t e = cudaMemsetAsync(ipos_bad, 0, 4, st);
-    if (e != cudaSuccess) return pgld_cuda_fail(h, e, "memset");
-    unsigned blocks = (unsigned)std::max<long long>(1, std::min<long long>((n + 255) / 256, h->n_sm * 8));
-    pos_to_int_kernel<<<blocks, 256, 0, st>>>(a.pos, n, ipos, ipos_bad);
-    e = cudaGetLastError();
-    if (e != cudaSuccess) return pgld_cuda_fail(h, e, "pos_to_int_kernel");
-  }
+  rc = pgld_tc_int_positions(h, a.pos, n, ipos, ipos_bad, st);
+  if (rc) return rc;
   CUtensorMap maps[2];
   for (int p = 0; p < P; ++p) {
     rc = make_map(h, &maps[p], ops[p], 2 * n_op, k_pad[p]);
