@@ -102,6 +102,46 @@ int pgld_pack_haplotypes(pgld_handle h, const int8_t* hap, int64_t ld, int64_t n
                          const int32_t* rows, int32_t n_rows, uint32_t* planes,
                          uint32_t* valid, int32_t* flags, void* stream);
 
+/* pgld_pack_haplotypes of the kept sites only: site s goes to row before[s] of
+ * the planes if before[s + 1] > before[s] (pgld_keep_sites), and is dropped
+ * otherwise, without a look at its flags.  before NULL: every site.  The
+ * column gather of HaplotypeMatrix.apply_biallelic_filter
+ * (haplotype_matrix.py:724-789) in the packing pass. */
+int pgld_pack_haplotypes_kept(pgld_handle h, const int8_t* hap, int64_t ld, int64_t n_snp,
+                              const int32_t* rows, int32_t n_rows, const int32_t* before,
+                              uint32_t* planes, uint32_t* valid, int32_t* flags, void* stream);
+
+/* Per site of an int8 matrix, over the listed rows (NULL = 0..n_rows-1), each
+ * output nullable and overwritten: sum of the values above 0, number of values
+ * >= 0, and flags: bit 0 a value 0, bit 1 a value 1, bit 2 a value above 1.
+ * The reductions of apply_biallelic_filter (haplotype_matrix.py:724-789),
+ * ld_statistics.py:250-277 and moments_ld.py:256-280, 346-388. */
+int pgld_site_counts(pgld_handle h, const int8_t* x, int64_t ld, int64_t n_snp, const int32_t* rows,
+                     int32_t n_rows, int32_t* sum, int32_t* valid, uint32_t* flags, void* stream);
+
+/* Sites that a rule keeps, from pgld_site_counts' outputs: before[s] = kept
+ * sites below s (device int32 [n_snp + 1]), index = the kept sites in order
+ * (device int32, room for n_snp), *n_kept their number (synchronises).
+ * BIALLELIC: a value 0, a value 1, none above 1 (flags); SEGREGATING: 0 < sum <
+ * valid; DIPLOID: 0 < sum < 2 valid and valid >= 2. */
+#define PGLD_KEEP_BIALLELIC 0
+#define PGLD_KEEP_SEGREGATING 1
+#define PGLD_KEEP_DIPLOID 2
+int pgld_keep_sites(pgld_handle h, int32_t rule, const int32_t* sum, const int32_t* valid,
+                    const uint32_t* flags, int64_t n_snp, int32_t* before, int32_t* index,
+                    int64_t* n_kept, void* stream);
+
+/* Heterozygosity sums H_ij (i <= j) of the moments convention over all sites,
+ * from each population's pgld_site_counts sums: alt = sum, n = ploidy x valid
+ * (valid NULL, or valid[p] NULL: ploidy x n_rows[p]), H_ii = sum of 2 (n - alt)
+ * alt / (n (n - 1)), H_ij = sum of ((n_i - alt_i) alt_j + alt_i (n_j - alt_j)) /
+ * (n_i n_j).  out: device float64 [n_pops (n_pops + 1) / 2].  sum, valid and
+ * n_rows are HOST arrays (of device pointers).  Replaces
+ * moments_ld._compute_heterozygosity (moments_ld.py:346-388). */
+int pgld_heterozygosity(pgld_handle h, int32_t n_pops, const int32_t* const* sum,
+                        const int32_t* const* valid, const int32_t* n_rows, int32_t ploidy,
+                        int64_t n_snp, double* out, void* stream);
+
 /* Joint counts [n11, n10, n01, n00] of listed SNP pairs for one
  * population; counts row stride counts_ld (int32 elements, >= 4).
  * n_valid (nullable) receives the pairwise-valid n.
@@ -329,6 +369,12 @@ typedef struct {
 int pgld_pack_genotypes(pgld_handle h, const int8_t* geno, int64_t ld, int64_t n_snp,
                         const int32_t* rows, int32_t n_rows, uint32_t* planes, uint32_t* valid,
                         uint32_t* ext, int32_t* flags, void* stream);
+
+/* pgld_pack_genotypes of the kept sites only (as pgld_pack_haplotypes_kept). */
+int pgld_pack_genotypes_kept(pgld_handle h, const int8_t* geno, int64_t ld, int64_t n_snp,
+                             const int32_t* rows, int32_t n_rows, const int32_t* before,
+                             uint32_t* planes, uint32_t* valid, uint32_t* ext, int32_t* flags,
+                             void* stream);
 
 /* 9-way counts [n00, n01, n02, n10, ..., n22] (row stride counts_ld >= 9)
  * of listed SNP pairs and the pairwise-valid n (nullable).  Replaces

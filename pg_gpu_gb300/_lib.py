@@ -78,6 +78,12 @@ _SIGS = {
     "pgld_last_error": ([_P], ctypes.c_char_p),
     "pgld_device_status": ([_P, ctypes.POINTER(_I32), _P], ctypes.c_int),
     "pgld_pack_haplotypes": ([_P, _P, _I64, _I64, _P, _I32, _P, _P, _P, _P], ctypes.c_int),
+    "pgld_pack_haplotypes_kept": ([_P, _P, _I64, _I64, _P, _I32, _P, _P, _P, _P, _P], ctypes.c_int),
+    "pgld_site_counts": ([_P, _P, _I64, _I64, _P, _I32, _P, _P, _P, _P], ctypes.c_int),
+    "pgld_keep_sites": ([_P, _I32, _P, _P, _P, _I64, _P, _P, ctypes.POINTER(_I64), _P],
+                        ctypes.c_int),
+    "pgld_heterozygosity": ([_P, _I32, ctypes.POINTER(_P), ctypes.POINTER(_P),
+                             ctypes.POINTER(_I32), _I32, _I64, _P, _P], ctypes.c_int),
     "pgld_hap_counts_pairs": ([_P, _P, _P, _I32, _I64, _P, _P, _I64, _P, _I64, _P, _P],
                               ctypes.c_int),
     "pgld_hap_tally": ([_P, _P, _P, _I32, _I64, _P, _P, _P], ctypes.c_int),
@@ -97,6 +103,8 @@ _SIGS = {
     "pgld_pairs_by_bin": ([_P, _P, _I32, _P, _I64, _P, _P, _I32, _P, _P, _P], ctypes.c_int),
     "pgld_segment_kth": ([_P, _P, _P, _I32, _P, _I32, _P, _P], ctypes.c_int),
     "pgld_pack_genotypes": ([_P, _P, _I64, _I64, _P, _I32, _P, _P, _P, _P, _P], ctypes.c_int),
+    "pgld_pack_genotypes_kept": ([_P, _P, _I64, _I64, _P, _I32, _P, _P, _P, _P, _P, _P],
+                                 ctypes.c_int),
     "pgld_geno_counts_pairs": ([_P, _P, _P, _P, _I32, _I64, _P, _P, _I64, _P, _I64, _P, _P],
                                ctypes.c_int),
     "pgld_geno_stat_terms": ([_I32, _P, _I32, ctypes.POINTER(_I32), ctypes.POINTER(_I32)],

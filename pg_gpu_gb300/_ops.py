@@ -98,13 +98,65 @@ def _host_readable(hap):
             and hap.dim() == 2 and hap.stride(1) == 1 and hap.is_pinned())
 
 
-def pack(hap, rows=None):
+# rules of kept_sites (pgld_keep_sites)
+KEEP_BIALLELIC, KEEP_SEGREGATING, KEEP_DIPLOID = range(3)
+
+
+def site_counts(x, rows=None, sums=True, flags=False):
+    """Per-site counts of an int8 matrix (device, or a pinned host tensor read
+    in place) over `rows` (None: all): int32 (sum of the values above 0, number
+    of values >= 0, presence bits of 0 / 1 / above 1), None where not asked."""
+    torch = _torch()
+    dev = x.device if x.is_cuda else torch.device("cuda", torch.cuda.current_device())
+    n_total, n = x.shape
+    rows_t = None if rows is None else _check_rows(rows, n_total)
+    out = [torch.empty(n, dtype=torch.int32, device=dev) if want else None
+           for want in (sums, sums, flags)]
+    h = L.handle()
+    L.check(L.lib().pgld_site_counts(h, L.ptr(x), x.stride(0), n, L.ptr(rows_t),
+                                     n_total if rows_t is None else rows_t.numel(),
+                                     *(L.ptr(t) for t in out), L.stream_ptr()), h)
+    if not x.is_cuda:
+        torch.cuda.current_stream().synchronize()  # the host matrix is read in place
+    return tuple(out)
+
+
+def kept_sites(rule, counts):
+    """(before: int32 (n + 1) kept sites below each site, index: int32 kept
+    sites in order) of a KEEP_* rule on site_counts' outputs, on the device."""
+    torch = _torch()
+    n, dev = next((t.numel(), t.device) for t in counts if t is not None)
+    before = torch.empty(n + 1, dtype=torch.int32, device=dev)
+    index = torch.empty(n, dtype=torch.int32, device=dev)
+    kept = ctypes.c_int64()
+    h = L.handle()
+    L.check(L.lib().pgld_keep_sites(h, rule, *(L.ptr(t) for t in counts), n, L.ptr(before),
+                                    L.ptr(index), ctypes.byref(kept), L.stream_ptr()), h)
+    return before, index[:kept.value]
+
+
+def heterozygosity(sums, valids, n_rows, ploidy):
+    """float64 H_ij (i <= j) on the host from per-population site sums (and
+    valid counts, or None where every row counts)."""
+    torch = _torch()
+    P = len(sums)
+    out = torch.empty(P * (P + 1) // 2, dtype=torch.float64, device=sums[0].device)
+    ptrs = [(ctypes.c_void_p * P)(*(t.data_ptr() if t is not None else None for t in ts))
+            for ts in (sums, valids)]
+    h = L.handle()
+    L.check(L.lib().pgld_heterozygosity(h, P, *ptrs, (ctypes.c_int32 * P)(*n_rows), ploidy,
+                                        sums[0].numel(), L.ptr(out), L.stream_ptr()), h)
+    return out.cpu().numpy()
+
+
+def pack(hap, rows=None, kept=None):
     """Pack the rows of an int8 (H x M) matrix into bit planes on the device.
 
     hap is a device matrix (or anything as_device accepts, copied first); an
     int8 CPU tensor in pinned memory is read in place by the packing kernel,
     so only the packed planes are written to device memory (the call then
-    returns once the kernel is done with the host matrix)."""
+    returns once the kernel is done with the host matrix).  kept: the result
+    of kept_sites, to pack those sites only."""
     torch = _torch()
     if not _host_readable(hap):
         hap = L.as_device(hap, np.int8)
@@ -119,18 +171,20 @@ def pack(hap, rows=None):
         n_rows = n_total
     W = max(1, (n_rows + 31) // 32)
     dev = hap.device if hap.is_cuda else torch.device("cuda", torch.cuda.current_device())
-    planes = torch.empty((n_snp, 2 * W), dtype=torch.int32, device=dev)
-    valid = torch.empty((n_snp, W), dtype=torch.int32, device=dev)
+    before, n_out = (None, n_snp) if kept is None else (kept[0], kept[1].numel())
+    planes = torch.empty((n_out, 2 * W), dtype=torch.int32, device=dev)
+    valid = torch.empty((n_out, W), dtype=torch.int32, device=dev)
     flags = torch.zeros(2, dtype=torch.int32, device=dev)
     if n_rows == 0:
         planes.zero_()
         valid.zero_()
     else:
         h = L.handle()
-        L.check(L.lib().pgld_pack_haplotypes(h, L.ptr(hap), hap.stride(0), n_snp, L.ptr(rows_t),
-                                             n_rows, L.ptr(planes), L.ptr(valid), L.ptr(flags),
-                                             L.stream_ptr()), h)
-    pk = PackedPop.pending(planes, valid, W, n_rows, n_snp, flags)
+        L.check(L.lib().pgld_pack_haplotypes_kept(h, L.ptr(hap), hap.stride(0), n_snp,
+                                                  L.ptr(rows_t), n_rows, L.ptr(before),
+                                                  L.ptr(planes), L.ptr(valid), L.ptr(flags),
+                                                  L.stream_ptr()), h)
+    pk = PackedPop.pending(planes, valid, W, n_rows, n_out, flags)
     if not hap.is_cuda:
         pk._resolve()  # the host matrix is read in place: finish before returning
     return pk
@@ -498,17 +552,16 @@ class PackedGeno:
         return self.ext if self.has_other else None
 
 
-def pack_geno(geno, rows=None):
-    """Pack the rows of an int8 (n_individuals x M) device dosage matrix."""
+def pack_geno(geno, rows=None, kept=None):
+    """Pack the rows of an int8 (n_individuals x M) device dosage matrix (kept:
+    the result of kept_sites, to pack those sites only)."""
     torch = _torch()
     g = L.as_device(geno, np.int8)
     if g.dim() != 2:
         raise ValueError("genotypes must be 2-D (n_individuals, n_variants)")
     n_total, n_snp = g.shape
     if rows is not None:
-        rows_t = L.as_device(rows, np.int32)
-        if rows_t.numel() and (int(rows_t.min()) < 0 or int(rows_t.max()) >= n_total):
-            raise IndexError("population row index out of range")
+        rows_t = _check_rows(rows, n_total)
         n_rows = rows_t.numel()
     else:
         rows_t = None
@@ -516,26 +569,30 @@ def pack_geno(geno, rows=None):
     if n_rows > MAX_GENO_N:
         raise ValueError(f"{n_rows} individuals exceed {MAX_GENO_N} per population")
     W = max(1, (n_rows + 31) // 32)
-    planes = torch.empty((n_snp, 3 * W), dtype=torch.int32, device=g.device)
-    valid = torch.empty((n_snp, W), dtype=torch.int32, device=g.device)
+    before, n_out = (None, n_snp) if kept is None else (kept[0], kept[1].numel())
+    planes = torch.empty((n_out, 3 * W), dtype=torch.int32, device=g.device)
+    valid = torch.empty((n_out, W), dtype=torch.int32, device=g.device)
     flags = torch.zeros(2, dtype=torch.int32, device=g.device)
     ext = None
+
+    def run():
+        h = L.handle()
+        L.check(L.lib().pgld_pack_genotypes_kept(h, L.ptr(g), g.stride(0), n_snp, L.ptr(rows_t),
+                                                 n_rows, L.ptr(before), L.ptr(planes),
+                                                 L.ptr(valid), L.ptr(ext), L.ptr(flags),
+                                                 L.stream_ptr()), h)
+
     if n_rows == 0:
         planes.zero_()
         valid.zero_()
     else:
-        h = L.handle()
-        L.check(L.lib().pgld_pack_genotypes(h, L.ptr(g), g.stride(0), n_snp, L.ptr(rows_t), n_rows,
-                                            L.ptr(planes), L.ptr(valid), None, L.ptr(flags),
-                                            L.stream_ptr()), h)
-        if int(flags[1]):
-            # dosages above 2: the planes of the values 3..8 as well
-            ext = torch.empty((n_snp, 6 * W), dtype=torch.int32, device=g.device)
-            L.check(L.lib().pgld_pack_genotypes(h, L.ptr(g), g.stride(0), n_snp, L.ptr(rows_t),
-                                                n_rows, L.ptr(planes), L.ptr(valid), L.ptr(ext),
-                                                L.ptr(flags), L.stream_ptr()), h)
+        run()
     f = flags.cpu().numpy()
-    return PackedGeno(planes, valid, W, n_rows, n_snp, bool(f[0]), bool(f[1]), ext)
+    if f[1]:
+        # dosages above 2: the planes of the values 3..8 as well
+        ext = torch.empty((n_out, 6 * W), dtype=torch.int32, device=g.device)
+        run()
+    return PackedGeno(planes, valid, W, n_rows, n_out, bool(f[0]), bool(f[1]), ext)
 
 
 def geno_panel(pops):

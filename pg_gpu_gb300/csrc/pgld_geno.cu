@@ -21,53 +21,6 @@ namespace pgld {
 namespace geno {
 
 // ---------------------------------------------------------------------------
-// packing: grid (ceil(n_snp/256), W), thread = one SNP x one 32-individual word
-// ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) pack_geno_kernel(const int8_t* __restrict__ geno, i64 ld,
-                                                        i64 n_snp, const int32_t* __restrict__ rows,
-                                                        int n_rows, int W,
-                                                        uint32_t* __restrict__ planes,
-                                                        uint32_t* __restrict__ valid,
-                                                        uint32_t* __restrict__ ext,
-                                                        int32_t* __restrict__ flags) {
-  const i64 s = (i64)blockIdx.x * 256 + threadIdx.x;
-  const int w = blockIdx.y;
-  uint32_t p0 = 0, p1 = 0, p2 = 0, vw = 0;
-  uint32_t x[6] = {0, 0, 0, 0, 0, 0};
-  bool miss = false, other = false;
-  if (s < n_snp) {
-    for (int r = 0; r < 32; ++r) {
-      const int row = w * 32 + r;
-      if (row >= n_rows) break;
-      const i64 gr = rows ? (i64)__ldg(rows + row) : (i64)row;
-      const int v = __ldg(geno + gr * ld + s);
-      p0 |= (uint32_t)(v == 0) << r;
-      p1 |= (uint32_t)(v == 1) << r;
-      p2 |= (uint32_t)(v == 2) << r;
-      vw |= (uint32_t)(v >= 0) << r;
-#pragma unroll
-      for (int e = 0; e < 6; ++e) x[e] |= (uint32_t)(v == 3 + e) << r;
-      miss |= v < 0;
-      other |= v > 2;
-    }
-    uint32_t* o = planes + s * 3 * W;
-    o[w] = p0;
-    o[W + w] = p1;
-    o[2 * W + w] = p2;
-    if (valid) valid[s * W + w] = vw;
-    if (ext)
-#pragma unroll
-      for (int e = 0; e < 6; ++e) ext[s * 6 * W + e * W + w] = x[e];
-  }
-  const unsigned any_miss = __ballot_sync(0xffffffffu, miss);
-  const unsigned any_other = __ballot_sync(0xffffffffu, other);
-  if ((threadIdx.x & 31) == 0) {
-    if (any_miss) atomicOr(flags, 1);
-    if (any_other) atomicOr(flags + 1, 1);
-  }
-}
-
-// ---------------------------------------------------------------------------
 // counts of listed pairs: a group of G lanes per pair, words strided by G
 // ---------------------------------------------------------------------------
 template <int G>
@@ -466,29 +419,6 @@ int launch_geno_band(pgld_context* h, const BandArgs& a, cudaStream_t st) {
 // ---------------------------------------------------------------------------
 // entry points
 // ---------------------------------------------------------------------------
-extern "C" int pgld_pack_genotypes(pgld_handle h, const int8_t* geno, int64_t ld, int64_t n_snp,
-                                   const int32_t* rows, int32_t n_rows, uint32_t* planes,
-                                   uint32_t* valid, uint32_t* ext, int32_t* flags, void* stream) {
-  PGLD_REQUIRE(h, h != nullptr, "pgld_pack_genotypes: NULL handle");
-  PGLD_REQUIRE(h, n_snp >= 0 && n_rows >= 0, "pgld_pack_genotypes: negative size");
-  PGLD_REQUIRE(h, planes && flags && (geno || n_snp == 0 || n_rows == 0),
-               "pgld_pack_genotypes: NULL buffer");
-  PGLD_REQUIRE(h, ld >= n_snp, "pgld_pack_genotypes: row stride %lld < n_snp %lld",
-               (long long)ld, (long long)n_snp);
-  PGLD_REQUIRE(h, n_rows <= pgld::geno::kMaxGenoN,
-               "pgld_pack_genotypes: %d individuals exceed %d per population", n_rows,
-               pgld::geno::kMaxGenoN);
-  const int W = (n_rows + 31) / 32;
-  if (n_snp == 0 || W == 0) return PGLD_OK;
-  PGLD_CHECK_CUDA(h, cudaSetDevice(h->device));
-  dim3 grid((unsigned)((n_snp + 255) / 256), (unsigned)W);
-  pgld::geno::pack_geno_kernel<<<grid, 256, 0, (cudaStream_t)stream>>>(geno, ld, n_snp, rows,
-                                                                       n_rows, W, planes, valid,
-                                                                       ext, flags);
-  PGLD_CHECK_CUDA(h, cudaGetLastError());
-  return PGLD_OK;
-}
-
 extern "C" int pgld_geno_counts_pairs(pgld_handle h, const uint32_t* planes, const uint32_t* valid,
                                       const uint32_t* ext, int32_t n_words, int64_t n_snp,
                                       const int32_t* idx_i,

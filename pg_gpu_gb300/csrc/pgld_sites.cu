@@ -1,0 +1,500 @@
+// Per-site work on int8 matrices (rows = haplotypes or individuals, columns =
+// sites): bit-plane packing, allele counts and presence flags, the lists of
+// kept sites, and the heterozygosity sums.
+//
+// All of it is one pass over the matrix, four sites of a row per 32-bit load
+// and four values per instruction: a comparison with a small constant leaves
+// 0x80 in the bytes that match.  Rows start at any byte (the row stride is the
+// number of sites), so a lane whose four bytes straddle two aligned words
+// loads both and shifts; each such word holds at least one byte of the row.
+// The kernels move the matrix once; packing writes three (haplotypes) or four
+// (genotypes) bits per value.
+#include <cuda_runtime.h>
+
+#include <algorithm>
+
+#include "pgld_geno.cuh"
+#include "pgld_internal.cuh"
+
+using pgld::i64;
+
+namespace pgld {
+namespace sites {
+
+constexpr int kWarps = 8;
+constexpr int kThreads = kWarps * 32;
+constexpr int kWarpSites = 128;       // four per lane
+constexpr uint32_t kTop = 0x80808080u, kLow = 0x7f7f7f7fu;
+
+// the bytes at p[0 .. 3], of which n exist (the others read as 0)
+__device__ __forceinline__ uint32_t load4(const int8_t* p, i64 n) {
+  if (n >= 4) {
+    const int a = (int)((uintptr_t)p & 3);
+    const uint32_t* w = reinterpret_cast<const uint32_t*>(p - a);
+    if (a == 0) return __ldg(w);
+    return __funnelshift_r(__ldg(w), __ldg(w + 1), 8 * a);
+  }
+  uint32_t v = 0;
+  for (int k = 0; k < (int)n; ++k) v |= (uint32_t)(uint8_t)__ldg(p + k) << (8 * k);
+  return v;
+}
+
+// 0x80 in every byte equal to c (0 <= c < 0x80): adding 0x7f to the low seven
+// bits of v ^ c sets the top bit unless they are all zero
+__device__ __forceinline__ uint32_t equal4(uint32_t v, uint32_t c) {
+  return ~((((v ^ (c * 0x01010101u)) & kLow) + kLow) | v) & kTop;
+}
+__device__ __forceinline__ uint32_t minus_one4(uint32_t v) { return ~((~v & kLow) + kLow) & v & kTop; }
+
+// planes of one value: haplotypes carrier, reference, valid
+struct HapPlanes {
+  static constexpr int N = 3, kValid = 2, kMain = 2, kExt = 0;
+  __device__ static void split(uint32_t v, uint32_t (&m)[N], uint32_t& miss, uint32_t& other) {
+    m[0] = equal4(v, 1);
+    m[1] = equal4(v, 0);
+    m[2] = ~v & kTop;
+    const uint32_t none = minus_one4(v);
+    miss |= none;
+    other |= ~(m[0] | m[1] | none) & kTop;
+  }
+};
+// genotypes: dosages 0, 1, 2, valid, and (EXT) the values 3 .. 8
+template <bool EXT>
+struct GenoPlanes {
+  static constexpr int N = EXT ? 10 : 4, kValid = 3, kMain = 3, kExt = EXT ? 6 : 0;
+  __device__ static void split(uint32_t v, uint32_t (&m)[N], uint32_t& miss, uint32_t& other) {
+    m[0] = equal4(v, 0);
+    m[1] = equal4(v, 1);
+    m[2] = equal4(v, 2);
+    m[3] = ~v & kTop;
+    miss |= v & kTop;
+    other |= m[3] & ~(m[0] | m[1] | m[2]);
+#pragma unroll
+    for (int e = 0; e < kExt; ++e) m[4 + e] = equal4(v, 3 + e);
+  }
+};
+
+struct PackArgs {
+  const int8_t* x;
+  i64 ld, n_snp;
+  const int32_t* rows;    // row of each haplotype / individual (NULL: 0 .. n_rows - 1)
+  int n_rows, W;
+  const int32_t* before;  // kept sites before each site, [n_snp + 1] (NULL: all kept)
+  uint32_t *planes, *valid, *ext;
+  int32_t* flags;
+  int words;              // words per block (a power of two, at most kWarps)
+};
+
+// A warp turns 32 rows x 128 sites into one word per site and plane: per row
+// the comparison's bytes shift into a register per plane and eight rows, byte
+// transposes then give the words.  The block's `words` words of a site are
+// stored together (32-byte segments at eight words), through shared memory.
+template <class S>
+__global__ void __launch_bounds__(kThreads) pack_kernel(PackArgs a) {
+  constexpr int kPitch = kWarps + 1;
+  __shared__ uint32_t out[S::N][kWarpSites * kPitch];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int chunks = kWarps / a.words;          // 128-site chunks per block
+  const int word = blockIdx.y * a.words + warp % a.words;
+  const i64 s0 = ((i64)blockIdx.x * chunks + warp / a.words) * kWarpSites + 4 * lane;
+  const int live = min(32, a.n_rows - 32 * word);  // rows of the word (none for a padding word)
+  uint32_t acc[S::N][4];
+#pragma unroll
+  for (int p = 0; p < S::N; ++p) acc[p][0] = acc[p][1] = acc[p][2] = acc[p][3] = 0;
+  uint32_t miss = 0, other = 0;
+  const i64 left = a.n_snp - s0;
+  const int mine = lane < live ? (a.rows ? __ldg(a.rows + 32 * word + lane) : 32 * word + lane) : 0;
+#pragma unroll
+  for (int o = 0; o < 4; ++o) {
+    uint32_t v[8];
+#pragma unroll
+    for (int r = 0; r < 8; ++r) {
+      const i64 row = __shfl_sync(0xffffffffu, mine, 8 * o + r);
+      v[r] = 8 * o + r < live && left > 0 ? load4(a.x + row * a.ld + s0, left) : 0u;
+    }
+#pragma unroll
+    for (int r = 0; r < 8; ++r) {
+      if (8 * o + r < live) {
+        uint32_t m[S::N];
+        S::split(v[r], m, miss, other);
+#pragma unroll
+        for (int p = 0; p < S::N; ++p) acc[p][o] |= m[p] >> (7 - r);
+      }
+    }
+  }
+  // the lane's sites that exist and are kept
+  uint32_t kept = 0;
+#pragma unroll
+  for (int k = 0; k < 4; ++k)
+    if (k < left && (!a.before || a.before[s0 + k + 1] > a.before[s0 + k])) kept |= 0x80u << (8 * k);
+#pragma unroll
+  for (int p = 0; p < S::N; ++p) {
+    const uint32_t l0 = __byte_perm(acc[p][0], acc[p][1], 0x5140), l1 = __byte_perm(acc[p][0], acc[p][1], 0x7362);
+    const uint32_t h0 = __byte_perm(acc[p][2], acc[p][3], 0x5140), h1 = __byte_perm(acc[p][2], acc[p][3], 0x7362);
+    uint32_t* o = out[p] + 4 * lane * kPitch + warp;
+    o[0] = __byte_perm(l0, h0, 0x5410);
+    o[kPitch] = __byte_perm(l0, h0, 0x7632);
+    o[2 * kPitch] = __byte_perm(l1, h1, 0x5410);
+    o[3 * kPitch] = __byte_perm(l1, h1, 0x7632);
+  }
+  const bool any_miss = __any_sync(0xffffffffu, (miss & kept) != 0);
+  const bool any_other = __any_sync(0xffffffffu, (other & kept) != 0);
+  if (lane == 0) {
+    if (any_miss) atomicOr(a.flags, 1);
+    if (any_other) atomicOr(a.flags + 1, 1);
+  }
+  __syncthreads();
+  // consecutive threads: the words of a site, then the next site of the block
+  const i64 b0 = (i64)blockIdx.x * chunks * kWarpSites;
+  for (int t = threadIdx.x; t < chunks * kWarpSites * a.words; t += kThreads) {
+    const int w = t % a.words, at = t / a.words;
+    const int W0 = blockIdx.y * a.words + w;
+    const i64 s = b0 + at;
+    if (W0 >= a.W || s >= a.n_snp) continue;
+    i64 d = s;
+    if (a.before) {
+      d = a.before[s];
+      if (a.before[s + 1] == d) continue;
+    }
+    const int from = (at % kWarpSites) * kPitch + (at / kWarpSites) * a.words + w;
+#pragma unroll
+    for (int p = 0; p < S::kMain; ++p) a.planes[d * S::kMain * a.W + p * a.W + W0] = out[p][from];
+    if (a.valid) a.valid[d * a.W + W0] = out[S::kValid][from];
+#pragma unroll
+    for (int e = 0; e < S::kExt; ++e) a.ext[d * S::kExt * a.W + e * a.W + W0] = out[S::kValid + 1 + e][from];
+  }
+}
+
+template <class S>
+int launch_pack(pgld_context* h, PackArgs a, cudaStream_t st) {
+  a.words = 1;
+  while (a.words < a.W && a.words < kWarps) a.words <<= 1;
+  const i64 per_block = (i64)(kWarps / a.words) * kWarpSites;
+  const dim3 grid((unsigned)((a.n_snp + per_block - 1) / per_block),
+                  (unsigned)((a.W + a.words - 1) / a.words));
+  pack_kernel<S><<<grid, kThreads, 0, st>>>(a);
+  PGLD_CHECK_CUDA(h, cudaGetLastError());
+  return PGLD_OK;
+}
+
+// ---------------------------------------------------------------------------
+// per-site sums of the non-negative values, valid counts, presence flags
+// ---------------------------------------------------------------------------
+// block: 128 sites x a share of the rows, one row in eight per warp; at most
+// 255 rows per warp, so byte counters and 16-bit sums (127 each) never carry
+__global__ void __launch_bounds__(kThreads) site_counts_kernel(
+    const int8_t* __restrict__ x, i64 ld, i64 n_snp, const int32_t* __restrict__ rows, int n_rows,
+    int share, int32_t* __restrict__ sum, int32_t* __restrict__ valid,
+    uint32_t* __restrict__ flags) {
+  __shared__ int s_sum[kWarpSites], s_valid[kWarpSites], s_flag[kWarpSites];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (threadIdx.x < kWarpSites) s_sum[threadIdx.x] = s_valid[threadIdx.x] = s_flag[threadIdx.x] = 0;
+  __syncthreads();
+  const i64 s0 = (i64)blockIdx.x * kWarpSites + 4 * lane, left = n_snp - s0;
+  const int r_end = min(n_rows, (int)(blockIdx.y + 1) * share);
+  uint32_t even = 0, odd = 0, nv = 0, zero = 0, one = 0, bits = 0;
+  if (left > 0) {
+#pragma unroll 8
+    for (int r = (int)blockIdx.y * share + warp; r < r_end; r += kWarps) {
+      const i64 row = rows ? (i64)__ldg(rows + r) : (i64)r;
+      const uint32_t v = load4(x + row * ld + s0, left);
+      const uint32_t neg = v & kTop;
+      const uint32_t pos = v & ~((neg - (neg >> 7)) | neg);  // negative bytes cleared
+      even += pos & 0x00ff00ffu;
+      odd += (pos >> 8) & 0x00ff00ffu;
+      nv += (~v >> 7) & 0x01010101u;
+      zero |= equal4(v, 0);
+      one |= equal4(v, 1);
+      bits |= pos;
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const uint32_t half = (k & 1) ? odd : even;
+      atomicAdd(&s_sum[4 * lane + k], (int)((half >> (k & 2 ? 16 : 0)) & 0xffffu));
+      atomicAdd(&s_valid[4 * lane + k], (int)((nv >> (8 * k)) & 0xffu));
+      const int f = (int)((zero >> (8 * k + 7)) & 1u) | (int)((one >> (8 * k + 7)) & 1u) << 1 |
+                    (((bits >> (8 * k)) & 0x7eu) ? 4 : 0);
+      if (f) atomicOr(&s_flag[4 * lane + k], f);
+    }
+  }
+  __syncthreads();
+  const i64 s = (i64)blockIdx.x * kWarpSites + threadIdx.x;
+  if (threadIdx.x < kWarpSites && s < n_snp) {
+    // several blocks share a site when the rows are split (outputs zeroed before)
+    if (sum) atomicAdd(sum + s, s_sum[threadIdx.x]);
+    if (valid) atomicAdd(valid + s, s_valid[threadIdx.x]);
+    if (flags && s_flag[threadIdx.x]) atomicOr(flags + s, (uint32_t)s_flag[threadIdx.x]);
+  }
+}
+
+// ---------------------------------------------------------------------------
+// kept sites: rule, counts before each site and the list, in two launches (a
+// block of the second adds up the totals of the tiles before its own)
+// ---------------------------------------------------------------------------
+constexpr int kKeepThreads = 256;
+constexpr int kKeepTile = kKeepThreads * 16;
+
+__device__ __forceinline__ bool keeps(int rule, const int32_t* sum, const int32_t* valid,
+                                      const uint32_t* flags, i64 s) {
+  if (rule == PGLD_KEEP_BIALLELIC) return (flags[s] & 7u) == 3u;
+  const int a = sum[s], n = valid[s];
+  if (rule == PGLD_KEEP_SEGREGATING) return a > 0 && a < n;
+  return a > 0 && a < 2 * n && n >= 2;
+}
+
+// exclusive prefix of v over the block's threads; *total the block's sum
+__device__ __forceinline__ int block_scan(int v, int* sh, int* total) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  int x = v;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y = __shfl_up_sync(0xffffffffu, x, o);
+    if (lane >= o) x += y;
+  }
+  if (lane == 31) sh[warp] = x;
+  __syncthreads();
+  int before = 0, all = 0;
+#pragma unroll
+  for (int w = 0; w < kKeepThreads / 32; ++w) {
+    if (w < warp) before += sh[w];
+    all += sh[w];
+  }
+  __syncthreads();
+  *total = all;
+  return before + x - v;
+}
+
+__global__ void __launch_bounds__(kKeepThreads) keep_totals_kernel(
+    int rule, const int32_t* sum, const int32_t* valid, const uint32_t* flags, i64 n,
+    int32_t* __restrict__ part) {
+  const i64 base = (i64)blockIdx.x * kKeepTile;
+  int c = 0;
+  for (int k = threadIdx.x; k < kKeepTile; k += kKeepThreads)
+    if (base + k < n) c += keeps(rule, sum, valid, flags, base + k);
+  __shared__ int sh[kKeepThreads / 32];
+  int tot;
+  block_scan(c, sh, &tot);
+  if (threadIdx.x == 0) part[blockIdx.x] = tot;
+}
+
+__global__ void __launch_bounds__(kKeepThreads) keep_apply_kernel(
+    int rule, const int32_t* sum, const int32_t* valid, const uint32_t* flags, i64 n,
+    const int32_t* __restrict__ part, int32_t* __restrict__ before, int32_t* __restrict__ index) {
+  __shared__ int sh[kKeepThreads / 32];
+  const i64 base = (i64)blockIdx.x * kKeepTile;
+  int c = 0;
+  for (int k = threadIdx.x; k < (int)blockIdx.x; k += kKeepThreads) c += part[k];
+  int at;
+  block_scan(c, sh, &at);
+  for (int k0 = 0; k0 < kKeepTile; k0 += kKeepThreads) {
+    const i64 s = base + k0 + threadIdx.x;
+    const bool keep = s < n && keeps(rule, sum, valid, flags, s);
+    int tot;
+    const int off = at + block_scan(keep, sh, &tot);
+    at += tot;
+    if (s <= n) before[s] = off;  // s == n: the total
+    if (keep) index[off] = (int32_t)s;
+  }
+  // n a multiple of the tile: no thread stood at s == n
+  if (threadIdx.x == 0 && blockIdx.x == gridDim.x - 1 && base + kKeepTile == n) before[n] = at;
+}
+
+// ---------------------------------------------------------------------------
+// heterozygosity sums of moments (moments_ld.py:346-388): H_ij for i <= j, the
+// same float64 expressions per site as the reference's arrays
+// ---------------------------------------------------------------------------
+struct HetArgs {
+  const int32_t* sum[PGLD_MAX_POPS];
+  const int32_t* valid[PGLD_MAX_POPS];  // NULL: n_rows everywhere
+  double n_rows[PGLD_MAX_POPS];
+  int n_pops;
+  double per;  // allele copies per row
+};
+
+__global__ void __launch_bounds__(256) het_kernel(HetArgs a, i64 n, double* __restrict__ out) {
+  __shared__ double sh[8];
+  double tot[10] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
+  for (i64 s = (i64)blockIdx.x * 256 + threadIdx.x; s < n; s += (i64)gridDim.x * 256) {
+    double alt[PGLD_MAX_POPS], ref[PGLD_MAX_POPS], m[PGLD_MAX_POPS];
+#pragma unroll
+    for (int p = 0; p < PGLD_MAX_POPS; ++p)
+      if (p < a.n_pops) {
+        alt[p] = (double)a.sum[p][s];
+        m[p] = a.per * (a.valid[p] ? (double)a.valid[p][s] : a.n_rows[p]);
+        ref[p] = m[p] - alt[p];
+      }
+    int k = 0;
+#pragma unroll
+    for (int i = 0; i < PGLD_MAX_POPS; ++i)
+#pragma unroll
+      for (int j = i; j < PGLD_MAX_POPS; ++j, ++k)
+        if (j < a.n_pops)
+          tot[k] += i == j ? 2.0 * ref[i] * alt[i] / (m[i] * (m[i] - 1.0))
+                           : (ref[i] * alt[j] + alt[i] * ref[j]) / (m[i] * m[j]);
+  }
+  int k = 0, o = 0;
+#pragma unroll
+  for (int i = 0; i < PGLD_MAX_POPS; ++i)
+#pragma unroll
+    for (int j = i; j < PGLD_MAX_POPS; ++j, ++k) {
+      if (j >= a.n_pops) continue;
+      double v = tot[k];
+#pragma unroll
+      for (int d = 16; d > 0; d >>= 1) v += __shfl_xor_sync(0xffffffffu, v, d);
+      __syncthreads();
+      if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = v;
+      __syncthreads();
+      if (threadIdx.x == 0) {
+        for (int w = 1; w < 8; ++w) v += sh[w];
+        atomicAdd(out + o, v);
+      }
+      ++o;
+    }
+}
+
+}  // namespace sites
+}  // namespace pgld
+
+// ---------------------------------------------------------------------------
+// entry points
+// ---------------------------------------------------------------------------
+extern "C" int pgld_pack_haplotypes_kept(pgld_handle h, const int8_t* hap, int64_t ld, int64_t n_snp,
+                                         const int32_t* rows, int32_t n_rows, const int32_t* before,
+                                         uint32_t* planes, uint32_t* valid, int32_t* flags,
+                                         void* stream) {
+  PGLD_REQUIRE(h, h != nullptr, "pgld_pack_haplotypes: NULL handle");
+  PGLD_REQUIRE(h, n_snp >= 0 && n_rows >= 0, "pgld_pack_haplotypes: negative size");
+  PGLD_REQUIRE(h, planes && flags && (hap || n_snp == 0 || n_rows == 0),
+               "pgld_pack_haplotypes: NULL buffer");
+  PGLD_REQUIRE(h, ld >= n_snp, "pgld_pack_haplotypes: row stride %lld < n_snp %lld",
+               (long long)ld, (long long)n_snp);
+  const int W = (n_rows + 31) / 32;
+  if (n_snp == 0 || W == 0) return PGLD_OK;
+  PGLD_REQUIRE(h, W <= 65535, "pgld_pack_haplotypes: too many rows");
+  PGLD_CHECK_CUDA(h, cudaSetDevice(h->device));
+  return pgld::sites::launch_pack<pgld::sites::HapPlanes>(
+      h, {hap, ld, n_snp, rows, n_rows, W, before, planes, valid, nullptr, flags, 0},
+      (cudaStream_t)stream);
+}
+
+extern "C" int pgld_pack_haplotypes(pgld_handle h, const int8_t* hap, int64_t ld, int64_t n_snp,
+                                    const int32_t* rows, int32_t n_rows, uint32_t* planes,
+                                    uint32_t* valid, int32_t* flags, void* stream) {
+  return pgld_pack_haplotypes_kept(h, hap, ld, n_snp, rows, n_rows, nullptr, planes, valid, flags,
+                                   stream);
+}
+
+extern "C" int pgld_pack_genotypes_kept(pgld_handle h, const int8_t* geno, int64_t ld, int64_t n_snp,
+                                        const int32_t* rows, int32_t n_rows, const int32_t* before,
+                                        uint32_t* planes, uint32_t* valid, uint32_t* ext,
+                                        int32_t* flags, void* stream) {
+  PGLD_REQUIRE(h, h != nullptr, "pgld_pack_genotypes: NULL handle");
+  PGLD_REQUIRE(h, n_snp >= 0 && n_rows >= 0, "pgld_pack_genotypes: negative size");
+  PGLD_REQUIRE(h, planes && flags && (geno || n_snp == 0 || n_rows == 0),
+               "pgld_pack_genotypes: NULL buffer");
+  PGLD_REQUIRE(h, ld >= n_snp, "pgld_pack_genotypes: row stride %lld < n_snp %lld",
+               (long long)ld, (long long)n_snp);
+  PGLD_REQUIRE(h, n_rows <= pgld::geno::kMaxGenoN,
+               "pgld_pack_genotypes: %d individuals exceed %d per population", n_rows,
+               pgld::geno::kMaxGenoN);
+  const int W = (n_rows + 31) / 32;
+  if (n_snp == 0 || W == 0) return PGLD_OK;
+  PGLD_CHECK_CUDA(h, cudaSetDevice(h->device));
+  const pgld::sites::PackArgs a{geno, ld, n_snp, rows, n_rows, W, before, planes, valid, ext, flags, 0};
+  if (ext) return pgld::sites::launch_pack<pgld::sites::GenoPlanes<true>>(h, a, (cudaStream_t)stream);
+  return pgld::sites::launch_pack<pgld::sites::GenoPlanes<false>>(h, a, (cudaStream_t)stream);
+}
+
+extern "C" int pgld_pack_genotypes(pgld_handle h, const int8_t* geno, int64_t ld, int64_t n_snp,
+                                   const int32_t* rows, int32_t n_rows, uint32_t* planes,
+                                   uint32_t* valid, uint32_t* ext, int32_t* flags, void* stream) {
+  return pgld_pack_genotypes_kept(h, geno, ld, n_snp, rows, n_rows, nullptr, planes, valid, ext, flags,
+                                  stream);
+}
+
+extern "C" int pgld_site_counts(pgld_handle h, const int8_t* x, int64_t ld, int64_t n_snp,
+                                const int32_t* rows, int32_t n_rows, int32_t* sum, int32_t* valid,
+                                uint32_t* flags, void* stream) {
+  using namespace pgld::sites;
+  PGLD_REQUIRE(h, h != nullptr, "pgld_site_counts: NULL handle");
+  PGLD_REQUIRE(h, n_snp >= 0 && n_rows >= 0 && ld >= n_snp, "pgld_site_counts: sizes");
+  PGLD_REQUIRE(h, x || n_snp == 0 || n_rows == 0, "pgld_site_counts: NULL matrix");
+  if (n_snp == 0) return PGLD_OK;
+  PGLD_CHECK_CUDA(h, cudaSetDevice(h->device));
+  cudaStream_t st = (cudaStream_t)stream;
+  if (sum) PGLD_CHECK_CUDA(h, cudaMemsetAsync(sum, 0, (size_t)n_snp * 4, st));
+  if (valid) PGLD_CHECK_CUDA(h, cudaMemsetAsync(valid, 0, (size_t)n_snp * 4, st));
+  if (flags) PGLD_CHECK_CUDA(h, cudaMemsetAsync(flags, 0, (size_t)n_snp * 4, st));
+  if (n_rows == 0) return PGLD_OK;
+  // rows are split until every SM has a few blocks (at least one row per warp,
+  // at most 255)
+  const i64 gx = (n_snp + kWarpSites - 1) / kWarpSites;
+  i64 gy = std::max<i64>(1, std::min<i64>((4 * h->n_sm + gx - 1) / gx, (n_rows + 4 * kWarps - 1) / (4 * kWarps)));
+  i64 share = (n_rows + gy - 1) / gy;
+  share = std::min<i64>((share + kWarps - 1) / kWarps, 255) * kWarps;
+  gy = (n_rows + share - 1) / share;
+  PGLD_REQUIRE(h, gy <= 65535, "pgld_site_counts: too many rows");
+  site_counts_kernel<<<dim3((unsigned)gx, (unsigned)gy), kThreads, 0, st>>>(
+      x, ld, n_snp, rows, n_rows, (int)share, sum, valid, flags);
+  PGLD_CHECK_CUDA(h, cudaGetLastError());
+  return PGLD_OK;
+}
+
+extern "C" int pgld_keep_sites(pgld_handle h, int32_t rule, const int32_t* sum, const int32_t* valid,
+                               const uint32_t* flags, int64_t n_snp, int32_t* before, int32_t* index,
+                               int64_t* n_kept, void* stream) {
+  using namespace pgld::sites;
+  PGLD_REQUIRE(h, h != nullptr, "pgld_keep_sites: NULL handle");
+  PGLD_REQUIRE(h, rule >= PGLD_KEEP_BIALLELIC && rule <= PGLD_KEEP_DIPLOID, "pgld_keep_sites: rule %d", rule);
+  PGLD_REQUIRE(h, n_snp >= 0 && n_snp < (int64_t(1) << 31) - 1, "pgld_keep_sites: n_snp");
+  PGLD_REQUIRE(h, before && n_kept && (index || n_snp == 0), "pgld_keep_sites: NULL output");
+  PGLD_REQUIRE(h, n_snp == 0 || (rule == PGLD_KEEP_BIALLELIC ? flags != nullptr : sum && valid),
+               "pgld_keep_sites: the rule's counts are missing");
+  PGLD_CHECK_CUDA(h, cudaSetDevice(h->device));
+  cudaStream_t st = (cudaStream_t)stream;
+  *n_kept = 0;
+  if (n_snp == 0) {
+    PGLD_CHECK_CUDA(h, cudaMemsetAsync(before, 0, 4, st));
+    return PGLD_OK;
+  }
+  const i64 tiles = (n_snp + kKeepTile - 1) / kKeepTile;
+  void* ws = nullptr;
+  int rc = pgld_workspace(h, (size_t)tiles * 4, &ws);
+  if (rc) return rc;
+  keep_totals_kernel<<<(unsigned)tiles, kKeepThreads, 0, st>>>(rule, sum, valid, flags, n_snp, (int32_t*)ws);
+  keep_apply_kernel<<<(unsigned)tiles, kKeepThreads, 0, st>>>(rule, sum, valid, flags, n_snp,
+                                                              (const int32_t*)ws, before, index);
+  PGLD_CHECK_CUDA(h, cudaGetLastError());
+  int32_t n = 0;
+  PGLD_CHECK_CUDA(h, cudaMemcpyAsync(&n, before + n_snp, 4, cudaMemcpyDeviceToHost, st));
+  PGLD_CHECK_CUDA(h, cudaStreamSynchronize(st));
+  *n_kept = n;
+  return PGLD_OK;
+}
+
+extern "C" int pgld_heterozygosity(pgld_handle h, int32_t n_pops, const int32_t* const* sum,
+                                   const int32_t* const* valid, const int32_t* n_rows,
+                                   int32_t ploidy, int64_t n_snp, double* out, void* stream) {
+  using namespace pgld::sites;
+  PGLD_REQUIRE(h, h != nullptr, "pgld_heterozygosity: NULL handle");
+  PGLD_REQUIRE(h, n_pops >= 1 && n_pops <= PGLD_MAX_POPS && n_snp >= 0 && ploidy >= 1,
+               "pgld_heterozygosity: sizes");
+  PGLD_REQUIRE(h, sum && n_rows && out, "pgld_heterozygosity: NULL argument");
+  HetArgs a{};
+  a.n_pops = n_pops;
+  a.per = ploidy;
+  for (int p = 0; p < n_pops; ++p) {
+    PGLD_REQUIRE(h, sum[p] != nullptr || n_snp == 0, "pgld_heterozygosity: counts of population %d", p);
+    a.sum[p] = sum[p];
+    a.valid[p] = valid ? valid[p] : nullptr;
+    a.n_rows[p] = n_rows[p];
+  }
+  PGLD_CHECK_CUDA(h, cudaSetDevice(h->device));
+  cudaStream_t st = (cudaStream_t)stream;
+  PGLD_CHECK_CUDA(h, cudaMemsetAsync(out, 0, (size_t)n_pops * (n_pops + 1) / 2 * 8, st));
+  if (n_snp == 0) return PGLD_OK;
+  const unsigned blocks = (unsigned)std::min<i64>((n_snp + 255) / 256, (i64)h->n_sm * 4);
+  het_kernel<<<blocks, 256, 0, st>>>(a, n_snp, out);
+  PGLD_CHECK_CUDA(h, cudaGetLastError());
+  return PGLD_OK;
+}

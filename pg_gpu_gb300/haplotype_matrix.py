@@ -458,19 +458,34 @@ class HaplotypeMatrix:
             return torch.cat([c1, c2], 1), nv1, nv2
         return torch.cat([c1, c2], 1), None, None
 
-    def _binned(self, bp_bins, pops):
+    def _binned(self, bp_bins, pops, ac_filter=False):
         bins = np.asarray(bp_bins, dtype=np.float64)
+        if ac_filter:
+            return self._binned_biallelic(bins, pops)
         packs = [self.packed(p) for p in pops]
         sums, cnt = _ops.binned_sums(packs, _ops.positions_f64(self._positions), bins)
+        return bins, sums.cpu().numpy(), cnt.cpu().numpy()
+
+    def _binned_biallelic(self, bins, pops):
+        """_binned of apply_biallelic_filter(): the sites are chosen and the
+        populations packed from the matrix itself, without the gathered copy."""
+        src = self._pinned if self._device == "CPU" else self._haplotypes
+        if src is None:
+            if self._haplotypes.dtype != np.int8:
+                return self.apply_biallelic_filter()._binned(bins, pops)
+            src = L.as_device(self._haplotypes, np.int8)
+        kept = _ops.kept_sites(_ops.KEEP_BIALLELIC, _ops.site_counts(src, sums=False, flags=True))
+        if kept[1].numel() == 0:
+            raise ValueError("genotypes cannot be empty")
+        packs = [_ops.pack(src, self._pop_rows(p), kept) for p in pops]
+        pos = _ops.positions_f64(self._positions).index_select(0, kept[1])
+        sums, cnt = _ops.binned_sums(packs, pos, bins)
         return bins, sums.cpu().numpy(), cnt.cpu().numpy()
 
     def compute_ld_statistics_gpu_single_pop(self, bp_bins, raw=False, ac_filter=True,
                                              chunk_size="auto"):
         """{(lo, hi): (DD, Dz, pi2)} sums or means per bin (haplotype_matrix.py:1592-1716)."""
-        if ac_filter:
-            return self.apply_biallelic_filter().compute_ld_statistics_gpu_single_pop(
-                bp_bins, raw=raw, ac_filter=False, chunk_size=chunk_size)
-        bins, sums, cnt = self._binned(bp_bins, [None])
+        bins, sums, cnt = self._binned(bp_bins, [None], ac_filter)
         out = {}
         for i in range(len(bins) - 1):
             key = (float(bins[i]), float(bins[i + 1]))
@@ -485,12 +500,9 @@ class HaplotypeMatrix:
     def compute_ld_statistics_gpu_two_pops(self, bp_bins, pop1, pop2, raw=False,
                                            ac_filter=True, chunk_size="auto"):
         """{(lo, hi): OrderedDict of the 15 statistics} (haplotype_matrix.py:1719-1866)."""
-        if ac_filter:
-            return self.apply_biallelic_filter().compute_ld_statistics_gpu_two_pops(
-                bp_bins, pop1, pop2, raw=raw, ac_filter=False, chunk_size=chunk_size)
         from .ld_pipeline import ld_names
         names = ld_names(2)
-        bins, sums, cnt = self._binned(bp_bins, [pop1, pop2])
+        bins, sums, cnt = self._binned(bp_bins, [pop1, pop2], ac_filter)
         out = {}
         for i in range(len(bins) - 1):
             key = (float(bins[i]), float(bins[i + 1]))

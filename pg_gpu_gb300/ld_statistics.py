@@ -176,13 +176,16 @@ def rogers_huff_r_squared(matrix, tile_size=None):
 # --------------------------------------------------------------------------
 # ZnS over windows (ld_statistics.py:534-735, windowed_analysis.py:2013-2062)
 # --------------------------------------------------------------------------
-def _segregating_index(hap):
-    """Indices of the sites with 0 < derived count < valid count (ld_statistics.py:250-277)."""
+def _segregating(hap, win_start, win_stop):
+    """The sites with 0 < derived count < valid count (ld_statistics.py:250-277)
+    as a device index, and each SNP window's range [b, e) of it on the host."""
     import torch
-    h = L.as_device(hap, np.int8)
-    dac = h.clamp(min=0).to(torch.int32).sum(0)
-    nv = (h >= 0).to(torch.int32).sum(0)
-    return ((dac > 0) & (dac < nv)).nonzero().flatten().to(torch.int32)
+    counts = _ops.site_counts(L.as_device(hap, np.int8))
+    before, index = _ops.kept_sites(_ops.KEEP_SEGREGATING, counts)
+    n = before.numel() - 1
+    ends = np.clip(np.stack([win_start, win_stop]), 0, n)
+    at = before[torch.as_tensor(ends, device=before.device)].cpu().numpy().astype(np.int64)
+    return index, at[0], at[1]
 
 
 def _zns_windows(matrix, win_start, win_stop, estimator):
@@ -196,10 +199,7 @@ def _zns_windows(matrix, win_start, win_stop, estimator):
     we = np.asarray(win_stop, np.int64)
     if ws.shape != we.shape:
         raise ValueError("win_start and win_stop must have the same shape")
-    seg = _segregating_index(matrix.haplotypes)
-    seg_np = seg.cpu().numpy()
-    b = np.searchsorted(seg_np, ws, side="left").astype(np.int64)
-    e = np.searchsorted(seg_np, we, side="left").astype(np.int64)
+    seg, b, e = _segregating(matrix.haplotypes, ws, we)
     sums, cnt = _ops.window_sums(matrix.packed(None), seg, b, e)
     s, c = sums.cpu().numpy(), cnt.cpu().numpy()
     out = np.zeros(len(ws))
@@ -399,10 +399,8 @@ def _omega_windows(hm, win_start, win_stop, column):
     column sums of the pair statistic (window column `column`) give every
     split point's block sums."""
     hm.transfer_to_gpu()
-    seg = _segregating_index(hm.haplotypes)
-    seg_np = seg.cpu().numpy()
-    b = np.searchsorted(seg_np, np.asarray(win_start, np.int64), side="left").astype(np.int64)
-    e = np.searchsorted(seg_np, np.asarray(win_stop, np.int64), side="left").astype(np.int64)
+    seg, b, e = _segregating(hm.haplotypes, np.asarray(win_start, np.int64),
+                             np.asarray(win_stop, np.int64))
     rows, cols, off = _ops.window_snp_sums(hm.packed(None), seg, b, e, column)
     rows, cols = rows.cpu().numpy(), cols.cpu().numpy()
     return np.array([_ops.omega_from_sums(rows[off[w]:off[w + 1]], cols[off[w]:off[w + 1]])

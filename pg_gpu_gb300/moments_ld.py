@@ -160,20 +160,15 @@ def _max_bp_for_r_dist(positions, gen_dists, max_r):
 
 def _compute_ld_sums(mat, pops, bins, gen_dists, max_bp, use_genotypes=False):
     """(n_bins, n_stats) float64 numpy sums (moments_ld.py:248-343)."""
-    import torch
     if use_genotypes:
         # variants polymorphic across the union of the populations (moments_ld.py:256-280)
-        g = mat.genotypes
+        g = L.as_device(mat.genotypes, np.int8)
         rows = sorted(set(i for p in pops for i in mat.sample_sets[p]))
-        sub = g[torch.as_tensor(rows, device=g.device)]
-        v = sub >= 0
-        alt = torch.where(v, sub, torch.zeros_like(sub)).to(torch.int64).sum(0)
-        nv = v.to(torch.int64).sum(0)
-        keep = ((alt > 0) & (alt < 2 * nv) & (nv >= 2)).nonzero().flatten()
-        data = g[:, keep].contiguous()
-        pos_d = L.as_device(mat.positions, np.float64)[keep].contiguous()
-        bc = None if gen_dists is None else L.as_device(gen_dists, np.float64)[keep].contiguous()
-        packs = [_ops.pack_geno(data, mat.sample_sets[p]) for p in pops]
+        kept = _ops.kept_sites(_ops.KEEP_DIPLOID, _ops.site_counts(g, rows))
+        pos_d = L.as_device(mat.positions, np.float64).index_select(0, kept[1])
+        bc = (None if gen_dists is None else
+              L.as_device(gen_dists, np.float64).index_select(0, kept[1]))
+        packs = [_ops.pack_geno(g, mat.sample_sets[p], kept) for p in pops]
         sums, _ = _ops.geno_binned_sums(packs, pos_d, bins, max_dist=max_bp, bin_coord=bc)
     else:
         pos_d = L.as_device(mat.positions, np.float64)
@@ -186,31 +181,15 @@ def _compute_ld_sums(mat, pops, bins, gen_dists, max_bp, use_genotypes=False):
 def _compute_heterozygosity(mat, pops, use_genotypes=False):
     """H_i_j of the moments convention (moments_ld.py:346-388)."""
     import torch
-    alt, ref, nh = [], [], []
-    for p in pops:
-        rows = torch.as_tensor(mat.sample_sets[p], device="cuda")
-        if use_genotypes:
-            d = mat.genotypes[rows]
-            v = d >= 0
-            a = torch.where(v, d, torch.zeros_like(d)).to(torch.float64).sum(0)
-            n = 2.0 * v.to(torch.float64).sum(0)
-        elif isinstance(mat, PackedVcf):
-            # biallelic alleles: the carriers of allele 1
-            a = mat.alt_counts(p)
-            n = torch.full_like(a, float(len(mat.sample_sets[p])))
-        else:
-            a = mat.haplotypes[rows].clamp(min=0).to(torch.float64).sum(0)
-            n = torch.full_like(a, float(len(mat.sample_sets[p])))
-        alt.append(a)
-        ref.append(n - a)
-        nh.append(n)
-    out = {}
-    P = len(pops)
-    for i in range(P):
-        for j in range(i, P):
-            if i == j:
-                val = (2.0 * ref[i] * alt[i] / (nh[i] * (nh[i] - 1))).sum()
-            else:
-                val = ((ref[i] * alt[j] + alt[i] * ref[j]) / (nh[i] * nh[j])).sum()
-            out[f"H_{i}_{j}"] = float(val)
-    return out
+    names = _het_names(len(pops))
+    if isinstance(mat, PackedVcf):
+        # biallelic alleles: the carriers of allele 1
+        counts = [(mat.alt_counts(p).to(torch.int32), None) for p in pops]
+    else:
+        x = L.as_device(mat.genotypes if use_genotypes else mat.haplotypes, np.int8)
+        counts = [_ops.site_counts(x, mat.sample_sets[p])[:2] for p in pops]
+    # every haplotype counts; of the genotypes the called ones
+    h = _ops.heterozygosity([c[0] for c in counts],
+                            [c[1] if use_genotypes else None for c in counts],
+                            [len(mat.sample_sets[p]) for p in pops], 2 if use_genotypes else 1)
+    return {name: float(v) for name, v in zip(names, h)}
