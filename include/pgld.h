@@ -465,6 +465,16 @@ int pgld_hap_window_snp_sums(pgld_handle h, const pgld_hap_panel* panel, const i
                              int32_t n_win, const int64_t* out_off, int32_t stat,
                              double* row_sums, double* col_sums, int64_t n_out, void* stream);
 
+/* Kim and Nielsen's omega of every window from pgld_hap_window_snp_sums'
+ * outputs (same window bounds and out_off, device int64; omega: device float64
+ * [n_win]): the largest ratio, over the splits l = 3 .. m - 2 of the window's m
+ * sites, of the mean within the two blocks to the mean across (0 where the sum
+ * across is not positive); 0 below 5 sites.  The split loop of ld_statistics.omega
+ * (ld_statistics.py:810-862). */
+int pgld_window_omega(pgld_handle h, const double* row_sums, const double* col_sums,
+                      const int64_t* win_begin, const int64_t* win_end, const int64_t* out_off,
+                      int32_t n_win, double* omega, void* stream);
+
 /* locate_unlinked pruning on the host (as the reference's): sliding windows
  * of `size` variants advanced by `step`; within a window, for still-active
  * variants i < j in order, j is dropped when r2 of the pair (i, j) exceeds

@@ -440,6 +440,24 @@ def window_snp_sums(pk, idx, win_begin, win_end, stat):
     return rows[:n_out], cols[:n_out], off
 
 
+def window_omega(rows, cols, off, win_begin, win_end):
+    """omega of each window on the host, from window_snp_sums' device sums and
+    host offsets (omega_from_sums on the device, one launch)."""
+    torch = _torch()
+    n_win = len(off) - 1
+    if n_win == 0:
+        return np.zeros(0)
+    if rows.numel() == 0:
+        return np.zeros(n_win)
+    out = torch.empty(n_win, dtype=torch.float64, device=rows.device)
+    wb, we, off_d = (L.as_device(np.ascontiguousarray(v), np.int64)
+                     for v in (win_begin, win_end, off[:-1]))
+    h = L.handle()
+    L.check(L.lib().pgld_window_omega(h, L.ptr(rows), L.ptr(cols), L.ptr(wb), L.ptr(we),
+                                      L.ptr(off_d), n_win, L.ptr(out), L.stream_ptr()), h)
+    return out.cpu().numpy()
+
+
 def omega_from_sums(row, col):
     """Kim and Nielsen's omega of m sites from the row sums row[i] = sum over
     j > i and column sums col[j] = sum over i < j of the pair statistic (the

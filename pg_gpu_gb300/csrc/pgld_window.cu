@@ -253,6 +253,87 @@ __global__ void __launch_bounds__(kThreads) window_kernel(Args a) {
   }
 }
 
+// Kim and Nielsen's omega of one window per CTA from its m row and column sums
+// (float64): with A[l], L[l] the sums of the first l rows / columns, split l
+// has L[l] within the left block, A[l] - L[l] across and A[m] - A[l] within
+// the right one; omega is the largest ratio of the within to the across mean
+// over l = 3 .. m - 2 with a positive across sum.  Two passes over the sums
+// (the total first), 256 splits at a time with a running prefix; a window of
+// some thousand sites takes microseconds, the host's prefix sums took 40.
+constexpr int kOmegaThreads = 256;
+
+__device__ __forceinline__ double2 omega_scan(double2 v, double2* sh, double2* total) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const double a = __shfl_up_sync(0xffffffffu, v.x, o), b = __shfl_up_sync(0xffffffffu, v.y, o);
+    if (lane >= o) {
+      v.x += a;
+      v.y += b;
+    }
+  }
+  __syncthreads();
+  if (lane == 31) sh[warp] = v;
+  __syncthreads();
+  double2 all = make_double2(0.0, 0.0);
+  for (int w = 0; w < kOmegaThreads / 32; ++w) {
+    if (w == warp) {
+      v.x += all.x;
+      v.y += all.y;
+    }
+    all.x += sh[w].x;
+    all.y += sh[w].y;
+  }
+  *total = all;
+  return v;  // inclusive
+}
+
+__global__ void __launch_bounds__(kOmegaThreads) window_omega_kernel(
+    const double* __restrict__ row, const double* __restrict__ col, const i64* __restrict__ off,
+    const i64* __restrict__ win_begin, const i64* __restrict__ win_end, double* __restrict__ out) {
+  __shared__ double2 sh[kOmegaThreads / 32];
+  const int w = blockIdx.x;
+  const i64 m = max((i64)0, win_end[w] - win_begin[w]);
+  const double *r = row + off[w], *c = col + off[w];
+  double best = -INFINITY;  // m >= 5 has a split
+  if (m >= 5) {
+    double2 tot, part = make_double2(0.0, 0.0);
+    for (i64 k = threadIdx.x; k < m; k += kOmegaThreads) part.x += r[k];
+    omega_scan(part, sh, &tot);
+    const double whole = tot.x;
+    double2 before = make_double2(0.0, 0.0);  // sums of the rows and columns below the block's
+    for (i64 k0 = 0; k0 < m - 2; k0 += kOmegaThreads) {
+      const i64 k = k0 + threadIdx.x;
+      const double2 v = k < m ? make_double2(r[k], c[k]) : make_double2(0.0, 0.0);
+      double2 blk;
+      const double2 s = omega_scan(v, sh, &blk);
+      const i64 l = k + 1;  // the first l sites form the left block
+      if (l >= 3 && l <= m - 2) {
+        const double A = before.x + s.x, left = before.y + s.y;
+        const double cross = A - left;
+        double ratio = 0.0;
+        if (cross > 0.0) {
+          const double n_within = (double)(l * (l - 1) / 2 + (m - l) * (m - l - 1) / 2);
+          ratio = (left + (whole - A)) / n_within / (cross / (double)(l * (m - l)));
+        }
+        best = max(best, ratio);
+      }
+      before.x += blk.x;
+      before.y += blk.y;
+    }
+  }
+  // the largest over the block
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) best = max(best, __shfl_xor_sync(0xffffffffu, best, o));
+  __syncthreads();
+  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5].x = best;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int k = 1; k < kOmegaThreads / 32; ++k) best = max(best, sh[k].x);
+    out[w] = m >= 5 ? best : 0.0;
+  }
+}
+
 }  // namespace win
 }  // namespace pgld
 
@@ -402,4 +483,22 @@ extern "C" int pgld_hap_window_snp_sums(pgld_handle h, const pgld_hap_panel* pan
   return window_run(h, panel, snp_idx, n_idx, reinterpret_cast<const i64*>(win_begin),
                     reinterpret_cast<const i64*>(win_end), n_win, nullptr, nullptr, (int)stat,
                     reinterpret_cast<const i64*>(out_off), row_sums, col_sums, st);
+}
+
+extern "C" int pgld_window_omega(pgld_handle h, const double* row_sums, const double* col_sums,
+                                 const int64_t* win_begin, const int64_t* win_end,
+                                 const int64_t* out_off, int32_t n_win, double* omega,
+                                 void* stream) {
+  PGLD_REQUIRE(h, h != nullptr, "pgld_window_omega: NULL handle");
+  PGLD_REQUIRE(h, n_win >= 0, "pgld_window_omega: n_win < 0");
+  if (n_win == 0) return PGLD_OK;
+  PGLD_REQUIRE(h, row_sums && col_sums && win_begin && win_end && out_off && omega,
+               "pgld_window_omega: NULL buffer");
+  PGLD_CHECK_CUDA(h, cudaSetDevice(h->device));
+  pgld::win::window_omega_kernel<<<(unsigned)n_win, pgld::win::kOmegaThreads, 0,
+                                   (cudaStream_t)stream>>>(
+      row_sums, col_sums, reinterpret_cast<const i64*>(out_off),
+      reinterpret_cast<const i64*>(win_begin), reinterpret_cast<const i64*>(win_end), omega);
+  PGLD_CHECK_CUDA(h, cudaGetLastError());
+  return PGLD_OK;
 }

@@ -402,9 +402,7 @@ def _omega_windows(hm, win_start, win_stop, column):
     seg, b, e = _segregating(hm.haplotypes, np.asarray(win_start, np.int64),
                              np.asarray(win_stop, np.int64))
     rows, cols, off = _ops.window_snp_sums(hm.packed(None), seg, b, e, column)
-    rows, cols = rows.cpu().numpy(), cols.cpu().numpy()
-    return np.array([_ops.omega_from_sums(rows[off[w]:off[w + 1]], cols[off[w]:off[w + 1]])
-                     for w in range(len(b))])
+    return _ops.window_omega(rows, cols, off, b, e)
 
 
 def omega(r2_matrix_or_matrix, missing_data="include", estimator="auto"):
