@@ -2,9 +2,8 @@
 // HaplotypeMatrix.pairwise_LD_v / pairwise_r2, haplotype_matrix.py:1092-1170)
 // and the distance-binned r^2 percentiles of windowed_r_squared
 // (haplotype_matrix.py:1235-1317) without moving the pair values to the host:
-// the valid pairs' r^2 are grouped by distance bin on the device and each
-// requested order statistic is found by an 8-bit radix select (one CTA per
-// order statistic, eight passes over its bin's values).
+// the valid pairs' r^2 are grouped by distance bin on the device and the
+// requested order statistics are found by radix selection.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -14,6 +13,9 @@
 #include "pgld_internal.cuh"
 
 using pgld::i64;
+
+int pgld_tc_int_positions(pgld_context* h, const double* pos, long long n, int* ipos, int* bad,
+                          cudaStream_t st);
 
 namespace pgld {
 namespace dense {
@@ -27,6 +29,7 @@ struct __align__(16) Smem {
   uint32_t ci[kKW][kPad], vi[kKW][kPad], cj[kKW][kPad], vj[kKW][kPad];
   double tr[kT][kT + 1];   // mirrored tile
   double bins[kMaxBins + 1];
+  int thr[kMaxBins + 1];
   int bin_cnt[kMaxBins];
   long long bin_base[kMaxBins];
 };
@@ -177,20 +180,44 @@ __device__ __forceinline__ int bin_index(const double* sb, int n_bins, double d)
   return lo;
 }
 
+// smallest integer distance of each bin edge
+__device__ __forceinline__ int int_edge(double b) {
+  const double c = ceil(b);
+  return c > 2147483647.0 ? 2147483647 : (c < -2147483647.0 ? -2147483647 : (int)c);
+}
+__device__ __forceinline__ int bin_index(const int* thr, int n_bins, int d) {
+  if (d < thr[0] || d >= thr[n_bins]) return -1;
+  int lo = 0, hi = n_bins;
+  while (hi - lo > 1) {
+    const int mid = (lo + hi) >> 1;
+    if (thr[mid] <= d) lo = mid; else hi = mid;
+  }
+  return lo;
+}
+
 // every pair i < j: its value (r^2 from the joint counts, or values[k] of the
 // condensed upper triangle), NaN skipped, binned by pos[j] - pos[i].
 // counts mode (out == NULL): bin_counts[b] += pairs; fill mode: the values
 // are written grouped by bin at cursor[b] (advanced atomically per tile).
+// The float64 pipe (two operations per SM and clock) bounds it: integer
+// positions are compared as integers, and counting asks only whether the
+// denominator is positive.  300 haplotypes x 5,001 SNPs: 0.50 ms for each of the
+// two passes when both divided and searched the bins in float64.
 __global__ void __launch_bounds__(kThreads) pairs_by_bin_kernel(
     const uint32_t* __restrict__ planes, int W, const double* __restrict__ values, i64 n,
-    const double* __restrict__ pos, const double* __restrict__ bins, int n_bins,
+    const double* __restrict__ pos, const int* __restrict__ ipos, const int* __restrict__ ipos_bad,
+    const double* __restrict__ bins, int n_bins,
     unsigned long long* __restrict__ bin_counts, unsigned long long* __restrict__ cursor,
     const unsigned long long* __restrict__ bin_end, double* __restrict__ out,
     int32_t* __restrict__ status) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   Smem& sm = *reinterpret_cast<Smem*>(smem_raw);
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  for (int x = threadIdx.x; x <= n_bins; x += kThreads) sm.bins[x] = bins[x];
+  for (int x = threadIdx.x; x <= n_bins; x += kThreads) {
+    sm.bins[x] = bins[x];
+    sm.thr[x] = int_edge(bins[x]);
+  }
+  const bool use_int = *ipos_bad == 0;
   const i64 nb = (n + kT - 1) / kT;
   const i64 n_tiles = nb * (nb + 1) / 2;
   for (i64 t = blockIdx.x; t < n_tiles; t += gridDim.x) {
@@ -213,9 +240,11 @@ __global__ void __launch_bounds__(kThreads) pairs_by_bin_kernel(
       bin[q] = -1;
       val[q] = 0.0;
       if (i < j && j < n) {
-        double v;
+        double v = 0.0;
+        bool defined;
         if (values) {
           v = values[i * (2 * n - i - 1) / 2 + (j - i - 1)];
+          defined = v == v;
         } else {
           // r^2 of ld_statistics.r_squared (haplotype_kernels.py:32-42):
           // (n11 n00 - n10 n01)^2 over pA (n - pA) pB (n - pB) of the pair's
@@ -225,11 +254,13 @@ __global__ void __launch_bounds__(kThreads) pairs_by_bin_kernel(
           const long long b = pa - a, c = pb - a, d = nn - pa - pb + a;
           const long long x = a * d - b * c;
           const long long den = pa * (nn - pa) * pb * (nn - pb);
-          v = den > 0 ? __ddiv_rn((double)(x * x), (double)den)
-                      : __longlong_as_double(0x7ff8000000000000LL);
+          defined = den > 0;
+          if (out && defined) v = __ddiv_rn((double)(x * x), (double)den);
         }
         val[q] = v;
-        if (v == v) bin[q] = bin_index(sm.bins, n_bins, pos[j] - pos[i]);
+        if (defined)
+          bin[q] = use_int ? bin_index(sm.thr, n_bins, ipos[j] - ipos[i])
+                           : bin_index(sm.bins, n_bins, pos[j] - pos[i]);
       }
       slot[q] = bin[q] >= 0 ? atomicAdd(&sm.bin_cnt[bin[q]], 1) : 0;
     }
@@ -258,61 +289,116 @@ __global__ void __launch_bounds__(kThreads) pairs_by_bin_kernel(
   }
 }
 
-// the rank-th smallest (0-based) value of each target's segment; values are
-// non-negative doubles, whose bit patterns order like the values: eight
-// passes over the segment, each fixing the next 8 bits of the answer from a
-// histogram of the values that share the bits fixed so far
-__global__ void __launch_bounds__(256) segment_kth_kernel(const double* __restrict__ values,
-                                                          const long long* __restrict__ seg_off,
-                                                          const long long* __restrict__ tseg,
-                                                          const long long* __restrict__ trank,
-                                                          double* __restrict__ out) {
-  __shared__ unsigned hist[8][256];
-  __shared__ unsigned long long prefix;
-  __shared__ long long rem;
-  const int t = blockIdx.x;
-  const long long seg = tseg[t];
-  const long long lo = seg_off[seg], hi = seg_off[seg + 1];
-  const int warp = threadIdx.x >> 5;
-  if (threadIdx.x == 0) {
-    prefix = 0ull;
-    rem = trank[t];
+// Order statistics of segments by radix selection: values are non-negative
+// doubles, whose bit patterns order like the values, so six passes over the
+// values fix 11, 11, 11, 11, 10 and 10 bits of every target.  A pass is one
+// launch over all segments (a block: one chunk of one segment, histograms of
+// the next digit in shared memory, one per distinct prefix among the segment's
+// targets) and one small launch that picks the targets' digits.  60 targets in
+// 12.5 million values (15 bins): 4.2 ms with one CTA per target and eight
+// passes of its own, 0.3 ms here.
+constexpr int kDigits = 6, kDigitBins = 2048;
+constexpr int kKthChunk = 1 << 15;
+constexpr int kKthGroup = 4;  // histograms per block at a time
+
+__host__ __device__ constexpr int digit_bits(int pass) { return pass < 4 ? 11 : 10; }
+__host__ __device__ constexpr int digit_shift(int pass) {
+  return pass < 4 ? 53 - 11 * pass : (pass == 4 ? 10 : 0);
+}
+
+struct KthArgs {
+  const double* values;
+  const long long* seg_off;    // [n_seg + 1]
+  const long long* chunk_off;  // [n_seg + 1] chunks of the segments before each
+  const int* tgt_off;          // [n_seg + 1] targets of the segments before each
+  long long* rank;             // [n_targets], rank among the values that share the prefix
+  unsigned long long* prefix;  // [n_targets], the bits fixed so far
+  int* rep;                    // [n_targets], first target with the same segment and prefix
+  unsigned* hist;              // [n_targets][kDigitBins]
+  int n_seg, n_targets;
+};
+
+__global__ void __launch_bounds__(256) kth_count_kernel(KthArgs a, int pass) {
+  __shared__ unsigned hist[kKthGroup][kDigitBins];
+  __shared__ int reps[kKthGroup];
+  int lo = 0, hi = a.n_seg;
+  while (hi - lo > 1) {
+    const int mid = (lo + hi) >> 1;
+    if (a.chunk_off[mid] <= (long long)blockIdx.x) lo = mid; else hi = mid;
   }
-  for (int pass = 0; pass < 8; ++pass) {
-    const int shift = 56 - 8 * pass;
-    for (int x = threadIdx.x; x < 8 * 256; x += blockDim.x) (&hist[0][0])[x] = 0u;
+  const long long v0 = a.seg_off[lo] + ((long long)blockIdx.x - a.chunk_off[lo]) * kKthChunk;
+  const long long v1 = min(a.seg_off[lo + 1], v0 + kKthChunk);
+  const int shift = digit_shift(pass), above = shift + digit_bits(pass);
+  const unsigned mask = (1u << digit_bits(pass)) - 1u;
+  for (int t = a.tgt_off[lo]; t < a.tgt_off[lo + 1];) {
+    // the next distinct prefixes
+    int n = 0;
     __syncthreads();
-    const unsigned long long want = pass == 0 ? 0ull : (prefix >> (shift + 8));
-    for (long long k = lo + threadIdx.x; k < hi; k += blockDim.x) {
-      const unsigned long long key = (unsigned long long)__double_as_longlong(values[k]);
-      if (pass == 0 || (key >> (shift + 8)) == want)
-        atomicAdd(&hist[warp][(unsigned)(key >> shift) & 255u], 1u);
-    }
-    __syncthreads();
-    {
-      unsigned v = 0;
-#pragma unroll
-      for (int w = 0; w < 8; ++w) v += hist[w][threadIdx.x];
-      __syncthreads();
-      hist[0][threadIdx.x] = v;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      long long r = rem;
-      int d = 255;
-      for (int x = 0; x < 256; ++x) {
-        if (r < (long long)hist[0][x]) {
-          d = x;
-          break;
-        }
-        r -= hist[0][x];
+    for (; t < a.tgt_off[lo + 1] && n < kKthGroup; ++t)
+      if (a.rep[t] == t) {
+        if (threadIdx.x == 0) reps[n] = t;
+        ++n;
       }
-      rem = r;
-      prefix |= (unsigned long long)d << shift;
+    for (int x = threadIdx.x; x < n * kDigitBins; x += 256) (&hist[0][0])[x] = 0u;
+    __syncthreads();
+    unsigned long long want[kKthGroup];
+#pragma unroll
+    for (int g = 0; g < kKthGroup; ++g)
+      want[g] = g < n && pass > 0 ? a.prefix[reps[g]] >> above : 0ull;
+#pragma unroll 4
+    for (long long k = v0 + threadIdx.x; k < v1; k += 256) {
+      const unsigned long long key = (unsigned long long)__double_as_longlong(a.values[k]);
+      const unsigned d = (unsigned)(key >> shift) & mask;
+      const unsigned long long top = pass > 0 ? key >> above : 0ull;
+#pragma unroll
+      for (int g = 0; g < kKthGroup; ++g)
+        if (g < n && top == want[g]) atomicAdd(&hist[g][d], 1u);
     }
     __syncthreads();
+    for (int x = threadIdx.x; x < n * kDigitBins; x += 256) {
+      const unsigned c = (&hist[0][0])[x];
+      if (c) atomicAdd(a.hist + (size_t)reps[x / kDigitBins] * kDigitBins + x % kDigitBins, c);
+    }
   }
-  if (threadIdx.x == 0) out[t] = __longlong_as_double((long long)prefix);
+}
+
+// a warp per target: the digit whose cumulative count passes the rank
+__global__ void __launch_bounds__(256) kth_pick_kernel(KthArgs a, int pass) {
+  const int t = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (t >= a.n_targets) return;
+  const unsigned* h = a.hist + (size_t)a.rep[t] * kDigitBins;
+  long long r = a.rank[t];
+  int digit = (1 << digit_bits(pass)) - 1;
+  for (int d0 = 0; d0 < (1 << digit_bits(pass)); d0 += 32) {
+    const unsigned c = h[d0 + lane];
+    unsigned incl = c;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const unsigned y = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += y;
+    }
+    const unsigned hit = __ballot_sync(0xffffffffu, (long long)incl > r);
+    if (hit) {
+      const int l = __ffs(hit) - 1;
+      r -= (long long)(__shfl_sync(0xffffffffu, incl, l) - __shfl_sync(0xffffffffu, c, l));
+      digit = d0 + l;
+      break;
+    }
+    r -= (long long)__shfl_sync(0xffffffffu, incl, 31);
+  }
+  if (lane == 0) {
+    a.rank[t] = r;
+    a.prefix[t] |= (unsigned long long)digit << digit_shift(pass);
+  }
+}
+
+// the first target of the same segment with the same prefix
+__global__ void kth_rep_kernel(KthArgs a, const int* __restrict__ tseg) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= a.n_targets) return;
+  int r = a.tgt_off[tseg[t]];
+  while (a.prefix[r] != a.prefix[t]) ++r;
+  a.rep[t] = r;
 }
 
 }  // namespace dense
@@ -374,13 +460,18 @@ extern "C" int pgld_pairs_by_bin(pgld_handle h, const uint32_t* planes, int32_t 
     for (int b = 0; b < n_bins; ++b) bin_counts[b] = 0;
   if (n_snp < 2) return PGLD_OK;
   PGLD_REQUIRE(h, pos != nullptr, "pgld_pairs_by_bin: NULL pos");
-  // workspace: counters [n_bins], cursors [n_bins], bin ends [n_bins]
+  // workspace: counters [n_bins], cursors [n_bins], bin ends [n_bins], integer
+  // positions and their flag
   void* ws = nullptr;
-  int rc = pgld_workspace(h, (size_t)3 * n_bins * 8, &ws);
+  int rc = pgld_workspace(h, (size_t)3 * n_bins * 8 + 16 + (size_t)n_snp * 4, &ws);
   if (rc) return rc;
   unsigned long long* cnt = (unsigned long long*)ws;
   unsigned long long* cur = cnt + n_bins;
   unsigned long long* end = cur + n_bins;
+  int* ipos_bad = (int*)(end + n_bins);
+  int* ipos = ipos_bad + 4;
+  rc = pgld_tc_int_positions(h, pos, n_snp, ipos, ipos_bad, st);
+  if (rc) return rc;
   std::vector<unsigned long long> host(2 * n_bins);
   if (values_out) {
     unsigned long long acc = 0;
@@ -402,8 +493,8 @@ extern "C" int pgld_pairs_by_bin(pgld_handle h, const uint32_t* planes, int32_t 
   PGLD_CHECK_CUDA(h, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   const int grid = dense_grid(h, (const void*)kern, smem, nb * (nb + 1) / 2);
   pgld_time_begin(h, st);
-  kern<<<grid, kThreads, smem, st>>>(planes, n_words, pair_values, n_snp, pos, bins, n_bins, cnt,
-                                     cur, end, values_out, h->dev_status);
+  kern<<<grid, kThreads, smem, st>>>(planes, n_words, pair_values, n_snp, pos, ipos, ipos_bad, bins,
+                                     n_bins, cnt, cur, end, values_out, h->dev_status);
   pgld_time_end(h, st);
   PGLD_CHECK_CUDA(h, cudaGetLastError());
   if (!values_out) {
@@ -435,25 +526,64 @@ extern "C" int pgld_segment_kth(pgld_handle h, const double* values, const int64
   }
   PGLD_CHECK_CUDA(h, cudaSetDevice(h->device));
   cudaStream_t st = (cudaStream_t)stream;
-  const size_t off_b = (size_t)(n_seg + 1) * 8, tb = (size_t)n_targets * 8;
-  void* ws = nullptr;
-  int rc = pgld_workspace(h, off_b + 3 * tb + 256, &ws);
-  if (rc) return rc;
-  long long* d_off = (long long*)ws;
-  long long* d_ts = d_off + (n_seg + 1);
-  long long* d_tr = d_ts + n_targets;
-  double* d_out = (double*)(d_tr + n_targets);
-  std::vector<long long> ts(n_targets), tr(n_targets);
+  // targets in segment order; chunks and targets of the segments before each
+  std::vector<int> by(n_targets), tseg(n_targets), tgt_off(n_seg + 1, 0);
+  for (int t = 0; t < n_targets; ++t) by[t] = t;
+  std::stable_sort(by.begin(), by.end(), [&](int x, int y) { return targets[2 * x] < targets[2 * y]; });
+  std::vector<long long> chunk_off(n_seg + 1, 0), rank(n_targets);
   for (int t = 0; t < n_targets; ++t) {
-    ts[t] = targets[2 * t];
-    tr[t] = targets[2 * t + 1];
+    tseg[t] = (int)targets[2 * by[t]];
+    rank[t] = targets[2 * by[t] + 1];
+    ++tgt_off[tseg[t] + 1];
   }
-  PGLD_CHECK_CUDA(h, cudaMemcpyAsync(d_off, seg_offsets, off_b, cudaMemcpyHostToDevice, st));
-  PGLD_CHECK_CUDA(h, cudaMemcpyAsync(d_ts, ts.data(), tb, cudaMemcpyHostToDevice, st));
-  PGLD_CHECK_CUDA(h, cudaMemcpyAsync(d_tr, tr.data(), tb, cudaMemcpyHostToDevice, st));
-  segment_kth_kernel<<<n_targets, 256, 0, st>>>(values, d_off, d_ts, d_tr, d_out);
-  PGLD_CHECK_CUDA(h, cudaGetLastError());
-  PGLD_CHECK_CUDA(h, cudaMemcpyAsync(out, d_out, tb, cudaMemcpyDeviceToHost, st));
+  for (int s = 0; s < n_seg; ++s) {
+    // only the segments that have targets are read
+    const long long len = tgt_off[s + 1] ? seg_offsets[s + 1] - seg_offsets[s] : 0;
+    chunk_off[s + 1] = chunk_off[s] + (len + kKthChunk - 1) / kKthChunk;
+    tgt_off[s + 1] += tgt_off[s];
+  }
+  std::vector<int> rep(n_targets);
+  for (int t = 0; t < n_targets; ++t) rep[t] = tgt_off[tseg[t]];
+  PGLD_REQUIRE(h, chunk_off[n_seg] < (1ll << 31), "pgld_segment_kth: too many values");
+  // one upload: offsets, chunk offsets, ranks, prefixes (0), then the int tables
+  const size_t nl = 2 * (size_t)(n_seg + 1) + 2 * (size_t)n_targets;
+  std::vector<long long> up(nl + ((size_t)(n_seg + 1) + 2 * (size_t)n_targets + 1) / 2, 0);
+  long long* u = up.data();
+  std::copy(seg_offsets, seg_offsets + n_seg + 1, u);
+  std::copy(chunk_off.begin(), chunk_off.end(), u + n_seg + 1);
+  std::copy(rank.begin(), rank.end(), u + 2 * (n_seg + 1));
+  int* ui = (int*)(u + nl);
+  std::copy(tgt_off.begin(), tgt_off.end(), ui);
+  std::copy(rep.begin(), rep.end(), ui + n_seg + 1);
+  std::copy(tseg.begin(), tseg.end(), ui + n_seg + 1 + n_targets);
+  const size_t up_b = (up.size() * 8 + 255) & ~size_t(255);
+  const size_t hist_b = (size_t)n_targets * kDigitBins * 4;
+  void* ws = nullptr;
+  int rc = pgld_workspace(h, up_b + hist_b, &ws);
+  if (rc) return rc;
+  KthArgs a{};
+  a.values = values;
+  a.seg_off = (long long*)ws;
+  a.chunk_off = a.seg_off + (n_seg + 1);
+  a.rank = (long long*)ws + 2 * (n_seg + 1);
+  a.prefix = (unsigned long long*)(a.rank + n_targets);
+  a.tgt_off = (int*)((long long*)ws + nl);
+  a.rep = (int*)((long long*)ws + nl) + (n_seg + 1);
+  a.hist = (unsigned*)((char*)ws + up_b);
+  a.n_seg = n_seg;
+  a.n_targets = n_targets;
+  const int* d_tseg = a.rep + n_targets;
+  PGLD_CHECK_CUDA(h, cudaMemcpyAsync(ws, u, up.size() * 8, cudaMemcpyHostToDevice, st));
+  for (int pass = 0; pass < kDigits; ++pass) {
+    PGLD_CHECK_CUDA(h, cudaMemsetAsync(a.hist, 0, hist_b, st));
+    kth_count_kernel<<<(unsigned)chunk_off[n_seg], 256, 0, st>>>(a, pass);
+    kth_pick_kernel<<<(unsigned)((n_targets + 7) / 8), 256, 0, st>>>(a, pass);
+    if (pass + 1 < kDigits) kth_rep_kernel<<<(unsigned)((n_targets + 255) / 256), 256, 0, st>>>(a, d_tseg);
+    PGLD_CHECK_CUDA(h, cudaGetLastError());
+  }
+  std::vector<double> got(n_targets);
+  PGLD_CHECK_CUDA(h, cudaMemcpyAsync(got.data(), a.prefix, (size_t)n_targets * 8, cudaMemcpyDeviceToHost, st));
   PGLD_CHECK_CUDA(h, cudaStreamSynchronize(st));
+  for (int t = 0; t < n_targets; ++t) out[by[t]] = got[t];
   return PGLD_OK;
 }
