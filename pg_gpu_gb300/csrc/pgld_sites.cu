@@ -26,17 +26,35 @@ constexpr int kThreads = kWarps * 32;
 constexpr int kWarpSites = 128;       // four per lane
 constexpr uint32_t kTop = 0x80808080u, kLow = 0x7f7f7f7fu;
 
-// the bytes at p[0 .. 3], of which n exist (the others read as 0)
-__device__ __forceinline__ uint32_t load4(const int8_t* p, i64 n) {
-  if (n >= 4) {
-    const int a = (int)((uintptr_t)p & 3);
-    const uint32_t* w = reinterpret_cast<const uint32_t*>(p - a);
-    if (a == 0) return __ldg(w);
-    return __funnelshift_r(__ldg(w), __ldg(w + 1), 8 * a);
-  }
+// the n < 4 bytes at p (the others read as 0)
+__device__ __forceinline__ uint32_t load_tail(const int8_t* p, i64 n) {
   uint32_t v = 0;
   for (int k = 0; k < (int)n; ++k) v |= (uint32_t)(uint8_t)__ldg(p + k) << (8 * k);
   return v;
+}
+// eight rows' four bytes at column s0: ALIGNED, one aligned word each, else the
+// two that the bytes lie in; all loads are issued before the first is used
+template <bool ALIGNED, class Row>
+__device__ __forceinline__ void load_rows(const int8_t* x, i64 ld, i64 s0, Row&& row,
+                                          uint32_t (&v)[8]) {
+  if constexpr (ALIGNED) {
+#pragma unroll
+    for (int r = 0; r < 8; ++r)
+      v[r] = __ldg(reinterpret_cast<const uint32_t*>(x + row(r) * ld + s0));
+  } else {
+    uint32_t hi[8], sh[8];
+#pragma unroll
+    for (int r = 0; r < 8; ++r) {
+      const int8_t* p = x + row(r) * ld + s0;
+      const int a = (int)((uintptr_t)p & 3);
+      const uint32_t* w = reinterpret_cast<const uint32_t*>(p - a);
+      sh[r] = 8 * a;
+      v[r] = __ldg(w);
+      hi[r] = __ldg(w + (a != 0));  // an aligned row's own word again
+    }
+#pragma unroll
+    for (int r = 0; r < 8; ++r) v[r] = __funnelshift_r(v[r], hi[r], sh[r]);
+  }
 }
 
 // 0x80 in every byte equal to c (0 <= c < 0x80): adding 0x7f to the low seven
@@ -44,34 +62,37 @@ __device__ __forceinline__ uint32_t load4(const int8_t* p, i64 n) {
 __device__ __forceinline__ uint32_t equal4(uint32_t v, uint32_t c) {
   return ~((((v ^ (c * 0x01010101u)) & kLow) + kLow) | v) & kTop;
 }
-__device__ __forceinline__ uint32_t minus_one4(uint32_t v) { return ~((~v & kLow) + kLow) & v & kTop; }
 
-// planes of one value: haplotypes carrier, reference, valid
+// The planes of a value.  split() leaves 0x80 in the bytes that belong to a
+// plane; neg1 / neg2 collect (in their top bits) the bytes equal to -1 and the
+// other negative ones: adding 1 to the low seven bits carries for -1 only.
+// over(): of one site's words, those above the values of the planes.
 struct HapPlanes {
   static constexpr int N = 3, kValid = 2, kMain = 2, kExt = 0;
-  __device__ static void split(uint32_t v, uint32_t (&m)[N], uint32_t& miss, uint32_t& other) {
+  __device__ static void split(uint32_t v, uint32_t (&m)[N], uint32_t& neg1, uint32_t& neg2) {
     m[0] = equal4(v, 1);
     m[1] = equal4(v, 0);
     m[2] = ~v & kTop;
-    const uint32_t none = minus_one4(v);
-    miss |= none;
-    other |= ~(m[0] | m[1] | none) & kTop;
+    const uint32_t up = (v & kLow) + 0x01010101u;
+    neg1 |= v & up;
+    neg2 |= v & ~up;
   }
+  static constexpr bool kAnyNegativeIsMissing = false;
 };
 // genotypes: dosages 0, 1, 2, valid, and (EXT) the values 3 .. 8
 template <bool EXT>
 struct GenoPlanes {
   static constexpr int N = EXT ? 10 : 4, kValid = 3, kMain = 3, kExt = EXT ? 6 : 0;
-  __device__ static void split(uint32_t v, uint32_t (&m)[N], uint32_t& miss, uint32_t& other) {
+  __device__ static void split(uint32_t v, uint32_t (&m)[N], uint32_t& neg1, uint32_t&) {
     m[0] = equal4(v, 0);
     m[1] = equal4(v, 1);
     m[2] = equal4(v, 2);
     m[3] = ~v & kTop;
-    miss |= v & kTop;
-    other |= m[3] & ~(m[0] | m[1] | m[2]);
+    neg1 |= v;
 #pragma unroll
     for (int e = 0; e < kExt; ++e) m[4 + e] = equal4(v, 3 + e);
   }
+  static constexpr bool kAnyNegativeIsMissing = true;
 };
 
 struct PackArgs {
@@ -85,11 +106,13 @@ struct PackArgs {
   int words;              // words per block (a power of two, at most kWarps)
 };
 
-// A warp turns 32 rows x 128 sites into one word per site and plane: per row
-// the comparison's bytes shift into a register per plane and eight rows, byte
+// A warp turns 32 rows x 128 sites into one word per site and plane: a row's
+// comparison bytes move to the row's bit (a high multiply, beside the
+// comparisons on the other pipe) in a register per plane and eight rows, byte
 // transposes then give the words.  The block's `words` words of a site are
 // stored together (32-byte segments at eight words), through shared memory.
-template <class S>
+// Values above the planes' show in the words themselves: valid, but in no plane.
+template <class S, bool ALIGNED>
 __global__ void __launch_bounds__(kThreads) pack_kernel(PackArgs a) {
   constexpr int kPitch = kWarps + 1;
   __shared__ uint32_t out[S::N][kWarpSites * kPitch];
@@ -101,24 +124,33 @@ __global__ void __launch_bounds__(kThreads) pack_kernel(PackArgs a) {
   uint32_t acc[S::N][4];
 #pragma unroll
   for (int p = 0; p < S::N; ++p) acc[p][0] = acc[p][1] = acc[p][2] = acc[p][3] = 0;
-  uint32_t miss = 0, other = 0;
+  uint32_t neg1 = 0, neg2 = 0;
   const i64 left = a.n_snp - s0;
-  const int mine = lane < live ? (a.rows ? __ldg(a.rows + 32 * word + lane) : 32 * word + lane) : 0;
+  // (rows past the last are loaded as the last one, and not used)
+  int mine = min(32 * word + lane, a.n_rows - 1);
+  if (a.rows) mine = __ldg(a.rows + mine);
+  const bool whole = s0 - 4 * lane + kWarpSites <= a.n_snp;  // a warp-uniform choice
 #pragma unroll
   for (int o = 0; o < 4; ++o) {
     uint32_t v[8];
+    auto row = [&](int r) { return (i64)__shfl_sync(0xffffffffu, mine, 8 * o + r); };
+    if (whole) {
+      load_rows<ALIGNED>(a.x, a.ld, s0, row, v);
+    } else {
 #pragma unroll
-    for (int r = 0; r < 8; ++r) {
-      const i64 row = __shfl_sync(0xffffffffu, mine, 8 * o + r);
-      v[r] = 8 * o + r < live && left > 0 ? load4(a.x + row * a.ld + s0, left) : 0u;
+      for (int r = 0; r < 8; ++r) {
+        const i64 at = row(r);
+        v[r] = 8 * o + r < live && left > 0 ? load_tail(a.x + at * a.ld + s0, min(left, (i64)4)) : 0u;
+      }
     }
 #pragma unroll
     for (int r = 0; r < 8; ++r) {
       if (8 * o + r < live) {
         uint32_t m[S::N];
-        S::split(v[r], m, miss, other);
+        S::split(v[r], m, neg1, neg2);
 #pragma unroll
-        for (int p = 0; p < S::N; ++p) acc[p][o] |= m[p] >> (7 - r);
+        for (int p = 0; p < S::N; ++p)  // m >> (7 - r), and add: the bits are apart
+          acc[p][o] = r == 7 ? acc[p][o] + m[p] : __umulhi(m[p], 1u << (25 + r)) + acc[p][o];
       }
     }
   }
@@ -127,18 +159,28 @@ __global__ void __launch_bounds__(kThreads) pack_kernel(PackArgs a) {
 #pragma unroll
   for (int k = 0; k < 4; ++k)
     if (k < left && (!a.before || a.before[s0 + k + 1] > a.before[s0 + k])) kept |= 0x80u << (8 * k);
+  uint32_t above[4];  // rows in a site's valid word and in no plane
 #pragma unroll
   for (int p = 0; p < S::N; ++p) {
     const uint32_t l0 = __byte_perm(acc[p][0], acc[p][1], 0x5140), l1 = __byte_perm(acc[p][0], acc[p][1], 0x7362);
     const uint32_t h0 = __byte_perm(acc[p][2], acc[p][3], 0x5140), h1 = __byte_perm(acc[p][2], acc[p][3], 0x7362);
     uint32_t* o = out[p] + 4 * lane * kPitch + warp;
-    o[0] = __byte_perm(l0, h0, 0x5410);
-    o[kPitch] = __byte_perm(l0, h0, 0x7632);
-    o[2 * kPitch] = __byte_perm(l1, h1, 0x5410);
-    o[3 * kPitch] = __byte_perm(l1, h1, 0x7632);
+    const uint32_t w[4] = {__byte_perm(l0, h0, 0x5410), __byte_perm(l0, h0, 0x7632),
+                           __byte_perm(l1, h1, 0x5410), __byte_perm(l1, h1, 0x7632)};
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      o[k * kPitch] = w[k];
+      if (p == 0) above[k] = ~w[k];
+      else if (p < S::kMain) above[k] &= ~w[k];
+      else if (p == S::kValid) above[k] &= w[k];
+    }
   }
-  const bool any_miss = __any_sync(0xffffffffu, (miss & kept) != 0);
-  const bool any_other = __any_sync(0xffffffffu, (other & kept) != 0);
+  uint32_t over = 0;
+#pragma unroll
+  for (int k = 0; k < 4; ++k)
+    if (kept & (0x80u << (8 * k))) over |= above[k];
+  const bool any_miss = __any_sync(0xffffffffu, (neg1 & kept) != 0);
+  const bool any_other = __any_sync(0xffffffffu, over != 0 || (!S::kAnyNegativeIsMissing && (neg2 & kept) != 0));
   if (lane == 0) {
     if (any_miss) atomicOr(a.flags, 1);
     if (any_other) atomicOr(a.flags + 1, 1);
@@ -172,7 +214,10 @@ int launch_pack(pgld_context* h, PackArgs a, cudaStream_t st) {
   const i64 per_block = (i64)(kWarps / a.words) * kWarpSites;
   const dim3 grid((unsigned)((a.n_snp + per_block - 1) / per_block),
                   (unsigned)((a.W + a.words - 1) / a.words));
-  pack_kernel<S><<<grid, kThreads, 0, st>>>(a);
+  if ((((uintptr_t)a.x | (uintptr_t)a.ld) & 3) == 0)
+    pack_kernel<S, true><<<grid, kThreads, 0, st>>>(a);
+  else
+    pack_kernel<S, false><<<grid, kThreads, 0, st>>>(a);
   PGLD_CHECK_CUDA(h, cudaGetLastError());
   return PGLD_OK;
 }
@@ -181,7 +226,9 @@ int launch_pack(pgld_context* h, PackArgs a, cudaStream_t st) {
 // per-site sums of the non-negative values, valid counts, presence flags
 // ---------------------------------------------------------------------------
 // block: 128 sites x a share of the rows, one row in eight per warp; at most
-// 255 rows per warp, so byte counters and 16-bit sums (127 each) never carry
+// 255 rows per warp, so byte counters and 16-bit sums (127 each) never carry.
+// SUMS: sum and valid; FLAGS: the presence bits.
+template <bool ALIGNED, bool SUMS, bool FLAGS>
 __global__ void __launch_bounds__(kThreads) site_counts_kernel(
     const int8_t* __restrict__ x, i64 ld, i64 n_snp, const int32_t* __restrict__ rows, int n_rows,
     int share, int32_t* __restrict__ sum, int32_t* __restrict__ valid,
@@ -191,30 +238,51 @@ __global__ void __launch_bounds__(kThreads) site_counts_kernel(
   if (threadIdx.x < kWarpSites) s_sum[threadIdx.x] = s_valid[threadIdx.x] = s_flag[threadIdx.x] = 0;
   __syncthreads();
   const i64 s0 = (i64)blockIdx.x * kWarpSites + 4 * lane, left = n_snp - s0;
+  const bool whole = s0 - 4 * lane + kWarpSites <= n_snp;
   const int r_end = min(n_rows, (int)(blockIdx.y + 1) * share);
   uint32_t even = 0, odd = 0, nv = 0, zero = 0, one = 0, bits = 0;
-  if (left > 0) {
-#pragma unroll 8
-    for (int r = (int)blockIdx.y * share + warp; r < r_end; r += kWarps) {
-      const i64 row = rows ? (i64)__ldg(rows + r) : (i64)r;
-      const uint32_t v = load4(x + row * ld + s0, left);
-      const uint32_t neg = v & kTop;
-      const uint32_t pos = v & ~((neg - (neg >> 7)) | neg);  // negative bytes cleared
+  auto add = [&](uint32_t v) {
+    uint32_t neg;  // 0xff for each negative byte (prmt's sign mode)
+    asm("prmt.b32 %0, %1, %1, 0xba98;" : "=r"(neg) : "r"(v));
+    const uint32_t pos = v & ~neg;
+    if (SUMS) {
       even += pos & 0x00ff00ffu;
-      odd += (pos >> 8) & 0x00ff00ffu;
-      nv += (~v >> 7) & 0x01010101u;
+      odd += __byte_perm(pos, 0u, 0x4341u);
+      nv += ~neg & 0x01010101u;
+    }
+    if (FLAGS) {
       zero |= equal4(v, 0);
       one |= equal4(v, 1);
       bits |= pos;
     }
+  };
+  auto at = [&](int r) { return rows ? (i64)__ldg(rows + r) : (i64)r; };
+  int r = (int)blockIdx.y * share + warp;
+  if (whole)
+    for (; r + 7 * kWarps < r_end; r += 8 * kWarps) {
+      uint32_t v[8];
+      load_rows<ALIGNED>(x, ld, s0, [&](int k) { return at(r + k * kWarps); }, v);
+#pragma unroll
+      for (int k = 0; k < 8; ++k) add(v[k]);
+    }
+  if (left > 0) {
+    for (; r < r_end; r += kWarps) {
+      const int8_t* p = x + at(r) * ld + s0;
+      add(ALIGNED && left >= 4 ? __ldg(reinterpret_cast<const uint32_t*>(p))
+                               : load_tail(p, min(left, (i64)4)));
+    }
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-      const uint32_t half = (k & 1) ? odd : even;
-      atomicAdd(&s_sum[4 * lane + k], (int)((half >> (k & 2 ? 16 : 0)) & 0xffffu));
-      atomicAdd(&s_valid[4 * lane + k], (int)((nv >> (8 * k)) & 0xffu));
-      const int f = (int)((zero >> (8 * k + 7)) & 1u) | (int)((one >> (8 * k + 7)) & 1u) << 1 |
-                    (((bits >> (8 * k)) & 0x7eu) ? 4 : 0);
-      if (f) atomicOr(&s_flag[4 * lane + k], f);
+      if (k >= left) break;
+      if (SUMS) {
+        atomicAdd(&s_sum[4 * lane + k], (int)((((k & 1) ? odd : even) >> (k & 2 ? 16 : 0)) & 0xffffu));
+        atomicAdd(&s_valid[4 * lane + k], (int)((nv >> (8 * k)) & 0xffu));
+      }
+      if (FLAGS) {
+        const int f = (int)((zero >> (8 * k + 7)) & 1u) | (int)((one >> (8 * k + 7)) & 1u) << 1 |
+                      (((bits >> (8 * k)) & 0x7eu) ? 4 : 0);
+        if (f) atomicOr(&s_flag[4 * lane + k], f);
+      }
     }
   }
   __syncthreads();
@@ -434,8 +502,13 @@ extern "C" int pgld_site_counts(pgld_handle h, const int8_t* x, int64_t ld, int6
   share = std::min<i64>((share + kWarps - 1) / kWarps, 255) * kWarps;
   gy = (n_rows + share - 1) / share;
   PGLD_REQUIRE(h, gy <= 65535, "pgld_site_counts: too many rows");
-  site_counts_kernel<<<dim3((unsigned)gx, (unsigned)gy), kThreads, 0, st>>>(
-      x, ld, n_snp, rows, n_rows, (int)share, sum, valid, flags);
+  const bool aligned = (((uintptr_t)x | (uintptr_t)ld) & 3) == 0;
+  const bool sums = sum || valid;
+  auto kern = !flags ? (aligned ? site_counts_kernel<true, true, false> : site_counts_kernel<false, true, false>)
+              : !sums ? (aligned ? site_counts_kernel<true, false, true> : site_counts_kernel<false, false, true>)
+                      : (aligned ? site_counts_kernel<true, true, true> : site_counts_kernel<false, true, true>);
+  kern<<<dim3((unsigned)gx, (unsigned)gy), kThreads, 0, st>>>(x, ld, n_snp, rows, n_rows, (int)share, sum,
+                                                              valid, flags);
   PGLD_CHECK_CUDA(h, cudaGetLastError());
   return PGLD_OK;
 }
