@@ -7,18 +7,16 @@
 // magnitude < 2^24, so it is formed exactly in float32 -- on the float32
 // pipes, with no integer-to-float conversions.
 //
-// Every numerator is rewritten as (at most) two products of such exact
-// integers -- e.g. DD: x (x + c2 + c3) - c1c4 n + (c1c4 + c2c3), pi2:
+// The numerators of one population are rewritten as (at most) two products of
+// such exact integers -- e.g. DD: x (x + c2 + c3) - c1c4 n + (c1c4 + c2c3), pi2:
 // c1c4 (n^2 - 4n + 2) + x (x + n - 1 - (n - 2)(c1 + c4)) -- and evaluated
 // with Kahan's algorithm for a*b + c*d (the rounding error of c*d recovered
 // exactly by an fma, one fma and one addition more), whose relative error is
 // at most 2u even under cancellation (Jeannerod, Louvet and Muller, "Further
 // analysis of Kahan's algorithm for the accurate computation of 2x2
-// determinants", Math. Comp. 82, 2013).  The one numerator with three
-// products, pi2(i,j,i,j), sums its two cubic products exactly as s + t
-// (TwoProduct / TwoSum: the low parts are integers below 2^22 and add exactly)
-// before one fma adds the quartic product, so it carries at most 3u (DD
-// likewise, its exact integer remainder added last).
+// determinants", Math. Comp. 82, 2013); DD, whose exact integer remainder is
+// added last, carries 3u.  The pi2 numerators of two populations are products
+// of distinct draws (Draws below).
 // 64-bit integer multiplies would run at the float64 rate on GB300.
 // Denominators come from per-CTA tables of reciprocals indexed by the valid
 // sample size n (1/n, 1/(n(n-1)), 1/(n(n-1)(n-2)), 1/(n(n-1)(n-2)(n-3)), each
@@ -168,30 +166,37 @@ PGLD_HD float pi2_num(const Pop& p) {
   const float w = fmaf(2.0f - p.ns, p.t, p.x + (p.ns - 1.0f));
   return dot2(p.a, pn, p.x, w);
 }
-// pi2 with population t three times and s once, times 2
-PGLD_HD float triple_num2(const Pop& t, const Pop& s) {
-  return dot2(t.pA * t.qA, t.qB * s.pB + t.pB * s.qB - 2.0f * s.qB, t.pA * t.c4 + t.c2 * t.qA,
-              s.qB - s.pB);
+// Draws from one population over distinct haplotypes, as whole features: X1 ..
+// X4 = pA pB - c1, pA qB - c2, qA pB - c3, qA qB - c4 (two draws; since pA pB =
+// n c1 - x, exact integers c1 (n - 1) - x and so on), T1, T2 = draws (A, a, b),
+// (A, a, B): pA X4 - c2 qA, pA X3 - c1 qA (one rounding).  The statistics of
+// both populations are then sums of non-negative products: pi2(t,t,t,s) times 2
+// and pi2(i,j,i,j) times 4 below, and pi2 of one population = T1 pB - (c1 X4 +
+// c3 X2), whose subtraction at most halves the first term: within 5u.  A third
+// fewer operations than the expanded polynomials with their error terms (33 of
+// 150 for two populations).
+struct Draws {
+  float X1, X2, X3, X4, T1, T2;
+};
+PGLD_HD Draws draws(const Pop& p) {
+  Draws d;
+  const float m = p.ns - 1.0f;
+  d.X1 = fmaf(p.c1, m, -p.x);
+  d.X2 = fmaf(p.c2, m, p.x);
+  d.X3 = fmaf(p.c3, m, p.x);
+  d.X4 = fmaf(p.c4, m, -p.x);
+  d.T1 = fmaf(p.pA, d.X4, -fmul(p.c2, p.qA));
+  d.T2 = fmaf(p.pA, d.X3, -fmul(p.c1, p.qA));
+  return d;
 }
-// pi2(i,j,i,j) times 4 (symmetric in the two populations).  The quartic and
-// cubic polynomial of the reference (ld_statistics.py:1349-1402) equals
-//   H_A H_B + (1 - n_A - n_B) K - x_A e_B - x_B e_A
-//   = K m_A m_B + x_B (m_A e_A) + x_A (m_B e_B + 4 x_B)
-// with H_A = qA_A pA_B + pA_A qA_B, H_B = qB_A pB_B + pB_A qB_B,
-// K = c1_A c4_B + c2_A c3_B + c3_A c2_B + c4_A c1_B and m = n - 1 (algebraic
-// identities, checked against the oracle in tests/test_epilogue_cpu.py).  The
-// two cubic products are summed exactly as s + t; K m_A m_B + s rounds once in
-// the fma and t (an integer below 2^22) is added last.
-PGLD_HD float ijij_num4(const Pop& A, const Pop& B) {
-  const float K = A.c1 * B.c4 + A.c2 * B.c3 + A.c3 * B.c2 + A.c4 * B.c1;
-  const float mA = A.ns - 1.0f, mB = B.ns - 1.0f;
-  const float y1 = mA * A.e, y2 = fmaf(mB, B.e, 4.0f * B.x);
-  const float p1 = fmul(B.x, y1), e1 = fmaf(B.x, y1, -p1);
-  const float p2 = fmul(A.x, y2), e2 = fmaf(A.x, y2, -p2);
-  const float s = fadd(p1, p2);
-  const float bb = fsub(s, p1);
-  const float t = fadd(fadd(fsub(p1, fsub(s, bb)), fsub(p2, bb)), fadd(e1, e2));
-  return fadd(fmaf(K, fmul(mA, mB), s), t);
+PGLD_HD float pi2_draws(const Pop& p, const Draws& d) {
+  return fmaf(d.T1, p.pB, -fmaf(p.c1, d.X4, fmul(p.c3, d.X2)));
+}
+PGLD_HD float triple_num2(const Draws& t, const Pop& s) {
+  return fmaf(s.pB, t.T1, fmul(s.qB, t.T2));
+}
+PGLD_HD float ijij_num4(const Draws& i, const Draws& j) {
+  return fmaf(i.X1, j.X4, fmaf(i.X2, j.X3, fmaf(i.X3, j.X2, fmul(i.X4, j.X1))));
 }
 
 // DD, Dz, pi2 of one population (moments order for one population)
@@ -217,6 +222,7 @@ PGLD_HD void stats2(const Pop& p, const Pop& q, const Recip& T, float o[15]) {
   const float r22 = T.r2[p.n] * T.r2[q.n];
   const float r31p = T.r3[p.n] * T.inv[q.n];  // 1 / (n_q * n_p(n_p-1)(n_p-2))
   const float r31q = T.r3[q.n] * T.inv[p.n];
+  const Draws dp = draws(p), dq = draws(q);
   o[0] = dd_num(p) * r4p;
   o[1] = (p.x * q.x) * r22;
   o[2] = dd_num(q) * r4q;
@@ -226,12 +232,12 @@ PGLD_HD void stats2(const Pop& p, const Pop& q, const Recip& T, float o[15]) {
   o[6] = (q.x * (p.e + p.dB * p.dA)) * r22;
   o[7] = (q.x * (q.dA * p.dB + q.dB * p.dA)) * (0.5f * r31q);
   o[8] = dz_num(q) * r4q;
-  o[9] = pi2_num(p) * r4p;
-  o[10] = triple_num2(p, q) * (0.5f * r31p);
+  o[9] = pi2_draws(p, dp) * r4p;
+  o[10] = triple_num2(dp, q) * (0.5f * r31p);
   o[11] = fmaf(p.pA * p.qA, q.pB * q.qB, (q.pA * q.qA) * (p.pB * p.qB)) * (0.5f * r22);
-  o[12] = ijij_num4(p, q) * (0.25f * r22);
-  o[13] = triple_num2(q, p) * (0.5f * r31q);
-  o[14] = pi2_num(q) * r4q;
+  o[12] = ijij_num4(dp, dq) * (0.25f * r22);
+  o[13] = triple_num2(dq, p) * (0.5f * r31q);
+  o[14] = pi2_draws(q, dq) * r4q;
 }
 
 }  // namespace fast

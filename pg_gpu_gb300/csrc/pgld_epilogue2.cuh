@@ -111,22 +111,27 @@ PGLD_HD V pi2_num(const Pop& p) {
   const V w = vfma(vsub(vs(2.0f), p.ns), p.t, vadd(p.x, p.m1));
   return dot2(p.a, pn, p.x, w);
 }
-// uA = pA qA of population t
-PGLD_HD V triple_num2(const Pop& t, const Pop& s, V uA) {
-  return dot2(uA, vsub(vfma(t.qB, s.pB, vmul(t.pB, s.qB)), vadd(s.qB, s.qB)),
-              vfma(t.pA, t.c4, vmul(t.c2, t.qA)), vsub(s.qB, s.pB));
+// fast::Draws of two pairs
+struct Draws {
+  V X1, X2, X3, X4, T1, T2;
+};
+PGLD_HD Draws draws(const Pop& p) {
+  Draws d;
+  const V nx = vneg(p.x);
+  d.X1 = vfma(p.c1, p.m1, nx);
+  d.X2 = vfma(p.c2, p.m1, p.x);
+  d.X3 = vfma(p.c3, p.m1, p.x);
+  d.X4 = vfma(p.c4, p.m1, nx);
+  d.T1 = vfma(p.pA, d.X4, vneg(vmul(p.c2, p.qA)));
+  d.T2 = vfma(p.pA, d.X3, vneg(vmul(p.c1, p.qA)));
+  return d;
 }
-PGLD_HD V ijij_num4(const Pop& A, const Pop& B) {
-  const V K = vfma(A.c1, B.c4, vfma(A.c2, B.c3, vfma(A.c3, B.c2, vmul(A.c4, B.c1))));
-  const V mA = A.m1, mB = B.m1;
-  const V x2 = vadd(B.x, B.x);
-  const V y1 = vmul(mA, A.e), y2 = vfma(mB, B.e, vadd(x2, x2));
-  const V p1 = vmul(B.x, y1), e1 = vfma(B.x, y1, vneg(p1));
-  const V p2 = vmul(A.x, y2), e2 = vfma(A.x, y2, vneg(p2));
-  const V s = vadd(p1, p2);
-  const V bb = vsub(s, p1);
-  const V t = vadd(vadd(vsub(p1, vsub(s, bb)), vsub(p2, bb)), vadd(e1, e2));
-  return vadd(vfma(K, vmul(mA, mB), s), t);
+PGLD_HD V pi2_draws(const Pop& p, const Draws& d) {
+  return vfma(d.T1, p.pB, vneg(vfma(p.c1, d.X4, vmul(p.c3, d.X2))));
+}
+PGLD_HD V triple_num2(const Draws& t, const Pop& s) { return vfma(s.pB, t.T1, vmul(s.qB, t.T2)); }
+PGLD_HD V ijij_num4(const Draws& i, const Draws& j) {
+  return vfma(i.X1, j.X4, vfma(i.X2, j.X3, vfma(i.X3, j.X2, vmul(i.X4, j.X1))));
 }
 
 // the reciprocal factors of the valid n of two lanes: 1/n, 1/(n(n-1)),
@@ -168,13 +173,14 @@ PGLD_HD void stats2_to(const Pop& p, const Pop& q, const float4* T4, Sink&& sink
   sink(2, dd_num(q), rq.r4);
   sink(3, dz_num(p, wp), rp.r4);
   sink(8, dz_num(q, wq), rq.r4);
-  sink(9, pi2_num(p), rp.r4);
-  sink(14, pi2_num(q), rq.r4);
   sink(5, vmul(p.x, wq), r22);
   sink(6, vmul(q.x, wp), r22);
   const V uAp = vmul(p.pA, p.qA), uAq = vmul(q.pA, q.qA);
   sink(11, vfma(uAp, vmul(q.pB, q.qB), vmul(uAq, vmul(p.pB, p.qB))), r22);  // x kPost11
-  sink(12, ijij_num4(p, q), r22);                                            // x kPost12
+  const Draws dp = draws(p), dq = draws(q);
+  sink(9, pi2_draws(p, dp), rp.r4);
+  sink(14, pi2_draws(q, dq), rq.r4);
+  sink(12, ijij_num4(dp, dq), r22);                                          // x kPost12
   const V dc = vfma(p.dA, q.dB, vmul(p.dB, q.dA));
 #if PGLD_F2_SSCALE
   const V h31p = vmul_s(rp.r3h, rq.inv);
@@ -182,14 +188,14 @@ PGLD_HD void stats2_to(const Pop& p, const Pop& q, const float4* T4, Sink&& sink
   const V h31p = vmul(rp.r3h, rq.inv);
 #endif
   sink(4, vmul(p.x, dc), h31p);
-  sink(10, triple_num2(p, q, uAp), h31p);
+  sink(10, triple_num2(dp, q), h31p);
 #if PGLD_F2_SSCALE
   const V h31q = vmul_s(rq.r3h, rp.inv);
 #else
   const V h31q = vmul(rq.r3h, rp.inv);
 #endif
   sink(7, vmul(q.x, dc), h31q);
-  sink(13, triple_num2(q, p, uAq), h31q);
+  sink(13, triple_num2(dq, p), h31q);
 }
 
 // the sink's products, statistics 11 and 12 still without their post factors
