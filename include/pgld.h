@@ -449,6 +449,14 @@ int pgld_hap_window_sums(pgld_handle h, const pgld_hap_panel* panel, const int32
                          int32_t n_win, double* sums, int64_t* counts, int32_t form,
                          void* stream);
 
+/* pgld_hap_window_sums for some of its columns (bit k of `columns`: column k of
+ * sums): the others, and the count of pairs with r^2 defined unless column 0
+ * is among them, may be left 0. */
+int pgld_hap_window_sums_columns(pgld_handle h, const pgld_hap_panel* panel, const int32_t* snp_idx,
+                                 int64_t n_idx, const int64_t* win_begin, const int64_t* win_end,
+                                 int32_t n_win, double* sums, int64_t* counts, int32_t columns,
+                                 int32_t form, void* stream);
+
 /* Per-SNP row and column sums of one window statistic, for Kim and Nielsen's
  * omega over batched windows (one launch).  Windows as pgld_hap_window_sums
  * (they may overlap).  For every pair of list positions a < b of window w

@@ -121,6 +121,8 @@ _SIGS = {
     "pgld_hap_window_sums": ([_P, ctypes.POINTER(HapPanel), _P, _I64, _P, _P, _I32, _P, _P, _I32,
                               _P],
                              ctypes.c_int),
+    "pgld_hap_window_sums_columns": ([_P, ctypes.POINTER(HapPanel), _P, _I64, _P, _P, _I32, _P, _P,
+                                      _I32, _I32, _P], ctypes.c_int),
     "pgld_hap_binned_sums_noalloc": ([ctypes.c_int, ctypes.POINTER(HapPanel), _P, _D, _P, _P, _I32,
                                       _P, _P, _P], ctypes.c_int),
     "pgld_noalloc_status": ([ctypes.c_int, ctypes.POINTER(_I32)], ctypes.c_int),

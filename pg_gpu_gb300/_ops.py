@@ -366,14 +366,18 @@ def band_pairs(pk, pos_d, max_dist, with_stats=True, form="auto", _tuning=False)
 WINDOW_COLUMNS = ("r2", "sigma_d2", "dd", "dz", "pi2", "r2_naive")
 
 
-def window_sums(pk, idx, win_begin, win_end, form="auto", _tuning=False):
+def window_sums(pk, idx, win_begin, win_end, form="auto", _tuning=False, columns=WINDOW_COLUMNS):
     """Per-window sums (n_win, 6) float64 and counts (n_win, 3) int64 over
     every pair inside each window (one launch for all windows).
 
     idx: int32 SNP indices (None: identity); window w covers
     idx[win_begin[w]:win_end[w]].  Columns: WINDOW_COLUMNS; counts: pairs,
     pairs with r^2 defined, pairs with n >= 4.  form: "tc", "plain" or
-    "auto" (tensor cores whenever they apply)."""
+    "auto" (tensor cores whenever they apply).  columns: those wanted (the
+    others, and the second count without "r2", may be left 0)."""
+    mask = 0
+    for c in columns:
+        mask |= 1 << WINDOW_COLUMNS.index(c)
     if form == "auto":
         form = "tc" if tc_applies([pk]) else "plain"
     if form == "tc" and not _tuning:
@@ -393,10 +397,11 @@ def window_sums(pk, idx, win_begin, win_end, form="auto", _tuning=False):
     ii = None if idx is None else L.as_device(idx, np.int32)
     n_idx = pk.n_snp if ii is None else ii.numel()
     h = L.handle()
-    L.check(L.lib().pgld_hap_window_sums(h, ctypes.byref(panel([pk])), L.ptr(ii), n_idx, L.ptr(wb),
-                                         L.ptr(we), n_win, L.ptr(sums), L.ptr(cnt),
-                                         L.FORM_TC if form == "tc" else L.FORM_PLAIN,
-                                         L.stream_ptr()), h)
+    L.check(L.lib().pgld_hap_window_sums_columns(h, ctypes.byref(panel([pk])), L.ptr(ii), n_idx,
+                                                 L.ptr(wb), L.ptr(we), n_win, L.ptr(sums),
+                                                 L.ptr(cnt), mask,
+                                                 L.FORM_TC if form == "tc" else L.FORM_PLAIN,
+                                                 L.stream_ptr()), h)
     st = torch.zeros(1, dtype=torch.int32)
     L.check(L.lib().pgld_device_status(h, ctypes.cast(st.data_ptr(), ctypes.POINTER(
         ctypes.c_int32)), L.stream_ptr()), h)

@@ -517,7 +517,7 @@ __global__ void __launch_bounds__(kThreads, 1)
             const fast2::Pop p = fast2::make(u2(r[o], r[o + 1]), u2(r[o + 4], r[o + 5]),
                                              u2(r[o + 2], r[o + 3]), u2(r[o + 6], r[o + 7]));
             const int gg = 2 * gp + g;
-            win::window_pair2(p, u2(r[o], r[o + 1]),
+            win::window_pair2<win::kAllColumns>(p, u2(r[o], r[o + 1]),
                               [&](int n) { return make_float2(T.inv[n], T.r4[n]); }, fi,
                               l0 ? wfj[2 * gg] : zero4,
                               l1 ? wfj[2 * gg + 1] : zero4, l0, l1, ws2, np, nr2, nfour);
@@ -1099,7 +1099,7 @@ int pgld_tc_wide_pairs(pgld_context* h, const pgld_hap_panel* panel, pgld::BandA
                        cudaStream_t st);
 int pgld_tc_wide_windows(pgld_context* h, const pgld_hap_panel* panel, const int32_t* idx,
                          long long n_idx, const long long* wb, const long long* we, int n_win,
-                         double* sums, unsigned long long* counts, cudaStream_t st);
+                         double* sums, unsigned long long* counts, int columns, cudaStream_t st);
 
 // per-pair outputs: 64 x 64 tiles unless the 64 x 128 layout (pgld_tc_wide.cu)
 // is configured (the output stores bound this form; at 2,000 haplotypes the
@@ -1151,11 +1151,12 @@ int pgld_site_freqs(pgld_context* h, const uint32_t* planes, const uint32_t* val
 // window is a contiguous range of operand rows.
 int pgld_tc_windows(pgld_context* h, const pgld_hap_panel* panel, const int32_t* idx,
                     long long n_idx, const long long* wb, const long long* we, int n_win,
-                    double* sums, unsigned long long* counts, cudaStream_t st) {
+                    double* sums, unsigned long long* counts, int columns, cudaStream_t st) {
   using namespace pgld::tc;
   // 64 x 128 tiles (pgld_tc_wide.cu) unless the square layout is configured
+  // (which forms every column)
   if (h->tc_layout != 1)
-    return pgld_tc_wide_windows(h, panel, idx, n_idx, wb, we, n_win, sums, counts, st);
+    return pgld_tc_wide_windows(h, panel, idx, n_idx, wb, we, n_win, sums, counts, columns, st);
   int rc = get_encode(h);
   if (rc) return rc;
   const long long n = panel->n_snp;

@@ -260,8 +260,8 @@ __device__ __forceinline__ bool role_wait(uint64_t* b, uint32_t parity, volatile
 
 // MODE kModeBinned: distance-binned sums of two populations (combined
 // operand); kModePairs: per-pair outputs of one population; kModeWindows:
-// per-window sums of one population
-template <int MODE>
+// per-window sums of one population (the columns COLS of them)
+template <int MODE, int COLS = win::kAllColumns>
 __global__ void __launch_bounds__(kThreads, 1)
     band_wide_kernel(const __grid_constant__ CUtensorMap map_a,
                      const __grid_constant__ CUtensorMap map_b, Params a) {
@@ -472,6 +472,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       if (cur_w >= 0) {
 #pragma unroll
         for (int s2 = 0; s2 < 6; ++s2) {
+          if (!((COLS >> s2) & 1)) continue;
           double v = (double)run[s2] + (double)comp[s2];
 #pragma unroll
           for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
@@ -619,8 +620,9 @@ __global__ void __launch_bounds__(kThreads, 1)
         // the naive-r^2 site terms of the lane's SNPs, loaded before the wait
         const float4 zero4 = make_float4(0.f, 0.f, 0.f, 0.f);
         float4 wfi[2], wfj[8];
+        constexpr bool kSites = (COLS & 61) != 0;  // sigma_D^2 needs the counts alone
         auto site_at = [&](long long pos) {
-          if (pos < wb_ || pos >= we_) return zero4;
+          if (!kSites || pos < wb_ || pos >= we_) return zero4;
           const long long sp = a.idx ? (long long)a.idx[pos] : pos;
           return (sp >= 0 && sp < a.n_panel) ? a.site[sp] : zero4;
         };
@@ -664,8 +666,8 @@ __global__ void __launch_bounds__(kThreads, 1)
             const bool iok = F || (is >= wb_ && is < we_);
             const float4 fi = wfi[hh];
             // the shorter form's n is the row SNP's nv: its r4 and n >= 4 once
-            const int nvi = fast::f2i_small(fi.y);
-            const float r4i = T4[nvi].w;
+            const int nvi = kSites ? fast::f2i_small(fi.y) : 0;
+            const float r4i = kSites ? T4[nvi].w : 0.f;
             const bool four_i = nvi >= 4;
 #pragma unroll
             for (int g = 0; g < 2; ++g) {
@@ -684,11 +686,12 @@ __global__ void __launch_bounds__(kThreads, 1)
               // (n = nv_i = nv_j), for every lane: the shorter form
               const bool same = (!l0 || (p.ns.x == fi.y && p.ns.x == sj0.y)) &&
                                 (!l1 || (p.ns.y == fi.y && p.ns.y == sj1.y));
-              if (__all_sync(0xffffffffu, same))
-                win::window_pair2_same(p, four_i, r4i, fi, sj0, sj1, l0, l1, ws2, np, nr2, nfour);
+              if (kSites && __all_sync(0xffffffffu, same))
+                win::window_pair2_same<COLS>(p, four_i, r4i, fi, sj0, sj1, l0, l1, ws2, np, nr2,
+                                             nfour);
               else
-                win::window_pair2(p, u2(r[o], r[o + 1]), tab, fi, sj0, sj1, l0, l1, ws2, np, nr2,
-                                  nfour);
+                win::window_pair2<COLS>(p, u2(r[o], r[o + 1]), tab, fi, sj0, sj1, l0, l1, ws2, np,
+                                        nr2, nfour);
             }
           }
         };
@@ -697,6 +700,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         // compensated (Neumaier) running sums of the lane's unit totals
 #pragma unroll
         for (int s2 = 0; s2 < 6; ++s2) {
+          if (!((COLS >> s2) & 1)) continue;
           const float v = __fadd_rn(ws2[s2].x, ws2[s2].y);
           const float sum = __fadd_rn(run[s2], v);
           const float err = fabsf(run[s2]) >= fabsf(v) ? __fadd_rn(__fsub_rn(run[s2], sum), v)
@@ -1208,7 +1212,7 @@ int pgld_site_freqs(pgld_context* h, const uint32_t* planes, const uint32_t* val
                     long long n_snp, float4* site, cudaStream_t st);
 
 // shared memory, stages and the register check of a one-population launch
-template <int MODE>
+template <int MODE, int COLS = pgld::win::kAllColumns>
 static int wide_one_pop_launch(pgld_context* h, pgld::tcw::Params& prm, const CUtensorMap& map_a,
                                const CUtensorMap& map_b, cudaStream_t st, const char* what) {
   using namespace pgld::tcw;
@@ -1226,7 +1230,7 @@ static int wide_one_pop_launch(pgld_context* h, pgld::tcw::Params& prm, const CU
   if (stages < 2) return pgld_fail(h, PGLD_ERR_TOO_LARGE, "%s: shared memory", what);
   prm.stages = stages;
   const size_t smem = (size_t)stages * kStage + fixed;
-  auto kern = band_wide_kernel<MODE>;
+  auto kern = band_wide_kernel<MODE, COLS>;
 #if PGLD_TCW_MAXNREG
   {
     cudaFuncAttributes fa;
@@ -1314,7 +1318,7 @@ int pgld_tc_wide_pairs(pgld_context* h, const pgld_hap_panel* panel, pgld::BandA
 // of operand rows; one launch over the tiles of every window.
 int pgld_tc_wide_windows(pgld_context* h, const pgld_hap_panel* panel, const int32_t* idx,
                          long long n_idx, const long long* wb, const long long* we, int n_win,
-                         double* sums, unsigned long long* counts, cudaStream_t st) {
+                         double* sums, unsigned long long* counts, int columns, cudaStream_t st) {
   using namespace pgld::tcw;
   int rc = get_encode(h);
   if (rc) return rc;
@@ -1349,7 +1353,11 @@ int pgld_tc_wide_windows(pgld_context* h, const pgld_hap_panel* panel, const int
   }
   rc = pgld::exclusive_scan_i64(h, tiles, n_win, w + off_scan, sb, st);
   if (rc) return rc;
-  if (n > 0) {
+  // the two estimators of ZnS each have a kernel of their column alone (400
+  // haplotypes, 512 windows of 500-20,000 SNPs: the whole ZnS call 50.8 ms with
+  // all columns, 23.3 ms with sigma_D^2 alone)
+  const bool sigma = columns == 2;
+  if (n > 0 && !sigma) {
     rc = pgld_site_freqs(h, panel->planes[0], nullptr, W, n, site, st);
     if (rc) return rc;
   }
@@ -1383,6 +1391,12 @@ int pgld_tc_wide_windows(pgld_context* h, const pgld_hap_panel* panel, const int
   prm.n_panel = n;
   prm.wsums = sums;
   prm.wcnt = counts;
-  return wide_one_pop_launch<pgld::kModeWindows>(h, prm, map_a, map_b, st,
-                                                 "band_wide_kernel (windows)");
+  if (sigma)
+    return wide_one_pop_launch<pgld::kModeWindows, 2>(h, prm, map_a, map_b, st,
+                                                      "band_wide_kernel (windows)");
+  if (columns == 32)
+    return wide_one_pop_launch<pgld::kModeWindows, 32>(h, prm, map_a, map_b, st,
+                                                       "band_wide_kernel (windows)");
+  return wide_one_pop_launch<pgld::kModeWindows, pgld::win::kAllColumns>(
+      h, prm, map_a, map_b, st, "band_wide_kernel (windows)");
 }

@@ -348,7 +348,7 @@ int pgld_site_freqs(pgld_context* h, const uint32_t* planes, const uint32_t* val
 int pgld_tc_supported(pgld_context* h, const pgld_hap_panel* panel);
 int pgld_tc_windows(pgld_context* h, const pgld_hap_panel* panel, const int32_t* idx,
                     long long n_idx, const long long* wb, const long long* we, int n_win,
-                    double* sums, unsigned long long* counts, cudaStream_t st);
+                    double* sums, unsigned long long* counts, int columns, cudaStream_t st);
 
 // the plain window kernel over windows [wb[w], we[w]) of the index list:
 // window sums (snp_stat < 0) or per-SNP row / column sums of statistic
@@ -421,7 +421,18 @@ extern "C" int pgld_hap_window_sums(pgld_handle h, const pgld_hap_panel* panel,
                                     const int64_t* win_begin, const int64_t* win_end,
                                     int32_t n_win, double* sums, int64_t* counts, int32_t form,
                                     void* stream) {
+  return pgld_hap_window_sums_columns(h, panel, snp_idx, n_idx, win_begin, win_end, n_win, sums,
+                                      counts, pgld::win::kAllColumns, form, stream);
+}
+
+extern "C" int pgld_hap_window_sums_columns(pgld_handle h, const pgld_hap_panel* panel,
+                                            const int32_t* snp_idx, int64_t n_idx,
+                                            const int64_t* win_begin, const int64_t* win_end,
+                                            int32_t n_win, double* sums, int64_t* counts,
+                                            int32_t columns, int32_t form, void* stream) {
   PGLD_REQUIRE(h, h != nullptr, "pgld_hap_window_sums: NULL handle");
+  PGLD_REQUIRE(h, columns > 0 && (columns & ~pgld::win::kAllColumns) == 0,
+               "pgld_hap_window_sums: columns %d", (int)columns);
   PGLD_REQUIRE(h, panel != nullptr && panel->n_pops == 1,
                "pgld_hap_window_sums: one population per call");
   PGLD_REQUIRE(h, panel->n_words[0] >= 1 && panel->n_snp >= 0, "pgld_hap_window_sums: panel");
@@ -444,7 +455,7 @@ extern "C" int pgld_hap_window_sums(pgld_handle h, const pgld_hap_panel* panel,
   if (form == PGLD_FORM_TC) {
     int rc = pgld_tc_windows(h, panel, snp_idx, n_idx, reinterpret_cast<const i64*>(win_begin),
                              reinterpret_cast<const i64*>(win_end), n_win, sums,
-                             reinterpret_cast<unsigned long long*>(counts), st);
+                             reinterpret_cast<unsigned long long*>(counts), columns, st);
     if (rc) return rc;
     // the workspace holds the tile offsets and the operand: finish before reuse
     PGLD_CHECK_CUDA(h, cudaStreamSynchronize(st));

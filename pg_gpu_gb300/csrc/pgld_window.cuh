@@ -60,47 +60,65 @@ __device__ __forceinline__ void window_pair(const fast::Pop& p, int n, float c1,
   }
 }
 
+// columns of the window sums that a call wants (bit k: column k)
+constexpr int kAllColumns = 63;
+
 // window_pair for two pairs (i, j0) and (i, j1) at once on packed float2
 // features (the tensor-core window kernels): the same statistics, with the
 // naive-r^2 numerator c1 v_i v_j - n d_i d_j by Kahan's two-product
 // algorithm; live.x / live.y select the pairs that belong to the window.
-// tab(n) gives (1/n, 1/(n(n-1)(n-2)(n-3))) of the reciprocal tables.
-template <class Tab>
+// tab(n) gives (1/n, 1/(n(n-1)(n-2)(n-3))) of the reciprocal tables.  Only the
+// columns of COLS are formed (n_r2 with column 0).
+template <int COLS, class Tab>
 __device__ __forceinline__ void window_pair2(const fast2::Pop& p, float2 c1, Tab&& tab,
                                              float4 si, float4 sj0, float4 sj1, bool live0,
                                              bool live1, float2 (&acc)[6], int& n_pairs,
                                              int& n_r2, int& n_four) {
   using namespace fast2;
-  const float2 t0 = tab(p.n0), t1 = tab(p.n1);
+  constexpr bool kMoments = (COLS & 28) != 0;
+  float2 t0 = make_float2(0.f, 0.f), t1 = t0;
+  if constexpr (kMoments || (COLS & 32) != 0) {
+    t0 = tab(p.n0);
+    t1 = tab(p.n1);
+  }
   n_pairs += (live0 ? 1 : 0) + (live1 ? 1 : 0);
-  const V rden = vmul(vmul(p.pA, p.qA), vmul(p.pB, p.qB));
-  const V xx = vmul(p.x, p.x);
-  const bool r0 = live0 && rden.x > 0.f, r1 = live1 && rden.y > 0.f;
-  n_r2 += (r0 ? 1 : 0) + (r1 ? 1 : 0);
-  acc[0] = vadd(acc[0], make_float2(r0 ? __fdividef(xx.x, rden.x) : 0.f,
-                                    r1 ? __fdividef(xx.y, rden.y) : 0.f));
+  if constexpr ((COLS & 1) != 0) {
+    const V rden = vmul(vmul(p.pA, p.qA), vmul(p.pB, p.qB));
+    const V xx = vmul(p.x, p.x);
+    const bool r0 = live0 && rden.x > 0.f, r1 = live1 && rden.y > 0.f;
+    n_r2 += (r0 ? 1 : 0) + (r1 ? 1 : 0);
+    acc[0] = vadd(acc[0], make_float2(r0 ? __fdividef(xx.x, rden.x) : 0.f,
+                                      r1 ? __fdividef(xx.y, rden.y) : 0.f));
+  }
   const bool f0 = live0 && p.n0 >= 4, f1 = live1 && p.n1 >= 4;
   n_four += (f0 ? 1 : 0) + (f1 ? 1 : 0);
-  if (f0 || f1) {
-    const V dd = dd_num(p), pi = pi2_num(p);
-    const V dz = dz_num(p, vfma(p.dA, p.dB, p.e));
-    const V r4 = make_float2(f0 ? t0.y : 0.f, f1 ? t1.y : 0.f);
-    acc[1] = vadd(acc[1], make_float2(f0 && pi.x != 0.f ? __fdividef(dd.x, pi.x) : 0.f,
-                                      f1 && pi.y != 0.f ? __fdividef(dd.y, pi.y) : 0.f));
-    acc[2] = vfma(dd, r4, acc[2]);
-    acc[3] = vfma(dz, r4, acc[3]);
-    acc[4] = vfma(pi, r4, acc[4]);
+  if constexpr ((COLS & 30) != 0) {
+    if (f0 || f1) {
+      const V dd = dd_num(p), pi = pi2_num(p);
+      if constexpr ((COLS & 2) != 0)
+        acc[1] = vadd(acc[1], make_float2(f0 && pi.x != 0.f ? __fdividef(dd.x, pi.x) : 0.f,
+                                          f1 && pi.y != 0.f ? __fdividef(dd.y, pi.y) : 0.f));
+      if constexpr (kMoments) {
+        const V dz = dz_num(p, vfma(p.dA, p.dB, p.e));
+        const V r4 = make_float2(f0 ? t0.y : 0.f, f1 ? t1.y : 0.f);
+        acc[2] = vfma(dd, r4, acc[2]);
+        acc[3] = vfma(dz, r4, acc[3]);
+        acc[4] = vfma(pi, r4, acc[4]);
+      }
+    }
   }
-  const bool s0 = live0 && si.w > 0.f && sj0.w > 0.f, s1 = live1 && si.w > 0.f && sj1.w > 0.f;
-  if (s0 || s1) {
-    // E = D v_i v_j from the integer c1 v_i v_j - n d_i d_j
-    const V ns = p.ns;
-    const V vv = make_float2(si.y * sj0.y, si.y * sj1.y), dd2 = make_float2(si.x * sj0.x, si.x * sj1.x);
-    const V num = dot2(c1, vv, vneg(ns), dd2);
-    const V Ev = vmul(num, make_float2(t0.x, t1.x));
-    const float E0 = p.n0 > 0 ? Ev.x : -dd2.x, E1 = p.n1 > 0 ? Ev.y : -dd2.y;
-    const V ww = make_float2(s0 ? si.w * sj0.w : 0.f, s1 ? si.w * sj1.w : 0.f);
-    acc[5] = vfma(vmul(make_float2(E0, E1), make_float2(E0, E1)), ww, acc[5]);
+  if constexpr ((COLS & 32) != 0) {
+    const bool s0 = live0 && si.w > 0.f && sj0.w > 0.f, s1 = live1 && si.w > 0.f && sj1.w > 0.f;
+    if (s0 || s1) {
+      // E = D v_i v_j from the integer c1 v_i v_j - n d_i d_j
+      const V ns = p.ns;
+      const V vv = make_float2(si.y * sj0.y, si.y * sj1.y), dd2 = make_float2(si.x * sj0.x, si.x * sj1.x);
+      const V num = dot2(c1, vv, vneg(ns), dd2);
+      const V Ev = vmul(num, make_float2(t0.x, t1.x));
+      const float E0 = p.n0 > 0 ? Ev.x : -dd2.x, E1 = p.n1 > 0 ? Ev.y : -dd2.y;
+      const V ww = make_float2(s0 ? si.w * sj0.w : 0.f, s1 ? si.w * sj1.w : 0.f);
+      acc[5] = vfma(vmul(make_float2(E0, E1), make_float2(E0, E1)), ww, acc[5]);
+    }
   }
 }
 
@@ -111,29 +129,37 @@ __device__ __forceinline__ void window_pair2(const fast2::Pop& p, float2 c1, Tab
 // (E = x), so one product serves both; DD, Dz, pi2 and sigma_D^2 as above.
 // n is the row SNP's nv for both pairs: four = (nv_i >= 4) and r4 =
 // 1/(n(n-1)(n-2)(n-3)) come from the caller, once per row.
+template <int COLS>
 __device__ __forceinline__ void window_pair2_same(const fast2::Pop& p, bool four, float r4n,
                                                   float4 si, float4 sj0, float4 sj1, bool live0,
                                                   bool live1, float2 (&acc)[6], int& n_pairs,
                                                   int& n_r2, int& n_four) {
   using namespace fast2;
   n_pairs += (live0 ? 1 : 0) + (live1 ? 1 : 0);
-  const V uu = vmul(vs(si.w), make_float2(sj0.w, sj1.w));
-  const bool r0 = live0 && uu.x > 0.f, r1 = live1 && uu.y > 0.f;
-  n_r2 += (r0 ? 1 : 0) + (r1 ? 1 : 0);
-  const V r2 = vmul(vmul(p.x, p.x), make_float2(live0 ? uu.x : 0.f, live1 ? uu.y : 0.f));
-  acc[0] = vadd(acc[0], r2);
-  acc[5] = vadd(acc[5], r2);
+  if constexpr ((COLS & 33) != 0) {
+    const V uu = vmul(vs(si.w), make_float2(sj0.w, sj1.w));
+    const bool r0 = live0 && uu.x > 0.f, r1 = live1 && uu.y > 0.f;
+    n_r2 += (r0 ? 1 : 0) + (r1 ? 1 : 0);
+    const V r2 = vmul(vmul(p.x, p.x), make_float2(live0 ? uu.x : 0.f, live1 ? uu.y : 0.f));
+    acc[0] = vadd(acc[0], r2);
+    acc[5] = vadd(acc[5], r2);
+  }
   const bool f0 = live0 && four, f1 = live1 && four;
   n_four += (f0 ? 1 : 0) + (f1 ? 1 : 0);
-  if (f0 || f1) {
-    const V dd = dd_num(p), pi = pi2_num(p);
-    const V dz = dz_num(p, vfma(p.dA, p.dB, p.e));
-    const V r4 = make_float2(f0 ? r4n : 0.f, f1 ? r4n : 0.f);
-    acc[1] = vadd(acc[1], make_float2(f0 && pi.x != 0.f ? __fdividef(dd.x, pi.x) : 0.f,
-                                      f1 && pi.y != 0.f ? __fdividef(dd.y, pi.y) : 0.f));
-    acc[2] = vfma(dd, r4, acc[2]);
-    acc[3] = vfma(dz, r4, acc[3]);
-    acc[4] = vfma(pi, r4, acc[4]);
+  if constexpr ((COLS & 30) != 0) {
+    if (f0 || f1) {
+      const V dd = dd_num(p), pi = pi2_num(p);
+      if constexpr ((COLS & 2) != 0)
+        acc[1] = vadd(acc[1], make_float2(f0 && pi.x != 0.f ? __fdividef(dd.x, pi.x) : 0.f,
+                                          f1 && pi.y != 0.f ? __fdividef(dd.y, pi.y) : 0.f));
+      if constexpr ((COLS & 28) != 0) {
+        const V dz = dz_num(p, vfma(p.dA, p.dB, p.e));
+        const V r4 = make_float2(f0 ? r4n : 0.f, f1 ? r4n : 0.f);
+        acc[2] = vfma(dd, r4, acc[2]);
+        acc[3] = vfma(dz, r4, acc[3]);
+        acc[4] = vfma(pi, r4, acc[4]);
+      }
+    }
   }
 }
 

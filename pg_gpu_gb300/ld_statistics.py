@@ -200,7 +200,8 @@ def _zns_windows(matrix, win_start, win_stop, estimator):
     if ws.shape != we.shape:
         raise ValueError("win_start and win_stop must have the same shape")
     seg, b, e = _segregating(matrix.haplotypes, ws, we)
-    sums, cnt = _ops.window_sums(matrix.packed(None), seg, b, e)
+    sums, cnt = _ops.window_sums(matrix.packed(None), seg, b, e, columns=(
+        "sigma_d2" if estimator == "sigma_d2" else "r2_naive",))
     s, c = sums.cpu().numpy(), cnt.cpu().numpy()
     out = np.zeros(len(ws))
     for w in range(len(ws)):
