@@ -260,6 +260,12 @@ int pgld_pairs_within(pgld_handle h, const double* pos, int64_t n_snp, double ma
                       int64_t i_begin, int64_t i_end, int32_t* idx_i, int32_t* idx_j,
                       int64_t n_pairs, void* stream);
 
+/* The same pairs from offsets that pgld_count_pairs_within filled (device
+ * int64): the pairs of the anchors [i_begin, i_end), offsets[i_end] -
+ * offsets[i_begin] of them.  Asynchronous. */
+int pgld_pairs_from_offsets(pgld_handle h, const int64_t* offsets, int64_t i_begin, int64_t i_end,
+                            int32_t* idx_i, int32_t* idx_j, void* stream);
+
 /* Per-pair outputs over the distance band of one population, in the
  * reference's pair order: counts [n_pairs][4] int32, n_valid [n_pairs]
  * (nullable), and stats [n_pairs][4] float32 = r^2, DD, Dz, pi2 (nullable).
@@ -399,6 +405,13 @@ int pgld_geno_stat_terms(int32_t n_pops, pgld_term* out, int32_t capacity, int32
 int pgld_geno_stats(pgld_handle h, const pgld_pair_counts* counts, int64_t n_pairs,
                     const pgld_term* terms, int32_t n_terms, int32_t n_stats, void* out,
                     int32_t out_dtype, int64_t out_ld, void* stream);
+
+/* Rogers-Huff r of every SNP pair i < j (condensed upper triangle, float64) of
+ * one population of n_rows individuals with dosages 0 / 1 / 2 and none missing;
+ * NaN where a SNP has no variance.  Replaces rogers_huff_r's tiles
+ * (ld_statistics.py:410-521). */
+int pgld_geno_rogers_huff(pgld_handle h, const uint32_t* planes, int32_t n_words, int32_t n_rows,
+                          int64_t n_snp, double* out, void* stream);
 
 /* Per-pair outputs over the distance band of one population, in the
  * reference's pair order: counts [n_pairs][9] int32 (nullable), n_valid

@@ -107,6 +107,10 @@ def rogers_huff_r(matrix):
     """Condensed upper-triangle Rogers-Huff r (ld_statistics.py:492-521)."""
     import torch
     g = dosage(matrix)
+    pk = _ops.pack_geno(g)
+    if not pk.has_other:
+        return _ops.rogers_huff_all(pk)
+    # dosages above 2 fold into the counts' classes
     m = g.shape[1]
     ii, jj = torch.triu_indices(m, m, offset=1, device=g.device)
     return rh_pairs(g, ii.to(torch.int32), jj.to(torch.int32))

@@ -93,6 +93,8 @@ _SIGS = {
                         _P, _I32, _I64, _P], ctypes.c_int),
     "pgld_count_pairs_within": ([_P, _P, _I64, _D, ctypes.POINTER(_I64), _P, _P], ctypes.c_int),
     "pgld_pairs_within": ([_P, _P, _I64, _D, _I64, _I64, _P, _P, _I64, _P], ctypes.c_int),
+    "pgld_pairs_from_offsets": ([_P, _P, _I64, _I64, _P, _P, _P], ctypes.c_int),
+    "pgld_geno_rogers_huff": ([_P, _P, _I32, _I32, _I64, _P, _P], ctypes.c_int),
     "pgld_hap_band_pairs": ([_P, ctypes.POINTER(HapPanel), _P, _D, _P, _P, _P, _I64, _I32, _P],
                             ctypes.c_int),
     "pgld_hap_binned_sums": ([_P, ctypes.POINTER(HapPanel), _P, _D, _P, _P, _I32, _P, _P, _I32,

@@ -323,13 +323,13 @@ def band_pair_count(pos_d, max_dist):
     return n
 
 
-def pairs_range(pos_d, max_dist, i_begin, i_end, n_pairs):
+def pairs_of_anchors(off, i_begin, i_end, n_pairs):
+    """(idx_i, idx_j) int32 of the anchors' pairs from band_offsets' offsets."""
     torch = _torch()
-    ii = torch.empty(n_pairs, dtype=torch.int32, device=pos_d.device)
-    jj = torch.empty(n_pairs, dtype=torch.int32, device=pos_d.device)
+    ii, jj = (torch.empty(n_pairs, dtype=torch.int32, device=off.device) for _ in range(2))
     h = L.handle()
-    L.check(L.lib().pgld_pairs_within(h, L.ptr(pos_d), pos_d.numel(), float(max_dist), i_begin,
-                                      i_end, L.ptr(ii), L.ptr(jj), n_pairs, L.stream_ptr()), h)
+    L.check(L.lib().pgld_pairs_from_offsets(h, L.ptr(off), i_begin, i_end, L.ptr(ii), L.ptr(jj),
+                                            L.stream_ptr()), h)
     return ii, jj
 
 
@@ -653,6 +653,19 @@ def geno_counts_pairs(pk, idx_i, idx_j):
         if int(st[0]):
             raise IndexError("pair index out of range of the variant axis")
     return counts, nv
+
+
+def rogers_huff_all(pk):
+    """Condensed upper-triangle Rogers-Huff r (float64) of a PackedGeno without
+    missing dosages or values above 2."""
+    torch = _torch()
+    m = pk.n_snp
+    out = torch.empty(m * (m - 1) // 2, dtype=torch.float64, device=pk.planes.device)
+    if out.numel():
+        h = L.handle()
+        L.check(L.lib().pgld_geno_rogers_huff(h, L.ptr(pk.planes), pk.n_words, pk.n_rows, m,
+                                              L.ptr(out), L.stream_ptr()), h)
+    return out
 
 
 def geno_spec_terms(P):

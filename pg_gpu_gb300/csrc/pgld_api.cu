@@ -427,6 +427,9 @@ extern "C" int pgld_device_status(pgld_handle h, int32_t* code_out, void* stream
   return PGLD_OK;
 }
 
+int pgld_tally_tiles(pgld_context* h, const uint32_t* planes, const uint32_t* valid, int W, i64 n,
+                     int32_t* counts, int32_t* n_valid, cudaStream_t st);
+
 // ---------------------------------------------------------------------------
 // counts of listed pairs: a group of G lanes per pair, words strided by G
 // ---------------------------------------------------------------------------
@@ -434,7 +437,7 @@ template <int G>
 __global__ void __launch_bounds__(256) counts_pairs_kernel(
     const uint32_t* __restrict__ planes, const uint32_t* __restrict__ valid, int W, i64 n_snp,
     const int32_t* __restrict__ idx_i, const int32_t* __restrict__ idx_j, i64 n_pairs,
-    i64 tri_m, int32_t* __restrict__ counts, i64 counts_ld, int32_t* __restrict__ n_valid,
+    int32_t* __restrict__ counts, i64 counts_ld, int32_t* __restrict__ n_valid,
     int32_t* __restrict__ status) {
   i64 g = ((i64)blockIdx.x * 256 + threadIdx.x) / G;
   int lane = threadIdx.x % G;
@@ -443,20 +446,8 @@ __global__ void __launch_bounds__(256) counts_pairs_kernel(
     bool live = k < n_pairs;
     i64 i = 0, j = 0;
     if (live) {
-      if (tri_m > 0) {
-        // row-major upper triangle of an m x m matrix: row i starts at i*m - i(i+1)/2
-        i64 lo = 0, hi = tri_m - 1;
-        while (hi - lo > 1) {
-          i64 mid = (lo + hi) >> 1;
-          i64 st = mid * tri_m - mid * (mid + 1) / 2;
-          if (st <= k) lo = mid; else hi = mid;
-        }
-        i = lo;
-        j = k - (i * tri_m - i * (i + 1) / 2) + i + 1;
-      } else {
-        i = idx_i[k];
-        j = idx_j[k];
-      }
+      i = idx_i[k];
+      j = idx_j[k];
       if (i < 0 || j < 0 || i >= n_snp || j >= n_snp) {
         if (lane == 0) atomicCAS(status, 0, 1001);
         live = false;
@@ -494,7 +485,7 @@ __global__ void __launch_bounds__(256) counts_pairs_kernel(
 
 static int launch_counts_pairs(pgld_context* h, const uint32_t* planes, const uint32_t* valid,
                                int W, i64 n_snp, const int32_t* ii, const int32_t* jj, i64 n,
-                               i64 tri_m, int32_t* counts, i64 ld, int32_t* nv, cudaStream_t st) {
+                               int32_t* counts, i64 ld, int32_t* nv, cudaStream_t st) {
   int G = 1;
   while (G < W && G < 32) G <<= 1;
   i64 groups_needed = n;
@@ -502,7 +493,7 @@ static int launch_counts_pairs(pgld_context* h, const uint32_t* planes, const ui
   blocks = std::min<i64>(std::max<i64>(blocks, 1), (i64)h->n_sm * 16);
 #define PGLD_LAUNCH_CP(GG)                                                                     \
   counts_pairs_kernel<GG><<<(unsigned)blocks, 256, 0, st>>>(planes, valid, W, n_snp, ii, jj, n, \
-                                                             tri_m, counts, ld, nv, h->dev_status)
+                                                             counts, ld, nv, h->dev_status)
   switch (G) {
     case 1: PGLD_LAUNCH_CP(1); break;
     case 2: PGLD_LAUNCH_CP(2); break;
@@ -527,7 +518,7 @@ extern "C" int pgld_hap_counts_pairs(pgld_handle h, const uint32_t* planes, cons
   PGLD_REQUIRE(h, planes && idx_i && idx_j && counts, "pgld_hap_counts_pairs: NULL buffer");
   PGLD_REQUIRE(h, counts_ld >= 4, "pgld_hap_counts_pairs: counts_ld < 4");
   PGLD_CHECK_CUDA(h, cudaSetDevice(h->device));
-  return launch_counts_pairs(h, planes, valid, n_words, n_snp, idx_i, idx_j, n_pairs, 0, counts,
+  return launch_counts_pairs(h, planes, valid, n_words, n_snp, idx_i, idx_j, n_pairs, counts,
                              counts_ld, n_valid, (cudaStream_t)stream);
 }
 
@@ -540,8 +531,7 @@ extern "C" int pgld_hap_tally(pgld_handle h, const uint32_t* planes, const uint3
   if (n_pairs <= 0) return PGLD_OK;
   PGLD_REQUIRE(h, planes && counts, "pgld_hap_tally: NULL buffer");
   PGLD_CHECK_CUDA(h, cudaSetDevice(h->device));
-  return launch_counts_pairs(h, planes, valid, n_words, n_snp, nullptr, nullptr, n_pairs, n_snp,
-                             counts, 4, n_valid, (cudaStream_t)stream);
+  return pgld_tally_tiles(h, planes, valid, n_words, n_snp, counts, n_valid, (cudaStream_t)stream);
 }
 
 // ---------------------------------------------------------------------------
@@ -555,24 +545,42 @@ struct StatsArgs {
   int n_pops;
 };
 
-template <typename T>
+// the term table as a kernel argument (no upload, nothing to wait for), or, for
+// very long lists, in device memory
+template <int N>
+struct TermTable {
+  pgld_term t[N];
+};
+struct TermPointer {
+  const pgld_term* t;
+};
+
+__device__ __forceinline__ pgld::PopC load_pop(const StatsArgs& a, int p, i64 k, bool wide) {
+  const int32_t* c = a.counts[p] + k * a.counts_ld[p];
+  int4 v;
+  if (wide) {
+    v = __ldg(reinterpret_cast<const int4*>(c));
+  } else {
+    v.x = c[0]; v.y = c[1]; v.z = c[2]; v.w = c[3];
+  }
+  const i64 n = a.nvalid[p] ? (i64)a.nvalid[p][k * a.nvalid_ld[p]] : (i64)v.x + v.y + v.z + v.w;
+  return pgld::make_pop(v.x, v.y, v.z, v.w, n);
+}
+
+// any term list: per pair, the table in order
+template <typename T, class Tab>
 __global__ void __launch_bounds__(256) stats_kernel(StatsArgs a, i64 n_pairs,
-                                                    const pgld_term* __restrict__ terms,
-                                                    int n_terms, T* __restrict__ out, i64 out_ld) {
+                                                    const __grid_constant__ Tab tab, int n_terms,
+                                                    T* __restrict__ out, i64 out_ld) {
   for (i64 k = (i64)blockIdx.x * 256 + threadIdx.x; k < n_pairs; k += (i64)gridDim.x * 256) {
     pgld::PopC P[PGLD_MAX_POPS];
-    for (int p = 0; p < a.n_pops; ++p) {
-      const int32_t* c = a.counts[p] + k * a.counts_ld[p];
-      i64 c1 = c[0], c2 = c[1], c3 = c[2], c4 = c[3];
-      i64 n = a.nvalid[p] ? (i64)a.nvalid[p][k * a.nvalid_ld[p]] : c1 + c2 + c3 + c4;
-      P[p] = pgld::make_pop(c1, c2, c3, c4, n);
-    }
+    for (int p = 0; p < a.n_pops; ++p) P[p] = load_pop(a, p, k, false);
     T* o = out + k * out_ld;
     int cur = -1;
     T acc = 0;
     int nt_in_stat = 0;
     for (int t = 0; t < n_terms; ++t) {
-      pgld_term tm = terms[t];
+      const pgld_term tm = tab.t[t];
       if (tm.stat != cur) {
         if (cur >= 0) o[cur] = acc;
         cur = tm.stat;
@@ -585,7 +593,7 @@ __global__ void __launch_bounds__(256) stats_kernel(StatsArgs a, i64 n_pairs,
       else
         v = (T)pgld::term_value_f32(tm.kind, tm.pops, P);
       // single weight-1 term: the value itself (NaN passes through); else sum of weighted terms
-      bool last_of_stat = (t + 1 == n_terms) || (terms[t + 1].stat != cur);
+      bool last_of_stat = (t + 1 == n_terms) || (tab.t[t + 1].stat != cur);
       if (nt_in_stat == 0 && last_of_stat && tm.weight == 1.0)
         acc = v;
       else
@@ -594,6 +602,136 @@ __global__ void __launch_bounds__(256) stats_kernel(StatsArgs a, i64 n_pairs,
     }
     if (cur >= 0) o[cur] = acc;
   }
+}
+
+// one weight-1 term of one or two populations, float64 (dd, dz, pi2, r, r^2, D'
+// of ld_statistics): a.counts[0], [1] are the term's roles.  The exact integer
+// numerator and denominator in registers, one quotient on the integer pipes.
+// 2.0 million pairs of one population: 81 us with the term interpreted from
+// memory and a float64 division, 17 us here.
+template <int ROLES>
+__global__ void __launch_bounds__(256) one_term_kernel(StatsArgs a, i64 n_pairs, int kind, bool wide,
+                                                       double* __restrict__ out, i64 out_ld) {
+  for (i64 k = (i64)blockIdx.x * 256 + threadIdx.x; k < n_pairs; k += (i64)gridDim.x * 256) {
+    pgld::PopC P[ROLES];
+#pragma unroll
+    for (int p = 0; p < ROLES; ++p) P[p] = load_pop(a, p, k, wide);
+    double v;
+    if constexpr (ROLES == 1) {
+      const pgld::PopC& p = P[0];
+      pgld::ND q = {0, 0};
+      bool nan = false;
+      switch (kind) {
+        case PGLD_DD_II: q = pgld::dd_ii(p); break;
+        case PGLD_DZ_III: q = pgld::dz_iii(p); break;
+        case PGLD_PI2_IIII: q = pgld::pi2_iiii(p); break;
+        case PGLD_DPRIME: q = {p.x, pgld::dprime_den(p)}; nan = true; break;
+        default: q = {p.x * p.x, pgld::r_den(p)}; nan = true; break;  // R2, R
+      }
+      if (kind == PGLD_R)
+        v = q.den > 0 ? (double)p.x / sqrt((double)q.den) : 0.0;
+      else
+        v = q.den > 0 ? pgld::quotient(q.num, q.den) : 0.0;
+      if (nan && q.den <= 0) v = __longlong_as_double(0x7ff8000000000000LL);
+    } else {
+      pgld::ND q = {0, 0};
+      switch (kind) {
+        case PGLD_DD_IJ: q = pgld::dd_ij(P[0], P[1]); break;
+        case PGLD_DZ_IIJ: q = pgld::dz_iij(P[0], P[1]); break;
+        case PGLD_DZ_IJI: q = pgld::dz_iji(P[0], P[1]); break;
+        case PGLD_DZ_IJJ: q = pgld::dz_ijj(P[0], P[1]); break;
+        case PGLD_PI2_TRIPLE: q = pgld::pi2_triple(P[0], P[1]); break;
+        case PGLD_PI2_IIKK: q = pgld::pi2_iikk(P[0], P[1]); break;
+        case PGLD_PI2_IIKK_SYM: q = pgld::pi2_iikk_sym(P[0], P[1]); break;
+        default: q = pgld::pi2_ijij(P[0], P[1]); break;
+      }
+      v = q.den > 0 ? pgld::quotient(q.num, q.den) : 0.0;
+    }
+    out[k * out_ld] = v;
+  }
+}
+// roles of a kind that one_term_kernel takes, else 0
+static int one_term_roles(int kind) {
+  switch (kind) {
+    case PGLD_DD_II: case PGLD_DZ_III: case PGLD_PI2_IIII:
+    case PGLD_R: case PGLD_R2: case PGLD_DPRIME:
+      return 1;
+    case PGLD_DD_IJ: case PGLD_DZ_IIJ: case PGLD_DZ_IJI: case PGLD_DZ_IJJ:
+    case PGLD_PI2_TRIPLE: case PGLD_PI2_IIKK: case PGLD_PI2_IIKK_SYM: case PGLD_PI2_IJIJ:
+      return 2;
+    default:
+      return 0;
+  }
+}
+
+// the moments tables of one and two populations (3 and 15 columns): each
+// column one exact integer ratio -- the calls that the table averages have one
+// denominator, and most of them one value -- divided once on the integer pipes.
+// A warp's rows leave through shared memory, so that the stores are whole
+// lines.  200,000 pairs of two populations: 176 us with the 27 terms of the
+// table interpreted, each with a float64 division, 24 us here.
+template <int P>
+__global__ void __launch_bounds__(256) table_kernel(StatsArgs a, i64 n_pairs, bool wide,
+                                                    double* __restrict__ out, i64 out_ld) {
+  constexpr int S = P == 1 ? 3 : 15;
+  __shared__ double rows[8][32 * S];
+  const int lane = threadIdx.x & 31;
+  double* mine = rows[threadIdx.x >> 5];
+  const i64 warps = (i64)gridDim.x * 8;
+  for (i64 k0 = ((i64)blockIdx.x * 8 + (threadIdx.x >> 5)) * 32; k0 < n_pairs; k0 += warps * 32) {
+    const i64 k = min(k0 + lane, n_pairs - 1);
+    double* o = mine + lane * S;
+    auto put = [&](int s, i64 num, i64 den) { o[s] = den > 0 ? pgld::quotient(num, den) : 0.0; };
+    auto put_nd = [&](int s, const pgld::ND& v) { put(s, v.num, v.den); };
+    const pgld::PopC p = load_pop(a, 0, k, wide);
+    if constexpr (P == 1) {
+      put_nd(0, pgld::dd_ii(p));
+      put_nd(1, pgld::dz_iii(p));
+      put_nd(2, pgld::pi2_iiii(p));
+    } else {
+      const pgld::PopC q = load_pop(a, 1, k, wide);
+      auto dz_mixed = [](const pgld::PopC& t, const pgld::PopC& u) {
+        const pgld::ND x = pgld::dz_iij(t, u), y = pgld::dz_iji(t, u);
+        return pgld::ND{x.num + y.num, 2 * x.den};
+      };
+      put_nd(0, pgld::dd_ii(p));
+      put_nd(1, pgld::dd_ij(p, q));
+      put_nd(2, pgld::dd_ii(q));
+      put_nd(3, pgld::dz_iii(p));
+      put_nd(4, dz_mixed(p, q));
+      put_nd(5, pgld::dz_ijj(p, q));
+      put_nd(6, pgld::dz_ijj(q, p));
+      put_nd(7, dz_mixed(q, p));
+      put_nd(8, pgld::dz_iii(q));
+      put_nd(9, pgld::pi2_iiii(p));
+      put_nd(10, pgld::pi2_triple(p, q));
+      put_nd(11, pgld::pi2_iikk_sym(p, q));
+      put_nd(12, pgld::pi2_ijij(p, q));
+      put_nd(13, pgld::pi2_triple(q, p));
+      put_nd(14, pgld::pi2_iiii(q));
+    }
+    __syncwarp();
+    const int live = (int)min((i64)32, n_pairs - k0);
+    if (out_ld == S) {
+      double* dst = out + k0 * S;
+      for (int x = lane; x < live * S; x += 32) dst[x] = mine[x];
+    } else {
+      for (int x = lane; x < live * S; x += 32) out[(k0 + x / S) * out_ld + x % S] = mine[x];
+    }
+    __syncwarp();
+  }
+}
+
+// whether terms are the moments table of n_pops populations
+static bool is_table(const pgld_term* terms, int n_terms, int n_stats, int n_pops) {
+  std::vector<pgld_term> t;
+  pgld_build_spec_terms(n_pops, t);
+  if ((int)t.size() != n_terms || n_stats != pgld_n_stats(n_pops)) return false;
+  for (int k = 0; k < n_terms; ++k)
+    if (t[k].stat != terms[k].stat || t[k].kind != terms[k].kind || t[k].weight != terms[k].weight ||
+        !std::equal(t[k].pops, t[k].pops + 4, terms[k].pops))
+      return false;
+  return true;
 }
 
 extern "C" int pgld_hap_stats(pgld_handle h, const pgld_pair_counts* counts, int64_t n_pairs,
@@ -632,21 +770,64 @@ extern "C" int pgld_hap_stats(pgld_handle h, const pgld_pair_counts* counts, int
   }
   PGLD_CHECK_CUDA(h, cudaSetDevice(h->device));
   cudaStream_t st = (cudaStream_t)stream;
-  void* ws = nullptr;
-  int rc = pgld_workspace(h, n_terms * sizeof(pgld_term), &ws);
-  if (rc) return rc;
-  PGLD_CHECK_CUDA(h, cudaMemcpyAsync(ws, terms, n_terms * sizeof(pgld_term),
-                                     cudaMemcpyHostToDevice, st));
-  i64 blocks = std::min<i64>((n_pairs + 255) / 256, (i64)h->n_sm * 8);
-  if (out_dtype == PGLD_F64)
-    stats_kernel<double><<<(unsigned)blocks, 256, 0, st>>>(a, n_pairs, (const pgld_term*)ws,
-                                                           n_terms, (double*)out, out_ld);
-  else
-    stats_kernel<float><<<(unsigned)blocks, 256, 0, st>>>(a, n_pairs, (const pgld_term*)ws,
-                                                          n_terms, (float*)out, out_ld);
+  const unsigned blocks = (unsigned)std::min<i64>((n_pairs + 255) / 256, (i64)h->n_sm * 8);
+  // 16-byte loads of the counts where every row allows them
+  auto is_wide = [&](int pops) {
+    bool w = true;
+    for (int p = 0; p < pops; ++p)
+      w = w && ((uintptr_t)a.counts[p] % 16 == 0) && a.counts_ld[p] % 4 == 0;
+    return w;
+  };
+  const int roles = n_terms == 1 && terms[0].weight == 1.0 ? one_term_roles(terms[0].kind) : 0;
+  if (out_dtype == PGLD_F64 && roles) {
+    StatsArgs r = a;
+    for (int p = 0; p < roles; ++p) {
+      const int q = terms[0].pops[p];
+      r.counts[p] = a.counts[q];
+      r.counts_ld[p] = a.counts_ld[q];
+      r.nvalid[p] = a.nvalid[q];
+      r.nvalid_ld[p] = a.nvalid_ld[q];
+    }
+    a = r;
+    double* o = (double*)out + terms[0].stat;
+    if (roles == 1)
+      one_term_kernel<1><<<blocks, 256, 0, st>>>(a, n_pairs, terms[0].kind, is_wide(1), o, out_ld);
+    else
+      one_term_kernel<2><<<blocks, 256, 0, st>>>(a, n_pairs, terms[0].kind, is_wide(2), o, out_ld);
+  } else if (out_dtype == PGLD_F64 && a.n_pops <= 2 && is_table(terms, n_terms, n_stats, a.n_pops)) {
+    if (a.n_pops == 1)
+      table_kernel<1><<<blocks, 256, 0, st>>>(a, n_pairs, is_wide(1), (double*)out, out_ld);
+    else
+      table_kernel<2><<<blocks, 256, 0, st>>>(a, n_pairs, is_wide(2), (double*)out, out_ld);
+  } else {
+    auto run = [&](const auto& tab) {
+      if (out_dtype == PGLD_F64)
+        stats_kernel<double><<<blocks, 256, 0, st>>>(a, n_pairs, tab, n_terms, (double*)out, out_ld);
+      else
+        stats_kernel<float><<<blocks, 256, 0, st>>>(a, n_pairs, tab, n_terms, (float*)out, out_ld);
+    };
+    constexpr int kMost = 512;  // 16 KB of kernel arguments
+    if (n_terms <= 64) {
+      TermTable<64> tab{};
+      std::copy(terms, terms + n_terms, tab.t);
+      run(tab);
+    } else if (n_terms <= kMost) {
+      TermTable<kMost> tab{};
+      std::copy(terms, terms + n_terms, tab.t);
+      run(tab);
+    } else {
+      void* ws = nullptr;
+      int rc = pgld_workspace(h, n_terms * sizeof(pgld_term), &ws);
+      if (rc) return rc;
+      PGLD_CHECK_CUDA(h, cudaMemcpyAsync(ws, terms, n_terms * sizeof(pgld_term),
+                                         cudaMemcpyHostToDevice, st));
+      run(TermPointer{(const pgld_term*)ws});
+      PGLD_CHECK_CUDA(h, cudaGetLastError());
+      // the term table lives in the workspace: keep it alive until the kernel ran
+      PGLD_CHECK_CUDA(h, cudaStreamSynchronize(st));
+    }
+  }
   PGLD_CHECK_CUDA(h, cudaGetLastError());
-  // the term table lives in the workspace: keep it alive until the kernel ran
-  PGLD_CHECK_CUDA(h, cudaStreamSynchronize(st));
   return PGLD_OK;
 }
 
@@ -760,6 +941,22 @@ extern "C" int pgld_pairs_within(pgld_handle h, const double* pos, int64_t n_snp
   PGLD_CHECK_CUDA(h, cudaGetLastError());
   // the offsets live in the workspace: finish before the next call reuses it
   PGLD_CHECK_CUDA(h, cudaStreamSynchronize(st));
+  return PGLD_OK;
+}
+
+extern "C" int pgld_pairs_from_offsets(pgld_handle h, const int64_t* offsets, int64_t i_begin,
+                                       int64_t i_end, int32_t* idx_i, int32_t* idx_j, void* stream) {
+  PGLD_REQUIRE(h, h != nullptr, "pgld_pairs_from_offsets: NULL handle");
+  PGLD_REQUIRE(h, 0 <= i_begin && i_begin <= i_end && i_end < (int64_t(1) << 31),
+               "pgld_pairs_from_offsets: anchors [%lld, %lld)", (long long)i_begin, (long long)i_end);
+  if (i_begin == i_end) return PGLD_OK;
+  PGLD_REQUIRE(h, offsets && idx_i && idx_j, "pgld_pairs_from_offsets: NULL buffer");
+  PGLD_CHECK_CUDA(h, cudaSetDevice(h->device));
+  const unsigned blocks =
+      (unsigned)std::max<i64>(1, std::min<i64>(((i_end - i_begin) * 32 + 255) / 256, (i64)h->n_sm * 16));
+  pairs_rows_kernel<<<blocks, 256, 0, (cudaStream_t)stream>>>(reinterpret_cast<const i64*>(offsets),
+                                                              i_begin, i_end, idx_i, idx_j);
+  PGLD_CHECK_CUDA(h, cudaGetLastError());
   return PGLD_OK;
 }
 

@@ -199,10 +199,9 @@ __device__ __forceinline__ int bin_index(const int* thr, int n_bins, int d) {
 // condensed upper triangle), NaN skipped, binned by pos[j] - pos[i].
 // counts mode (out == NULL): bin_counts[b] += pairs; fill mode: the values
 // are written grouped by bin at cursor[b] (advanced atomically per tile).
-// The float64 pipe (two operations per SM and clock) bounds it: integer
-// positions are compared as integers, and counting asks only whether the
-// denominator is positive.  300 haplotypes x 5,001 SNPs: 0.50 ms for each of the
-// two passes when both divided and searched the bins in float64.
+// The float64 pipe (two operations per SM and clock) would bound it: integer
+// positions are compared as integers, counting asks only whether the
+// XX
 __global__ void __launch_bounds__(kThreads) pairs_by_bin_kernel(
     const uint32_t* __restrict__ planes, int W, const double* __restrict__ values, i64 n,
     const double* __restrict__ pos, const int* __restrict__ ipos, const int* __restrict__ ipos_bad,
@@ -255,7 +254,7 @@ __global__ void __launch_bounds__(kThreads) pairs_by_bin_kernel(
           const long long x = a * d - b * c;
           const long long den = pa * (nn - pa) * pb * (nn - pb);
           defined = den > 0;
-          if (out && defined) v = __ddiv_rn((double)(x * x), (double)den);
+          if (out && defined) v = quotient(x * x, den);
         }
         val[q] = v;
         if (defined)
@@ -401,6 +400,161 @@ __global__ void kth_rep_kernel(KthArgs a, const int* __restrict__ tseg) {
   a.rep[t] = r;
 }
 
+// ---------------------------------------------------------------------------
+// all pairs of one population in upper-triangle order, 32 x 32 SNP tiles
+// ---------------------------------------------------------------------------
+// a chunk of 32 words of one plane of 32 SNPs, as [word][SNP]; rows of 36 words
+// so that a warp's four SNPs load as one 16-byte word
+constexpr int kRow = 36;
+__device__ __forceinline__ void stage_words(uint32_t (*dst)[kRow], const uint32_t* __restrict__ src,
+                                            i64 stride, i64 s0, i64 n, int w0, int W) {
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const int sl = wid * 4 + q;
+    const i64 s = s0 + sl;
+    dst[lane][sl] = s < n && w0 + lane < W ? __ldg(src + s * stride + w0 + lane) : 0u;
+  }
+}
+// first pair of row i of the condensed upper triangle
+__device__ __forceinline__ i64 tri_row(i64 i, i64 n) { return i * (2 * n - i - 1) / 2; }
+
+// joint counts of every pair (HaplotypeMatrix.tally_gpu_haplotypes): a warp's
+// stores are 32 consecutive pairs of a row.  2,000 SNPs x 200 haplotypes (2.0
+// million pairs, 32 MB): 279 us with a lane group per pair that searched the
+// triangle for its SNPs, 26 us here.
+template <bool VALID>
+__global__ void __launch_bounds__(kThreads) tally_kernel(const uint32_t* __restrict__ planes,
+                                                         const uint32_t* __restrict__ valid, int W,
+                                                         i64 n, int32_t* __restrict__ counts,
+                                                         bool aligned, int32_t* __restrict__ n_valid) {
+  __shared__ __align__(16) uint32_t ci[kKW][kRow], zi[kKW][kRow], cj[kKW][kRow], zj[kKW][kRow];
+  __shared__ __align__(16) uint32_t vi[VALID ? kKW : 1][kRow], vj[VALID ? kKW : 1][kRow];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const i64 nb = (n + kT - 1) / kT, n_tiles = nb * (nb + 1) / 2;
+  for (i64 t = blockIdx.x; t < n_tiles; t += gridDim.x) {
+    i64 bi, bj;
+    tri_decode(t, nb, bi, bj);
+    const i64 i0 = bi * kT, j0 = bj * kT;
+    int c[4][4] = {}, nv[4] = {};
+    for (int w0 = 0; w0 < W; w0 += kKW) {
+      __syncthreads();
+      stage_words(ci, planes, 2 * W, i0, n, w0, W);
+      stage_words(zi, planes + W, 2 * W, i0, n, w0, W);
+      stage_words(cj, planes, 2 * W, j0, n, w0, W);
+      stage_words(zj, planes + W, 2 * W, j0, n, w0, W);
+      if constexpr (VALID) {
+        stage_words(vi, valid, W, i0, n, w0, W);
+        stage_words(vj, valid, W, j0, n, w0, W);
+      }
+      __syncthreads();
+      const int nw = min(kKW, W - w0);
+#pragma unroll 4
+      for (int w = 0; w < nw; ++w) {
+        const uint32_t b1 = cj[w][lane], b0 = zj[w][lane];
+        const uint4 a1 = *reinterpret_cast<const uint4*>(&ci[w][wid * 4]);
+        const uint4 a0 = *reinterpret_cast<const uint4*>(&zi[w][wid * 4]);
+        const uint32_t x1[4] = {a1.x, a1.y, a1.z, a1.w}, x0[4] = {a0.x, a0.y, a0.z, a0.w};
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          c[q][0] += __popc(x1[q] & b1);
+          c[q][1] += __popc(x1[q] & b0);
+          c[q][2] += __popc(x0[q] & b1);
+          c[q][3] += __popc(x0[q] & b0);
+        }
+        if constexpr (VALID) {
+#pragma unroll
+          for (int q = 0; q < 4; ++q) nv[q] += __popc(vi[w][wid * 4 + q] & vj[w][lane]);
+        }
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const i64 i = i0 + wid * 4 + q, j = j0 + lane;
+      if (i < j && j < n) {
+        const i64 k = tri_row(i, n) + (j - i - 1);
+        if (aligned) {
+          reinterpret_cast<int4*>(counts)[k] = make_int4(c[q][0], c[q][1], c[q][2], c[q][3]);
+        } else {
+#pragma unroll
+          for (int x = 0; x < 4; ++x) counts[4 * k + x] = c[q][x];
+        }
+        if (n_valid) n_valid[k] = VALID ? nv[q] : c[q][0] + c[q][1] + c[q][2] + c[q][3];
+      }
+    }
+  }
+}
+
+// per-SNP dosage sum and n sum g^2 - (sum g)^2
+__global__ void dosage_site_kernel(const uint32_t* __restrict__ planes, int W, i64 m, int n,
+                                   int2* __restrict__ site) {
+  for (i64 s = (i64)blockIdx.x * blockDim.x + threadIdx.x; s < m; s += (i64)gridDim.x * blockDim.x) {
+    int one = 0, two = 0;
+    for (int w = 0; w < W; ++w) {
+      one += __popc(planes[s * 3 * W + W + w]);
+      two += __popc(planes[s * 3 * W + 2 * W + w]);
+    }
+    const int g = one + 2 * two;
+    site[s] = make_int2(g, n * (one + 4 * two) - g * g);
+  }
+}
+
+// Rogers-Huff r of every SNP pair of n individuals without missing dosages
+// (ld_statistics.py:410-443): cov = n sum g_i g_j - sum g_i sum g_j over
+// sqrt(var_i var_j), the exact integers of the general form (pgld_geno.cuh),
+// of which only sum g_i g_j depends on the pair: three popcounts a word, since
+// the individuals with dosages (1, 2) and (2, 1) are disjoint.  The float64
+// square root and division bound it (about 20 operations a pair on a pipe of
+// two a clock).  1,000 individuals x 3,000 SNPs: 2.30 ms with 36-byte counts
+// per pair, an index list and a kernel for the quotients, 0.21 ms here.
+__global__ void __launch_bounds__(kThreads) rogers_huff_kernel(const uint32_t* __restrict__ planes,
+                                                               int W, i64 m, int n,
+                                                               const int2* __restrict__ site,
+                                                               double* __restrict__ out) {
+  __shared__ __align__(16) uint32_t i1[kKW][kRow], i2[kKW][kRow], j1[kKW][kRow], j2[kKW][kRow];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const i64 nb = (m + kT - 1) / kT, n_tiles = nb * (nb + 1) / 2;
+  for (i64 t = blockIdx.x; t < n_tiles; t += gridDim.x) {
+    i64 bi, bj;
+    tri_decode(t, nb, bi, bj);
+    const i64 i0 = bi * kT, j0 = bj * kT;
+    int s[4] = {0, 0, 0, 0};
+    for (int w0 = 0; w0 < W; w0 += kKW) {
+      __syncthreads();
+      stage_words(i1, planes + W, 3 * W, i0, m, w0, W);
+      stage_words(i2, planes + 2 * W, 3 * W, i0, m, w0, W);
+      stage_words(j1, planes + W, 3 * W, j0, m, w0, W);
+      stage_words(j2, planes + 2 * W, 3 * W, j0, m, w0, W);
+      __syncthreads();
+      const int nw = min(kKW, W - w0);
+#pragma unroll 4
+      for (int w = 0; w < nw; ++w) {
+        const uint32_t b1 = j1[w][lane], b2 = j2[w][lane];
+        const uint4 a1 = *reinterpret_cast<const uint4*>(&i1[w][wid * 4]);
+        const uint4 a2 = *reinterpret_cast<const uint4*>(&i2[w][wid * 4]);
+        const uint32_t x1[4] = {a1.x, a1.y, a1.z, a1.w}, x2[4] = {a2.x, a2.y, a2.z, a2.w};
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+          s[q] += __popc(x1[q] & b1) + 2 * __popc((x1[q] & b2) | (x2[q] & b1)) +
+                  4 * __popc(x2[q] & b2);
+      }
+    }
+    const i64 j = j0 + lane;
+    const int2 sj = j < m ? site[j] : make_int2(0, 0);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const i64 i = i0 + wid * 4 + q;
+      if (i < j && j < m) {
+        const int2 si = site[i];
+        const int cov = n * s[q] - si.x * sj.x;
+        const i64 den = (i64)si.y * sj.y;
+        out[tri_row(i, m) + (j - i - 1)] = den > 0 ? (double)cov / sqrt(__ll2double_rn(den))
+                                                   : __longlong_as_double(0x7ff8000000000000LL);
+      }
+    }
+  }
+}
+
 }  // namespace dense
 }  // namespace pgld
 
@@ -412,6 +566,48 @@ static int dense_grid(pgld_context* h, const void* kern, size_t smem, i64 n_tile
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, pgld::dense::kThreads, smem);
   per_sm = std::max(1, per_sm);
   return (int)std::max<i64>(1, std::min<i64>(n_tiles, (i64)h->n_sm * per_sm));
+}
+
+int pgld_tally_tiles(pgld_context* h, const uint32_t* planes, const uint32_t* valid, int W, i64 n,
+                     int32_t* counts, int32_t* n_valid, cudaStream_t st) {
+  using namespace pgld::dense;
+  const bool aligned = ((uintptr_t)counts & 15) == 0;
+  const i64 nb = (n + kT - 1) / kT;
+  const bool v = valid && n_valid;
+  const void* kern = v ? (const void*)tally_kernel<true> : (const void*)tally_kernel<false>;
+  const int grid = dense_grid(h, kern, 0, nb * (nb + 1) / 2);
+  pgld_time_begin(h, st);
+  if (v)
+    tally_kernel<true><<<grid, kThreads, 0, st>>>(planes, valid, W, n, counts, aligned, n_valid);
+  else
+    tally_kernel<false><<<grid, kThreads, 0, st>>>(planes, nullptr, W, n, counts, aligned, n_valid);
+  pgld_time_end(h, st);
+  PGLD_CHECK_CUDA(h, cudaGetLastError());
+  return PGLD_OK;
+}
+
+extern "C" int pgld_geno_rogers_huff(pgld_handle h, const uint32_t* planes, int32_t n_words,
+                                     int32_t n_rows, int64_t n_snp, double* out, void* stream) {
+  using namespace pgld::dense;
+  PGLD_REQUIRE(h, h != nullptr, "pgld_geno_rogers_huff: NULL handle");
+  PGLD_REQUIRE(h, n_words >= 1 && n_rows >= 0 && n_rows <= 8192 && n_rows <= 32 * (int64_t)n_words && n_snp >= 0,
+               "pgld_geno_rogers_huff: sizes");
+  if (n_snp < 2) return PGLD_OK;
+  PGLD_REQUIRE(h, planes && out, "pgld_geno_rogers_huff: NULL buffer");
+  PGLD_CHECK_CUDA(h, cudaSetDevice(h->device));
+  cudaStream_t st = (cudaStream_t)stream;
+  void* ws = nullptr;
+  int rc = pgld_workspace(h, (size_t)n_snp * sizeof(int2), &ws);
+  if (rc) return rc;
+  const unsigned sb = (unsigned)std::max<i64>(1, std::min<i64>((n_snp + 255) / 256, h->n_sm * 8LL));
+  dosage_site_kernel<<<sb, 256, 0, st>>>(planes, n_words, n_snp, n_rows, (int2*)ws);
+  const i64 nb = (n_snp + kT - 1) / kT;
+  const int grid = dense_grid(h, (const void*)rogers_huff_kernel, 0, nb * (nb + 1) / 2);
+  pgld_time_begin(h, st);
+  rogers_huff_kernel<<<grid, kThreads, 0, st>>>(planes, n_words, n_snp, n_rows, (const int2*)ws, out);
+  pgld_time_end(h, st);
+  PGLD_CHECK_CUDA(h, cudaGetLastError());
+  return PGLD_OK;
 }
 
 extern "C" int pgld_hap_pairwise_ld(pgld_handle h, const uint32_t* planes, int32_t n_words,

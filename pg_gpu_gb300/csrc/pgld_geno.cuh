@@ -282,6 +282,7 @@ __host__ __device__ __forceinline__ GV term_gv(int kind, const int32_t* pp, cons
 
 __device__ __forceinline__ double gv_f64(const GV& v) {
   if (v.gated && !v.ok) return 0.0;
+  if (v.den > 0) return quotient(v.num, v.den);
   return __ll2double_rn(v.num) / __ll2double_rn(v.den);
 }
 
@@ -290,7 +291,7 @@ __device__ __forceinline__ double rh_f64(const int* c, bool square) {
   const RH m = rh_moments(c);
   const i64 den = m.vi * m.vj;
   if (den <= 0) return __longlong_as_double(0x7ff8000000000000ll);
-  if (square) return __ll2double_rn(m.cov * m.cov) / __ll2double_rn(den);
+  if (square) return quotient(m.cov * m.cov, den);
   return __ll2double_rn(m.cov) / sqrt(__ll2double_rn(den));
 }
 
@@ -299,8 +300,7 @@ __device__ __forceinline__ T term_value(const pgld_term& tm, const GPop* P, cons
   if (tm.kind == PGLD_G_SIGMA_D2) {
     const GV v = sigma_d2(P[tm.pops[0]]);
     if (!v.ok) return (T)__longlong_as_double(0x7ff8000000000000ll);
-    return sizeof(T) == 8 ? (T)(__ll2double_rn(v.num) / __ll2double_rn(v.den))
-                          : (T)(ll2f(v.num) / ll2f(v.den));
+    return sizeof(T) == 8 ? (T)quotient(v.num, v.den) : (T)(ll2f(v.num) / ll2f(v.den));
   }
   if (tm.kind == PGLD_G_RH_R || tm.kind == PGLD_G_RH_R2) {
     if (sizeof(T) == 4 && tm.kind == PGLD_G_RH_R2) return (T)rh2_f32(cc[tm.pops[0]]);

@@ -11,6 +11,7 @@
 #include <vector>
 
 #include "../../include/pgld.h"
+#include "pgld_quot.cuh"
 
 struct pgld_context {
   int device = 0;
@@ -220,15 +221,15 @@ __device__ __forceinline__ double term_value_f64(int kind, const int* pp, const 
     const PopC& p = P[pp[0]];
     if (kind == PGLD_DPRIME) {
       i64 dm = dprime_den(p);
-      return dm > 0 ? (double)p.x / (double)dm : __longlong_as_double(0x7ff8000000000000LL);
+      return dm > 0 ? quotient(p.x, dm) : __longlong_as_double(0x7ff8000000000000LL);
     }
     i64 den = r_den(p);
     if (den <= 0) return __longlong_as_double(0x7ff8000000000000LL);
     if (kind == PGLD_R) return (double)p.x / sqrt((double)den);
-    return (double)(p.x * p.x) / (double)den;
+    return quotient(p.x * p.x, den);
   }
   ND v = eval_case(kind, pp, P);
-  return v.den > 0 ? (double)v.num / (double)v.den : 0.0;
+  return v.den > 0 ? quotient(v.num, v.den) : 0.0;
 }
 
 // 64-bit integer to float32 in two 32-bit conversions of the magnitude:

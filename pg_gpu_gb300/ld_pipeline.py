@@ -61,7 +61,7 @@ def iter_pairs_within_distance(positions, max_dist, chunk_size):
         if npairs == 0:
             v_lo = v_hi
             continue
-        yield _ops.pairs_range(pos_d, max_dist, v_lo, v_hi, npairs)
+        yield _ops.pairs_of_anchors(off_d, v_lo, v_hi, npairs)
         v_lo = v_hi
 
 

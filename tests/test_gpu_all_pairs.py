@@ -1,0 +1,83 @@
+"""All-pairs kernels and the float64 statistics kernels: exact counts, the exact
+quotients of their integers (one rounding), Rogers-Huff r bit for bit."""
+import numpy as np
+import pytest
+
+from oracle import ld_oracle as O
+
+pytestmark = pytest.mark.gpu
+
+torch = pytest.importorskip("torch")
+if not torch.cuda.is_available():
+    pytest.skip("needs a CUDA device", allow_module_level=True)
+
+from pg_gpu_gb300 import _geno, _lib as L, _ops  # noqa: E402
+
+
+def np_(t):
+    return t.cpu().numpy()
+
+
+# SNPs: below, at and above a tile; haplotypes: one word, a chunk of words, more
+@pytest.mark.parametrize("M", [1, 2, 32, 33, 97])
+@pytest.mark.parametrize("H,missing,other", [(1, 0.0, 0.0), (33, 0.1, 0.0), (1024, 0.02, 0.0),
+                                             (1100, 0.0, 0.05), (70, 0.1, 0.05)])
+def test_tally(M, H, missing, other):
+    rng = np.random.default_rng(M * H)
+    x = rng.integers(0, 2, (H, M)).astype(np.int8)
+    x[rng.random(x.shape) < other] = 2
+    x[rng.random(x.shape) < missing] = -1
+    pk = _ops.pack(torch.as_tensor(x, device="cuda"))
+    c, nv = _ops.tally(pk)
+    i, j = np.triu_indices(M, 1)
+    want, wnv = O.counts_for_pairs(x, i, j)
+    assert np.array_equal(np_(c), want.reshape(-1, 4))
+    assert (nv is None) == (wnv is None)
+    if nv is not None:
+        assert np.array_equal(np_(nv), wnv)
+
+
+@pytest.mark.parametrize("m,n", [(1, 5), (2, 3), (32, 31), (33, 33), (70, 1030), (65, 8192)])
+def test_rogers_huff(m, n):
+    rng = np.random.default_rng(m + n)
+    g = rng.binomial(2, rng.beta(0.3, 0.3, m), (n, m)).astype(np.int8)
+    g[:, 0] = 1  # no variance
+    gd = torch.as_tensor(g, device="cuda")
+    got = _ops.rogers_huff_all(_ops.pack_geno(gd))
+    i, j = torch.triu_indices(m, m, 1, device="cuda").to(torch.int32)
+    want = _geno.rh_pairs(gd, i, j) if m > 1 else got
+    assert torch.equal(torch.nan_to_num(got, nan=9.0), torch.nan_to_num(want, nan=9.0))
+
+
+# sample sizes: below four (zero denominators), ordinary, numerators above 53 bits;
+# counts rows that 16-byte loads may and may not read
+@pytest.mark.parametrize("n", [3, 60, 1000, 20_000])
+@pytest.mark.parametrize("pad", [0, 1])
+def test_single_terms_and_tables(n, pad):
+    rng = np.random.default_rng(n + pad)
+    N = 700
+    c = rng.multinomial(n, [0.4, 0.2, 0.3, 0.1], (2, N)).astype(np.int32)
+    c[:, ::7, 1] = 0
+    c[:, ::11, :3] = 0
+    buf = torch.zeros((N, 8 + pad), dtype=torch.int32, device="cuda")
+    buf[:, :8] = torch.as_tensor(np.concatenate([c[0], c[1]], 1))
+    views = [buf[:, :4], buf[:, 4:8]]
+    nv = [None, torch.as_tensor(c[1].sum(1).astype(np.int32), device="cuda")]
+    one = [L.DD_II, L.DZ_III, L.PI2_IIII, L.R, L.R2, L.DPRIME]
+    two = [L.DD_IJ, L.DZ_IIJ, L.DZ_IJI, L.DZ_IJJ, L.PI2_TRIPLE, L.PI2_IIKK, L.PI2_IIKK_SYM,
+           L.PI2_IJIJ]
+    for kind in one + two:
+        for roles in ((0, 1), (1, 0)):
+            r = roles[:1] if kind in one else roles
+            # a list of two terms takes the general kernel
+            want = _ops.stats(views, nv, [(0, kind, r, 1.0), (1, kind, r, 0.5)], 2)[:, 0]
+            got = _ops.stats(views, nv, [(0, kind, r, 1.0)], 1)[:, 0]
+            assert torch.equal(torch.nan_to_num(got, nan=7.5), torch.nan_to_num(want, nan=7.5)), kind
+    from pg_gpu_gb300.ld_pipeline import spec_terms
+    for P, S in ((1, 3), (2, 15)):
+        got = np_(_ops.stats(views[:P], nv[:P], spec_terms(P), S))
+        # with a column more the list is not the table; the averages of two
+        # quotients differ from one quotient by roundings of the larger
+        more = spec_terms(P) + [(S, L.DD_II, (0,), 1.0)]
+        want = np_(_ops.stats(views[:P], nv[:P], more, S + 1))[:, :S]
+        np.testing.assert_allclose(got, want, rtol=1e-14, atol=1e-15 * np.abs(want).max())
