@@ -275,6 +275,12 @@ int pgld_pairs_from_offsets(pgld_handle h, const int64_t* offsets, int64_t i_beg
 int pgld_hap_band_pairs(pgld_handle h, const pgld_hap_panel* panel, const double* pos,
                         double max_dist, int32_t* counts, int32_t* n_valid, float* stats,
                         int64_t n_pairs, int32_t form, void* stream);
+/* The same with the offsets that pgld_count_pairs_within filled for pos and
+ * max_dist (n_pairs = offsets[n_snp], not read back): asynchronous. */
+int pgld_hap_band_pairs_at(pgld_handle h, const pgld_hap_panel* panel, const double* pos,
+                           double max_dist, const int64_t* offsets, int32_t* counts,
+                           int32_t* n_valid, float* stats, int64_t n_pairs, int32_t form,
+                           void* stream);
 
 /* Distance-binned sums of the moments LD statistics of n_pops (1..4)
  * populations over every pair i<j with pos[j]-pos[i] <= max_dist.
@@ -426,6 +432,11 @@ int pgld_geno_rogers_huff(pgld_handle h, const uint32_t* planes, int32_t n_words
 int pgld_geno_band_pairs(pgld_handle h, const pgld_geno_panel* panel, const double* pos,
                          double max_dist, int32_t* counts, int32_t* n_valid, float* stats,
                          int32_t stat_mask, int64_t n_pairs, int32_t form, void* stream);
+/* The same with given offsets (as pgld_hap_band_pairs_at). */
+int pgld_geno_band_pairs_at(pgld_handle h, const pgld_geno_panel* panel, const double* pos,
+                            double max_dist, const int64_t* offsets, int32_t* counts,
+                            int32_t* n_valid, float* stats, int32_t stat_mask, int64_t n_pairs,
+                            int32_t form, void* stream);
 
 /* Distance-binned sums of the moments genotype statistics of n_pops (1..4)
  * populations, arguments and bins as pgld_hap_binned_sums.  Replaces

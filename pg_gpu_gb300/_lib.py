@@ -94,6 +94,10 @@ _SIGS = {
     "pgld_count_pairs_within": ([_P, _P, _I64, _D, ctypes.POINTER(_I64), _P, _P], ctypes.c_int),
     "pgld_pairs_within": ([_P, _P, _I64, _D, _I64, _I64, _P, _P, _I64, _P], ctypes.c_int),
     "pgld_pairs_from_offsets": ([_P, _P, _I64, _I64, _P, _P, _P], ctypes.c_int),
+    "pgld_hap_band_pairs_at": ([_P, ctypes.POINTER(HapPanel), _P, _D, _P, _P, _P, _P, _I64, _I32,
+                                _P], ctypes.c_int),
+    "pgld_geno_band_pairs_at": ([_P, ctypes.POINTER(GenoPanel), _P, _D, _P, _P, _P, _P, _I32, _I64,
+                                 _I32, _P], ctypes.c_int),
     "pgld_geno_rogers_huff": ([_P, _P, _I32, _I32, _I64, _P, _P], ctypes.c_int),
     "pgld_hap_band_pairs": ([_P, ctypes.POINTER(HapPanel), _P, _D, _P, _P, _P, _I64, _I32, _P],
                             ctypes.c_int),
@@ -182,7 +186,7 @@ def check(rc, h=None):
 def handle(device=None):
     """The per-device libpgld handle of this process."""
     import torch
-    if not torch.cuda.is_available():
+    if not _handles and not torch.cuda.is_available():
         raise PgldError(-2, "no CUDA device: libpgld has no CPU path")
     dev = torch.cuda.current_device() if device is None else int(device)
     h = _handles.get(dev)
@@ -196,6 +200,13 @@ def handle(device=None):
                 h = p.value
                 _handles[dev] = h
     return h
+
+
+def device_status(h):
+    """Reads and clears the handle's device error word (synchronises)."""
+    st = ctypes.c_int32()
+    check(lib().pgld_device_status(h, ctypes.byref(st), stream_ptr()), h)
+    return st.value
 
 
 def stream_ptr():

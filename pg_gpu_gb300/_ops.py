@@ -18,6 +18,24 @@ def _torch():
 # --------------------------------------------------------------------------
 # packed haplotype planes
 # --------------------------------------------------------------------------
+class PackFlags:
+    """The flag pairs (missing, other) that packing launches write, read back
+    together on first use."""
+
+    def __init__(self, count, device):
+        self.device_flags = _torch().zeros(2 * count, dtype=_torch().int32, device=device)
+        self._host = None
+
+    def pair(self, k):
+        """The k-th launch's device pair."""
+        return self.device_flags[2 * k:2 * k + 2]
+
+    def read(self, k):
+        if self._host is None:
+            self._host = self.device_flags.cpu().numpy()
+        return bool(self._host[2 * k]), bool(self._host[2 * k + 1])
+
+
 class PackedPop:
     """Bit planes of one population (carrier / reference, optional validity).
 
@@ -37,18 +55,23 @@ class PackedPop:
         self._other = has_other
 
     @classmethod
-    def pending(cls, planes, valid, n_words, n_rows, n_snp, flags):
-        """Planes whose flags (a device int32[2] written by the packing kernel)
-        are read on first use, so that packing does not synchronise."""
+    def pending(cls, planes, valid, n_words, n_rows, n_snp, flags, k):
+        """Planes whose flags (pair k of a PackFlags, written by the packing
+        kernel) are read on first use, so that packing does not synchronise."""
         pk = cls(planes, valid, n_words, n_rows, n_snp, None, None)
-        pk._flags = flags
+        pk._flags = (flags, k)
         return pk
 
     def _resolve(self):
         if self._flags is not None:
-            f = self._flags.cpu().numpy()
-            self._missing, self._other = bool(f[0]), bool(f[1])
+            flags, k = self._flags
+            self._missing, self._other = flags.read(k)
             self._flags = None
+
+    @property
+    def unread(self):
+        """Whether the flags are still on the device."""
+        return self._flags is not None
 
     @property
     def has_missing(self):
@@ -66,10 +89,28 @@ class PackedPop:
         return self.valid if (self.has_other and self.has_missing) else None
 
 
+class Rows:
+    """Checked population row indices on the device (device_rows)."""
+
+    def __init__(self, tensor):
+        self.tensor = tensor
+
+
+def device_rows(row_lists, n_total):
+    """Rows of several populations' host index lists, checked against n_total
+    and uploaded together."""
+    host = [np.asarray(r).astype(np.int32, copy=False).reshape(-1) for r in row_lists]
+    whole = _check_rows(np.concatenate(host), n_total)
+    ends = np.cumsum([r.size for r in host])
+    return [Rows(whole[e - r.size:e]) for e, r in zip(ends, host)]
+
+
 def _check_rows(rows, n_total):
     """Population row indices as a device int32 tensor, checked against
     n_total (on the host for host indices, one device read otherwise)."""
     torch = _torch()
+    if isinstance(rows, Rows):
+        return rows.tensor
     if isinstance(rows, torch.Tensor) and rows.is_cuda:
         rows_t = L.as_device(rows, np.int32)
         if rows_t.numel():
@@ -149,14 +190,15 @@ def heterozygosity(sums, valids, n_rows, ploidy):
     return out.cpu().numpy()
 
 
-def pack(hap, rows=None, kept=None):
+def pack(hap, rows=None, kept=None, flags=None, k=0):
     """Pack the rows of an int8 (H x M) matrix into bit planes on the device.
 
     hap is a device matrix (or anything as_device accepts, copied first); an
     int8 CPU tensor in pinned memory is read in place by the packing kernel,
     so only the packed planes are written to device memory (the call then
     returns once the kernel is done with the host matrix).  kept: the result
-    of kept_sites, to pack those sites only."""
+    of kept_sites, to pack those sites only.  flags: a PackFlags shared by
+    several calls, of which this one writes pair k."""
     torch = _torch()
     if not _host_readable(hap):
         hap = L.as_device(hap, np.int8)
@@ -174,7 +216,8 @@ def pack(hap, rows=None, kept=None):
     before, n_out = (None, n_snp) if kept is None else (kept[0], kept[1].numel())
     planes = torch.empty((n_out, 2 * W), dtype=torch.int32, device=dev)
     valid = torch.empty((n_out, W), dtype=torch.int32, device=dev)
-    flags = torch.zeros(2, dtype=torch.int32, device=dev)
+    if flags is None:
+        flags, k = PackFlags(1, dev), 0
     if n_rows == 0:
         planes.zero_()
         valid.zero_()
@@ -182,9 +225,9 @@ def pack(hap, rows=None, kept=None):
         h = L.handle()
         L.check(L.lib().pgld_pack_haplotypes_kept(h, L.ptr(hap), hap.stride(0), n_snp,
                                                   L.ptr(rows_t), n_rows, L.ptr(before),
-                                                  L.ptr(planes), L.ptr(valid), L.ptr(flags),
-                                                  L.stream_ptr()), h)
-    pk = PackedPop.pending(planes, valid, W, n_rows, n_out, flags)
+                                                  L.ptr(planes), L.ptr(valid),
+                                                  L.ptr(flags.pair(k)), L.stream_ptr()), h)
+    pk = PackedPop.pending(planes, valid, W, n_rows, n_out, flags, k)
     if not hap.is_cuda:
         pk._resolve()  # the host matrix is read in place: finish before returning
     return pk
@@ -214,19 +257,19 @@ def counts_pairs(pk, idx_i, idx_j):
         raise ValueError("idx_i and idx_j must have the same shape")
     n = ii.numel()
     counts = torch.empty((n, 4), dtype=torch.int32, device=ii.device)
-    nv = torch.empty(n, dtype=torch.int32, device=ii.device) if pk.has_missing else None
+    # flags that are still on the device are read with the status, after the
+    # kernel: until then the validity plane gives n whatever the codes are
+    unread = n > 0 and pk.unread
+    nv = torch.empty(n, dtype=torch.int32, device=ii.device) if unread or pk.has_missing else None
     if n:
         h = L.handle()
-        v = pk.valid_for_n
+        v = pk.valid if unread else pk.valid_for_n
         L.check(L.lib().pgld_hap_counts_pairs(h, L.ptr(pk.planes), L.ptr(v), pk.n_words, pk.n_snp,
                                               L.ptr(ii), L.ptr(jj), n, L.ptr(counts), 4,
                                               L.ptr(nv), L.stream_ptr()), h)
-        st = torch.zeros(1, dtype=torch.int32)
-        L.check(L.lib().pgld_device_status(h, ctypes.cast(st.data_ptr(), ctypes.POINTER(
-            ctypes.c_int32)), L.stream_ptr()), h)
-        if int(st[0]):
+        if L.device_status(h):
             raise IndexError("pair index out of range of the variant axis")
-    return counts, nv
+    return counts, nv if pk.has_missing else None
 
 
 def tally(pk):
@@ -247,7 +290,9 @@ def tally(pk):
 # statistics
 # --------------------------------------------------------------------------
 def make_terms(term_list):
-    """[(stat, kind, pops, weight)] -> ctypes array of Term."""
+    """[(stat, kind, pops, weight)] (or such an array) -> ctypes array of Term."""
+    if isinstance(term_list, ctypes.Array):
+        return term_list
     arr = (L.Term * len(term_list))()
     for k, (stat, kind, pops, w) in enumerate(term_list):
         arr[k].stat = stat
@@ -308,19 +353,8 @@ def band_offsets(pos_d, max_dist):
 
 
 def band_pair_count(pos_d, max_dist):
-    """Pairs within max_dist of sorted device positions.  The count is kept
-    with the positions tensor (keyed by its version counter and max_dist), so
-    a call repeated on unchanged positions reads nothing from the device."""
-    key = float(max_dist)
-    cache = getattr(pos_d, "_pgld_npairs", None)
-    if cache is not None and cache[0] == pos_d._version and key in cache[1]:
-        return cache[1][key]
-    _, n = band_offsets(pos_d, max_dist)
-    if cache is None or cache[0] != pos_d._version:
-        cache = (pos_d._version, {})
-        pos_d._pgld_npairs = cache
-    cache[1][key] = n
-    return n
+    """Pairs within max_dist of sorted device positions."""
+    return band_offsets(pos_d, max_dist)[1]
 
 
 def pairs_of_anchors(off, i_begin, i_end, n_pairs):
@@ -350,16 +384,17 @@ def band_pairs(pk, pos_d, max_dist, with_stats=True, form="auto", _tuning=False)
         from . import autotune
         autotune.apply("pairs", [pk.n_words])
     torch = _torch()
-    n = band_pair_count(pos_d, max_dist)
+    off, n = band_offsets(pos_d, max_dist)
     dev = pos_d.device
     counts = torch.empty((n, 4), dtype=torch.int32, device=dev)
     nv = torch.empty(n, dtype=torch.int32, device=dev)
     st = torch.empty((n, 4), dtype=torch.float32, device=dev) if with_stats else None
     h = L.handle()
-    L.check(L.lib().pgld_hap_band_pairs(h, ctypes.byref(panel([pk])), L.ptr(pos_d),
-                                        float(max_dist), L.ptr(counts), L.ptr(nv), L.ptr(st), n,
-                                        L.FORM_TC if form == "tc" else L.FORM_PLAIN,
-                                        L.stream_ptr()), h)
+    L.check(L.lib().pgld_hap_band_pairs_at(h, ctypes.byref(panel([pk])), L.ptr(pos_d),
+                                           float(max_dist), L.ptr(off), L.ptr(counts), L.ptr(nv),
+                                           L.ptr(st), n,
+                                           L.FORM_TC if form == "tc" else L.FORM_PLAIN,
+                                           L.stream_ptr()), h)
     return counts, nv, st
 
 
@@ -402,11 +437,9 @@ def window_sums(pk, idx, win_begin, win_end, form="auto", _tuning=False, columns
                                                  L.ptr(cnt), mask,
                                                  L.FORM_TC if form == "tc" else L.FORM_PLAIN,
                                                  L.stream_ptr()), h)
-    st = torch.zeros(1, dtype=torch.int32)
-    L.check(L.lib().pgld_device_status(h, ctypes.cast(st.data_ptr(), ctypes.POINTER(
-        ctypes.c_int32)), L.stream_ptr()), h)
-    if int(st[0]):
-        raise IndexError(f"window or SNP index out of range (device status {int(st[0])})")
+    code = L.device_status(h)
+    if code:
+        raise IndexError(f"window or SNP index out of range (device status {code})")
     return sums, cnt
 
 
@@ -437,11 +470,9 @@ def window_snp_sums(pk, idx, win_begin, win_end, stat):
     L.check(L.lib().pgld_hap_window_snp_sums(h, ctypes.byref(panel([pk])), L.ptr(ii), n_idx,
                                              L.ptr(wb), L.ptr(we), n_win, L.ptr(off_d), int(stat),
                                              L.ptr(rows), L.ptr(cols), n_out, L.stream_ptr()), h)
-    st = torch.zeros(1, dtype=torch.int32)
-    L.check(L.lib().pgld_device_status(h, ctypes.cast(st.data_ptr(), ctypes.POINTER(
-        ctypes.c_int32)), L.stream_ptr()), h)
-    if int(st[0]):
-        raise IndexError(f"window or SNP index out of range (device status {int(st[0])})")
+    code = L.device_status(h)
+    if code:
+        raise IndexError(f"window or SNP index out of range (device status {code})")
     return rows[:n_out], cols[:n_out], off
 
 
@@ -497,6 +528,20 @@ def tc_applies(pops):
     return len(pops) <= 2 and all(pk.n_words <= 64 and pk.valid_for_n is None for pk in pops)
 
 
+def _sum_buffers(n_bins, n_stats, dev):
+    """(sums float64 (n_bins, n_stats), counts int64 (n_bins,)) in one allocation."""
+    torch = _torch()
+    buf = torch.empty(n_bins * (n_stats + 1), dtype=torch.float64, device=dev)
+    return buf[:n_bins * n_stats].view(n_bins, n_stats), buf[n_bins * n_stats:].view(torch.int64)
+
+
+def host_sums(sums, cnt):
+    """binned_sums' results on the host, in one copy."""
+    n, k = sums.shape
+    buf = sums.as_strided((n * (k + 1),), (1,)).cpu().numpy()
+    return buf[:n * k].reshape(n, k), buf[n * k:].view(np.int64)
+
+
 def binned_sums(pops, pos_d, bins, max_dist=None, bin_coord=None, form="auto", anchors=None,
                 _tuning=False):
     """(sums (n_bins, n_stats) float64 tensor, pair counts (n_bins,) int64).
@@ -520,8 +565,7 @@ def binned_sums(pops, pos_d, bins, max_dist=None, bin_coord=None, form="auto", a
     n_stats = {1: 3, 2: 15, 3: 45, 4: 105}[P]
     dev = pos_d.device
     bins_d = torch.as_tensor(bins_np, device=dev)
-    sums = torch.empty((n_bins, n_stats), dtype=torch.float64, device=dev)
-    cnt = torch.empty(n_bins, dtype=torch.int64, device=dev)
+    sums, cnt = _sum_buffers(n_bins, n_stats, dev)
     md = float(bins_np[-1]) if max_dist is None else float(max_dist)
     bc = None if bin_coord is None else L.as_device(bin_coord, np.float64)
     h = L.handle()
@@ -578,44 +622,51 @@ class PackedGeno:
 def pack_geno(geno, rows=None, kept=None):
     """Pack the rows of an int8 (n_individuals x M) device dosage matrix (kept:
     the result of kept_sites, to pack those sites only)."""
+    return pack_geno_all(geno, [rows], kept)[0]
+
+
+def pack_geno_all(geno, row_lists, kept=None):
+    """pack_geno of several populations of one matrix, their flags read together."""
     torch = _torch()
     g = L.as_device(geno, np.int8)
     if g.dim() != 2:
         raise ValueError("genotypes must be 2-D (n_individuals, n_variants)")
     n_total, n_snp = g.shape
-    if rows is not None:
-        rows_t = _check_rows(rows, n_total)
-        n_rows = rows_t.numel()
-    else:
-        rows_t = None
-        n_rows = n_total
-    if n_rows > MAX_GENO_N:
-        raise ValueError(f"{n_rows} individuals exceed {MAX_GENO_N} per population")
-    W = max(1, (n_rows + 31) // 32)
     before, n_out = (None, n_snp) if kept is None else (kept[0], kept[1].numel())
-    planes = torch.empty((n_out, 3 * W), dtype=torch.int32, device=g.device)
-    valid = torch.empty((n_out, W), dtype=torch.int32, device=g.device)
-    flags = torch.zeros(2, dtype=torch.int32, device=g.device)
-    ext = None
+    flags = PackFlags(len(row_lists), g.device)
 
-    def run():
+    def run(rows_t, n_rows, planes, valid, ext, k):
         h = L.handle()
         L.check(L.lib().pgld_pack_genotypes_kept(h, L.ptr(g), g.stride(0), n_snp, L.ptr(rows_t),
                                                  n_rows, L.ptr(before), L.ptr(planes),
-                                                 L.ptr(valid), L.ptr(ext), L.ptr(flags),
+                                                 L.ptr(valid), L.ptr(ext), L.ptr(flags.pair(k)),
                                                  L.stream_ptr()), h)
 
-    if n_rows == 0:
-        planes.zero_()
-        valid.zero_()
-    else:
-        run()
-    f = flags.cpu().numpy()
-    if f[1]:
-        # dosages above 2: the planes of the values 3..8 as well
-        ext = torch.empty((n_out, 6 * W), dtype=torch.int32, device=g.device)
-        run()
-    return PackedGeno(planes, valid, W, n_rows, n_out, bool(f[0]), bool(f[1]), ext)
+    parts = []
+    for k, rows in enumerate(row_lists):
+        rows_t = None if rows is None else _check_rows(rows, n_total)
+        n_rows = n_total if rows_t is None else rows_t.numel()
+        if n_rows > MAX_GENO_N:
+            raise ValueError(f"{n_rows} individuals exceed {MAX_GENO_N} per population")
+        W = max(1, (n_rows + 31) // 32)
+        planes = torch.empty((n_out, 3 * W), dtype=torch.int32, device=g.device)
+        valid = torch.empty((n_out, W), dtype=torch.int32, device=g.device)
+        if n_rows == 0:
+            planes.zero_()
+            valid.zero_()
+        else:
+            run(rows_t, n_rows, planes, valid, None, k)
+        parts.append((rows_t, n_rows, W, planes, valid))
+    packs = []
+    for k, (rows_t, n_rows, W, planes, valid) in enumerate(parts):
+        missing, other = flags.read(k)
+        ext = None
+        if other:
+            # dosages above 2: the planes of the values 3..8 as well
+            ext = torch.empty((n_out, 6 * W), dtype=torch.int32, device=g.device)
+            run(rows_t, n_rows, planes, valid, ext, k)
+        packs.append(PackedGeno(planes, valid, W, n_rows, n_out, missing, other, ext))
+    return packs
 
 
 def geno_panel(pops):
@@ -647,10 +698,7 @@ def geno_counts_pairs(pk, idx_i, idx_j):
         L.check(L.lib().pgld_geno_counts_pairs(h, L.ptr(pk.planes), L.ptr(pk.valid_for_n),
                                                L.ptr(pk.ext_planes), pk.n_words, pk.n_snp, L.ptr(ii), L.ptr(jj), n,
                                                L.ptr(counts), 9, L.ptr(nv), L.stream_ptr()), h)
-        st = torch.zeros(1, dtype=torch.int32)
-        L.check(L.lib().pgld_device_status(h, ctypes.cast(st.data_ptr(), ctypes.POINTER(
-            ctypes.c_int32)), L.stream_ptr()), h)
-        if int(st[0]):
+        if L.device_status(h):
             raise IndexError("pair index out of range of the variant axis")
     return counts, nv
 
@@ -698,16 +746,17 @@ def geno_band_pairs(pk, pos_d, max_dist, with_counts=True, with_stats=True,
             raise ValueError(f"unknown column {c!r}")
         mask |= 1 << GENO_BAND_COLUMNS.index(c)
     torch = _torch()
-    n = band_pair_count(pos_d, max_dist)
+    off, n = band_offsets(pos_d, max_dist)
     dev = pos_d.device
     counts = torch.empty((n, 9), dtype=torch.int32, device=dev) if with_counts else None
     nv = torch.empty(n, dtype=torch.int32, device=dev)
     st = torch.empty((n, 4), dtype=torch.float32, device=dev) if with_stats else None
     h = L.handle()
-    L.check(L.lib().pgld_geno_band_pairs(h, ctypes.byref(geno_panel([pk])), L.ptr(pos_d),
-                                         float(max_dist), L.ptr(counts), L.ptr(nv), L.ptr(st),
-                                         mask, n, L.FORM_TC if form == "tc" else L.FORM_PLAIN,
-                                         L.stream_ptr()), h)
+    L.check(L.lib().pgld_geno_band_pairs_at(h, ctypes.byref(geno_panel([pk])), L.ptr(pos_d),
+                                            float(max_dist), L.ptr(off), L.ptr(counts), L.ptr(nv),
+                                            L.ptr(st), mask, n,
+                                            L.FORM_TC if form == "tc" else L.FORM_PLAIN,
+                                            L.stream_ptr()), h)
     return counts, nv, st
 
 
@@ -742,8 +791,7 @@ def geno_binned_sums(pops, pos_d, bins, max_dist=None, bin_coord=None, form="aut
     n_stats = {1: 3, 2: 15, 3: 45, 4: 105}[len(pops)]
     dev = pos_d.device
     bins_d = torch.as_tensor(bins_np, device=dev)
-    sums = torch.empty((n_bins, n_stats), dtype=torch.float64, device=dev)
-    cnt = torch.empty(n_bins, dtype=torch.int64, device=dev)
+    sums, cnt = _sum_buffers(n_bins, n_stats, dev)
     md = float(bins_np[-1]) if max_dist is None else float(max_dist)
     bc = None if bin_coord is None else L.as_device(bin_coord, np.float64)
     h = L.handle()
@@ -800,11 +848,9 @@ def pairs_by_bin(pos_d, bins, pk=None, pair_values=None):
         L.check(L.lib().pgld_pairs_by_bin(h, L.ptr(planes), W, L.ptr(pv), m, L.ptr(pos_d),
                                           L.ptr(bins_d), n_bins, c_ptr, L.ptr(vals),
                                           L.stream_ptr()), h)
-        st = torch.zeros(1, dtype=torch.int32)
-        L.check(L.lib().pgld_device_status(h, ctypes.cast(st.data_ptr(), ctypes.POINTER(
-            ctypes.c_int32)), L.stream_ptr()), h)
-        if int(st[0]):
-            raise RuntimeError(f"pairs changed between counting and filling (status {int(st[0])})")
+        code = L.device_status(h)
+        if code:
+            raise RuntimeError(f"pairs changed between counting and filling (status {code})")
     return vals[:int(counts.sum())], counts
 
 

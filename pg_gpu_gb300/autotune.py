@@ -25,6 +25,7 @@ is missing; with PGLD_AUTOTUNE=1 a missing key is tuned first).
 """
 from __future__ import annotations
 
+import functools
 import json
 import os
 import threading
@@ -44,11 +45,16 @@ ONE_POP_CANDIDATES = [(layout, stages) for layout in (2, 1) for stages in (0, 4,
 OTHER_CANDIDATES = [(0, stages) for stages in (0, 4, 3, 2)]
 
 
-def _device_key():
+@functools.lru_cache(maxsize=None)
+def _device_name(dev):
     import torch
-    dev = torch.cuda.current_device()
     p = torch.cuda.get_device_properties(dev)
     return f"{p.name}|{p.multi_processor_count}"
+
+
+def _device_key():
+    import torch
+    return _device_name(torch.cuda.current_device())
 
 
 def key(kind, words):

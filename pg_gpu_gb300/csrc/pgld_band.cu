@@ -329,9 +329,11 @@ int pgld_tc_binned(pgld_context* h, const pgld_hap_panel* panel, pgld::BandArgs&
 int pgld_tc_pairs(pgld_context* h, const pgld_hap_panel* panel, pgld::BandArgs& a,
                   cudaStream_t st);
 
-extern "C" int pgld_hap_band_pairs(pgld_handle h, const pgld_hap_panel* panel, const double* pos,
-                                   double max_dist, int32_t* counts, int32_t* n_valid,
-                                   float* stats, int64_t n_pairs, int32_t form, void* stream) {
+// offsets: the band offsets of pos and max_dist (n_pairs = offsets[n_snp]), or
+// NULL: computed here, and their total checked against n_pairs (synchronises)
+static int band_pairs(pgld_context* h, const pgld_hap_panel* panel, const double* pos, double max_dist,
+                      const int64_t* offsets, int32_t* counts, int32_t* n_valid, float* stats,
+                      int64_t n_pairs, int32_t form, void* stream) {
   PGLD_REQUIRE(h, h != nullptr, "pgld_hap_band_pairs: NULL handle");
   int rc = check_panel(h, panel, "pgld_hap_band_pairs");
   if (rc) return rc;
@@ -348,6 +350,7 @@ extern "C" int pgld_hap_band_pairs(pgld_handle h, const pgld_hap_panel* panel, c
                  (long long)n_pairs, (long long)n);
     return PGLD_OK;
   }
+  if (offsets && n_pairs == 0) return PGLD_OK;
   PGLD_REQUIRE(h, pos && counts, "pgld_hap_band_pairs: NULL buffer");
   PGLD_REQUIRE(h, ((uintptr_t)counts & 15) == 0 && (!stats || ((uintptr_t)stats & 15) == 0),
                "pgld_hap_band_pairs: counts/stats must be 16-byte aligned");
@@ -356,36 +359,62 @@ extern "C" int pgld_hap_band_pairs(pgld_handle h, const pgld_hap_panel* panel, c
   const i64 nb = (n + pgld::kTile - 1) / pgld::kTile;
   size_t sb1 = pgld::scan_scratch_bytes(n), sb2 = pgld::scan_scratch_bytes(nb);
   size_t off_bytes = (size_t)(n + 1) * 8, it_bytes = (size_t)(nb + 1) * 8;
-  void* ws = nullptr;
-  rc = pgld_workspace(h, off_bytes + it_bytes + sb1 + sb2 + 512, &ws);
-  if (rc) return rc;
-  char* w = (char*)ws;
-  i64* off = (i64*)w;
-  i64* items = (i64*)(w + ((off_bytes + 255) & ~size_t(255)));
-  char* scratch = (char*)items + ((it_bytes + 255) & ~size_t(255));
-  rc = pgld_band_offsets(h, pos, n, max_dist, off, scratch, std::max(sb1, sb2), st);
-  if (rc) return rc;
-  i64 tot = 0;
-  PGLD_CHECK_CUDA(h, cudaMemcpyAsync(&tot, off + n, 8, cudaMemcpyDeviceToHost, st));
-  PGLD_CHECK_CUDA(h, cudaStreamSynchronize(st));
-  if (tot != n_pairs)
-    return pgld_fail(h, PGLD_ERR_INVALID_ARG, "pgld_hap_band_pairs: n_pairs %lld != %lld in band",
-                     (long long)n_pairs, (long long)tot);
-  rc = pgld::band_schedule(h, pos, n, max_dist, items, scratch, std::max(sb1, sb2), st);
-  if (rc) return rc;
+  const i64* off = reinterpret_cast<const i64*>(offsets);
+  i64* items = nullptr;
+  char* scratch = nullptr;
+  if (!offsets || form == PGLD_FORM_PLAIN) {
+    void* ws = nullptr;
+    rc = pgld_workspace(h, off_bytes + it_bytes + sb1 + sb2 + 512, &ws);
+    if (rc) return rc;
+    char* w = (char*)ws;
+    items = (i64*)(w + ((off_bytes + 255) & ~size_t(255)));
+    scratch = (char*)items + ((it_bytes + 255) & ~size_t(255));
+    if (!offsets) {
+      rc = pgld_band_offsets(h, pos, n, max_dist, (i64*)w, scratch, std::max(sb1, sb2), st);
+      if (rc) return rc;
+      off = (const i64*)w;
+      i64 tot = 0;
+      PGLD_CHECK_CUDA(h, cudaMemcpyAsync(&tot, off + n, 8, cudaMemcpyDeviceToHost, st));
+      PGLD_CHECK_CUDA(h, cudaStreamSynchronize(st));
+      if (tot != n_pairs)
+        return pgld_fail(h, PGLD_ERR_INVALID_ARG, "pgld_hap_band_pairs: n_pairs %lld != %lld in band",
+                         (long long)n_pairs, (long long)tot);
+    }
+  }
   pgld::BandArgs a{};
   a.status = h->dev_status;
   fill_panel(a, panel);
   a.pos = pos;
   a.max_dist = max_dist;
-  a.item_off = items;
-  a.n_blocks = nb;
-  a.pair_off = off;
   a.counts = counts;
   a.nvalid = n_valid;
   a.stats = stats;
-  if (form == PGLD_FORM_TC) return pgld_tc_pairs(h, panel, a, st);
+  if (form == PGLD_FORM_TC) {
+    // the tensor-core forms lay out their own workspace, which may move ours:
+    // they take the caller's offsets or compute their own
+    a.pair_off = reinterpret_cast<const i64*>(offsets);
+    return pgld_tc_pairs(h, panel, a, st);
+  }
+  rc = pgld::band_schedule(h, pos, n, max_dist, items, scratch, std::max(sb1, sb2), st);
+  if (rc) return rc;
+  a.item_off = items;
+  a.n_blocks = nb;
+  a.pair_off = off;
   return pgld::launch_band_plain(h, a, pgld::kModePairs, st);
+}
+
+extern "C" int pgld_hap_band_pairs(pgld_handle h, const pgld_hap_panel* panel, const double* pos,
+                                   double max_dist, int32_t* counts, int32_t* n_valid,
+                                   float* stats, int64_t n_pairs, int32_t form, void* stream) {
+  return band_pairs(h, panel, pos, max_dist, nullptr, counts, n_valid, stats, n_pairs, form, stream);
+}
+
+extern "C" int pgld_hap_band_pairs_at(pgld_handle h, const pgld_hap_panel* panel, const double* pos,
+                                      double max_dist, const int64_t* offsets, int32_t* counts,
+                                      int32_t* n_valid, float* stats, int64_t n_pairs, int32_t form,
+                                      void* stream) {
+  PGLD_REQUIRE(h, offsets != nullptr, "pgld_hap_band_pairs_at: NULL offsets");
+  return band_pairs(h, panel, pos, max_dist, offsets, counts, n_valid, stats, n_pairs, form, stream);
 }
 
 namespace pgld {

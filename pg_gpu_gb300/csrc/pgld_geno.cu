@@ -548,13 +548,14 @@ static void fill_geno_panel(pgld::BandArgs& a, const pgld_geno_panel* panel) {
 }
 
 int pgld_geno_tc_pairs(pgld_context* h, const pgld_geno_panel* panel, const double* pos,
-                       double max_dist, int32_t* counts, int32_t* n_valid, float* stats,
-                       int32_t stat_mask, cudaStream_t st);
+                       double max_dist, const long long* offsets, int32_t* counts, int32_t* n_valid,
+                       float* stats, int32_t stat_mask, cudaStream_t st);
 
-extern "C" int pgld_geno_band_pairs(pgld_handle h, const pgld_geno_panel* panel, const double* pos,
-                                    double max_dist, int32_t* counts, int32_t* n_valid,
-                                    float* stats, int32_t stat_mask, int64_t n_pairs,
-                                    int32_t form, void* stream) {
+// offsets as for the haplotype pairs: the caller's, or NULL
+static int geno_band_pairs(pgld_context* h, const pgld_geno_panel* panel, const double* pos,
+                           double max_dist, const int64_t* offsets, int32_t* counts,
+                           int32_t* n_valid, float* stats, int32_t stat_mask, int64_t n_pairs,
+                           int32_t form, void* stream) {
   PGLD_REQUIRE(h, h != nullptr, "pgld_geno_band_pairs: NULL handle");
   int rc = check_geno_panel(h, panel, "pgld_geno_band_pairs");
   if (rc) return rc;
@@ -580,24 +581,32 @@ extern "C" int pgld_geno_band_pairs(pgld_handle h, const pgld_geno_panel* panel,
   const i64 nb = (n + pgld::geno::kT - 1) / pgld::geno::kT;
   const size_t sb1 = pgld::scan_scratch_bytes(n), sb2 = pgld::scan_scratch_bytes(nb);
   const size_t off_bytes = (size_t)(n + 1) * 8, it_bytes = (size_t)(nb + 1) * 8;
-  void* ws = nullptr;
-  rc = pgld_workspace(h, off_bytes + it_bytes + std::max(sb1, sb2) + 768, &ws);
-  if (rc) return rc;
-  char* w = (char*)ws;
-  i64* off = (i64*)w;
-  i64* items = (i64*)(w + ((off_bytes + 255) & ~size_t(255)));
-  char* scratch = (char*)items + ((it_bytes + 255) & ~size_t(255));
-  rc = pgld_band_offsets(h, pos, n, max_dist, off, scratch, std::max(sb1, sb2), st);
-  if (rc) return rc;
-  i64 tot = 0;
-  PGLD_CHECK_CUDA(h, cudaMemcpyAsync(&tot, off + n, 8, cudaMemcpyDeviceToHost, st));
-  PGLD_CHECK_CUDA(h, cudaStreamSynchronize(st));
-  if (tot != n_pairs)
-    return pgld_fail(h, PGLD_ERR_INVALID_ARG, "pgld_geno_band_pairs: n_pairs %lld != %lld in band",
-                     (long long)n_pairs, (long long)tot);
-  if (tot == 0) return PGLD_OK;
+  const i64* off = reinterpret_cast<const i64*>(offsets);
+  i64* items = nullptr;
+  char* scratch = nullptr;
+  if (!offsets || form == PGLD_FORM_PLAIN) {
+    void* ws = nullptr;
+    rc = pgld_workspace(h, off_bytes + it_bytes + std::max(sb1, sb2) + 768, &ws);
+    if (rc) return rc;
+    char* w = (char*)ws;
+    items = (i64*)(w + ((off_bytes + 255) & ~size_t(255)));
+    scratch = (char*)items + ((it_bytes + 255) & ~size_t(255));
+    if (!offsets) {
+      rc = pgld_band_offsets(h, pos, n, max_dist, (i64*)w, scratch, std::max(sb1, sb2), st);
+      if (rc) return rc;
+      off = (const i64*)w;
+      i64 tot = 0;
+      PGLD_CHECK_CUDA(h, cudaMemcpyAsync(&tot, off + n, 8, cudaMemcpyDeviceToHost, st));
+      PGLD_CHECK_CUDA(h, cudaStreamSynchronize(st));
+      if (tot != n_pairs)
+        return pgld_fail(h, PGLD_ERR_INVALID_ARG, "pgld_geno_band_pairs: n_pairs %lld != %lld in band",
+                         (long long)n_pairs, (long long)tot);
+    }
+  }
+  if (n_pairs == 0) return PGLD_OK;
   if (form == PGLD_FORM_TC)
-    return pgld_geno_tc_pairs(h, panel, pos, max_dist, counts, n_valid, stats, stat_mask, st);
+    return pgld_geno_tc_pairs(h, panel, pos, max_dist, reinterpret_cast<const i64*>(offsets), counts,
+                              n_valid, stats, stat_mask, st);
   rc = pgld::band_schedule(h, pos, n, max_dist, items, scratch, std::max(sb1, sb2), st,
                            pgld::geno::kT);
   if (rc) return rc;
@@ -614,6 +623,24 @@ extern "C" int pgld_geno_band_pairs(pgld_handle h, const pgld_geno_panel* panel,
   a.stats = stats;
   a.stat_mask = stat_mask;
   return pgld::geno::launch_geno_band<pgld::kModePairs, 1>(h, a, st);
+}
+
+extern "C" int pgld_geno_band_pairs(pgld_handle h, const pgld_geno_panel* panel, const double* pos,
+                                    double max_dist, int32_t* counts, int32_t* n_valid,
+                                    float* stats, int32_t stat_mask, int64_t n_pairs,
+                                    int32_t form, void* stream) {
+  return geno_band_pairs(h, panel, pos, max_dist, nullptr, counts, n_valid, stats, stat_mask, n_pairs,
+                         form, stream);
+}
+
+extern "C" int pgld_geno_band_pairs_at(pgld_handle h, const pgld_geno_panel* panel,
+                                       const double* pos, double max_dist, const int64_t* offsets,
+                                       int32_t* counts, int32_t* n_valid, float* stats,
+                                       int32_t stat_mask, int64_t n_pairs, int32_t form,
+                                       void* stream) {
+  PGLD_REQUIRE(h, offsets != nullptr, "pgld_geno_band_pairs_at: NULL offsets");
+  return geno_band_pairs(h, panel, pos, max_dist, offsets, counts, n_valid, stats, stat_mask, n_pairs,
+                         form, stream);
 }
 
 int pgld_geno_tc_binned(pgld_context* h, const pgld_geno_panel* panel, const pgld::BandArgs& ba,

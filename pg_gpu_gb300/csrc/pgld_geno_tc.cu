@@ -926,8 +926,8 @@ __global__ void __launch_bounds__(kThreads, 1)
 // Genotype band pairs on the tensor cores: one population, dosages 0/1/2
 // (missing allowed), no values above 2.  a carries the band and outputs.
 int pgld_geno_tc_pairs(pgld_context* h, const pgld_geno_panel* panel, const double* pos,
-                       double max_dist, int32_t* counts, int32_t* n_valid, float* stats,
-                       int32_t stat_mask, cudaStream_t st) {
+                       double max_dist, const long long* offsets, int32_t* counts, int32_t* n_valid,
+                       float* stats, int32_t stat_mask, cudaStream_t st) {
   using namespace pgld::gtc;
   int rc = pgld::tchost::get_encode(h);
   if (rc) return rc;
@@ -941,16 +941,20 @@ int pgld_geno_tc_pairs(pgld_context* h, const pgld_geno_panel* panel, const doub
   const size_t sb = pgld::scan_scratch_bytes(std::max<long long>(nb, n));
   auto al = [](size_t x) { return (x + 1023) & ~size_t(1023); };
   const size_t off_items = 0, off_scan = al((nb + 1) * 8), off_op = off_scan + al(sb),
-               off_poff = off_op + al(op_bytes), total = off_poff + al((size_t)(n + 1) * 8);
+               off_poff = off_op + al(op_bytes),
+               total = off_poff + (offsets ? 0 : al((size_t)(n + 1) * 8));
   void* ws = nullptr;
   rc = pgld_workspace(h, total, &ws);
   if (rc) return rc;
   char* w = (char*)ws;
   long long* items = (long long*)(w + off_items);
-  long long* poff = (long long*)(w + off_poff);
   unsigned char* op = (unsigned char*)(w + off_op);
-  rc = pgld_band_offsets(h, pos, n, max_dist, poff, w + off_scan, sb, st);
-  if (rc) return rc;
+  const long long* poff = offsets;
+  if (!poff) {
+    poff = (long long*)(w + off_poff);
+    rc = pgld_band_offsets(h, pos, n, max_dist, (long long*)(w + off_poff), w + off_scan, sb, st);
+    if (rc) return rc;
+  }
   {
     const unsigned blocks = (unsigned)std::max<long long>(1, (nb * kBlkRows + 7) / 8);
     pack_gtc_kernel<<<blocks, 256, 0, st>>>(panel->planes[0], W, n, nb, k_pad, (uint32_t*)op);

@@ -1,6 +1,7 @@
 // Exclusive prefix sum of int64 counts, in place, n -> n+1 entries
-// (entry n receives the total).  Three launches: tile sums, scan of the
-// tile sums in one block, then the per-tile scans.
+// (entry n receives the total).  Two launches: tile sums, then the per-tile
+// scans, each block adding up the sums of the tiles before its own (a few
+// hundred values at 10^6 entries).
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -58,25 +59,15 @@ static __global__ void __launch_bounds__(kScanThreads) scan_tile_sums(const long
   if (threadIdx.x == 0) part[blockIdx.x] = tot;
 }
 
-static __global__ void __launch_bounds__(kScanThreads) scan_partials(long long* __restrict__ part, long long m) {
-  __shared__ long long sh[kScanThreads / 32 + 1];
-  long long carry = 0;
-  for (long long b = 0; b < m; b += kScanThreads) {
-    long long k = b + threadIdx.x;
-    long long v = k < m ? part[k] : 0;
-    long long tot;
-    long long e = block_excl_scan(v, sh, &tot);
-    if (k < m) part[k] = carry + e;
-    carry += tot;
-  }
-  if (threadIdx.x == 0) part[m] = carry;
-}
-
 static __global__ void __launch_bounds__(kScanThreads) scan_apply(long long* __restrict__ a, long long n,
                                                           const long long* __restrict__ part,
                                                           long long m) {
   __shared__ long long sh[kScanThreads / 32 + 1];
   long long base = (long long)blockIdx.x * kScanTile + (long long)threadIdx.x * kScanPerThread;
+  long long before = 0;
+  for (long long k = threadIdx.x; k < (long long)blockIdx.x; k += kScanThreads) before += part[k];
+  long long first;
+  block_excl_scan(before, sh, &first);
   long long v[kScanPerThread];
   long long s = 0;
 #pragma unroll
@@ -85,13 +76,13 @@ static __global__ void __launch_bounds__(kScanThreads) scan_apply(long long* __r
     s += v[q];
   }
   long long tot;
-  long long e = block_excl_scan(s, sh, &tot) + part[blockIdx.x];
+  long long e = block_excl_scan(s, sh, &tot) + first;
 #pragma unroll
   for (int q = 0; q < kScanPerThread; ++q) {
     if (base + q < n) a[base + q] = e;
     e += v[q];
   }
-  if (blockIdx.x == 0 && threadIdx.x == 0) a[n] = part[m];
+  if (blockIdx.x == m - 1 && threadIdx.x == 0) a[n] = first + tot;
 }
 
 inline int exclusive_scan_i64(pgld_context* h, long long* a, long long n, void* scratch,
@@ -105,7 +96,6 @@ inline int exclusive_scan_i64(pgld_context* h, long long* a, long long n, void* 
     return pgld_fail(h, PGLD_ERR_INVALID_ARG, "scan scratch too small");
   long long* part = (long long*)scratch;
   scan_tile_sums<<<(unsigned)tiles, kScanThreads, 0, st>>>(a, n, part);
-  scan_partials<<<1, kScanThreads, 0, st>>>(part, tiles);
   scan_apply<<<(unsigned)tiles, kScanThreads, 0, st>>>(a, n, part, tiles);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return pgld_cuda_fail(h, e, "exclusive_scan_i64");

@@ -989,14 +989,15 @@ static int tc_launch(pgld_context* h, const pgld_hap_panel* panel, pgld::BandArg
   const size_t off_items = 0, off_scan = al((nb + 1) * 8), off_op0 = off_scan + al(sb),
                off_op1 = off_op0 + al(op_bytes[0]), off_ipos = off_op1 + al(op_bytes[1]),
                off_bad = off_ipos + al((size_t)n * 4), off_poff = off_bad + 1024,
-               total = off_poff + (mode == pgld::kModePairs ? al((size_t)(n + 1) * 8) : 0);
+               total = off_poff + (mode == pgld::kModePairs && !a.pair_off ? al((size_t)(n + 1) * 8) : 0);
   void* ws = nullptr;
   rc = pgld_workspace(h, total, &ws);
   if (rc) return rc;
   char* w = (char*)ws;
-  long long* poff = mode == pgld::kModePairs ? (long long*)(w + off_poff) : nullptr;
-  if (poff) {
-    rc = pgld_band_offsets(h, a.pos, n, a.max_dist, poff, w + off_scan, sb, st);
+  const long long* poff = a.pair_off;
+  if (mode == pgld::kModePairs && !poff) {
+    poff = (long long*)(w + off_poff);
+    rc = pgld_band_offsets(h, a.pos, n, a.max_dist, (long long*)(w + off_poff), w + off_scan, sb, st);
     if (rc) return rc;
   }
   long long* items = (long long*)(w + off_items);

@@ -1253,7 +1253,7 @@ static int wide_one_pop_launch(pgld_context* h, pgld::tcw::Params& prm, const CU
 
 // Per-pair outputs of one population (<= 2,048 haplotypes, no validity
 // plane) over the distance band: a's pair_off / counts / nvalid / stats as
-// for the square form; the band offsets are rebuilt in this call's workspace.
+// for the square form.
 int pgld_tc_wide_pairs(pgld_context* h, const pgld_hap_panel* panel, pgld::BandArgs& a,
                        cudaStream_t st) {
   using namespace pgld::tcw;
@@ -1270,16 +1270,20 @@ int pgld_tc_wide_pairs(pgld_context* h, const pgld_hap_panel* panel, pgld::BandA
   const size_t sb = pgld::scan_scratch_bytes(std::max<long long>(n_rb, n));
   auto al = [](size_t x) { return (x + 1023) & ~size_t(1023); };
   const size_t off_items = 0, off_scan = al((n_rb + 1) * 8), off_op = off_scan + al(sb),
-               off_poff = off_op + al(op_bytes), total = off_poff + al((size_t)(n + 1) * 8);
+               off_poff = off_op + al(op_bytes),
+               total = off_poff + (a.pair_off ? 0 : al((size_t)(n + 1) * 8));
   void* ws = nullptr;
   rc = pgld_workspace(h, total, &ws);
   if (rc) return rc;
   char* w = (char*)ws;
   long long* items = (long long*)(w + off_items);
   unsigned char* op = (unsigned char*)(w + off_op);
-  long long* poff = (long long*)(w + off_poff);
-  rc = pgld_band_offsets(h, a.pos, n, a.max_dist, poff, w + off_scan, sb, st);
-  if (rc) return rc;
+  const long long* poff = a.pair_off;
+  if (!poff) {
+    poff = (long long*)(w + off_poff);
+    rc = pgld_band_offsets(h, a.pos, n, a.max_dist, (long long*)(w + off_poff), w + off_scan, sb, st);
+    if (rc) return rc;
+  }
   {
     const unsigned blocks = (unsigned)((2 * n_op + 7) / 8);
     pack_wide_kernel<<<blocks, 256, 0, st>>>(panel->planes[0], W, panel->planes[0], 0, n, 2 * n_op,

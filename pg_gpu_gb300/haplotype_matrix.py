@@ -434,6 +434,20 @@ class HaplotypeMatrix:
             self._packed[key] = _ops.pack(src, rows)
         return self._packed[key]
 
+    def packed_all(self, pops, rows=None):
+        """packed() of several populations, whose flags are read back together
+        (rows: their device_rows, if the caller has them)."""
+        src = self._pinned if (self._device == "CPU" and self._pinned is not None) else None
+        if src is None:
+            self.transfer_to_gpu()
+            src = self._haplotypes
+        new = [p for p in dict.fromkeys(pops) if p not in self._packed]
+        flags = _ops.PackFlags(len(new), "cuda" if not src.is_cuda else src.device) if new else None
+        for k, p in enumerate(new):
+            r = self._pop_rows(p) if rows is None else rows[pops.index(p)]
+            self._packed[p] = _ops.pack(src, r, flags=flags, k=k)
+        return [self._packed[p] for p in pops]
+
     # ------------------------------------------------------------ LD methods
     def tally_gpu_haplotypes(self, pop=None):
         """All-pairs [n11,n10,n01,n00] and n_valid or None (haplotype_matrix.py:1320-1434).
@@ -462,9 +476,9 @@ class HaplotypeMatrix:
         bins = np.asarray(bp_bins, dtype=np.float64)
         if ac_filter:
             return self._binned_biallelic(bins, pops)
-        packs = [self.packed(p) for p in pops]
+        packs = self.packed_all(pops)
         sums, cnt = _ops.binned_sums(packs, _ops.positions_f64(self._positions), bins)
-        return bins, sums.cpu().numpy(), cnt.cpu().numpy()
+        return (bins, *_ops.host_sums(sums, cnt))
 
     def _binned_biallelic(self, bins, pops):
         """_binned of apply_biallelic_filter(): the sites are chosen and the
@@ -477,10 +491,14 @@ class HaplotypeMatrix:
         kept = _ops.kept_sites(_ops.KEEP_BIALLELIC, _ops.site_counts(src, sums=False, flags=True))
         if kept[1].numel() == 0:
             raise ValueError("genotypes cannot be empty")
-        packs = [_ops.pack(src, self._pop_rows(p), kept) for p in pops]
+        rows = [self._pop_rows(p) for p in pops]
+        if None not in rows:
+            rows = _ops.device_rows(rows, src.shape[0])
+        flags = _ops.PackFlags(len(pops), kept[1].device)
+        packs = [_ops.pack(src, r, kept, flags, k) for k, r in enumerate(rows)]
         pos = _ops.positions_f64(self._positions).index_select(0, kept[1])
         sums, cnt = _ops.binned_sums(packs, pos, bins)
-        return bins, sums.cpu().numpy(), cnt.cpu().numpy()
+        return (bins, *_ops.host_sums(sums, cnt))
 
     def compute_ld_statistics_gpu_single_pop(self, bp_bins, raw=False, ac_filter=True,
                                              chunk_size="auto"):

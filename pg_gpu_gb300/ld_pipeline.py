@@ -6,6 +6,8 @@ torch tensors, CuPy arrays (``__cuda_array_interface__``) or NumPy arrays.
 """
 from __future__ import annotations
 
+import functools
+
 import numpy as np
 
 from . import _lib as L
@@ -131,8 +133,7 @@ def compute_two_pop_statistics_batch(counts_pop1, counts_pop2, n_valid1, n_valid
     """
     c1, c2 = _pc(counts_pop1), _pc(counts_pop2)
     n1, n2 = _nv(n_valid1), _nv(n_valid2)
-    terms = spec_terms(2)
-    return _ops.stats([c1, c2], [n1, n2], terms, 15)
+    return _ops.stats([c1, c2], [n1, n2], _table_terms(2), 15)
 
 
 def compute_single_pop_statistics_batch(counts, n_valid, ld_statistics=None):
@@ -267,6 +268,12 @@ def specs_to_terms(stat_specs):
 
 def spec_terms(num_pops):
     return specs_to_terms(generate_stat_specs(num_pops))
+
+
+@functools.lru_cache(maxsize=None)
+def _table_terms(num_pops):
+    """spec_terms as the library's term array."""
+    return _ops.make_terms(spec_terms(num_pops))
 
 
 class PopData:

@@ -103,10 +103,10 @@ def compute_ld_statistics(vcf_file=None, rec_map_file=None, pop_file=None, pops=
             print(f"  {sum(len(r) for r in mat.sample_sets.values())} hap, "
                   f"{mat.num_variants:,} variants")
 
-    pos_np = (mat.positions if isinstance(mat, PackedVcf) else mat._pos_np()).astype(np.float64)
     if r_bins is not None:
         if rec_map_file is None:
             raise ValueError("rec_map_file required with r_bins")
+        pos_np = (mat.positions if isinstance(mat, PackedVcf) else mat._pos_np()).astype(np.float64)
         bins = np.asarray(r_bins, dtype=np.float64)
         gen = _interpolate_genetic_distances(pos_np, rec_map_file)
         max_bp = _max_bp_for_r_dist(pos_np, gen, float(bins[-1]))
@@ -117,8 +117,15 @@ def compute_ld_statistics(vcf_file=None, rec_map_file=None, pop_file=None, pops=
     n_bins = len(bins) - 1
     if report:
         print(f"  Computing LD ({n_bins} bins, {num_pops} pops) ...")
-    ld_sums = _compute_ld_sums(mat, pops, bins, gen, max_bp, use_genotypes)
-    het = _compute_heterozygosity(mat, pops, use_genotypes)
+    rows = None
+    if not isinstance(mat, PackedVcf):
+        if use_genotypes:
+            lists, n = [mat.sample_sets[p] for p in pops], mat.genotypes.shape[0]
+        else:
+            lists, n = [mat._pop_rows(p) for p in pops], mat.haplotypes.shape[0]
+        rows = _ops.device_rows(lists, n)
+    ld_sums = _compute_ld_sums(mat, pops, bins, gen, max_bp, use_genotypes, rows)
+    het = _compute_heterozygosity(mat, pops, use_genotypes, rows)
     if report:
         print("  Done.")
     bin_tuples = [(float(bins[i]), float(bins[i + 1])) for i in range(n_bins)]
@@ -158,8 +165,9 @@ def _max_bp_for_r_dist(positions, gen_dists, max_r):
     return min(max_r / min_rate * 1.1, chrom_len)
 
 
-def _compute_ld_sums(mat, pops, bins, gen_dists, max_bp, use_genotypes=False):
-    """(n_bins, n_stats) float64 numpy sums (moments_ld.py:248-343)."""
+def _compute_ld_sums(mat, pops, bins, gen_dists, max_bp, use_genotypes=False, pop_rows=None):
+    """(n_bins, n_stats) float64 numpy sums (moments_ld.py:248-343); pop_rows: the
+    populations' device_rows, if the caller has them."""
     if use_genotypes:
         # variants polymorphic across the union of the populations (moments_ld.py:256-280)
         g = L.as_device(mat.genotypes, np.int8)
@@ -168,17 +176,18 @@ def _compute_ld_sums(mat, pops, bins, gen_dists, max_bp, use_genotypes=False):
         pos_d = L.as_device(mat.positions, np.float64).index_select(0, kept[1])
         bc = (None if gen_dists is None else
               L.as_device(gen_dists, np.float64).index_select(0, kept[1]))
-        packs = [_ops.pack_geno(g, mat.sample_sets[p], kept) for p in pops]
+        packs = _ops.pack_geno_all(g, pop_rows or [mat.sample_sets[p] for p in pops], kept)
         sums, _ = _ops.geno_binned_sums(packs, pos_d, bins, max_dist=max_bp, bin_coord=bc)
     else:
         pos_d = L.as_device(mat.positions, np.float64)
         bc = None if gen_dists is None else L.as_device(gen_dists, np.float64)
-        packs = [mat.packs[p] if isinstance(mat, PackedVcf) else mat.packed(p) for p in pops]
+        packs = ([mat.packs[p] for p in pops] if isinstance(mat, PackedVcf)
+                 else mat.packed_all(pops, pop_rows))
         sums, _ = _ops.binned_sums(packs, pos_d, bins, max_dist=max_bp, bin_coord=bc)
     return sums.cpu().numpy()
 
 
-def _compute_heterozygosity(mat, pops, use_genotypes=False):
+def _compute_heterozygosity(mat, pops, use_genotypes=False, pop_rows=None):
     """H_i_j of the moments convention (moments_ld.py:346-388)."""
     import torch
     names = _het_names(len(pops))
@@ -187,7 +196,8 @@ def _compute_heterozygosity(mat, pops, use_genotypes=False):
         counts = [(mat.alt_counts(p).to(torch.int32), None) for p in pops]
     else:
         x = L.as_device(mat.genotypes if use_genotypes else mat.haplotypes, np.int8)
-        counts = [_ops.site_counts(x, mat.sample_sets[p])[:2] for p in pops]
+        counts = [_ops.site_counts(x, r)[:2]
+                  for r in pop_rows or [mat.sample_sets[p] for p in pops]]
     # every haplotype counts; of the genotypes the called ones
     h = _ops.heterozygosity([c[0] for c in counts],
                             [c[1] if use_genotypes else None for c in counts],
