@@ -10,8 +10,9 @@
 //   d31(i,j)     n_i(n_i-1)(n_i-2) n_j     Dz_iij, pi2_iiij
 //   d211(s,a,b)  n_s(n_s-1) n_a n_b        Dz_sab, pi2_ssab, pi2_sasb
 //   d1111        n_0 n_1 n_2 n_3           the three pi2 of four populations
-// so a pair takes one reciprocal per class (15 for three populations, 35 for
-// four) instead of one division per term (63 and 315 terms).
+// so a pair takes one reciprocal per class, two where haplotype denominators of
+// one class round apart (21 for three populations, 53 for four) instead of one
+// division per term (63 and 315 terms).
 //
 // Features per population are exact float32 integers, or one rounding of an
 // exact integer, for sample sizes up to kMaxN.  Products of draws from one
@@ -22,8 +23,8 @@
 // each, where the expanded polynomials needed 64-bit integers.
 //
 // A quotient is num * (r + rl): r the approximate reciprocal of the
-// denominator den (one float32 rounding of the exact integer: a product of
-// two exact factors below 2^24), rl = r (1 - den r) its correction, added
+// denominator den (the exact integer in float32: a product of two exact
+// factors below 2^24, rounded as round_den says), rl = r (1 - den r) its correction, added
 // before the product rounds.  So a quotient carries no bias that repeats over
 // the pairs of equal sample size, as a rounded reciprocal would: sums over
 // 10^8 pairs keep an error near 1e-9.
@@ -50,16 +51,36 @@ __host__ __device__ constexpr int group_size(int P, int g) {
 struct Den {
   float r, rl;
 };
-// den: the rounded denominator; 0 (too few samples) gives quotient 0
+// a b, exact factors below 2^23 (haplotype denominators): the float32 of M a b
+// over M, as the two 32-bit conversions of the 64-bit product round it -- its
+// bits from 2^31 on, plus the rounded rest.  M is the factor that the term
+// table's denominator carries (1, 2 or 4).  From n = 152 on this is not always
+// the nearest float32 of a b; where one sample size is frequent (n = 390, 4%
+// missing) the difference would shift a bin's sum by 1e-8 of a statistic.
+template <int M>
+PGLD_HD float round_den(float a, float b) {
+  constexpr float G = 1.5f * 18014398509481984.0f / M;  // ulp 2^31 / M
+#ifdef __CUDA_ARCH__
+  const float s = __fmaf_rd(a, b, G);
+#else
+  constexpr double U = 2147483648.0 / M;
+  const double fl = (double)(long long)((double)a * b / U) * U;
+  const float s = (float)(G + fl);
+#endif
+  const float low = fmaf(a, b, G - s);
+  return (s - G) + low;
+}
+// den: the rounded denominator.  Where it is 0 (fewer samples than draws) the
+// numerators count no draws and are exactly 0, so any other value will do
 PGLD_HD Den make_den(float den) {
   Den d;
+  den = fmaxf(den, 1.0f);
 #ifdef __CUDA_ARCH__
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(d.r) : "f"(den));
 #else
   d.r = 1.0f / den;
 #endif
   d.rl = d.r * fmaf(-den, d.r, 1.0f);
-  if (!(den > 0.0f)) d.r = d.rl = 0.0f;
   return d;
 }
 PGLD_HD float quot(float num, Den d) { return fmaf(num, d.r, fast::fmul(num, d.rl)); }
@@ -74,6 +95,18 @@ PGLD_HD Size make_size(float n) {
   s.k = n - 2.0f;
   s.m2b = s.k * (n - 3.0f);
   return s;
+}
+
+// A statistic that averages quotients of two kinds adds them term by term, in
+// the table's order (a, a, b, b or a, a, a, a, b, b, b, b; the factor of the
+// first is left out here: two_two is (a + a + b + b) / 2, four_four a
+// quarter).  At small sample sizes every numerator is an exact float32, the
+// same few quotients recur in all pairs, and their roundings do not average
+// out: the sum of the terms and the quotient of the summed numerators differ
+// by up to 2e-9 of a bin of 10^8 pairs.
+PGLD_HD float two_two(float a, float b) { return fmaf(b, 0.5f, fmaf(b, 0.5f, a)); }
+PGLD_HD float four_four(float a, float b) {
+  return fmaf(b, 0.25f, fmaf(b, 0.25f, fmaf(b, 0.25f, fmaf(b, 0.25f, a))));
 }
 
 // ---- haplotypes ------------------------------------------------------------
@@ -114,8 +147,9 @@ PGLD_HD float ijij(const Hap& i, const Hap& j) {
   return fmaf(i.X1, j.X4, fmaf(i.X2, j.X3, fmaf(i.X3, j.X2, fast::fmul(i.X4, j.X1))));
 }
 PGLD_HD float dz31(const Hap& t, const Hap& s) { return t.x * (t.dA * s.dB + t.dB * s.dA); }
-PGLD_HD float triple(const Hap& t, const Hap& s) {
-  return fmaf(s.pB, t.T1, fast::fmul(s.qB, t.T2));
+// the four terms of pi2_ttts are equal
+PGLD_HD float triple(const Hap& t, const Hap& s, Den d, bool) {
+  return quot(fmaf(s.pB, t.T1, fast::fmul(s.qB, t.T2)), d);
 }
 PGLD_HD float dz211(const Hap& s, const Hap& a, const Hap& b) {
   return s.x * (a.dA * b.dB + b.dA * a.dB);
@@ -206,8 +240,11 @@ PGLD_HD float dz31(const Geno& t, const Geno& s) {
                              fast::fadd(pe, qe));
   return fast::fsub(fmaf(t.y, t.m3 * s.m1 + t.m1 * s.m3, -h), l);
 }
-PGLD_HD float triple(const Geno& t, const Geno& s) {
-  return fmaf(t.TA1, s.S2, fast::fmul(t.TA2, s.Q2)) + fmaf(t.TB1, s.R2, fast::fmul(t.TB2, s.P2));
+// t twice at the first SNP, and twice at the second
+PGLD_HD float triple(const Geno& t, const Geno& s, Den d, bool first) {
+  const float a = quot(fmaf(t.TA1, s.S2, fast::fmul(t.TA2, s.Q2)), d);
+  const float b = quot(fmaf(t.TB1, s.R2, fast::fmul(t.TB2, s.P2)), d);
+  return first ? two_two(a, b) : two_two(b, a);
 }
 PGLD_HD float dz211(const Geno& s, const Geno& a, const Geno& b) {
   return s.y * (a.m3 * b.m1 + b.m3 * a.m1);
@@ -217,6 +254,12 @@ PGLD_HD float mixB(const Geno& a, const Geno& b) { return a.z.n * b.z.n - a.m1 *
 PGLD_HD float shared(const Geno& s, const Geno& a, const Geno& b) {
   return fmaf(a.R2, fmaf(s.X1, b.S2, fast::fmul(s.X2, b.Q2)),
               fast::fmul(a.P2, fmaf(s.X3, b.S2, fast::fmul(s.X4, b.Q2))));
+}
+
+// denominator M a b of a class
+template <class F, int M>
+PGLD_HD Den class_den(float a, float b) {
+  return make_den(F::geno ? a * b : round_den<M>(a, b));
 }
 
 // D of one population (x of the haplotype, y of the genotype features)
@@ -232,7 +275,7 @@ PGLD_HD void eval(const F (&f)[P], Sink&& sink) {
   if (G0) {
 #pragma unroll
     for (int i = 0; i < P; ++i) {
-      const Den d = make_den(f[i].z.m2 * f[i].z.m2b);
+      const Den d = class_den<F, 1>(f[i].z.m2, f[i].z.m2b);
       sink(k++, quot(f[i].dd, d));
       sink(k++, quot(f[i].dz, d));
       sink(k++, quot(f[i].pi, d));
@@ -241,21 +284,22 @@ PGLD_HD void eval(const F (&f)[P], Sink&& sink) {
     for (int i = 0; i < P; ++i)
 #pragma unroll
       for (int j = i + 1; j < P; ++j) {
-        const Den d = make_den(f[i].z.m2 * f[j].z.m2);
+        const Den d = class_den<F, 1>(f[i].z.m2, f[j].z.m2);
+        const Den d4 = class_den<F, 4>(f[i].z.m2, f[j].z.m2);
         sink(k++, quot(dval(f[i]) * dval(f[j]), d));
         sink(k++, quot(dval(f[i]) * f[j].w, d));
         sink(k++, quot(dval(f[j]) * f[i].w, d));
-        sink(k++, quot(fmaf(f[i].hA, f[j].hB, fast::fmul(f[j].hA, f[i].hB)), d));
-        sink(k++, quot(ijij(f[i], f[j]), d));
+        sink(k++, quot(fast::fmul(f[i].hA, f[j].hB), d) + quot(fast::fmul(f[j].hA, f[i].hB), d));
+        sink(k++, quot(ijij(f[i], f[j]), d4));
       }
 #pragma unroll
     for (int i = 0; i < P; ++i)
 #pragma unroll
       for (int j = 0; j < P; ++j)
         if (j != i) {
-          const Den d = make_den(f[i].z.m2 * (f[i].z.k * f[j].z.n));
+          const Den d = class_den<F, 2>(f[i].z.m2, f[i].z.k * f[j].z.n);
           sink(k++, quot(dz31(f[i], f[j]), d));
-          sink(k++, quot(triple(f[i], f[j]), d));
+          sink(k++, triple(f[i], f[j], d, i < j));
         }
   }
   if (G1) {
@@ -266,18 +310,23 @@ PGLD_HD void eval(const F (&f)[P], Sink&& sink) {
 #pragma unroll
         for (int b = a + 1; b < P; ++b)
           if (a != s && b != s) {
-            const Den d = make_den(f[s].z.m2 * (f[a].z.n * f[b].z.n));
+            const Den d = class_den<F, 2>(f[s].z.m2, f[a].z.n * f[b].z.n);
+            const Den d4 = class_den<F, 4>(f[s].z.m2, f[a].z.n * f[b].z.n);
             sink(k++, quot(dz211(f[s], f[a], f[b]), d));
-            sink(k++, quot(fmaf(f[s].hA, mixB(f[a], f[b]), fast::fmul(f[s].hB, mixA(f[a], f[b]))), d));
-            sink(k++, quot(shared(f[s], f[a], f[b]) + shared(f[s], f[b], f[a]), d));
+            // the table lists the pair with the smaller population first
+            const float sA = quot(fast::fmul(f[s].hA, mixB(f[a], f[b])), d);
+            const float sB = quot(fast::fmul(f[s].hB, mixA(f[a], f[b])), d);
+            sink(k++, s < a ? two_two(sA, sB) : two_two(sB, sA));
+            sink(k++, four_four(quot(shared(f[s], f[a], f[b]), d4), quot(shared(f[s], f[b], f[a]), d4)));
           }
     if (P == 4) {
-      const Den d = make_den((f[0].z.n * f[1].z.n) * (f[P - 2].z.n * f[P - 1].z.n));
+      const Den d = class_den<F, 4>(f[0].z.n * f[1].z.n, f[P - 2].z.n * f[P - 1].z.n);
 #pragma unroll
       for (int b = 1; b < 4; ++b) {
         const int c = b == 1 ? 2 : 1, e = b == 3 ? 2 : 3;  // the other two
         const F &f0 = f[0], &f1 = f[b % P], &f2 = f[c % P], &f3 = f[e % P];
-        sink(k++, quot(fmaf(mixA(f0, f1), mixB(f2, f3), fast::fmul(mixA(f2, f3), mixB(f0, f1))), d));
+        sink(k++, four_four(quot(fast::fmul(mixA(f0, f1), mixB(f2, f3)), d),
+                            quot(fast::fmul(mixA(f2, f3), mixB(f0, f1)), d)));
       }
     }
   }

@@ -38,3 +38,16 @@ extern "C" void pgld_check_multi(const int* counts, int N, int P, int geno, floa
   if (P == 3) rows<3>(counts, N, geno != 0, out, S);
   if (P == 4) rows<4>(counts, N, geno != 0, out, S);
 }
+
+// float32 denominators M a b / M (M = 1, 2, 4) and the two conversions' of M a b
+extern "C" void pgld_check_den(const float* a, const float* b, int N, float* out) {
+  for (int k = 0; k < N; ++k, out += 6) {
+    out[0] = multi::round_den<1>(a[k], b[k]);
+    out[1] = multi::round_den<2>(a[k], b[k]);
+    out[2] = multi::round_den<4>(a[k], b[k]);
+    for (int m = 0; m < 3; ++m) {
+      const long long x = ((long long)a[k] * (long long)b[k]) << m;
+      out[3 + m] = fmaf((float)(int)(x >> 31), 2147483648.0f, (float)(int)(x & 0x7fffffff)) / (1 << m);
+    }
+  }
+}

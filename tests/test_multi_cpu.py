@@ -30,6 +30,7 @@ def check_lib(tmp_path_factory):
     L = ctypes.CDLL(so)
     L.pgld_check_multi.argtypes = [ctypes.c_void_p, ctypes.c_int, ctypes.c_int, ctypes.c_int,
                                    ctypes.c_void_p, ctypes.c_int]
+    L.pgld_check_den.argtypes = [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int, ctypes.c_void_p]
     return L
 
 
@@ -53,3 +54,25 @@ def test_multi_population_statistics_match_oracle(check_lib, P, geno, nmax):
     err = np.abs(out - ref)
     bad = np.argwhere(err > tol)
     assert len(bad) == 0, [(O.ld_names(P)[s], ref[k, s], out[k, s]) for k, s in bad[:5]]
+
+
+def test_denominators_round_as_the_two_conversions(check_lib):
+    n = np.arange(0, 2049, dtype=np.float64)
+    rng = np.random.default_rng(5)
+    i, j, k = (rng.choice(n, 200_000) for _ in range(3))
+    a = np.concatenate([i * (i - 1), n * (n - 1)]).astype(np.float32)
+    b = np.concatenate([j * k, np.maximum(n - 2, 0) * np.maximum(n - 3, 0)]).astype(np.float32)
+    out = np.empty((len(a), 6), np.float32)
+    check_lib.pgld_check_den(a.ctypes.data, b.ctypes.data, len(a), out.ctypes.data)
+    np.testing.assert_array_equal(out[:, :3], out[:, 3:])
+
+
+@pytest.mark.parametrize("P", [3, 4])
+def test_too_few_haplotypes_give_zero(check_lib, P):
+    rng = np.random.default_rng(P)
+    c = np.stack([rng.multinomial(n, np.full(4, 0.25)) for n in rng.integers(0, 5, 4000 * P)])
+    c = c.reshape(-1, P, 4).astype(np.int32)
+    ref = O.multi_pop_stats([c[:, p] for p in range(P)], [None] * P)
+    out = np.full(ref.shape, np.nan, np.float32)
+    check_lib.pgld_check_multi(c.ctypes.data, len(c), P, 0, out.ctypes.data, ref.shape[1])
+    np.testing.assert_allclose(out, np.nan_to_num(ref, nan=0.0), rtol=1e-6, atol=0)
