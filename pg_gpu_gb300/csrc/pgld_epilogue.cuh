@@ -76,6 +76,15 @@ PGLD_HD int f2i_small(float f) {
 #endif
 }
 
+// two float32 integers in [-2^15, 2^15) as the int16 halves of a word
+PGLD_HD uint32_t f2i_pair(float lo, float hi) {
+#ifdef __CUDA_ARCH__
+  return __byte_perm(__float_as_uint(lo + 12582912.0f), __float_as_uint(hi + 12582912.0f), 0x5410);
+#else
+  return (uint32_t)(uint16_t)(int16_t)lo | (uint32_t)(uint16_t)(int16_t)hi << 16;
+#endif
+}
+
 // an integer held exactly as s + e
 struct X2 {
   float s, e;

@@ -87,9 +87,9 @@ PGLD_GM_HD void to_counts(const Mom& o, int* c) {
   }
 #pragma unroll
   for (int a = 0; a < 3; ++a) {
-    c[3 * a + 0] = (q[a][2] - q[a][1]) / 4;
-    c[3 * a + 1] = (2 * (q[a][0] - q[a][2])) / 4;
-    c[3 * a + 2] = (q[a][2] + q[a][1]) / 4;
+    c[3 * a + 0] = (q[a][2] - q[a][1]) >> 2;
+    c[3 * a + 1] = (q[a][0] - q[a][2]) >> 1;
+    c[3 * a + 2] = (q[a][2] + q[a][1]) >> 2;
   }
 }
 

@@ -80,7 +80,15 @@ struct Params {
   int stat_mask;
   int32_t* status;
   int stages;
+  int groups;  // epilogue groups of four warps (2-4)
 };
+
+constexpr int kMaxGroups = 4;
+constexpr int kPairThreads = (4 + 4 * kMaxGroups) * 32;
+constexpr int kMomWords = kCntPitch / 2;     // words (two int16 moments) per row of a moment block
+constexpr int kMomBytes = 96 * kMomWords * 4;
+constexpr int kCtrlBytes = 512;             // the control block, 16-byte aligned end
+constexpr int kCountStage = (9 * 32 + 4) * 4;  // bytes of a warp's staged counts, any alignment
 
 constexpr int kChunkItems = 16;  // consecutive tiles a CTA takes per turn (resident form)
 
@@ -88,8 +96,11 @@ constexpr int kChunkItems = 16;  // consecutive tiles a CTA takes per turn (resi
 // B barriers and the per-stage tile flags the producer hands the MMA issuer
 struct GCtrl : Ctrl {
   uint64_t bfull, bempty;
+  uint64_t gfull[kMaxGroups], gempty[kMaxGroups];  // the pairs kernel's accumulator stages
   int meta[8];  // first stage of a tile: bit 0 = first tile of a strip, bit 1 = last
 };
+
+static_assert(sizeof(GCtrl) <= kCtrlBytes, "control block");
 
 // the t-th tile of this CTA: turns of `chunk` consecutive items, round robin
 // over the CTAs (chunk 1: item blockIdx.x + t * gridDim.x)
@@ -114,15 +125,43 @@ __device__ __forceinline__ long long advance_block(const long long* item_off, lo
   return lo;
 }
 
+// The nine counts of the warp's pairs first + lane (lanes lo <= lane < hi) to
+// counts[][9].  The lanes' values lie 36 bytes apart: stored one by one, each of
+// nine stores would touch every sector of the row.  They pass through the
+// warp's staging words, placed as the row lies to a 16-byte boundary, and leave
+// as 16-byte stores, the ends of the row word by word.
+__device__ __forceinline__ void store_counts(int32_t* counts, long long first, int lo, int hi,
+                                             int lane, uint32_t* stage, const int (&c)[9]) {
+  int32_t* row = counts + first * 9;
+  const int a0 = (int)((reinterpret_cast<uintptr_t>(row) >> 2) & 3);
+  __syncwarp();  // the previous row has left the staging words
+#pragma unroll
+  for (int x = 0; x < 9; ++x) stage[a0 + 9 * lane + x] = (uint32_t)c[x];
+  __syncwarp();
+  if (lo >= hi) return;
+  const int w0 = a0 + 9 * lo, w1 = a0 + 9 * hi;  // the row's words of the stage
+  row -= a0;
+#pragma unroll
+  for (int q = 0; q < 3; ++q) {
+    const int s = 4 * (lane + 32 * q);
+    if (s >= w0 && s + 4 <= w1)
+      __stcs(reinterpret_cast<int4*>(row + s), *reinterpret_cast<const int4*>(stage + s));
+  }
+  // the words of the first and last quarters that are not whole
+  const int f = w0 & ~3, l = w1 & ~3;
+  const int s = lane < 4 ? f + lane : l + lane - 4;
+  const bool part = lane < 4 ? f < w0 || f + 4 > w1 : lane < 8 && l < w1 && l != f;
+  if (part && s >= w0 && s < w1) __stcs(row + s, (int)stage[s]);
+}
+
 // MASK: the statistic columns when fixed at compile time (-1: a.stat_mask).
+// A (M = 128 with 32 zero rows) is the column block j, B (N = 96) the row block
+// i: accumulator lanes are planes of the SNPs j, columns planes of the SNPs i.
 // RES: the resident form -- the row block's 96 operand rows (every K chunk)
-// stay in shared memory as the B operand (N = 96) for a strip of consecutive
-// tiles of that row block, and only the column block streams (A, M = 128 with
-// 32 zero rows); the accumulator is then transposed (lanes: planes of the
-// SNPs j, columns: planes of the SNPs i).  Otherwise both blocks stream per
-// K chunk (A = row block, B = column block).
+// stay in shared memory for a strip of consecutive tiles of that row block, and
+// only the column block streams.  Otherwise both blocks stream per K chunk.
 template <int MASK, bool RES>
-__global__ void __launch_bounds__(kThreads, 1)
+__global__ void __launch_bounds__(kPairThreads, 1)
     gtc_pairs_kernel(const __grid_constant__ CUtensorMap map, Params a) {
   extern __shared__ unsigned char smem_dyn[];
   unsigned char* base = smem_dyn + ((1024 - (smem_u32(smem_dyn) & 1023)) & 1023);
@@ -132,7 +171,10 @@ __global__ void __launch_bounds__(kThreads, 1)
   unsigned char* ring = base;
   unsigned char* bres = ring + (size_t)stages * kStage;  // resident B (RES only)
   GCtrl* ctrl = reinterpret_cast<GCtrl*>(bres + (RES ? (size_t)a.kchunks * kBBytes : 0));
-  int16_t* cnt = reinterpret_cast<int16_t*>(ctrl + 1);  // [2][96][kCntPitch]
+  unsigned char* moms = reinterpret_cast<unsigned char*>(ctrl) + kCtrlBytes;  // [groups][96][kMomWords]
+  const int groups = a.groups;
+  unsigned char* stage_c = moms + (size_t)groups * kMomBytes;  // [4 * groups][kCountStage]
+  const uint32_t tmem_cols = groups > 2 ? 512u : kTmemCols;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   volatile int* abort_flag = &ctrl->abort_flag;
 
@@ -141,9 +183,9 @@ __global__ void __launch_bounds__(kThreads, 1)
       mbar_init(&ctrl->full[s], 1);
       mbar_init(&ctrl->empty[s], 1);
     }
-    for (int s = 0; s < 2; ++s) {
-      mbar_init(&ctrl->tfull[s], 1);
-      mbar_init(&ctrl->tempty[s], kEpiWarps / 2);  // the four warps of epilogue group s
+    for (int s = 0; s < groups; ++s) {
+      mbar_init(&ctrl->gfull[s], 1);
+      mbar_init(&ctrl->gempty[s], 4);  // the four warps of epilogue group s
     }
     mbar_init(&ctrl->drain, 1);
     mbar_init(&ctrl->bfull, 1);
@@ -155,7 +197,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   if (warp == 1) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
                      smem_u32(&ctrl->tmem_base)),
-                 "r"(kTmemCols)
+                 "r"(tmem_cols)
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
@@ -221,9 +263,9 @@ __global__ void __launch_bounds__(kThreads, 1)
             tma_load_2d(sa, &map, &ctrl->full[stage], kc * kKChunk, (int)(jb * kBlkRows));
           } else {
             mbar_expect_tx(&ctrl->full[stage], 2 * kBBytes);
-            tma_load_2d(sa, &map, &ctrl->full[stage], kc * kKChunk, (int)(lo * kBlkRows));
+            tma_load_2d(sa, &map, &ctrl->full[stage], kc * kKChunk, (int)(jb * kBlkRows));
             tma_load_2d(sa + kABytes, &map, &ctrl->full[stage], kc * kKChunk,
-                        (int)(jb * kBlkRows));
+                        (int)(lo * kBlkRows));
           }
           ++issued;
           if (++stage == stages) {
@@ -258,11 +300,15 @@ __global__ void __launch_bounds__(kThreads, 1)
       uint32_t phase = 0;
       int consumed = 0, strips = 0;
       bool any = false;
+      int acc = -1;
+      uint32_t aph = 1;
       for (int t = 0; !*abort_flag; ++t) {
         if (tile_item(t, chunk) >= n_items) break;
-        const int acc = t & 1;
-        const uint32_t aph = (uint32_t)((t >> 1) & 1);
-        if (!mbar_wait_role(&ctrl->tempty[acc], aph ^ 1, abort_flag)) {
+        if (++acc == groups || t == 0) {
+          acc = 0;
+          aph ^= 1;
+        }
+        if (!mbar_wait_role(&ctrl->gempty[acc], aph ^ 1, abort_flag)) {
           set_abort(ctrl, a.status, 4003);
           break;
         }
@@ -304,7 +350,7 @@ __global__ void __launch_bounds__(kThreads, 1)
           }
         }
         if (!ok) break;
-        mma_commit(&ctrl->tfull[acc]);
+        mma_commit(&ctrl->gfull[acc]);
         if (RES && last) mma_commit(&ctrl->bempty);  // the strip's MMAs are all issued
       }
       if (*abort_flag && any) {
@@ -314,17 +360,19 @@ __global__ void __launch_bounds__(kThreads, 1)
     }
   } else if (warp >= 4) {
     // ---------------- epilogue ----------------
-    // Two groups of four warps take alternate tiles (group g: tiles g, g + 2,
+    // Groups of four warps take the tiles in turn (group g: tiles g, g + groups,
     // ... of this CTA, accumulator stage g, moment buffer g), so one group's
-    // copy and the other's statistics overlap.  Within a group the warp of
-    // TMEM lane quarter q < 3 copies plane q's 96 moment columns, and all four
-    // warps turn the 1,024 pairs into outputs (8 per thread).
+    // copy and the others' statistics overlap.  Within a group the warp of
+    // TMEM lane quarter q < 3 copies plane q's 96 moment columns, two int16
+    // moments (rows i, i + 1) to a word, and all four warps turn the 1,024
+    // pairs into outputs (8 per thread).
     const int e = warp - 4;
     const int grp = e >> 2;
-    const int wq = warp & 3;  // TMEM lanes 32q..32q+31: plane q of the SNPs i (j if RES)
+    const int wq = warp & 3;  // TMEM lanes 32q..32q+31: plane q of the SNPs j
     const uint32_t lane_base = (uint32_t)(wq * 32) << 16;
     const uint32_t bar_id = 1u + (uint32_t)grp;
-    int16_t* buf = cnt + grp * 96 * kCntPitch;
+    uint32_t* buf = reinterpret_cast<uint32_t*>(moms + (size_t)grp * kMomBytes);
+    uint32_t* cstage = reinterpret_cast<uint32_t*>(stage_c + (size_t)e * kCountStage);
     int t = grp;
     long long item = tile_item(t, chunk);
 
@@ -361,7 +409,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 
     for (int u = 0; item < n_items; ++u) {
       bool ready = true;
-      if (lane == 0) ready = mbar_wait(&ctrl->tfull[grp], (uint32_t)(u & 1), abort_flag);
+      if (lane == 0) ready = mbar_wait(&ctrl->gfull[grp], (uint32_t)(u & 1), abort_flag);
       ready = __shfl_sync(0xffffffffu, ready ? 1 : 0, 0) != 0;
       if (!ready && lane == 0) set_abort(ctrl, a.status, 4005);
       // the group meets before overwriting its buffer (every warp is done
@@ -379,7 +427,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       if (any_abort) break;
       tc_fence_after();
       if (wq < 3) {
-        int16_t* row = buf + (wq * 32 + lane) * kCntPitch;
+        uint32_t* row = buf + (wq * 32 + lane) * kMomWords;
 #pragma unroll 1
         for (int h = 0; h < 2; ++h) {
           uint32_t r[3][16];
@@ -390,57 +438,59 @@ __global__ void __launch_bounds__(kThreads, 1)
 #pragma unroll
           for (int c = 0; c < 3; ++c)
 #pragma unroll
-            for (int v = 0; v < 16; ++v)
-              row[48 * h + 16 * c + v] = (int16_t)fast::f2i_small(__uint_as_float(r[c][v]));
+            for (int v = 0; v < 8; ++v)
+              row[24 * h + 8 * c + v] =
+                  fast::f2i_pair(__uint_as_float(r[c][2 * v]), __uint_as_float(r[c][2 * v + 1]));
         }
       }
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(&ctrl->tempty[grp]);
+      if (lane == 0) mbar_arrive(&ctrl->gempty[grp]);
       asm volatile("bar.sync %0, 128;" ::"r"(bar_id) : "memory");
 
       const bool want_nv = a.nvalid != nullptr;
       // this tile's location; the next tile's offsets load during the pairs
       const long long ti0 = i0, tj0 = j0, toff = off_lo;
       const int tn = off_n;
-      t += 2;
+      t += groups;
       const long long next = tile_item(t, chunk);
       if (next < n_items) nv = lo + 1 + lane <= a.n_blocks ? a.item_off[lo + 1 + lane] : LLONG_MAX;
 
-      // eight pairs per thread; every value is computed and only the stores
-      // depend on the pair lying in the band.  The outputs go out as
-      // streaming global stores (st.global.cs): they are not re-read, and
-      // being global-space they cannot alias the shared-memory moments, so
-      // the loads of later pairs may move ahead of earlier pairs' stores.
+      // eight pairs per thread, two rows at a time; every value is computed and
+      // only the stores depend on the pair lying in the band.  The outputs go
+      // out as streaming global stores (st.global.cs): they are not re-read,
+      // and being global-space they cannot alias the shared-memory moments.
 #pragma unroll
-      for (int k = 0; k < 8; ++k) {
-        const int il = wq + 4 * k, jl = lane;
-        const long long row_off = __shfl_sync(0xffffffffu, toff, il);
-        const int row_n = __shfl_sync(0xffffffffu, tn, il);
-        const int d = (int)(tj0 - ti0) + jl - il - 1;  // j - i - 1
-        // d < row_n keeps j inside the band and below n_snp
-        const bool ok = d >= 0 && d < row_n;
-        gmom::Mom mo;
+      for (int k = 0; k < 4; ++k) {
+        const uint32_t* w0 = buf + lane * kMomWords + wq + 4 * k;
+        uint32_t w[9];
 #pragma unroll
         for (int x = 0; x < 3; ++x)
 #pragma unroll
-          for (int y = 0; y < 3; ++y)
-            mo.m[3 * x + y] = RES ? buf[(y * 32 + jl) * kCntPitch + x * 32 + il]
-                                  : buf[(x * 32 + il) * kCntPitch + y * 32 + jl];
-        const long long kk = row_off + d;
-        if (a.counts) {
-          int c9[9];
-          gmom::to_counts(mo, c9);
-          if (ok) {
-            int32_t* o = a.counts + kk * 9;
+          for (int y = 0; y < 3; ++y) w[3 * x + y] = w0[y * 32 * kMomWords + x * 16];
 #pragma unroll
-            for (int x = 0; x < 9; ++x) __stcs(o + x, c9[x]);
+        for (int z = 0; z < 2; ++z) {
+          const int il = 2 * (wq + 4 * k) + z;
+          const long long row_off = __shfl_sync(0xffffffffu, toff, il);
+          const int row_n = __shfl_sync(0xffffffffu, tn, il);
+          const int d0 = (int)(tj0 - ti0) - il - 1;  // j - i - 1 of lane 0
+          const int d = d0 + lane;
+          // d < row_n keeps j inside the band and below n_snp
+          const bool ok = d >= 0 && d < row_n;
+          gmom::Mom mo;
+#pragma unroll
+          for (int x = 0; x < 9; ++x) mo.m[x] = z ? (int)w[x] >> 16 : (int)(short)(w[x] & 0xffff);
+          const long long kk = row_off + d;
+          if (a.counts) {
+            int c9[9];
+            gmom::to_counts(mo, c9);
+            store_counts(a.counts, row_off + d0, max(0, -d0), min(32, row_n - d0), lane, cstage, c9);
           }
-        }
-        st_cs_if(ok && want_nv, a.nvalid + kk, mo.m[0]);
-        if (a.stats) {
-          const float4 o = gmom::stats_f32<MASK>(mo, a.stat_mask);
-          st_cs_if(ok, reinterpret_cast<float4*>(a.stats) + kk, o);
+          st_cs_if(ok && want_nv, a.nvalid + kk, mo.m[0]);
+          if (a.stats) {
+            const float4 o = gmom::stats_f32<MASK>(mo, a.stat_mask);
+            st_cs_if(ok, reinterpret_cast<float4*>(a.stats) + kk, o);
+          }
         }
       }
       item = next;
@@ -454,7 +504,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   if (warp == 1) {
     tc_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base),
-                 "r"(kTmemCols)
+                 "r"(tmem_cols)
                  : "memory");
   }
 }
@@ -977,22 +1027,25 @@ int pgld_geno_tc_pairs(pgld_context* h, const pgld_geno_panel* panel, const doub
   prm.stats = stats;
   prm.stat_mask = stat_mask;
   prm.status = h->dev_status;
-  const size_t fixed = sizeof(GCtrl) + (size_t)2 * 96 * kCntPitch * 2 + 1024;
   int max_smem = 0;
   cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, h->device);
-  // the resident form when the row block (every K chunk) fits beside at
-  // least four 16 KB A stages: up to 1,280 individuals
+  // the resident form when the row block (every K chunk) fits beside at least
+  // three 16 KB A stages, with as many epilogue groups as leave three
   const long long res_bytes = (long long)prm.kchunks * kBBytes;
-  const long long res_stages =
-      std::min<long long>(8, ((long long)max_smem - (long long)fixed - res_bytes) / kABytes);
-  const bool res = res_stages >= 4;
-  const int stages = res ? (int)res_stages
-                         : (int)std::min<long long>(
-                               8, ((long long)max_smem - (long long)fixed) / kGStageBytes);
+  auto fixed = [](int g) { return (long long)kCtrlBytes + 1024 + g * (kMomBytes + 4ll * kCountStage); };
+  auto ring = [&](int g, long long resident, int stage) {
+    return (int)std::min<long long>(8, (max_smem - fixed(g) - resident) / stage);
+  };
+  int g = kMaxGroups;
+  while (g > 2 && ring(g, res_bytes, kABytes) < 3) --g;
+  const bool res = ring(g, res_bytes, kABytes) >= 3;
+  if (!res) g = 3;
+  const int stages = res ? ring(g, res_bytes, kABytes) : ring(g, 0, kGStageBytes);
   if (stages < 2) return pgld_fail(h, PGLD_ERR_TOO_LARGE, "genotype tensor-core form: shared memory");
   prm.stages = stages;
+  prm.groups = g;
   const size_t smem =
-      res ? (size_t)stages * kABytes + (size_t)res_bytes + fixed : (size_t)stages * kGStageBytes + fixed;
+      (size_t)fixed(g) + (res ? (size_t)stages * kABytes + (size_t)res_bytes : (size_t)stages * kGStageBytes);
   // the two column sets of the band workloads get their own instantiation
   void (*kern)(CUtensorMap, Params);
   if (res)
@@ -1008,7 +1061,7 @@ int pgld_geno_tc_pairs(pgld_context* h, const pgld_geno_panel* panel, const doub
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return pgld_cuda_fail(h, e, "gtc smem attribute");
   pgld_time_begin(h, st);
-  kern<<<(unsigned)h->n_sm, kThreads, smem, st>>>(map, prm);
+  kern<<<(unsigned)h->n_sm, (4 + 4 * g) * 32, smem, st>>>(map, prm);
   pgld_time_end(h, st);
   e = cudaGetLastError();
   if (e != cudaSuccess) return pgld_cuda_fail(h, e, "gtc_pairs_kernel");
