@@ -8,7 +8,7 @@
 // m0 = n, the pairwise-valid count).  The tensor-core kernel gets them
 // straight from the MMA (operand planes 1, c and c^2 per SNP); from counts
 // they are nine small linear forms.  Let
-//   U = m1^2 - m2,  V = m3^2 - m6,  T = m1 m3 m4 - m1 m7 - m3 m5.
+//   U = m1^2 - m2,  V = m3^2 - m6,  S = m1 m7 + m3 m5,  T = m1 m3 m4 - S.
 // As identities of polynomials in the nine counts (expanded with sympy and
 // checked term by term against the reference's expressions):
 //   16 dd_poly + D16^2      = 16 [(n-1)(n-2) m4^2 - n(n-1) m8 - 2(n-1) T + U V]
@@ -17,12 +17,18 @@
 //                             - 4 T + 2 m4^2 - 6 m8
 // so DD = [..] / (4 d4), Dz = [..] / (2 d4), pi2 = [..] / (16 d4) with
 // d4 = n(n-1)(n-2)(n-3), each gated on n >= 4 like the reference kernels.
+// They are evaluated over y = n m4 - m1 m3 (the Rogers-Huff covariance) and
+// G = U m6 + m2 m3^2, which leaves one 32 x 32 -> 64 bit product per term:
+//   [dd]  = y^2 - (3n-2) m4^2 + 2 m1 m3 m4 - n(n-1) m8 + 2(n-1) S - G
+//   [dz]  = m1 m3 y + m1 m3 m4 - (n+1) S - (n-1) m4^2 + 2 n m8 + G
+//   [pi2] = (n(n-1) - U) ((n-2)(n-3) - V) + (4n-6) V - 4 m1 m3 m4 + 4 S
+//           + 2 m4^2 - 6 m8
 // Rogers-Huff: cov = n m4 - m1 m3, var_I = n m6 - m3^2, var_J = n m2 - m1^2.
 //
-// Every |m| <= n < 2^15, so U, V, m4^2, m1 m3 and the polynomials in n are
-// 32-bit integers, every product below is 32 x 32 -> 64 bits or a 64-bit
-// value times a 16-bit one, and every partial sum stays below 2^62: the
-// numerators are exact for populations below 32,768 individuals.
+// Every |m| <= n < 2^15, so U, V, S, m4^2, m1 m3, y (a covariance: |y| <= n^2)
+// and the polynomials in n are 32-bit integers, every product below is
+// 32 x 32 -> 64 bits, and every partial sum stays below 2^62: the numerators
+// are exact for populations below 32,768 individuals.
 #pragma once
 #include <stdint.h>
 
@@ -78,37 +84,42 @@ PGLD_GM_HD Mom from_counts(const int* c) {
 // E1 = (2, 0, -2), E2 = (0, 1, 1); the division by 4 is exact
 PGLD_GM_HD void to_counts(const Mom& o, int* c) {
   const int* m = o.m;
-  int q[3][3];  // q[a][y] = sum_x E_a[x] m[3 x + y]
+  int q0[3], q1[3], q2[3];  // sum_x E_a[x] m[3 x + y]; half of it for a = 1
 #pragma unroll
   for (int y = 0; y < 3; ++y) {
-    q[0][y] = m[6 + y] - m[3 + y];
-    q[1][y] = 2 * (m[y] - m[6 + y]);
-    q[2][y] = m[6 + y] + m[3 + y];
+    q0[y] = m[6 + y] - m[3 + y];
+    q1[y] = m[y] - m[6 + y];
+    q2[y] = m[6 + y] + m[3 + y];
   }
-#pragma unroll
-  for (int a = 0; a < 3; ++a) {
-    c[3 * a + 0] = (q[a][2] - q[a][1]) >> 2;
-    c[3 * a + 1] = (q[a][0] - q[a][2]) >> 1;
-    c[3 * a + 2] = (q[a][2] + q[a][1]) >> 2;
-  }
+  c[0] = (q0[2] - q0[1]) >> 2;
+  c[1] = (q0[0] - q0[2]) >> 1;
+  c[2] = (q0[2] + q0[1]) >> 2;
+  c[3] = (q1[2] - q1[1]) >> 1;
+  c[4] = q1[0] - q1[2];
+  c[5] = (q1[2] + q1[1]) >> 1;
+  c[6] = (q2[2] - q2[1]) >> 2;
+  c[7] = (q2[0] - q2[2]) >> 1;
+  c[8] = (q2[2] + q2[1]) >> 2;
 }
 
 struct Terms {
-  i64 T;    // m1 m3 m4 - m1 m7 - m3 m5
-  i64 UV;   // (m1^2 - m2)(m3^2 - m6)
-  int UpV;  // (m1^2 - m2) + (m3^2 - m6)
-  int m44;  // m4^2
+  int y;         // n m4 - m1 m3
+  int m13, m44;  // m1 m3, m4^2
+  int U, V, S;
+  i64 G;         // U m6 + m2 m3^2
 };
 
 PGLD_GM_HD Terms terms(const Mom& o) {
   const int* m = o.m;
   Terms t;
-  const int U = m[1] * m[1] - m[2];
-  const int V = m[3] * m[3] - m[6];
-  t.T = (i64)(m[1] * m[3]) * m[4] - ((i64)(m[1] * m[7]) + (i64)(m[3] * m[5]));
-  t.UV = (i64)U * V;
-  t.UpV = U + V;
+  const int m33 = m[3] * m[3];
+  t.m13 = m[1] * m[3];
   t.m44 = m[4] * m[4];
+  t.y = (int)((unsigned)m[0] * (unsigned)m[4] - (unsigned)t.m13);
+  t.U = m[1] * m[1] - m[2];
+  t.V = m33 - m[6];
+  t.S = m[1] * m[7] + m[3] * m[5];
+  t.G = (i64)t.U * m[6] + (i64)m[2] * m33;
   return t;
 }
 
@@ -117,19 +128,30 @@ PGLD_GM_HD i64 d4(int n) { return (i64)(n * (n - 1)) * ((n - 2) * (n - 3)); }
 // numerator over 4 d4
 PGLD_GM_HD i64 dd_num(const Mom& o, const Terms& t) {
   const int n = o.m[0];
-  return (i64)((n - 1) * (n - 2)) * t.m44 - (i64)(n * (n - 1)) * o.m[8] -
-         2 * (i64)(n - 1) * t.T + t.UV;
+  i64 v = (i64)t.y * t.y - t.G;
+  v += (i64)(2 - 3 * n) * t.m44;
+  v += (i64)t.m13 * (2 * o.m[4]);
+  v += (i64)(n * (1 - n)) * o.m[8];
+  return v + (i64)(2 * n - 2) * t.S;
 }
 // numerator over 2 d4
 PGLD_GM_HD i64 dz_num(const Mom& o, const Terms& t) {
   const int n = o.m[0];
-  return (i64)(n + 1) * t.T - (i64)(n - 1) * t.m44 + (i64)(2 * n) * o.m[8] - t.UV;
+  i64 v = (i64)t.m13 * t.y + t.G;
+  v += (i64)t.m13 * o.m[4];
+  v += (i64)(1 - n) * t.m44;
+  v += (i64)(2 * n) * o.m[8];
+  return v - (i64)(n + 1) * t.S;
 }
-// numerator over 16 d4
+// numerator over 16 d4: non-negative (sixteen times a count of distinct draws)
 PGLD_GM_HD i64 pi2_num(const Mom& o, const Terms& t) {
   const int n = o.m[0];
-  return d4(n) - (i64)((n - 2) * (n - 3)) * t.UpV + t.UV - 4 * t.T + 2 * (i64)t.m44 -
-         6 * (i64)o.m[8];
+  i64 v = (i64)(n * (n - 1) - t.U) * ((n - 2) * (n - 3) - t.V);
+  v += (i64)(4 * n - 6) * t.V;
+  v -= (i64)t.m13 * (4 * o.m[4]);
+  v += (i64)t.S * 4;
+  v += (i64)t.m44 * 2;
+  return v - (i64)o.m[8] * 6;
 }
 
 struct RHm {
@@ -164,7 +186,7 @@ __device__ __forceinline__ float4 stats_f32(const Mom& o, int mask_rt) {
   const int* m = o.m;
   const int n = m[0];
   if (mask & 1) {
-    const int cov = n * m[4] - m[1] * m[3];
+    const int cov = terms(o).y;
     const int vi = n * m[6] - m[3] * m[3];
     const int vj = n * m[2] - m[1] * m[1];
     const float fc = (float)cov;
@@ -174,10 +196,10 @@ __device__ __forceinline__ float4 stats_f32(const Mom& o, int mask_rt) {
   if (mask & 14) {
     const Terms t = terms(o);
     const bool ok = n >= 4;
-    const float r = __fdividef(1.0f, pgld::ll2f(d4(n)));  // unused where !ok
+    const float r = __fdividef(1.0f, pgld::ull2f(d4(n)));  // unused where !ok
     if (mask & 2) out.y = ok ? pgld::ll2f(dd_num(o, t)) * (0.25f * r) : 0.f;
     if (mask & 4) out.z = ok ? pgld::ll2f(dz_num(o, t)) * (0.5f * r) : 0.f;
-    if (mask & 8) out.w = ok ? pgld::ll2f(pi2_num(o, t)) * (0.0625f * r) : 0.f;
+    if (mask & 8) out.w = ok ? pgld::ull2f(pi2_num(o, t)) * (0.0625f * r) : 0.f;
   }
   return out;
 }

@@ -85,7 +85,7 @@ struct Params {
 
 constexpr int kMaxGroups = 4;
 constexpr int kPairThreads = (4 + 4 * kMaxGroups) * 32;
-constexpr int kMomWords = kCntPitch / 2;     // words (two int16 moments) per row of a moment block
+constexpr int kMomWords = 25;                // pitch of a half tile's 24 moment words (odd)
 constexpr int kMomBytes = 96 * kMomWords * 4;
 constexpr int kCtrlBytes = 512;             // the control block, 16-byte aligned end
 constexpr int kCountStage = (9 * 32 + 4) * 4;  // bytes of a warp's staged counts, any alignment
@@ -362,10 +362,12 @@ __global__ void __launch_bounds__(kPairThreads, 1)
     // ---------------- epilogue ----------------
     // Groups of four warps take the tiles in turn (group g: tiles g, g + groups,
     // ... of this CTA, accumulator stage g, moment buffer g), so one group's
-    // copy and the others' statistics overlap.  Within a group the warp of
-    // TMEM lane quarter q < 3 copies plane q's 96 moment columns, two int16
-    // moments (rows i, i + 1) to a word, and all four warps turn the 1,024
-    // pairs into outputs (8 per thread).
+    // copy and the others' statistics overlap.  A group takes its tile in two
+    // halves of 16 rows i: the warp of TMEM lane quarter q < 3 copies plane q's
+    // 48 moment columns of the half, two int16 moments (rows i, i + 1) to a
+    // word, and all four warps turn its 512 pairs into outputs (4 per thread).
+    // Whole tiles would take 28 KB more of shared memory, two of the stages
+    // that keep the column block streaming.
     const int e = warp - 4;
     const int grp = e >> 2;
     const int wq = warp & 3;  // TMEM lanes 32q..32q+31: plane q of the SNPs j
@@ -426,28 +428,6 @@ __global__ void __launch_bounds__(kPairThreads, 1)
           : "memory");
       if (any_abort) break;
       tc_fence_after();
-      if (wq < 3) {
-        uint32_t* row = buf + (wq * 32 + lane) * kMomWords;
-#pragma unroll 1
-        for (int h = 0; h < 2; ++h) {
-          uint32_t r[3][16];
-#pragma unroll
-          for (int c = 0; c < 3; ++c)
-            tmem_ld16(tmem_base + lane_base + (uint32_t)(grp * 128 + 48 * h + 16 * c), r[c]);
-          tmem_wait_ld();
-#pragma unroll
-          for (int c = 0; c < 3; ++c)
-#pragma unroll
-            for (int v = 0; v < 8; ++v)
-              row[24 * h + 8 * c + v] =
-                  fast::f2i_pair(__uint_as_float(r[c][2 * v]), __uint_as_float(r[c][2 * v + 1]));
-        }
-      }
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&ctrl->gempty[grp]);
-      asm volatile("bar.sync %0, 128;" ::"r"(bar_id) : "memory");
-
       const bool want_nv = a.nvalid != nullptr;
       // this tile's location; the next tile's offsets load during the pairs
       const long long ti0 = i0, tj0 = j0, toff = off_lo;
@@ -456,40 +436,70 @@ __global__ void __launch_bounds__(kPairThreads, 1)
       const long long next = tile_item(t, chunk);
       if (next < n_items) nv = lo + 1 + lane <= a.n_blocks ? a.item_off[lo + 1 + lane] : LLONG_MAX;
 
-      // eight pairs per thread, two rows at a time; every value is computed and
-      // only the stores depend on the pair lying in the band.  The outputs go
-      // out as streaming global stores (st.global.cs): they are not re-read,
-      // and being global-space they cannot alias the shared-memory moments.
+#pragma unroll 1
+      for (int h = 0; h < 2; ++h) {
+        if (wq < 3) {
+          uint32_t* row = buf + (wq * 32 + lane) * kMomWords;
+          uint32_t r[3][16];
 #pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        const uint32_t* w0 = buf + lane * kMomWords + wq + 4 * k;
-        uint32_t w[9];
+          for (int x = 0; x < 3; ++x)
+            tmem_ld16(tmem_base + lane_base + (uint32_t)(grp * 128 + 32 * x + 16 * h), r[x]);
+          tmem_wait_ld();
+          if (h) asm volatile("bar.sync %0, 128;" ::"r"(bar_id) : "memory");  // half 0 is read
 #pragma unroll
-        for (int x = 0; x < 3; ++x)
+          for (int x = 0; x < 3; ++x)
 #pragma unroll
-          for (int y = 0; y < 3; ++y) w[3 * x + y] = w0[y * 32 * kMomWords + x * 16];
+            for (int v = 0; v < 8; ++v)
+              row[8 * x + v] =
+                  fast::f2i_pair(__uint_as_float(r[x][2 * v]), __uint_as_float(r[x][2 * v + 1]));
+        } else if (h) {
+          asm volatile("bar.sync %0, 128;" ::"r"(bar_id) : "memory");
+        }
+        if (h) {
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&ctrl->gempty[grp]);
+        }
+        asm volatile("bar.sync %0, 128;" ::"r"(bar_id) : "memory");
+
+        // four pairs per thread, two rows at a time; every value is computed
+        // and only the stores depend on the pair lying in the band.  The
+        // outputs go out as streaming global stores (st.global.cs): they are
+        // not re-read, and being global-space they cannot alias the
+        // shared-memory moments.
+#pragma unroll 1
+        for (int k = 0; k < 2; ++k) {
+          const uint32_t* w0 = buf + lane * kMomWords + wq + 4 * k;
+          uint32_t w[9];
 #pragma unroll
-        for (int z = 0; z < 2; ++z) {
-          const int il = 2 * (wq + 4 * k) + z;
-          const long long row_off = __shfl_sync(0xffffffffu, toff, il);
-          const int row_n = __shfl_sync(0xffffffffu, tn, il);
-          const int d0 = (int)(tj0 - ti0) - il - 1;  // j - i - 1 of lane 0
-          const int d = d0 + lane;
-          // d < row_n keeps j inside the band and below n_snp
-          const bool ok = d >= 0 && d < row_n;
-          gmom::Mom mo;
+          for (int x = 0; x < 3; ++x)
 #pragma unroll
-          for (int x = 0; x < 9; ++x) mo.m[x] = z ? (int)w[x] >> 16 : (int)(short)(w[x] & 0xffff);
-          const long long kk = row_off + d;
-          if (a.counts) {
-            int c9[9];
-            gmom::to_counts(mo, c9);
-            store_counts(a.counts, row_off + d0, max(0, -d0), min(32, row_n - d0), lane, cstage, c9);
-          }
-          st_cs_if(ok && want_nv, a.nvalid + kk, mo.m[0]);
-          if (a.stats) {
-            const float4 o = gmom::stats_f32<MASK>(mo, a.stat_mask);
-            st_cs_if(ok, reinterpret_cast<float4*>(a.stats) + kk, o);
+            for (int y = 0; y < 3; ++y) w[3 * x + y] = w0[y * 32 * kMomWords + x * 8];
+#pragma unroll
+          for (int z = 0; z < 2; ++z) {
+            const int il = 16 * h + 2 * (wq + 4 * k) + z;
+            const long long row_off = __shfl_sync(0xffffffffu, toff, il);
+            const int row_n = __shfl_sync(0xffffffffu, tn, il);
+            const int d0 = (int)(tj0 - ti0) - il - 1;  // j - i - 1 of lane 0
+            const int d = d0 + lane;
+            // d < row_n keeps j inside the band and below n_snp
+            const bool ok = d >= 0 && d < row_n;
+            gmom::Mom mo;
+#pragma unroll
+            for (int x = 0; x < 9; ++x)
+              mo.m[x] = z ? (int)w[x] >> 16 : (int)(short)(w[x] & 0xffff);
+            const long long kk = row_off + d;
+            if (a.counts) {
+              int c9[9];
+              gmom::to_counts(mo, c9);
+              store_counts(a.counts, row_off + d0, max(0, -d0), min(32, row_n - d0), lane, cstage,
+                           c9);
+            }
+            st_cs_if(ok && want_nv, a.nvalid + kk, mo.m[0]);
+            if (a.stats) {
+              const float4 o = gmom::stats_f32<MASK>(mo, a.stat_mask);
+              st_cs_if(ok, reinterpret_cast<float4*>(a.stats) + kk, o);
+            }
           }
         }
       }
@@ -1030,15 +1040,19 @@ int pgld_geno_tc_pairs(pgld_context* h, const pgld_geno_panel* panel, const doub
   int max_smem = 0;
   cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, h->device);
   // the resident form when the row block (every K chunk) fits beside at least
-  // three 16 KB A stages, with as many epilogue groups as leave three
+  // four 16 KB A stages, with as many epilogue groups as leave six: a copy
+  // takes about 1.6 us under load, so the stages in flight set the pace of long
+  // rows (1,000 individuals, 1.0e8 pairs: two groups and six stages 2.17 ms, three
+  // and five 2.24, four and four 2.31; short rows are bound by the statistics,
+  // which four groups do in 1.39 ms at 250 individuals)
   const long long res_bytes = (long long)prm.kchunks * kBBytes;
   auto fixed = [](int g) { return (long long)kCtrlBytes + 1024 + g * (kMomBytes + 4ll * kCountStage); };
   auto ring = [&](int g, long long resident, int stage) {
     return (int)std::min<long long>(8, (max_smem - fixed(g) - resident) / stage);
   };
   int g = kMaxGroups;
-  while (g > 2 && ring(g, res_bytes, kABytes) < 3) --g;
-  const bool res = ring(g, res_bytes, kABytes) >= 3;
+  while (g > 2 && ring(g, res_bytes, kABytes) < 6) --g;
+  const bool res = ring(g, res_bytes, kABytes) >= 4;
   if (!res) g = 3;
   const int stages = res ? ring(g, res_bytes, kABytes) : ring(g, 0, kGStageBytes);
   if (stages < 2) return pgld_fail(h, PGLD_ERR_TOO_LARGE, "genotype tensor-core form: shared memory");

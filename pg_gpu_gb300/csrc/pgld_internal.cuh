@@ -246,6 +246,11 @@ __device__ __forceinline__ float ll2f(i64 x) {
   return x < 0 ? -f : f;
 }
 
+// ll2f of a non-negative integer
+__device__ __forceinline__ float ull2f(i64 x) {
+  return fmaf(__int2float_rn((int)(x >> 31)), 2147483648.0f, __int2float_rn((int)(x & 0x7fffffffll)));
+}
+
 __device__ __forceinline__ float term_value_f32(int kind, const int* pp, const PopC* P) {
   if (kind >= PGLD_R) {
     const PopC& p = P[pp[0]];
