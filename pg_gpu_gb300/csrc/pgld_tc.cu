@@ -868,7 +868,9 @@ __global__ void __launch_bounds__(256) pack_tc_kernel(const uint32_t* __restrict
                                                       long long n_snp, long long n_rows,
                                                       const int32_t* __restrict__ idx, int k_pad,
                                                       int grouped, uint32_t* __restrict__ out,
-                                                      int32_t* __restrict__ status) {
+                                                      int32_t* __restrict__ status,
+                                                      const int* __restrict__ skip = nullptr) {
+  if (skip && *skip) return;
   const long long rows_out = 2 * (grouped ? (n_rows + 7) / 8 * 8 : n_rows);
   const long long rowi = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
@@ -1112,14 +1114,14 @@ int pgld_tc_pairs(pgld_context* h, const pgld_hap_panel* panel, pgld::BandArgs& 
 }
 
 // the E4M3 operand rows of a population's bit planes over an index list
-// (pack_tc_kernel, rows grouped by 8 positions)
+// (pack_tc_kernel, rows grouped by 8 positions); nothing where *skip is set
 int pgld_tc_pack_rows(pgld_context* h, const uint32_t* planes, int W, long long n_snp,
                       long long n_rows, const int32_t* idx, int k_pad, unsigned char* out,
-                      cudaStream_t st) {
+                      const int* skip, cudaStream_t st) {
   const long long rows_out = 2 * ((n_rows + 7) / 8 * 8);
   const unsigned blocks = (unsigned)std::max<long long>(1, (rows_out + 7) / 8);
   pgld::tc::pack_tc_kernel<<<blocks, 256, 0, st>>>(planes, W, n_snp, n_rows, idx, k_pad, 1,
-                                                   (uint32_t*)out, h->dev_status);
+                                                   (uint32_t*)out, h->dev_status, skip);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return pgld_cuda_fail(h, e, "pack_tc_kernel");
   return PGLD_OK;

@@ -48,6 +48,7 @@
 #include "pgld_tc_common.cuh"
 #include "pgld_tcgen05.cuh"
 #include "pgld_window.cuh"
+#include "pgld_window_complete.cuh"
 
 #ifndef PGLD_TCW_MAXNREG
 #define PGLD_TCW_MAXNREG 1
@@ -142,14 +143,10 @@ struct Params {
   long long n_panel;           // SNPs of the panel (bound of idx values)
   double* wsums;               // [n_win][6]
   unsigned long long* wcnt;    // [n_win][3]
+  const wcomp::State* state;   // a complete list (or NULL: none) has its own kernel
 };
 
-// windows mode: row block b of a window of C column blocks holds the column
-// blocks b / 2 .. C - 1; the tiles before row block b
-__host__ __device__ __forceinline__ long long wtiles_before(long long b, long long C) {
-  const long long k = b >> 1;
-  return b * C - ((b & 1) ? k * k : k * (k - 1));
-}
+using wcomp::tiles_before;
 
 // a work item's tile: first list positions of its rows i0 and columns j0,
 // and (windows mode) its window [begin, end) and index
@@ -179,19 +176,11 @@ __device__ __forceinline__ WideTile window_tile(const Params& a, long long item,
   const long long base = a.win_begin[lo] & ~7ll, m = a.win_end[lo] - base;
   const long long R = (m + kRowSnp - 1) / kRowSnp, C = (m + kColSnp - 1) / kColSnp;
   const long long t = item - a.tile_off[lo];
-  // the row block: the largest b < R with wtiles_before(b, C) <= t.  For even
-  // b, wtiles_before = b C - b^2 / 4 + b / 2, whose root in b, (2C + 1) -
-  // sqrt((2C + 1)^2 - 4 t), starts the search; the steps below make it exact
-  // (wtiles_before rises by C - floor(b / 2) >= 1 per row block)
-  const long long c2 = 2 * C + 1;
-  const float disc = (float)(c2 * c2 - 4 * t);
-  long long rlo = (long long)((float)c2 - sqrtf(disc > 0.f ? disc : 0.f));
-  rlo = rlo < 0 ? 0 : (rlo > R - 1 ? R - 1 : rlo);
-  while (rlo > 0 && wtiles_before(rlo, C) > t) --rlo;
-  while (rlo + 1 < R && wtiles_before(rlo + 1, C) <= t) ++rlo;
+  long long rlo, first;
+  wcomp::row_block(t, R, C, rlo, first);
   WideTile r;
   r.i0 = base + rlo * kRowSnp;
-  r.j0 = base + ((rlo >> 1) + (t - wtiles_before(rlo, C))) * kColSnp;
+  r.j0 = base + ((rlo >> 1) + (t - first)) * kColSnp;
   r.begin = a.win_begin[lo];
   r.end = a.win_end[lo];
   r.w = lo;
@@ -330,6 +319,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     if (threadIdx.x == 0) set_abort(ctrl, a.status, 3001);
     n_items = 0;
   }
+  if (MODE == kModeWindows && a.state && a.state->complete) n_items = 0;
   if (MODE == kModeBinned && n_items > 0 && a.n_anchor < a.n_snp)
     n_items = a.item_off[(a.n_anchor + kRowSnp - 1) / kRowSnp];
 
@@ -1061,19 +1051,29 @@ __global__ void pos_to_int_kernel_w(const double* __restrict__ pos, long long n,
 }
 
 // 64 x 128 tiles of each window's upper triangle (list positions from
-// win_begin & ~7); bad ranges get none and set the status
+// win_begin & ~7); bad ranges get none and set the status.  A complete list has
+// 128 x 256 tiles, and its pair counts follow from the window's
+// length
 __global__ void wide_window_tiles_kernel(const long long* __restrict__ wb,
                                          const long long* __restrict__ we, int n_win,
-                                         long long n_idx, long long* __restrict__ tiles,
+                                         long long n_idx, const wcomp::State* __restrict__ state,
+                                         long long* __restrict__ tiles,
+                                         unsigned long long* __restrict__ wcnt,
                                          int32_t* __restrict__ status) {
+  const bool complete = state && state->complete;
   for (int w = blockIdx.x * blockDim.x + threadIdx.x; w < n_win; w += gridDim.x * blockDim.x) {
     const long long lo = wb[w], hi = we[w];
     long long T = 0;
     if (lo < 0 || hi < lo || hi > n_idx) {
       atomicCAS(status, 0, 3100);
+    } else if (hi > lo && complete) {
+      const long long m = hi - (lo & ~7ll), pairs = (hi - lo) * (hi - lo - 1) / 2;
+      T = tiles_before((m + 127) / 128, (m + 255) / 256);
+      wcnt[3 * w] = (unsigned long long)pairs;
+      if (state->n >= 4) wcnt[3 * w + 2] = (unsigned long long)pairs;
     } else if (hi > lo) {
       const long long m = hi - (lo & ~7ll);
-      T = wtiles_before((m + kRowSnp - 1) / kRowSnp, (m + kColSnp - 1) / kColSnp);
+      T = tiles_before((m + kRowSnp - 1) / kRowSnp, (m + kColSnp - 1) / kColSnp);
     }
     tiles[w] = T;
   }
@@ -1207,7 +1207,7 @@ int pgld_tc_wide_binned(pgld_context* h, const pgld_hap_panel* panel, pgld::Band
 // ---------------------------------------------------------------------------
 int pgld_tc_pack_rows(pgld_context* h, const uint32_t* planes, int W, long long n_snp,
                       long long n_rows, const int32_t* idx, int k_pad, unsigned char* out,
-                      cudaStream_t st);
+                      const int* skip, cudaStream_t st);
 int pgld_site_freqs(pgld_context* h, const uint32_t* planes, const uint32_t* valid, int W,
                     long long n_snp, float4* site, cudaStream_t st);
 
@@ -1341,7 +1341,9 @@ int pgld_tc_wide_windows(pgld_context* h, const pgld_hap_panel* panel, const int
   auto al = [](size_t x) { return (x + 1023) & ~size_t(1023); };
   const size_t off_tiles = 0, off_scan = al((size_t)(n_win + 1) * 8), off_op = off_scan + al(sb),
                off_site = off_op + al(op_bytes),
-               total = off_site + al((size_t)std::max<long long>(n, 1) * 16);
+               off_list = off_site + al((size_t)std::max<long long>(n, 1) * 16),
+               off_state = off_list + al((size_t)std::max<long long>(n_idx, 1) * 8),
+               total = off_state + al(sizeof(pgld::wcomp::State));
   void* ws = nullptr;
   rc = pgld_workspace(h, total, &ws);
   if (rc) return rc;
@@ -1349,9 +1351,19 @@ int pgld_tc_wide_windows(pgld_context* h, const pgld_hap_panel* panel, const int
   long long* tiles = (long long*)(w + off_tiles);
   unsigned char* op = (unsigned char*)(w + off_op);
   float4* site = (float4*)(w + off_site);
+  float2* list_site = (float2*)(w + off_list);
+  // a list whose SNPs all have the same valid haplotypes takes the kernel of
+  // complete lists; which of the two has the windows is decided on the device
+  pgld::wcomp::State* state = nullptr;
+  if (n_idx > 0 && n > 0) {
+    state = (pgld::wcomp::State*)(w + off_state);
+    rc = pgld_window_complete_pack(h, panel->planes[0], W, n, n_idx, idx, state, op, list_site, st);
+    if (rc) return rc;
+  }
   {
     const unsigned gb = (unsigned)std::max<long long>(1, std::min<long long>((n_win + 255) / 256, h->n_sm * 4LL));
-    wide_window_tiles_kernel<<<gb, 256, 0, st>>>(wb, we, n_win, n_idx, tiles, h->dev_status);
+    wide_window_tiles_kernel<<<gb, 256, 0, st>>>(wb, we, n_win, n_idx, state, tiles, counts,
+                                                 h->dev_status);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return pgld_cuda_fail(h, e, "wide_window_tiles_kernel");
   }
@@ -1366,7 +1378,8 @@ int pgld_tc_wide_windows(pgld_context* h, const pgld_hap_panel* panel, const int
     if (rc) return rc;
   }
   if (n_idx > 0) {
-    rc = pgld_tc_pack_rows(h, panel->planes[0], W, n, n_idx, idx, k_pad, op, st);
+    rc = pgld_tc_pack_rows(h, panel->planes[0], W, n, n_idx, idx, k_pad, op,
+                           state ? &state->complete : nullptr, st);
     if (rc) return rc;
   }
   {
@@ -1395,6 +1408,12 @@ int pgld_tc_wide_windows(pgld_context* h, const pgld_hap_panel* panel, const int
   prm.n_panel = n;
   prm.wsums = sums;
   prm.wcnt = counts;
+  prm.state = state;
+  if (state) {
+    rc = pgld_window_complete_sums(h, state, W, n_idx, op, list_site, wb, we, n_win, tiles, sums,
+                                   counts, columns, st);
+    if (rc) return rc;
+  }
   if (sigma)
     return wide_one_pop_launch<pgld::kModeWindows, 2>(h, prm, map_a, map_b, st,
                                                       "band_wide_kernel (windows)");
