@@ -297,7 +297,7 @@ __global__ void __launch_bounds__(kThreads) pairs_by_bin_kernel(
 // the next digit in shared memory, one per distinct prefix among the segment's
 // targets) and one small launch that picks the targets' digits.  60 targets in
 // 12.5 million values (15 bins): 4.2 ms with one CTA per target and eight
-// passes of its own, 0.3 ms here.
+// passes of its own, 0.17 ms here.
 constexpr int kDigits = 6, kDigitBins = 2048;
 constexpr int kKthChunk = 1 << 15;
 constexpr int kKthGroup = 4;  // histograms per block at a time
@@ -363,34 +363,96 @@ __global__ void __launch_bounds__(256) kth_count_kernel(KthArgs a, int pass) {
   }
 }
 
-// a warp per target: the digit whose cumulative count passes the rank
-__global__ void __launch_bounds__(256) kth_pick_kernel(KthArgs a, int pass) {
-  const int t = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-  if (t >= a.n_targets) return;
-  const unsigned* h = a.hist + (size_t)a.rep[t] * kDigitBins;
-  long long r = a.rank[t];
-  int digit = (1 << digit_bits(pass)) - 1;
-  for (int d0 = 0; d0 < (1 << digit_bits(pass)); d0 += 32) {
-    const unsigned c = h[d0 + lane];
-    unsigned incl = c;
+// inclusive sum over the block of one count per thread; total: the block's sum
+template <int THREADS>
+__device__ __forceinline__ unsigned block_scan(unsigned v, unsigned* warp_sums, unsigned& total) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  unsigned incl = v;
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const unsigned y = __shfl_up_sync(0xffffffffu, incl, o);
-      if (lane >= o) incl += y;
-    }
-    const unsigned hit = __ballot_sync(0xffffffffu, (long long)incl > r);
-    if (hit) {
-      const int l = __ffs(hit) - 1;
-      r -= (long long)(__shfl_sync(0xffffffffu, incl, l) - __shfl_sync(0xffffffffu, c, l));
-      digit = d0 + l;
-      break;
-    }
-    r -= (long long)__shfl_sync(0xffffffffu, incl, 31);
+  for (int o = 1; o < 32; o <<= 1) {
+    const unsigned y = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += y;
   }
-  if (lane == 0) {
+  if (lane == 31) warp_sums[warp] = incl;
+  __syncthreads();
+  unsigned before = 0;
+  total = 0;
+#pragma unroll
+  for (int w = 0; w < THREADS / 32; ++w) {
+    const unsigned x = warp_sums[w];
+    if (w < warp) before += x;
+    total += x;
+  }
+  __syncthreads();
+  return incl + before;
+}
+
+// a block per target: the digit whose cumulative count passes the rank, eight
+// digits to a thread
+__global__ void __launch_bounds__(256) kth_pick_kernel(KthArgs a, int pass) {
+  __shared__ unsigned warp_sums[8];
+  const int t = blockIdx.x;
+  const uint4* h = reinterpret_cast<const uint4*>(a.hist + (size_t)a.rep[t] * kDigitBins);
+  const uint4 x = h[2 * threadIdx.x], y = h[2 * threadIdx.x + 1];
+  const unsigned c[8] = {x.x, x.y, x.z, x.w, y.x, y.y, y.z, y.w};
+  unsigned sum = 0, total;
+#pragma unroll
+  for (int k = 0; k < 8; ++k) sum += c[k];
+  long long r = a.rank[t];
+  r -= (long long)(block_scan<256>(sum, warp_sums, total) - sum);
+  if (r >= 0 && r < (long long)sum) {  // one thread: the rank is below the total
+    int k = 0;
+    while (r >= (long long)c[k]) r -= (long long)c[k++];
     a.rank[t] = r;
-    a.prefix[t] |= (unsigned long long)digit << digit_shift(pass);
+    a.prefix[t] |= (unsigned long long)(8 * threadIdx.x + k) << digit_shift(pass);
   }
+}
+
+// Short segments: a block per target does all passes by itself, one launch
+// instead of 23.  34 targets in 17 segments of 15,000 values: 104 us of the device
+// and 170 us of the call in passes over the grid, 18 us and none here; 16 in 8 of
+// 140,000: 164 and 140 us; 30 in 15 of 830,000: 171 and 825 us.
+constexpr int kSmallSeg = 1 << 17;
+constexpr int kSmallCopies = 4;
+__global__ void __launch_bounds__(1024) kth_small_kernel(KthArgs a, const int* __restrict__ tseg) {
+  __shared__ unsigned hist[kSmallCopies][kDigitBins];
+  __shared__ unsigned warp_sums[32];
+  __shared__ unsigned long long s_prefix;
+  __shared__ long long s_rank;
+  const int t = blockIdx.x;
+  const long long v0 = a.seg_off[tseg[t]], v1 = a.seg_off[tseg[t] + 1];
+  unsigned long long prefix = 0;
+  long long rank = a.rank[t];
+  unsigned* mine = hist[(threadIdx.x >> 5) & (kSmallCopies - 1)];
+  for (int pass = 0; pass < kDigits; ++pass) {
+    const int shift = digit_shift(pass), above = shift + digit_bits(pass);
+    const unsigned mask = (1u << digit_bits(pass)) - 1u;
+    for (int x = threadIdx.x; x < kSmallCopies * kDigitBins; x += 1024) (&hist[0][0])[x] = 0u;
+    __syncthreads();
+    const unsigned long long want = pass > 0 ? prefix >> above : 0ull;
+#pragma unroll 8
+    for (long long k = v0 + threadIdx.x; k < v1; k += 1024) {
+      const unsigned long long key = (unsigned long long)__double_as_longlong(a.values[k]);
+      if (pass == 0 || key >> above == want) atomicAdd(mine + ((unsigned)(key >> shift) & mask), 1u);
+    }
+    __syncthreads();
+    unsigned c0 = 0, c1 = 0, total;
+#pragma unroll
+    for (int w = 0; w < kSmallCopies; ++w) {
+      c0 += hist[w][2 * threadIdx.x];
+      c1 += hist[w][2 * threadIdx.x + 1];
+    }
+    long long r = rank - (long long)(block_scan<1024>(c0 + c1, warp_sums, total) - (c0 + c1));
+    if (r >= 0 && r < (long long)(c0 + c1)) {  // one thread
+      const bool second = r >= (long long)c0;
+      s_rank = second ? r - (long long)c0 : r;
+      s_prefix = prefix | (unsigned long long)(2 * threadIdx.x + second) << shift;
+    }
+    __syncthreads();
+    rank = s_rank;
+    prefix = s_prefix;
+  }
+  if (threadIdx.x == 0) a.prefix[t] = prefix;
 }
 
 // the first target of the same segment with the same prefix
@@ -755,7 +817,11 @@ extern "C" int pgld_segment_kth(pgld_handle h, const double* values, const int64
   std::copy(rep.begin(), rep.end(), ui + n_seg + 1);
   std::copy(tseg.begin(), tseg.end(), ui + n_seg + 1 + n_targets);
   const size_t up_b = (up.size() * 8 + 255) & ~size_t(255);
-  const size_t hist_b = (size_t)n_targets * kDigitBins * 4;
+  long long longest = 0;
+  for (int t = 0; t < n_targets; ++t)
+    longest = std::max<long long>(longest, seg_offsets[tseg[t] + 1] - seg_offsets[tseg[t]]);
+  const bool small = longest <= kSmallSeg;
+  const size_t hist_b = small ? 0 : (size_t)n_targets * kDigitBins * 4;
   void* ws = nullptr;
   int rc = pgld_workspace(h, up_b + hist_b, &ws);
   if (rc) return rc;
@@ -772,10 +838,14 @@ extern "C" int pgld_segment_kth(pgld_handle h, const double* values, const int64
   a.n_targets = n_targets;
   const int* d_tseg = a.rep + n_targets;
   PGLD_CHECK_CUDA(h, cudaMemcpyAsync(ws, u, up.size() * 8, cudaMemcpyHostToDevice, st));
-  for (int pass = 0; pass < kDigits; ++pass) {
+  if (small) {
+    kth_small_kernel<<<(unsigned)n_targets, 1024, 0, st>>>(a, d_tseg);
+    PGLD_CHECK_CUDA(h, cudaGetLastError());
+  }
+  for (int pass = 0; pass < kDigits && !small; ++pass) {
     PGLD_CHECK_CUDA(h, cudaMemsetAsync(a.hist, 0, hist_b, st));
     kth_count_kernel<<<(unsigned)chunk_off[n_seg], 256, 0, st>>>(a, pass);
-    kth_pick_kernel<<<(unsigned)((n_targets + 7) / 8), 256, 0, st>>>(a, pass);
+    kth_pick_kernel<<<(unsigned)n_targets, 256, 0, st>>>(a, pass);
     if (pass + 1 < kDigits) kth_rep_kernel<<<(unsigned)((n_targets + 255) / 256), 256, 0, st>>>(a, d_tseg);
     PGLD_CHECK_CUDA(h, cudaGetLastError());
   }

@@ -44,6 +44,14 @@ def test_segment_kth(sizes, kind):
     assert np.array_equal(got, np.asarray(want)[mix])
 
 
+# segments on both sides of the length up to which a block does all passes
+@pytest.mark.parametrize("sizes", [[1 << 17, 5], [(1 << 17) + 1, 1, 0, 300], [200_000, 1 << 17]])
+def test_segment_kth_long(sizes):
+    test_segment_kth(sizes, "ties")
+    test_segment_kth(sizes, "r2")
+    test_segment_kth(sizes, "close")
+
+
 # whole and fractional positions: the same bins (right-open) and values
 @pytest.mark.parametrize("shift", [0.0, 0.5])
 def test_pairs_by_bin(shift):
