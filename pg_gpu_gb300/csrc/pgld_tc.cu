@@ -43,15 +43,18 @@ namespace tc {
 
 constexpr int kTileSnp = 64;
 constexpr int kEpiWarps = 8;
-// pairs mode: per epilogue warp two staging buffers of the counts and the
-// float32 statistics of one step (8 rows i x 16 columns j, rows padded to 17
-// entries of 16 bytes), written out by bulk copies of each row's band range
+// pairs mode: two sets of eight epilogue warps on alternate tiles, and per warp
+// a staging buffer of the counts and the float32 statistics of one step (8 rows
+// i x 16 columns j, rows padded to 17 entries of 16 bytes), written out by bulk
+// copies of each row's band range
 constexpr int kStgRow = 17 * 16;
 constexpr int kStgArr = 8 * kStgRow;
-constexpr int kStgBuf = 2 * kStgArr;
-constexpr int kStgWarp = 2 * kStgBuf;
-constexpr int kEpiThreads = kEpiWarps * 32;
-constexpr int kThreads = (4 + kEpiWarps) * 32;
+constexpr int kStgN = 8 * 33 * 4;  // the sample sizes of two steps (8 rows x 32 columns)
+constexpr int kStgWarp = 2 * kStgArr + kStgN;
+__host__ __device__ constexpr int epi_warps(int mode) { return mode == kModePairs ? 16 : kEpiWarps; }
+__host__ __device__ constexpr int threads_of(int mode) { return (4 + epi_warps(mode)) * 32; }
+// reciprocal tables by n: four of them, the pairs mode one (1/(n(n-1)(n-2)(n-3)))
+__host__ __device__ constexpr int n_tables(int mode) { return mode == kModePairs ? 1 : 4; }
 constexpr uint32_t kTmemCols = 512;
 #ifndef PGLD_TC_MAXNREG
 #define PGLD_TC_MAXNREG 0
@@ -175,10 +178,11 @@ __device__ __forceinline__ TileRef decode_item(const Params& a, long long item,
 // MODE kModeBinned: distance-binned moments sums of P populations;
 // kModePairs: per-pair counts / n / (r^2, DD, Dz, pi2) of one population
 template <int P, int MODE>
-__global__ void __launch_bounds__(kThreads, 1)
+__global__ void __launch_bounds__(threads_of(MODE), 1)
     band_tc_kernel(const __grid_constant__ CUtensorMap map0, const __grid_constant__ CUtensorMap map1,
                    Params a) {
   constexpr int S = (P == 1) ? 3 : 15;
+  constexpr int kEpiThreads = epi_warps(MODE) * 32;
   extern __shared__ unsigned char smem_dyn[];
   // 1024-byte aligned base for the swizzled stages
   unsigned char* base =
@@ -193,9 +197,9 @@ __global__ void __launch_bounds__(kThreads, 1)
   unsigned long long* kcnt =
       reinterpret_cast<unsigned long long*>(kacc + kEpiWarps * a.n_bins * S);  // [kEpiWarps][n_bins]
   // reciprocal tables by n, 4 x (nmax + 1) floats: four arrays (1/n,
-  // 1/(n(n-1)), 1/(n(n-1)(n-2)), 1/(n(n-1)(n-2)(n-3))) for the per-pair and
-  // window modes, one interleaved float4 array for the binned mode (one load
-  // per population and pair)
+  // 1/(n(n-1)), 1/(n(n-1)(n-2)), 1/(n(n-1)(n-2)(n-3))) for the window mode (the
+  // per-pair mode needs the last alone), one interleaved float4 array for the
+  // binned mode (one load per population and pair)
   unsigned char* tables_u8 = reinterpret_cast<unsigned char*>(kcnt + kEpiWarps * a.n_bins);
   tables_u8 += (16 - (smem_u32(tables_u8) & 15)) & 15;  // 16-byte aligned for float4 loads
   float* tables = reinterpret_cast<float*>(tables_u8);
@@ -203,10 +207,10 @@ __global__ void __launch_bounds__(kThreads, 1)
   T.inv = tables;
   T.r2 = tables + (a.nmax + 1);
   T.r3 = tables + 2 * (a.nmax + 1);
-  T.r4 = tables + 3 * (a.nmax + 1);
+  T.r4 = tables + (n_tables(MODE) - 1) * (a.nmax + 1);
   const float4* T4 = reinterpret_cast<const float4*>(tables);
   // pairs mode: the epilogue warps' staging buffers, after the tables
-  unsigned char* stg = reinterpret_cast<unsigned char*>(tables + 4 * (a.nmax + 1));
+  unsigned char* stg = reinterpret_cast<unsigned char*>(tables + n_tables(MODE) * (a.nmax + 1));
   stg += (16 - (smem_u32(stg) & 15)) & 15;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -242,7 +246,10 @@ __global__ void __launch_bounds__(kThreads, 1)
     for (int x = t; x <= a.nmax; x += kEpiThreads)
       if constexpr (MODE == kModeBinned)
         fast2::recip_entry4(x, reinterpret_cast<float4*>(tables) + x);
-      else
+      else if constexpr (MODE == kModePairs) {
+        float inv, r2, r3;
+        fast::recip_entry(x, &inv, &r2, &r3, tables + x);
+      } else
         fast::recip_entry(x, tables + x, tables + (a.nmax + 1) + x, tables + 2 * (a.nmax + 1) + x,
                           tables + 3 * (a.nmax + 1) + x);
     for (int x = t; MODE == kModeBinned && x <= n_bins; x += kEpiThreads) {
@@ -375,18 +382,20 @@ __global__ void __launch_bounds__(kThreads, 1)
     // ---------------- epilogue ----------------
     // Warp e reads TMEM lane quarter (warp & 3) and column half (e >> 2): the
     // 16 x 32 sub-tile i in i0 + 16*quarter + [0,16), j in j0 + 32*half + [0,32).
+    // Pairs mode: warps 0-7 on the even tiles of the CTA, 8-15 on the odd ones.
     const int e = warp - 4;
     const int quarter = warp & 3;
-    const int half = e >> 2;
+    const int half = (e >> 2) & 1;
+    constexpr int kSets = epi_warps(MODE) / 8;
     const double maxd = a.max_dist;
     const int maxd_int = maxd >= 2147483647.0 ? 2147483647 : (int)floor(maxd);
     const bool use_int = MODE != kModeWindows && (a.bcoord == nullptr) && (*a.ipos_bad == 0);
     Slot* my_acc = kacc + (size_t)e * n_bins * S;
     unsigned long long* my_cnt = kcnt + (size_t)e * n_bins;
-    int t = 0;
+    int t = kSets == 2 ? e >> 3 : 0;
     long long row_hint = 0;
-    int stg_step = 0;  // pairs mode: the warp's steps so far (staging buffer stg_step % 2)
-    for (long long item = blockIdx.x; item < n_items; item += gridDim.x, ++t) {
+    for (long long item = blockIdx.x + (long long)t * gridDim.x; item < n_items;
+         item += (long long)kSets * gridDim.x, t += kSets) {
       const int acc = t & 1;
       const uint32_t aph = (uint32_t)((t >> 1) & 1);
       const TileRef tr = decode_item<MODE>(a, item, row_hint);
@@ -454,16 +463,17 @@ __global__ void __launch_bounds__(kThreads, 1)
 
       // pairs mode: the band offsets of the thread's two rows, loaded before
       // the accumulator wait
-      long long pf_off0 = 0, pf_np0 = 0, pf_off1 = 0, pf_np1 = 0;
+      long long pf_off0 = 0, pf_off1 = 0;
+      int pf_np0 = 0, pf_np1 = 0;  // pairs of the row, none past the last SNP
       if constexpr (MODE == kModePairs) {
         const long long ibp = i0 + 16 * quarter + (lane >> 2);
         if (ibp < a.n_snp) {
           pf_off0 = a.pair_off[ibp];
-          pf_np0 = a.pair_off[ibp + 1] - pf_off0;
+          pf_np0 = (int)min(a.pair_off[ibp + 1] - pf_off0, a.n_snp - ibp - 1);
         }
         if (ibp + 8 < a.n_snp) {
           pf_off1 = a.pair_off[ibp + 8];
-          pf_np1 = a.pair_off[ibp + 9] - pf_off1;
+          pf_np1 = (int)min(a.pair_off[ibp + 9] - pf_off1, a.n_snp - ibp - 9);
         }
       }
 
@@ -551,12 +561,12 @@ __global__ void __launch_bounds__(kThreads, 1)
         // x 16 columns j) go through a shared-memory staging buffer: the lane
         // of each row then writes the row's band range with one bulk copy per
         // array (contiguous output rows, whole sectors); n goes out directly.
-        const long long ib = i0 + 16 * quarter + (lane >> 2);
-        const long long off0 = pf_off0, np0 = pf_np0, off1 = pf_off1, np1 = pf_np1;
+        // j - i - 1 of the lane's row of half 0 with the sub-tile's first column
+        const int dj = (int)(sj0 - si0) - (lane >> 2) - 1;
         unsigned char* wst = stg + (size_t)e * kStgWarp;
 #pragma unroll 1
         for (int c = 0; c < 4; ++c) {
-          const int hh = c & 1, gp = c >> 1;
+          const int hh = c >> 1, gp = c & 1;
           uint32_t r[16];
           tmem_ld16x256_x4(tmem_base + ((uint32_t)(quarter * 32 + hh * 16) << 16) +
                                (uint32_t)(acc * 256 + half * 64 + gp * 32),
@@ -567,15 +577,16 @@ __global__ void __launch_bounds__(kThreads, 1)
             __syncwarp();
             if (lane == 0) mbar_arrive(&ctrl->tempty[acc]);
           }
-          const long long is = ib + 8 * hh;
-          const long long offh = hh ? off1 : off0, nph = hh ? np1 : np0;
-          // this step's buffer is free once the copies issued from it two
-          // steps ago have read it (one bulk group per row lane and step)
-          unsigned char* buf = wst + (size_t)(stg_step & 1) * kStgBuf;
-          bulk_wait_read<1>();
+          const long long offh = hh ? pf_off1 : pf_off0;
+          const int nph = hh ? pf_np1 : pf_np0;
+          const int d0 = dj - 8 * hh + 16 * gp;  // j - i - 1 of the step's first column
+          // the buffer is free once the copies of the previous step have read
+          // it (one bulk group per row lane and step)
+          bulk_wait_read<0>();
           __syncwarp();
-          int4* cst = reinterpret_cast<int4*>(buf) + (lane >> 2) * 17;
-          float4* sst = reinterpret_cast<float4*>(buf + kStgArr) + (lane >> 2) * 17;
+          int4* cst = reinterpret_cast<int4*>(wst) + (lane >> 2) * 17;
+          float4* sst = reinterpret_cast<float4*>(wst + kStgArr) + (lane >> 2) * 17;
+          int* nst = reinterpret_cast<int*>(wst + 2 * kStgArr);
           auto u2 = [](uint32_t x, uint32_t y) {
             return make_float2(__uint_as_float(x), __uint_as_float(y));
           };
@@ -584,45 +595,50 @@ __global__ void __launch_bounds__(kThreads, 1)
             // the pairs (is, j) and (is, j + 1), two lanes of the packed epilogue
             const int o = 8 * g;
             const int jj = 8 * g + 2 * (lane & 3);  // column in the step's 16
-            const long long j = j0 + 32 * half + 16 * gp + jj;
             // a pair is written exactly when the band offsets list it
-            const bool ok0 = is < j && j < a.n_snp && (j - is - 1) < nph;
-            const bool ok1 = is < j + 1 && j + 1 < a.n_snp && (j - is) < nph;
+            const int d = d0 + jj;
+            const bool ok0 = d >= 0 && d < nph, ok1 = d + 1 >= 0 && d + 1 < nph;
             if (!ok0 && !ok1) continue;
             const fast2::Pop p = fast2::make(u2(r[o], r[o + 1]), u2(r[o + 4], r[o + 5]),
                                              u2(r[o + 2], r[o + 3]), u2(r[o + 6], r[o + 7]));
-            const long long k = offh + (j - is - 1);  // row of (is, j); (is, j + 1) follows
             float4 st[2];
             if (a.stats) fast2::pair_outputs(p, make_float2(T.r4[p.n0], T.r4[p.n1]), st);
 #pragma unroll
             for (int y = 0; y < 2; ++y) {
               const int q = o + y;
-              cst[jj + y] = make_int4(fast::f2i_small(__uint_as_float(r[q])),
-                                      fast::f2i_small(__uint_as_float(r[q + 4])),
-                                      fast::f2i_small(__uint_as_float(r[q + 2])),
-                                      fast::f2i_small(__uint_as_float(r[q + 6])));
+              // (the conversion unit is idle here, the integer pipe is not)
+              cst[jj + y] = make_int4(__float2int_rz(__uint_as_float(r[q])),
+                                      __float2int_rz(__uint_as_float(r[q + 4])),
+                                      __float2int_rz(__uint_as_float(r[q + 2])),
+                                      __float2int_rz(__uint_as_float(r[q + 6])));
               if (a.stats) sst[jj + y] = st[y];
-              if (a.nvalid) st_cs_if(y ? ok1 : ok0, a.nvalid + (k + y), y ? p.n1 : p.n0);
+              if (a.nvalid) nst[(lane >> 2) * 33 + 16 * gp + jj + y] = y ? p.n1 : p.n0;
             }
           }
           fence_proxy_async_smem();
           __syncwarp();
           if ((lane & 3) == 0) {
-            // the row's pairs in this step: columns jlo..jhi (j <= is + nph)
-            const long long jb = j0 + 32 * half + 16 * gp;
-            const long long jlo = jb > is + 1 ? jb : is + 1;
-            long long jhi = jb + 15 < a.n_snp - 1 ? jb + 15 : a.n_snp - 1;
-            if (is + nph < jhi) jhi = is + nph;
-            if (jlo <= jhi) {
-              const long long k0 = offh + (jlo - is - 1);
-              const uint32_t bytes = (uint32_t)(jhi - jlo + 1) * 16u;
-              const int q0 = (int)(jlo - jb);
+            // the row's pairs in this step: columns q0 .. q1 - 1
+            const int q0 = max(0, -d0), q1 = min(16, nph - d0);
+            if (q0 < q1) {
+              const long long k0 = offh + (d0 + q0);
+              const uint32_t bytes = (uint32_t)(q1 - q0) * 16u;
               bulk_store(reinterpret_cast<int4*>(a.counts) + k0, cst + q0, bytes);
               if (a.stats) bulk_store(reinterpret_cast<float4*>(a.stats) + k0, sst + q0, bytes);
             }
             bulk_commit();
           }
-          ++stg_step;
+          // n a row at a time, 32 columns: as 4-byte stores of each lane's pairs
+          // the sectors went out in pieces (n cost more than r^2, DD, Dz, pi2)
+          if (gp == 1 && a.nvalid) {
+#pragma unroll
+            for (int rr = 0; rr < 8; ++rr) {
+              const long long off = __shfl_sync(0xffffffffu, offh, 4 * rr);
+              const int np = __shfl_sync(0xffffffffu, nph, 4 * rr);
+              const int d = (int)(sj0 - si0) - 8 * hh - rr - 1 + lane;
+              if (d >= 0 && d < np) a.nvalid[off + d] = nst[rr * 33 + lane];
+            }
+          }
         }
         continue;
       }
@@ -1062,8 +1078,8 @@ static int tc_launch(pgld_context* h, const pgld_hap_panel* panel, pgld::BandArg
 
   const size_t fixed = sizeof(Ctrl) + (pgld::kMaxBins + 1) * 8 + (pgld::kMaxBins + 2) * 4 +
                        (size_t)kEpiWarps * a.n_bins * (S + 1) * 8 +
-                       (size_t)4 * (prm.nmax + 1) * sizeof(float) + 1024 +
-                       (mode == pgld::kModePairs ? (size_t)kEpiWarps * kStgWarp + 16 : 0);
+                       (size_t)n_tables(mode) * (prm.nmax + 1) * sizeof(float) + 1024 +
+                       (mode == pgld::kModePairs ? (size_t)epi_warps(mode) * kStgWarp + 32 : 0);
   int max_smem = 0;
   cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, h->device);
   int stages = (int)std::min<long long>(8, ((long long)max_smem - (long long)fixed) / kStageBytes);
@@ -1080,7 +1096,7 @@ static int tc_launch(pgld_context* h, const pgld_hap_panel* panel, pgld::BandArg
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return pgld_cuda_fail(h, e, "band_tc smem attribute");
   pgld_time_begin(h, st);
-  kern<<<(unsigned)h->n_sm, kThreads, smem, st>>>(maps[0], maps[1], prm);
+  kern<<<(unsigned)h->n_sm, threads_of(mode), smem, st>>>(maps[0], maps[1], prm);
   pgld_time_end(h, st);
   e = cudaGetLastError();
   if (e != cudaSuccess) return pgld_cuda_fail(h, e, "band_tc_kernel");
@@ -1238,7 +1254,7 @@ int pgld_tc_windows(pgld_context* h, const pgld_hap_panel* panel, const int32_t*
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return pgld_cuda_fail(h, e, "tc windows smem attribute");
   pgld_time_begin(h, st);
-  kern<<<(unsigned)h->n_sm, kThreads, smem, st>>>(map, map, prm);
+  kern<<<(unsigned)h->n_sm, threads_of(pgld::kModeWindows), smem, st>>>(map, map, prm);
   pgld_time_end(h, st);
   e = cudaGetLastError();
   if (e != cudaSuccess) return pgld_cuda_fail(h, e, "band_tc_kernel (windows)");
