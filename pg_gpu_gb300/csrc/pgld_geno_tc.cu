@@ -521,46 +521,49 @@ __global__ void __launch_bounds__(kPairThreads, 1)
 
 // operand rows: row 96 * (s / 32) + 32 * plane + s % 32 holds, per
 // individual, plane 0: 1 if the dosage at SNP s is known, plane 1: c = dosage
-// - 1 (+1, 0, -1; 0 if missing), plane 2: c^2.  A block
-// writes 8 rows, a warp one row in 16-byte chunks (16 individuals, one
-// nibble-to-bytes step per 4).
-__device__ __forceinline__ uint32_t e4m3_nibble(uint32_t mag, uint32_t neg) {
-  // byte q = (bit q of mag ? 1.0 : 0) with the sign bit from neg
-  uint32_t v = 0;
-#pragma unroll
-  for (int q = 0; q < 4; ++q)
-    v |= ((mag >> q & 1u) ? kOne : 0u) << (8 * q) | ((neg >> q & 1u) ? 0x80u : 0u) << (8 * q);
-  return v;
-}
-
+// - 1 (+1, 0, -1; 0 if missing), plane 2: c^2.  A warp
+// writes the three rows of its SNPs in 16-byte chunks (16 individuals), the
+// bit planes read once (1,000 individuals, 100,000 SNPs, 307 MB written: 104 us
+// with a warp per row, 53 us).
+constexpr int kPackSnps = 2;  // SNPs in flight per warp
 __global__ void __launch_bounds__(256) pack_gtc_kernel(const uint32_t* __restrict__ planes, int W,
                                                        long long n_snp, long long n_blocks,
                                                        int k_pad, uint32_t* __restrict__ out) {
-  const long long row = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
-  const int lane = threadIdx.x & 31;
-  if (row >= n_blocks * kBlkRows) return;
-  const int chunks = k_pad / 16;
-  uint4* dst = reinterpret_cast<uint4*>(out) + row * chunks;
-  const long long blk = row / kBlkRows;
-  const int within = (int)(row - blk * kBlkRows);
-  const int plane = within >> 5;
-  const long long s = blk * kTileSnp + (within & 31);
-  const uint32_t* ps = planes + (s < n_snp ? s : 0) * 3 * W;
-  for (int c = lane; c < chunks; c += 32) {
-    const int h0 = 16 * c;
-    const int w = h0 >> 5;
-    uint32_t mag = 0, neg = 0;
-    if (s < n_snp && w < W) {
-      const uint32_t g0 = __ldg(ps + w), g2 = __ldg(ps + 2 * W + w);
-      const uint32_t word = plane == 0 ? (g0 | __ldg(ps + W + w) | g2) : (g0 | g2);
-      mag = (word >> (h0 & 31)) & 0xFFFFu;
-      if (plane == 1) neg = (g0 >> (h0 & 31)) & 0xFFFFu;
-    }
-    uint32_t v[4];
+  const int lane = threadIdx.x & 31, chunks = k_pad / 16;
+  uint4* rows = reinterpret_cast<uint4*>(out);
+  const long long n_out = n_blocks * kTileSnp, step = (long long)gridDim.x * 8 * kPackSnps;
+  for (long long s0 = ((long long)blockIdx.x * 8 + (threadIdx.x >> 5)) * kPackSnps; s0 < n_out;
+       s0 += step) {
+    for (int c = lane; c < chunks; c += 32) {
+      const int w = c >> 1, sh = 16 * (c & 1);
+      uint32_t g[kPackSnps][3];
 #pragma unroll
-    for (int q = 0; q < 4; ++q) v[q] = e4m3_nibble(mag >> (4 * q), neg >> (4 * q));
-    dst[c] = make_uint4(v[0], v[1], v[2], v[3]);
+      for (int k = 0; k < kPackSnps; ++k)
+#pragma unroll
+        for (int d = 0; d < 3; ++d)
+          g[k][d] = s0 + k < n_snp && w < W ? __ldg(planes + (s0 + k) * 3 * W + d * W + w) >> sh : 0u;
+#pragma unroll
+      for (int k = 0; k < kPackSnps; ++k) {
+        const long long s = s0 + k;
+        uint4* dst = rows + ((s / kTileSnp) * kBlkRows + (s % kTileSnp)) * chunks + c;
+        const uint32_t hom = g[k][0] | g[k][2], known = hom | g[k][1];
+        uint32_t v[3][4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          v[0][q] = nibble_bytes(known >> (4 * q)) * kOne;
+          v[2][q] = nibble_bytes(hom >> (4 * q)) * kOne;
+          v[1][q] = v[2][q] | nibble_bytes(g[k][0] >> (4 * q)) * 0x80u;  // the sign bit
+        }
+#pragma unroll
+        for (int d = 0; d < 3; ++d)
+          dst[(long long)d * kTileSnp * chunks] = make_uint4(v[d][0], v[d][1], v[d][2], v[d][3]);
+      }
+    }
   }
+}
+static unsigned pack_gtc_blocks(const pgld_context* h, long long n_blocks) {
+  return (unsigned)std::max<long long>(
+      1, std::min<long long>((n_blocks * kTileSnp + 8 * kPackSnps - 1) / (8 * kPackSnps), h->n_sm * 16LL));
 }
 
 // ---------------------------------------------------------------------------
@@ -1016,8 +1019,7 @@ int pgld_geno_tc_pairs(pgld_context* h, const pgld_geno_panel* panel, const doub
     if (rc) return rc;
   }
   {
-    const unsigned blocks = (unsigned)std::max<long long>(1, (nb * kBlkRows + 7) / 8);
-    pack_gtc_kernel<<<blocks, 256, 0, st>>>(panel->planes[0], W, n, nb, k_pad, (uint32_t*)op);
+    pack_gtc_kernel<<<pack_gtc_blocks(h, nb), 256, 0, st>>>(panel->planes[0], W, n, nb, k_pad, (uint32_t*)op);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return pgld_cuda_fail(h, e, "pack_gtc_kernel");
   }
@@ -1115,8 +1117,7 @@ int pgld_geno_tc_binned(pgld_context* h, const pgld_geno_panel* panel, const pgl
   long long* items = (long long*)(w + off_items);
   unsigned char* op = (unsigned char*)(w + off_op);
   for (int p = 0; p < P; ++p) {
-    const unsigned blocks = (unsigned)std::max<long long>(1, (nb * kBlkRows + 7) / 8);
-    pack_gtc_kernel<<<blocks, 256, 0, st>>>(panel->planes[p], panel->n_words[p], n, nb, k_pad,
+    pack_gtc_kernel<<<pack_gtc_blocks(h, nb), 256, 0, st>>>(panel->planes[p], panel->n_words[p], n, nb, k_pad,
                                             (uint32_t*)(op + op_pop * p));
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return pgld_cuda_fail(h, e, "pack_gtc_kernel");

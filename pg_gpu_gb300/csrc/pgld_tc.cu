@@ -878,8 +878,9 @@ __global__ void pos_to_int_kernel(const double* __restrict__ pos, long long n, i
 // ---------------------------------------------------------------------------
 // Row order: interleaved (row 2r + plane: SNP r) or, with grouped, by groups of
 // 8 SNPs (row 16g + 8 plane + k: SNP 8g + k; n_rows rounded up to 8, rows of
-// SNPs past n_rows zero).  A block writes 8 operand rows, a warp one row in
-// 16-byte chunks (16 haplotypes: one nibble-to-bytes lookup per 4).
+// SNPs past n_rows zero).  A warp writes its rows in 16-byte chunks (16
+// haplotypes: one nibble-to-bytes product per 4).
+constexpr int kPackRows = 4;  // rows in flight per warp
 __global__ void __launch_bounds__(256) pack_tc_kernel(const uint32_t* __restrict__ planes, int W,
                                                       long long n_snp, long long n_rows,
                                                       const int32_t* __restrict__ idx, int k_pad,
@@ -888,43 +889,47 @@ __global__ void __launch_bounds__(256) pack_tc_kernel(const uint32_t* __restrict
                                                       const int* __restrict__ skip = nullptr) {
   if (skip && *skip) return;
   const long long rows_out = 2 * (grouped ? (n_rows + 7) / 8 * 8 : n_rows);
-  const long long rowi = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
-  const int lane = threadIdx.x & 31;
-  if (rowi >= rows_out) return;
-  const int chunks = k_pad / 16;
-  uint4* dst = reinterpret_cast<uint4*>(out) + rowi * chunks;
-  long long r;
-  int plane;
-  if (grouped) {
-    r = (rowi >> 4) * 8 + (rowi & 7);
-    plane = (int)((rowi >> 3) & 1);
-  } else {
-    r = rowi >> 1;
-    plane = (int)(rowi & 1);
-  }
-  long long s = -1;
-  if (r < n_rows) {
-    s = idx ? (long long)idx[r] : r;
-    if (s < 0 || s >= n_snp) {
-      if (status && lane == 0) atomicCAS(status, 0, 3102);
-      s = -1;
-    }
-  }
-  const uint32_t* src = planes + (s < 0 ? 0 : s) * 2 * W + plane * W;
-  for (int c = lane; c < chunks; c += 32) {
-    const int h0 = 16 * c;
-    const int w = h0 >> 5;
-    const uint32_t bits = (s >= 0 && w < W) ? (__ldg(src + w) >> (h0 & 31)) & 0xFFFFu : 0u;
-    uint32_t v[4];
+  const int lane = threadIdx.x & 31, chunks = k_pad / 16;
+  // a warp's rows in turn, kPackRows of them in flight
+  const long long step = (long long)gridDim.x * 8 * kPackRows;
+  for (long long row0 = ((long long)blockIdx.x * 8 + (threadIdx.x >> 5)) * kPackRows; row0 < rows_out;
+       row0 += step) {
+    const uint32_t* src[kPackRows];
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const uint32_t nib = (bits >> (4 * q)) & 0xFu;
-      // byte b of v[q] = E4M3 1.0 where bit b of the nibble is set
-      v[q] = (nib & 1u ? kOne : 0u) | (nib & 2u ? kOne << 8 : 0u) | (nib & 4u ? kOne << 16 : 0u) |
-             (nib & 8u ? kOne << 24 : 0u);
+    for (int k = 0; k < kPackRows; ++k) {
+      const long long rowi = row0 + k;
+      const long long r = grouped ? (rowi >> 4) * 8 + (rowi & 7) : rowi >> 1;
+      const int plane = (int)((grouped ? rowi >> 3 : rowi) & 1);
+      src[k] = nullptr;
+      if (rowi < rows_out && r < n_rows) {
+        const long long s = idx ? (long long)idx[r] : r;
+        if (s >= 0 && s < n_snp)
+          src[k] = planes + s * 2 * W + plane * W;
+        else if (status && lane == 0)
+          atomicCAS(status, 0, 3102);
+      }
     }
-    dst[c] = make_uint4(v[0], v[1], v[2], v[3]);
+    for (int c = lane; c < chunks; c += 32) {
+      const int w = c >> 1, sh = 16 * (c & 1);
+      uint32_t bits[kPackRows];
+#pragma unroll
+      for (int k = 0; k < kPackRows; ++k) bits[k] = src[k] && w < W ? __ldg(src[k] + w) >> sh : 0u;
+#pragma unroll
+      for (int k = 0; k < kPackRows; ++k) {
+        if (row0 + k >= rows_out) break;
+        uint32_t v[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+          v[q] = nibble_bytes(bits[k] >> (4 * q)) * kOne;
+        reinterpret_cast<uint4*>(out)[(row0 + k) * chunks + c] = make_uint4(v[0], v[1], v[2], v[3]);
+      }
+    }
   }
+}
+
+static unsigned pack_blocks(const pgld_context* h, long long rows) {
+  return (unsigned)std::max<long long>(
+      1, std::min<long long>((rows + 8 * kPackRows - 1) / (8 * kPackRows), h->n_sm * 16LL));
 }
 
 }  // namespace tc
@@ -1023,8 +1028,7 @@ static int tc_launch(pgld_context* h, const pgld_hap_panel* panel, pgld::BandArg
 
   // operands
   for (int p = 0; p < P; ++p) {
-    const unsigned blocks = (unsigned)((2 * n_op + 7) / 8);
-    pack_tc_kernel<<<std::max(1u, blocks), 256, 0, st>>>(panel->planes[p], panel->n_words[p], n,
+    pack_tc_kernel<<<pack_blocks(h, 2 * n_op), 256, 0, st>>>(panel->planes[p], panel->n_words[p], n,
                                                           n, nullptr, k_pad[p], grouped,
                                                           (uint32_t*)ops[p], h->dev_status);
     cudaError_t e = cudaGetLastError();
@@ -1135,8 +1139,7 @@ int pgld_tc_pack_rows(pgld_context* h, const uint32_t* planes, int W, long long 
                       long long n_rows, const int32_t* idx, int k_pad, unsigned char* out,
                       const int* skip, cudaStream_t st) {
   const long long rows_out = 2 * ((n_rows + 7) / 8 * 8);
-  const unsigned blocks = (unsigned)std::max<long long>(1, (rows_out + 7) / 8);
-  pgld::tc::pack_tc_kernel<<<blocks, 256, 0, st>>>(planes, W, n_snp, n_rows, idx, k_pad, 1,
+  pgld::tc::pack_tc_kernel<<<pgld::tc::pack_blocks(h, rows_out), 256, 0, st>>>(planes, W, n_snp, n_rows, idx, k_pad, 1,
                                                    (uint32_t*)out, h->dev_status, skip);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return pgld_cuda_fail(h, e, "pack_tc_kernel");
@@ -1211,8 +1214,7 @@ int pgld_tc_windows(pgld_context* h, const pgld_hap_panel* panel, const int32_t*
     if (rc) return rc;
   }
   if (n_idx > 0) {
-    const unsigned blocks = (unsigned)((2 * n_op + 7) / 8);
-    pack_tc_kernel<<<blocks, 256, 0, st>>>(panel->planes[0], W, n, n_idx, idx, k_pad, 1, (uint32_t*)op,
+    pack_tc_kernel<<<pack_blocks(h, 2 * n_op), 256, 0, st>>>(panel->planes[0], W, n, n_idx, idx, k_pad, 1, (uint32_t*)op,
                                            h->dev_status);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return pgld_cuda_fail(h, e, "pack_tc_kernel");

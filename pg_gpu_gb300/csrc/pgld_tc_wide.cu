@@ -1002,40 +1002,38 @@ __global__ void __launch_bounds__(kThreads, 1)
 // Both populations' bit planes -> one E4M3 operand (rows grouped by 8 SNPs:
 // row 16g + 8 plane + k is plane `plane` of SNP 8g + k; SNPs past n_snp are
 // zero rows).  Bytes [0, k0) of a row: population 0 (1.0), [k0, k0 + k1):
-// population 1 (64.0).  A block writes 8 rows, a warp one row in 16-byte
-// chunks.
+// population 1 (64.0).  A warp writes its rows in 16-byte chunks.
+constexpr int kPackRows = 4;  // rows in flight per warp
 __global__ void __launch_bounds__(256) pack_wide_kernel(const uint32_t* __restrict__ pl0, int W0,
                                                         const uint32_t* __restrict__ pl1, int W1,
                                                         long long n_snp, long long rows_out, int k0,
                                                         int k1, uint32_t* __restrict__ out) {
-  const long long rowi = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
-  const int lane = threadIdx.x & 31;
-  if (rowi >= rows_out) return;
-  const int chunks0 = k0 / 16, chunks = (k0 + k1) / 16;
-  uint4* dst = reinterpret_cast<uint4*>(out) + rowi * chunks;
-  const long long r = (rowi >> 4) * 8 + (rowi & 7);
-  const int plane = (int)((rowi >> 3) & 1);
-  const bool live = r < n_snp;
-  const uint32_t* src0 = pl0 + (live ? r : 0) * 2 * W0 + plane * W0;
-  const uint32_t* src1 = pl1 + (live ? r : 0) * 2 * W1 + plane * W1;
-  for (int c = lane; c < chunks; c += 32) {
-    const bool p1 = c >= chunks0;
-    const int h0 = 16 * (p1 ? c - chunks0 : c);
-    const int w = h0 >> 5;
-    const uint32_t one = p1 ? kOne64 : kOne;
-    uint32_t bits = 0u;
-    if (live) {
-      if (!p1 && w < W0) bits = (__ldg(src0 + w) >> (h0 & 31)) & 0xFFFFu;
-      if (p1 && w < W1) bits = (__ldg(src1 + w) >> (h0 & 31)) & 0xFFFFu;
-    }
-    uint32_t v[4];
+  const int lane = threadIdx.x & 31, chunks0 = k0 / 16, chunks = (k0 + k1) / 16;
+  const long long step = (long long)gridDim.x * 8 * kPackRows;
+  for (long long row0 = ((long long)blockIdx.x * 8 + (threadIdx.x >> 5)) * kPackRows; row0 < rows_out;
+       row0 += step) {
+    for (int c = lane; c < chunks; c += 32) {
+      const bool p1 = c >= chunks0;
+      const int h0 = 16 * (p1 ? c - chunks0 : c), w = h0 >> 5, W = p1 ? W1 : W0;
+      const uint32_t* pl = p1 ? pl1 : pl0;
+      const uint32_t one = p1 ? kOne64 : kOne;
+      uint32_t bits[kPackRows];
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const uint32_t nib = (bits >> (4 * q)) & 0xFu;
-      v[q] = (nib & 1u ? one : 0u) | (nib & 2u ? one << 8 : 0u) | (nib & 4u ? one << 16 : 0u) |
-             (nib & 8u ? one << 24 : 0u);
+      for (int k = 0; k < kPackRows; ++k) {
+        const long long rowi = row0 + k, r = (rowi >> 4) * 8 + (rowi & 7);
+        const int plane = (int)((rowi >> 3) & 1);
+        bits[k] = rowi < rows_out && r < n_snp && w < W
+                      ? __ldg(pl + r * 2 * W + plane * W + w) >> (h0 & 31) : 0u;
+      }
+#pragma unroll
+      for (int k = 0; k < kPackRows; ++k) {
+        if (row0 + k >= rows_out) break;
+        uint32_t v[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) v[q] = nibble_bytes(bits[k] >> (4 * q)) * one;
+        reinterpret_cast<uint4*>(out)[(row0 + k) * chunks + c] = make_uint4(v[0], v[1], v[2], v[3]);
+      }
     }
-    dst[c] = make_uint4(v[0], v[1], v[2], v[3]);
   }
 }
 
@@ -1121,7 +1119,8 @@ int pgld_tc_wide_binned(pgld_context* h, const pgld_hap_panel* panel, pgld::Band
   long long* items = (long long*)(w + off_items);
   unsigned char* op = (unsigned char*)(w + off_op);
   {
-    const unsigned blocks = (unsigned)((2 * n_op + 7) / 8);
+    const unsigned blocks = (unsigned)std::max<long long>(
+        1, std::min<long long>((2 * n_op + 8 * kPackRows - 1) / (8 * kPackRows), h->n_sm * 16LL));
     pack_wide_kernel<<<blocks, 256, 0, st>>>(panel->planes[0], panel->n_words[0], panel->planes[1],
                                              panel->n_words[1], n, 2 * n_op, k0, k1, (uint32_t*)op);
     cudaError_t e = cudaGetLastError();
@@ -1285,7 +1284,8 @@ int pgld_tc_wide_pairs(pgld_context* h, const pgld_hap_panel* panel, pgld::BandA
     if (rc) return rc;
   }
   {
-    const unsigned blocks = (unsigned)((2 * n_op + 7) / 8);
+    const unsigned blocks = (unsigned)std::max<long long>(
+        1, std::min<long long>((2 * n_op + 8 * kPackRows - 1) / (8 * kPackRows), h->n_sm * 16LL));
     pack_wide_kernel<<<blocks, 256, 0, st>>>(panel->planes[0], W, panel->planes[0], 0, n, 2 * n_op,
                                              k0, 0, (uint32_t*)op);
     cudaError_t e = cudaGetLastError();

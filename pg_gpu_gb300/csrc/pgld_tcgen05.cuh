@@ -250,6 +250,11 @@ __device__ __forceinline__ void st_cs_if(bool p, int4* ptr, int4 v) {
       "l"(ptr), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w));
 }
 
+// bit b of a nibble to bit 0 of byte b (the four products share no bit)
+__device__ __forceinline__ uint32_t nibble_bytes(uint32_t x) {
+  return ((x & 0xFu) * 0x00204081u) & 0x01010101u;
+}
+
 struct Ctrl {
   uint64_t full[8], empty[8], tfull[2], tempty[2], drain;
   uint32_t tmem_base;

@@ -164,9 +164,7 @@ __global__ void __launch_bounds__(256) pack_complete_kernel(
         const uint32_t bits = (lane & 1) ? word >> 16 : word & 0xffffu;
         uint32_t v[4];
 #pragma unroll
-        for (int y = 0; y < 4; ++y)
-          // bit b of the nibble to byte b (the four products share no bit)
-          v[y] = ((((bits >> (4 * y)) & 0xfu) * 0x00204081u) & 0x01010101u) * kOne;
+        for (int y = 0; y < 4; ++y) v[y] = nibble_bytes(bits >> (4 * y)) * kOne;
         if (ch < 2 * W) dst[ch] = make_uint4(v[0], v[1], v[2], v[3]);
       }
     }
