@@ -5,28 +5,26 @@
 // from the nine centred moments m[3 x + y] = sum c_i^x c_j^y over the
 // individuals valid at both SNPs, c = dosage - 1 in {-1, 0, 1}
 // (pgld_geno_mom.cuh).  Those are dot products over the individuals: with A =
-// the planes (valid, c, c^2) of 32 SNPs i and B the same for 32 SNPs j,
+// the planes (valid, c, c^2) of 32 SNPs j and B the same for 32 SNPs i,
 // D = A B^T holds m[3 x + y] for all 1,024 pairs of the tile.  The operand
 // rows are plane-major within a 32-SNP block (row = 96 * block + 32 * plane
-// + SNP), so D[32 x + i][32 y + j] = m[3 x + y](i, j); the A tile's rows
+// + SNP), so D[32 y + j][32 x + i] = m[3 x + y](i, j); the A tile's rows
 // 96..127 (M = 128) are zero rows kept in shared memory.
 // Operands are E4M3 bytes (0x38 = 1.0, 0xB8 = -1.0) in K-major rows padded to
 // 128 bytes; the float32 accumulators hold integers of magnitude below 2^24,
 // so the moments are exact.
 //
 // One CTA per SM:
-//   warp 0      TMA producer (96-row x 128-byte boxes, SWIZZLE_128B; 28 KB
-//               stages, so six are in flight)
-//   warp 1      allocates 256 TMEM columns; one lane issues M=128 N=96 K=32
-//               kind::f8f6f4 MMAs (the B rows of planes 0-2) into
-//               accumulator stage t % 2
-//   warps 4-11  epilogue: two groups of four warps on alternate tiles
-//               (accumulator stage and moment buffer per group); in a group
-//               the warps of TMEM lane quarters 0-2 (planes 0-2) copy the
-//               3 x 3 moment blocks to shared memory, then all four turn
-//               1,024 pairs into outputs (8 per thread)
+//   warp 0      TMA producer (96-row x 128-byte boxes, SWIZZLE_128B)
+//   warp 1      allocates the TMEM columns; one lane issues M=128 N=96 K=32
+//               kind::f8f6f4 MMAs (the B rows of planes 0-2) into the tile's
+//               accumulator stage
+//   warps 4-    epilogue: two to four groups of four warps take the tiles in
+//               turn; in a group the warps of TMEM lane quarters 0-2 (planes
+//               0-2) copy the moments to shared memory, then all four turn the
+//               pairs into outputs or sums
 // Every mbarrier wait is bounded; the warps of an epilogue group meet at
-// their named barrier twice per tile and agree on aborting at the first.
+// their named barrier and agree on aborting at the first meeting of a tile.
 #include <cuda.h>
 #include <cuda_runtime.h>
 
@@ -48,8 +46,6 @@ namespace gtc {
 using namespace pgld::tc;
 
 constexpr int kTileSnp = 32;          // SNPs per tile side (4 planes = 128 rows)
-constexpr int kEpiWarps = 8;
-constexpr int kThreads = (4 + kEpiWarps) * 32;
 constexpr uint32_t kTmemCols = 256;   // two accumulator stages of 128 columns
 constexpr int kBlkRows = 96;          // operand rows of a 32-SNP block (3 planes)
 constexpr int kABytes = kBoxBytes;     // A: 96 loaded rows + 32 zero rows (M = 128)
@@ -96,7 +92,8 @@ constexpr int kChunkItems = 16;  // consecutive tiles a CTA takes per turn (resi
 // B barriers and the per-stage tile flags the producer hands the MMA issuer
 struct GCtrl : Ctrl {
   uint64_t bfull, bempty;
-  uint64_t gfull[kMaxGroups], gempty[kMaxGroups];  // the pairs kernel's accumulator stages
+  uint64_t gfull[kMaxGroups];   // an epilogue group's next tile is accumulated
+  uint64_t gempty[kMaxGroups];  // an accumulator stage is copied
   int meta[8];  // first stage of a tile: bit 0 = first tile of a strip, bit 1 = last
 };
 
@@ -578,9 +575,15 @@ static unsigned pack_gtc_blocks(const pgld_context* h, long long n_blocks) {
 // fewer than four valid individuals in a population, where the reference's
 // thresholds and zero denominators differ from statistic to statistic, goes
 // through the exact term table by itself.  Sums per distance bin in float64
-// slots of the CTA.  G epilogue groups take alternate tiles: G = 2 for at most
-// two populations (two accumulator stages of 256 columns), G = 1 for three or
-// four (one stage of 384 columns).
+// slots of the CTA.  G epilogue groups take the tiles in turn, each with a
+// moment buffer of its own; the accumulator stages (four of one population, two
+// of two, one of three or four) are freed once copied.  Bound by the
+// statistics' instructions, about 600 a pair of two populations: 500
+// individuals, 100,000 SNPs, 12 bins to 100 kb (1.0e8 pairs) 4.1 ms with two
+// groups, 3.6 with three (sixteen warps in two groups: 5.1, registers and totals
+// of four steps); three populations of 200, 20,000 SNPs 1.78 and 1.41 ms with one
+// group of eight warps and two of four; one population of 200, 60,000 SNPs: 1.5 ms
+// with distances and bins in 64 bits and a butterfly per total, 0.86 here.
 // ---------------------------------------------------------------------------
 struct BParams {
   int kchunks;
@@ -627,14 +630,22 @@ __device__ __noinline__ void term_table_pair(const gmom::Mom* mo, const BParams&
   }
 }
 
+// G groups of kGW epilogue warps take the tiles in turn, A accumulator stages
+// (four populations leave room for one group's moments only)
 template <int P>
-__global__ void __launch_bounds__(kThreads, 1)
+struct Binned {
+  static constexpr int G = P == 1 ? 4 : P == 2 ? 3 : P == 3 ? 2 : 1;
+  static constexpr int kGW = P <= 2 ? 4 : 8 / G;
+  static constexpr int A = P == 1 ? 4 : P == 2 ? 2 : 1;
+  static constexpr int kThreads = (4 + G * kGW) * 32;
+};
+template <int P>
+__global__ void __launch_bounds__(Binned<P>::kThreads, 1)
     gtc_binned_kernel(const __grid_constant__ CUtensorMap map, const __grid_constant__ BParams a,
                       const __grid_constant__ multi::Places pl) {
-  constexpr int G = P <= 2 ? 2 : 1;
-  constexpr int kGW = kEpiWarps / G;   // warps per epilogue group
+  constexpr int G = Binned<P>::G, A = Binned<P>::A, kGW = Binned<P>::kGW;
   constexpr int kRows = 32 / kGW;      // rows of a tile per warp
-  constexpr uint32_t kStageCols = G == 2 ? 256u : 0u;
+  constexpr uint32_t kStageCols = 512u / A;
   extern __shared__ unsigned char smem_dyn[];
   unsigned char* base = smem_dyn + ((1024 - (smem_u32(smem_dyn) & 1023)) & 1023);
   const int stages = a.stages;
@@ -655,10 +666,8 @@ __global__ void __launch_bounds__(kThreads, 1)
       mbar_init(&ctrl->full[s], 1);
       mbar_init(&ctrl->empty[s], 1);
     }
-    for (int s = 0; s < G; ++s) {
-      mbar_init(&ctrl->tfull[s], 1);
-      mbar_init(&ctrl->tempty[s], kGW);
-    }
+    for (int s = 0; s < G; ++s) mbar_init(&ctrl->gfull[s], 1);
+    for (int s = 0; s < A; ++s) mbar_init(&ctrl->gempty[s], kGW);
     mbar_init(&ctrl->drain, 1);
     ctrl->abort_flag = 0;
     ctrl->consumed = 0;
@@ -716,9 +725,9 @@ __global__ void __launch_bounds__(kThreads, 1)
             unsigned char* sa = ring + (size_t)stage * kGStageBytes;
             mbar_expect_tx(&ctrl->full[stage], 2 * kBBytes);
             tma_load_2d(sa, &map, &ctrl->full[stage], kc * kKChunk,
-                        p * a.pop_rows + (int)(lo * kBlkRows));
-            tma_load_2d(sa + kABytes, &map, &ctrl->full[stage], kc * kKChunk,
                         p * a.pop_rows + (int)(jb * kBlkRows));
+            tma_load_2d(sa + kABytes, &map, &ctrl->full[stage], kc * kKChunk,
+                        p * a.pop_rows + (int)(lo * kBlkRows));
             ++issued;
             if (++stage == stages) {
               stage = 0;
@@ -748,9 +757,9 @@ __global__ void __launch_bounds__(kThreads, 1)
       bool any = false, ok = true;
       for (int t = 0; ok && !*abort_flag; ++t) {
         if ((long long)blockIdx.x + (long long)t * gridDim.x >= n_items) break;
-        const int sg = t % G;
-        const uint32_t tph = (uint32_t)((t / G) & 1);
-        if (!mbar_wait_role(&ctrl->tempty[sg], tph ^ 1, abort_flag)) {
+        const int sg = t % A;
+        const uint32_t tph = (uint32_t)((t / A) & 1);
+        if (!mbar_wait_role(&ctrl->gempty[sg], tph ^ 1, abort_flag)) {
           set_abort(ctrl, a.status, 4103);
           break;
         }
@@ -779,7 +788,7 @@ __global__ void __launch_bounds__(kThreads, 1)
           }
         }
         if (!ok) break;
-        mma_commit(&ctrl->tfull[sg]);
+        mma_commit(&ctrl->gfull[t % G]);
       }
       if (*abort_flag && any) {
         mma_commit(&ctrl->drain);
@@ -791,18 +800,21 @@ __global__ void __launch_bounds__(kThreads, 1)
     const int e = warp - 4;
     const int grp = e / kGW;
     const int gi = e % kGW;                // warp within the group
-    const int wq = warp & 3;               // TMEM lane quarter: plane wq of the SNPs i
+    const int wq = warp & 3;               // TMEM lane quarter: plane wq of the SNPs j
     const uint32_t lane_base = (uint32_t)(wq * 32) << 16;
     const uint32_t bar_id = 1u + (uint32_t)grp;
     int16_t* gbuf = cnt + (size_t)grp * P * 96 * kCntPitch;
     const bool use_int = a.bcoord == nullptr && *a.ipos_bad == 0;
     const int maxd_int = a.max_dist >= 2147483647.0 ? 2147483647 : (int)floor(a.max_dist);
     long long lo = 0;
+    // the tile is ready on the group's own barrier, whose phases the group alone
+    // follows (a stage's would pass through other groups' tiles)
     for (int t = grp, u = 0;; t += G, ++u) {
+      const int sg = t % A;  // accumulator stage
       const long long item = (long long)blockIdx.x + (long long)t * gridDim.x;
       if (item >= n_items) break;
       bool ready = true;
-      if (lane == 0) ready = mbar_wait(&ctrl->tfull[grp], (uint32_t)(u & 1), abort_flag);
+      if (lane == 0) ready = mbar_wait(&ctrl->gfull[grp], (uint32_t)(u & 1), abort_flag);
       ready = __shfl_sync(0xffffffffu, ready ? 1 : 0, 0) != 0;
       if (!ready && lane == 0) set_abort(ctrl, a.status, 4105);
       // the group meets before overwriting its moment buffers and takes one
@@ -822,27 +834,28 @@ __global__ void __launch_bounds__(kThreads, 1)
       if (wq < 3) {
         const int half = gi >> 2;   // 0 with four warps per group
         for (int p = half; p < P; p += kGW / 4) {
-          int16_t* row = gbuf + ((size_t)p * 96 + wq * 32 + lane) * kCntPitch;
+          uint32_t* row = reinterpret_cast<uint32_t*>(gbuf + ((size_t)p * 96 + wq * 32 + lane) * kCntPitch);
 #pragma unroll 1
           for (int h = 0; h < 2; ++h) {
             uint32_t r[3][16];
 #pragma unroll
             for (int c = 0; c < 3; ++c)
               tmem_ld16(tmem_base + lane_base +
-                            ((uint32_t)grp * kStageCols + (uint32_t)(p * 96 + 48 * h + 16 * c)),
+                            ((uint32_t)sg * kStageCols + (uint32_t)(p * 96 + 48 * h + 16 * c)),
                         r[c]);
             tmem_wait_ld();
 #pragma unroll
             for (int c = 0; c < 3; ++c)
 #pragma unroll
-              for (int v = 0; v < 16; ++v)
-                row[48 * h + 16 * c + v] = (int16_t)fast::f2i_small(__uint_as_float(r[c][v]));
+              for (int v = 0; v < 8; ++v)
+                row[24 * h + 8 * c + v] =
+                    fast::f2i_pair(__uint_as_float(r[c][2 * v]), __uint_as_float(r[c][2 * v + 1]));
           }
         }
       }
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(&ctrl->tempty[grp]);
+      if (lane == 0) mbar_arrive(&ctrl->gempty[sg]);
       asm volatile("bar.sync %0, %1;" ::"r"(bar_id), "r"(kGW * 32) : "memory");
 
       lo = advance_block(a.item_off, a.n_blocks, lo, item);
@@ -891,7 +904,7 @@ __global__ void __launch_bounds__(kThreads, 1)
             for (int x = 0; x < 3; ++x)
 #pragma unroll
               for (int y = 0; y < 3; ++y)
-                mo[p].m[3 * x + y] = bp[(x * 32 + il) * kCntPitch + y * 32 + jl];
+                mo[p].m[3 * x + y] = bp[(y * 32 + jl) * kCntPitch + x * 32 + il];
             n_least = min(n_least, mo[p].m[0]);
           }
           const bool live = pair < multi::kGroupPairs;
@@ -917,50 +930,77 @@ __global__ void __launch_bounds__(kThreads, 1)
         continue;
       }
       // one population: DD, Dz, pi2 in float32 from the moments
-      // (gmom::stats_f32, within 1e-6 relative of each exact value)
-      const double pj = j_ok ? a.pos[j] : 0.0;
-      const double cj = (j_ok && a.bcoord) ? a.bcoord[j] : 0.0;
+      // (gmom::stats_f32, within 1e-6 relative of each exact value), summed over
+      // each row's pairs of a bin; eight rows at a time, whose totals take 24
+      // exchanges together instead of 15 each (the sums are the same: every step
+      // adds the same two halves)
+      const int pj = use_int && j_ok ? a.ipos[j] : 0;
+      const int pi = use_int && i0 + lane < a.n_snp ? a.ipos[i0 + lane] : 0;
+      const double pj64 = !use_int && j_ok ? a.pos[j] : 0.0;
+      const double cj = j_ok && a.bcoord ? a.bcoord[j] : 0.0;
 #pragma unroll 1
-      for (int k = 0; k < 32 / kGW; ++k) {
-        const int il = gi + kGW * k;
-        const long long i = i0 + il;
-        bool ok = i < j && j_ok;
-        double dpos = 0.0;
-        if (ok) {
-          dpos = pj - a.pos[i];
-          ok = dpos <= a.max_dist;
-        }
-        int b = -1;
-        if (ok) {
-          const double d = a.bcoord ? fabs(cj - a.bcoord[i]) : dpos;
-          b = bin_of_f64(sbins, a.n_bins, d);
-        }
-        unsigned pending = __ballot_sync(0xffffffffu, b >= 0);
-        if (!pending) continue;
-        gmom::Mom mo;
+      for (int k0 = 0; k0 < kRows; k0 += 8) {
+        float v[24];
+        int bins[8];  // bin of the lane's pair of each row
+        unsigned more = 0;  // rows with pairs of another bin than the first
 #pragma unroll
-        for (int x = 0; x < 3; ++x)
-#pragma unroll
-          for (int y = 0; y < 3; ++y)
-            mo.m[3 * x + y] = gbuf[(x * 32 + il) * kCntPitch + y * 32 + lane];
-        const float4 o4 = gmom::stats_f32<14>(mo, 14);
-        while (pending) {
-          const int bb = __shfl_sync(0xffffffffu, b, __ffs(pending) - 1);
-          const bool mine = (b == bb);
-          const unsigned grpm = __ballot_sync(0xffffffffu, mine);
-          float v[3] = {mine ? o4.y : 0.f, mine ? o4.z : 0.f, mine ? o4.w : 0.f};
-#pragma unroll
-          for (int q = 0; q < 3; ++q) {
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) v[q] += __shfl_xor_sync(0xffffffffu, v[q], o);
+        for (int k = 0; k < 8; ++k) {
+          const int il = gi + kGW * (k0 + k);
+          const long long i = i0 + il;
+          int b = -1;
+          if (use_int) {
+            const int d = pj - __shfl_sync(0xffffffffu, pi, il);
+            if (i < j && j_ok && d <= maxd_int) b = bin_of_int(thr, a.n_bins, d);
+          } else if (i < j && j_ok) {
+            const double dpos = pj64 - a.pos[i];
+            if (dpos <= a.max_dist)
+              b = bin_of_f64(sbins, a.n_bins, a.bcoord ? fabs(cj - a.bcoord[i]) : dpos);
           }
-          if (lane == 0) {
-#pragma unroll
-            for (int q = 0; q < 3; ++q) atomicAdd(&acc[bb * 3 + q], (double)v[q]);
-            atomicAdd(&bcnt[bb], (unsigned long long)__popc(grpm));
-          }
-          pending &= ~grpm;
+          bins[k] = b;
         }
+        float4 o4[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+          const int il = gi + kGW * (k0 + k);
+          gmom::Mom mo;
+#pragma unroll
+          for (int x = 0; x < 3; ++x)
+#pragma unroll
+            for (int y = 0; y < 3; ++y)
+              mo.m[3 * x + y] = gbuf[(y * 32 + lane) * kCntPitch + x * 32 + il];
+          o4[k] = gmom::stats_f32<14>(mo, 14);
+        }
+        unsigned pending[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) pending[k] = __ballot_sync(0xffffffffu, bins[k] >= 0);
+        do {
+          int slot = -1;  // lane k: the bin of row k in this turn
+          more = 0;
+#pragma unroll
+          for (int k = 0; k < 8; ++k) {
+            v[3 * k] = v[3 * k + 1] = v[3 * k + 2] = 0.f;
+            if (!pending[k]) continue;
+            const int bb = __shfl_sync(0xffffffffu, bins[k], __ffs(pending[k]) - 1);
+            const bool mine = bins[k] == bb;
+            const unsigned same = __ballot_sync(0xffffffffu, mine);
+            if (mine) {
+              v[3 * k] = o4[k].y;
+              v[3 * k + 1] = o4[k].z;
+              v[3 * k + 2] = o4[k].w;
+            }
+            if (lane == k) {
+              slot = bb;
+              atomicAdd(&bcnt[bb], (unsigned long long)__popc(same));
+            }
+            pending[k] &= ~same;
+            more |= pending[k];
+          }
+          // lane l: the totals of value multi::halved<24>(0)
+          multi::halve_plain<24>(v);
+          const int at = multi::halved<24>(0);
+          const int bb = __shfl_sync(0xffffffffu, slot, at < 0 ? 0 : at / 3);
+          if (at >= 0 && bb >= 0) atomicAdd(&acc[bb * 3 + at % 3], (double)v[0]);
+        } while (more);
       }
     }
   }
@@ -1152,9 +1192,11 @@ int pgld_geno_tc_binned(pgld_context* h, const pgld_geno_panel* panel, const pgl
   prm.sums = ba.sums;
   prm.pair_counts = reinterpret_cast<unsigned long long*>(ba.pair_counts);
   prm.status = h->dev_status;
-  const int G = P <= 2 ? 2 : 1;
-  const size_t group_bytes = G == 2 ? 2 * sizeof(pgld::multi::Groups<kEpiWarps / 2>)
-                                    : sizeof(pgld::multi::Groups<kEpiWarps>);
+  const int G = P == 1 ? Binned<1>::G : P == 2 ? Binned<2>::G : P == 3 ? Binned<3>::G : Binned<4>::G;
+  const int threads = P == 1   ? Binned<1>::kThreads
+                      : P == 2 ? Binned<2>::kThreads
+                      : P == 3 ? Binned<3>::kThreads : Binned<4>::kThreads;
+  const size_t group_bytes = P == 1 ? 0 : G * sizeof(pgld::multi::Groups<8>);
   const size_t fixed = sizeof(GCtrl) + (size_t)G * P * 96 * kCntPitch * 2 +
                        (size_t)(pgld::kMaxBins + 1) * 8 + (size_t)ba.n_bins * ba.n_stats * 8 +
                        (size_t)ba.n_bins * 8 + (size_t)(pgld::kMaxBins + 2) * 4 + group_bytes + 1024;
@@ -1173,7 +1215,7 @@ int pgld_geno_tc_binned(pgld_context* h, const pgld_geno_panel* panel, const pgl
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return pgld_cuda_fail(h, e, "gtc binned smem attribute");
   pgld_time_begin(h, st);
-  kern<<<(unsigned)h->n_sm, kThreads, smem, st>>>(map, prm, pl);
+  kern<<<(unsigned)h->n_sm, threads, smem, st>>>(map, prm, pl);
   pgld_time_end(h, st);
   e = cudaGetLastError();
   if (e != cudaSuccess) return pgld_cuda_fail(h, e, "gtc_binned_kernel");

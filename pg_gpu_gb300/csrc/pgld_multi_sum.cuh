@@ -52,6 +52,18 @@ __device__ __forceinline__ void halve(float* v, float* e) {
   }
   if constexpr (O > 1) halve<H, O / 2>(v, e);
 }
+// the same without the errors: each total is the butterfly's
+template <int N, int O = 16>
+__device__ __forceinline__ void halve_plain(float* v) {
+  constexpr int H = (N + 1) / 2;
+  const bool up = (threadIdx.x & O) != 0;
+#pragma unroll
+  for (int k = 0; k < H; ++k) {
+    const float hi = k + H < N ? v[k + H] : 0.f;
+    v[k] = __fadd_rn(up ? hi : v[k], __shfl_xor_sync(0xffffffffu, up ? v[k] : hi, O));
+  }
+  if constexpr (O > 1) halve_plain<H, O / 2>(v);
+}
 template <int N, int O = 16>
 __device__ __forceinline__ constexpr int halved_len() {
   if constexpr (O == 0)
