@@ -18,6 +18,7 @@
 #include "pgld_band.cuh"
 #include "pgld_epilogue.cuh"
 #include "pgld_internal.cuh"
+#include "pgld_multi_sum.cuh"
 #include "pgld_scan.cuh"
 #include "pgld_window.cuh"
 
@@ -29,6 +30,7 @@ namespace win {
 constexpr int kT = 32;
 constexpr int kKW = 32;
 constexpr int kPad = 33;
+constexpr int kPadRows = 36;  // 16-byte aligned rows
 constexpr int kThreads = 256;
 constexpr int kCols = 6;  // r2, sigma_D^2, DD, Dz, pi2, naive r2
 constexpr int kCnts = 3;  // pairs, pairs with r2 defined, pairs with n >= 4
@@ -90,34 +92,55 @@ __global__ void site_freq_kernel(const uint32_t* __restrict__ planes,
   }
 }
 
-__device__ __forceinline__ void stage(uint32_t (*dst)[kPad], const uint32_t* __restrict__ src,
-                                      const int32_t* __restrict__ idx, i64 a0, i64 a_end,
-                                      i64 stride, int w0, int W, i64 n_snp, int32_t* status) {
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-#pragma unroll
-  for (int q = 0; q < kT / (kThreads / 32); ++q) {
-    const int sl = wid * (kT / (kThreads / 32)) + q;
-    const i64 a = a0 + sl;
-    const int w = w0 + lane;
-    uint32_t v = 0;
-    if (a < a_end && w < W) {
-      const i64 s = idx ? (i64)idx[a] : a;
-      if (s >= 0 && s < n_snp)
-        v = __ldg(src + s * stride + w);
-      else
-        atomicCAS(status, 0, 3101);
+struct __align__(16) Smem {
+  uint32_t ci[kKW][kPadRows], zi[kKW][kPadRows], vi[kKW][kPadRows];
+  uint32_t cj[kKW][kPad], zj[kKW][kPad], vj[kKW][kPad];
+};
+
+// the words [w0, w0 + 32) of the planes of the tile's rows (list positions from
+// a0) and columns (from b0), zeros past the list's end.  L (8, 16 or 32, at least
+// the words staged) lanes to a SNP, which look its index up once for both
+// planes.  Row r is kept at 4 (r % 8) + r / 8, so that the four rows of warp w
+// (w, w + 8, w + 16, w + 24) are one 16-byte load.
+__device__ __forceinline__ void stage(Smem& sm, const Args& a, i64 a0, i64 b0, i64 end, int w0, int lsh) {
+  const int L = 1 << lsh, w = threadIdx.x & (L - 1);
+  const bool wok = w0 + w < a.W;
+  for (int x = threadIdx.x; x < 2 * kT * L; x += kThreads) {
+    const int row = x >> lsh, r = row & (kT - 1);
+    const bool col = row >= kT;
+    const i64 at = (col ? b0 : a0) + r;
+    uint32_t c = 0, z = 0, v = 0;
+    if (at < end && wok) {
+      const i64 s = a.idx ? (i64)a.idx[at] : at;
+      if (s >= 0 && s < a.n_snp) {
+        const uint32_t* p = a.planes + s * 2 * a.W + w0 + w;
+        c = __ldg(p);
+        z = __ldg(p + a.W);
+        if (a.valid) v = __ldg(a.valid + s * a.W + w0 + w);
+      } else {
+        atomicCAS(a.status, 0, 3101);
+      }
     }
-    dst[lane][sl] = v;
+    if (col) {
+      sm.cj[w][r] = c;
+      sm.zj[w][r] = z;
+      if (a.valid) sm.vj[w][r] = v;
+    } else {
+      const int k = 4 * (r & 7) + (r >> 3);
+      sm.ci[w][k] = c;
+      sm.zi[w][k] = z;
+      if (a.valid) sm.vi[w][k] = v;
+    }
   }
 }
 
-struct __align__(16) Smem {
-  uint32_t ci[kKW][kPad], zi[kKW][kPad], cj[kKW][kPad], zj[kKW][kPad];
-  uint32_t vi[kKW][kPad], vj[kKW][kPad];
-};
-
+// Bound by issue: staging, 12 instructions per word and pair for the counts and
+// the statistic.  Per-SNP sums of r^2, 200 windows of 200-2,000 SNPs, 401
+// haplotypes (8.8e7 pairs): 1.18 ms with a lane of 32 per staged word, an index
+// lookup per plane and a butterfly per row, 0.99 ms here (four CTAs per SM: with
+// more registers than 64 it waits for its loads, 1.33 ms at 80).
 template <bool SNP>
-__global__ void __launch_bounds__(kThreads) window_kernel(Args a) {
+__global__ void __launch_bounds__(kThreads, 4) window_kernel(Args a) {
   __shared__ Smem sm;
   extern __shared__ float tabs[];  // 1/n and 1/(n(n-1)(n-2)(n-3)), n = 0..nmax
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -129,24 +152,40 @@ __global__ void __launch_bounds__(kThreads) window_kernel(Args a) {
   }
   __syncthreads();
   i64 n_items = a.tile_off[a.n_win];
+  const int lsh = a.W <= 8 ? 3 : a.W <= 16 ? 4 : 5;
+  int w = 0;
   for (i64 item = blockIdx.x; item < n_items; item += gridDim.x) {
-    // window of the item, then its tile (bi, bj), bj >= bi, in row-major order
-    int lo = 0, hi = a.n_win;
-    while (hi - lo > 1) {
-      const int mid = (lo + hi) >> 1;
-      if (a.tile_off[mid] <= item) lo = mid; else hi = mid;
+    // window of the item (a CTA's items ascend: a few steps forward, else a
+    // search), then its tile (bi, bj), bj >= bi, in row-major order: row bi
+    // starts at bi T - bi (bi - 1) / 2, whose root starts the search
+    int steps = 0;
+    while (w + 1 < a.n_win && a.tile_off[w + 1] <= item && steps < 4) {
+      ++w;
+      ++steps;
     }
-    const int w = lo;
+    if (steps == 4) {
+      int hi = a.n_win;
+      while (hi - w > 1) {
+        const int mid = (w + hi) >> 1;
+        if (a.tile_off[mid] <= item) w = mid; else hi = mid;
+      }
+    }
     const i64 base = a.win_begin[w], m = a.win_end[w] - base;
-    const i64 T = (m + kT - 1) / kT;
-    const i64 t = item - a.tile_off[w];
-    i64 rlo = 0, rhi = T;  // row bi starts at bi*T - bi(bi-1)/2
-    while (rhi - rlo > 1) {
-      const i64 mid = (rlo + rhi) >> 1;
-      if (mid * T - mid * (mid - 1) / 2 <= t) rlo = mid; else rhi = mid;
-    }
-    const i64 bi = rlo, bj = bi + (t - (bi * T - bi * (bi - 1) / 2));
+    const i64 T = (m + kT - 1) / kT, t = item - a.tile_off[w], c2 = 2 * T + 1;
+    const float disc = (float)(c2 * c2 - 8 * t);
+    i64 bi = (i64)(0.5f * ((float)c2 - sqrtf(disc > 0.f ? disc : 0.f)));
+    bi = bi < 0 ? 0 : (bi > T - 1 ? T - 1 : bi);
+    while (bi > 0 && bi * T - bi * (bi - 1) / 2 > t) --bi;
+    while (bi + 1 < T && (bi + 1) * T - (bi + 1) * bi / 2 <= t) ++bi;
+    const i64 bj = bi + (t - (bi * T - bi * (bi - 1) / 2));
     const i64 a0 = base + bi * kT, b0 = base + bj * kT, end = base + m;
+    // sites: of the per-SNP statistics the naive r^2 alone uses them
+    const bool sites = !SNP || a.snp_stat == 5;
+    auto site_at = [&](i64 at) {
+      if (!sites || at >= end) return make_float4(0.f, 0.f, 0.f, 0.f);
+      const i64 s = a.idx ? (i64)a.idx[at] : at;
+      return s >= 0 && s < a.n_snp ? a.site[s] : make_float4(0.f, 0.f, 0.f, 0.f);
+    };
 
     int c[4][4], nv[4];
 #pragma unroll
@@ -156,40 +195,35 @@ __global__ void __launch_bounds__(kThreads) window_kernel(Args a) {
     }
     const int W = a.W;
     for (int w0 = 0; w0 < W; w0 += kKW) {
-      stage(sm.ci, a.planes, a.idx, a0, end, 2 * W, w0, W, a.n_snp, a.status);
-      stage(sm.zi, a.planes + W, a.idx, a0, end, 2 * W, w0, W, a.n_snp, a.status);
-      stage(sm.cj, a.planes, a.idx, b0, end, 2 * W, w0, W, a.n_snp, a.status);
-      stage(sm.zj, a.planes + W, a.idx, b0, end, 2 * W, w0, W, a.n_snp, a.status);
-      if (a.valid) {
-        stage(sm.vi, a.valid, a.idx, a0, end, W, w0, W, a.n_snp, a.status);
-        stage(sm.vj, a.valid, a.idx, b0, end, W, w0, W, a.n_snp, a.status);
-      }
+      stage(sm, a, a0, b0, end, w0, lsh);
       __syncthreads();
       const int nw = min(kKW, W - w0);
       for (int k = 0; k < nw; ++k) {
         const uint32_t cj = sm.cj[k][lane], zj = sm.zj[k][lane];
+        const uint4 c4 = *reinterpret_cast<const uint4*>(&sm.ci[k][4 * wid]);
+        const uint4 z4 = *reinterpret_cast<const uint4*>(&sm.zi[k][4 * wid]);
+        const uint32_t ci[4] = {c4.x, c4.y, c4.z, c4.w}, zi[4] = {z4.x, z4.y, z4.z, z4.w};
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
-          const int r = wid + 8 * q;
-          const uint32_t ci = sm.ci[k][r], zi = sm.zi[k][r];
-          c[q][0] += __popc(ci & cj);
-          c[q][1] += __popc(ci & zj);
-          c[q][2] += __popc(zi & cj);
-          c[q][3] += __popc(zi & zj);
+          c[q][0] += __popc(ci[q] & cj);
+          c[q][1] += __popc(ci[q] & zj);
+          c[q][2] += __popc(zi[q] & cj);
+          c[q][3] += __popc(zi[q] & zj);
         }
       }
       if (a.valid)
         for (int k = 0; k < nw; ++k) {
           const uint32_t vj = sm.vj[k][lane];
 #pragma unroll
-          for (int q = 0; q < 4; ++q) nv[q] += __popc(sm.vi[k][wid + 8 * q] & vj);
+          for (int q = 0; q < 4; ++q) nv[q] += __popc(sm.vi[k][4 * wid + q] & vj);
         }
       __syncthreads();
     }
 
+    const float4 fj = site_at(b0 + lane);
     if constexpr (SNP) {
       // row totals of the warp's 4 rows, column totals of its lane's column
-      float colv = 0.f;
+      float colv = 0.f, rv[4];
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
         const i64 ia = a0 + wid + 8 * q, jb = b0 + lane;
@@ -199,19 +233,17 @@ __global__ void __launch_bounds__(kThreads) window_kernel(Args a) {
                       c4 = (float)c[q][3];
           const fast::Pop p = fast::make(c1, c2, c3, c4);
           const int n = a.valid ? nv[q] : p.n;
-          const i64 si = a.idx ? (i64)a.idx[ia] : ia, sj = a.idx ? (i64)a.idx[jb] : jb;
-          const bool sok = si >= 0 && si < a.n_snp && sj >= 0 && sj < a.n_snp;
-          const float4 fi = sok ? a.site[si] : make_float4(0.f, 0.f, 0.f, 0.f);
-          const float4 fj = sok ? a.site[sj] : make_float4(0.f, 0.f, 0.f, 0.f);
-          x = pair_stat(a.snp_stat, p, n, c1, tinv[n], tr4[n], fi, fj);
+          x = pair_stat(a.snp_stat, p, n, c1, tinv[n], tr4[n], site_at(ia), fj);
         }
         colv += x;
-        float rv = x;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) rv += __shfl_xor_sync(0xffffffffu, rv, o);
-        if (lane == 0 && rv != 0.f && ia < end)
-          atomicAdd(a.row_sums + a.snp_off[w] + (ia - base), (double)rv);
+        rv[q] = x;
       }
+      // the rows' totals: six exchanges for the four (each total the butterfly's)
+      multi::halve_plain<4>(rv);
+      const int q = multi::halved<4>(0);
+      const i64 ia = a0 + wid + 8 * q;
+      if (q >= 0 && rv[0] != 0.f && ia < end)
+        atomicAdd(a.row_sums + a.snp_off[w] + (ia - base), (double)rv[0]);
       if (colv != 0.f && b0 + lane < end)
         atomicAdd(a.col_sums + a.snp_off[w] + (b0 + lane - base), (double)colv);
       continue;
@@ -228,11 +260,7 @@ __global__ void __launch_bounds__(kThreads) window_kernel(Args a) {
       const fast::Pop p = fast::make(c1, c2, c3, c4);
       const int n = a.valid ? nv[q] : p.n;
       ++n_pairs;
-      const i64 si = a.idx ? (i64)a.idx[ia] : ia, sj = a.idx ? (i64)a.idx[jb] : jb;
-      const bool sok = si >= 0 && si < a.n_snp && sj >= 0 && sj < a.n_snp;
-      const float4 fi = sok ? a.site[si] : make_float4(0.f, 0.f, 0.f, 0.f);
-      const float4 fj = sok ? a.site[sj] : make_float4(0.f, 0.f, 0.f, 0.f);
-      window_pair(p, n, c1, tinv[n], tr4[n], fi, fj, acc, n_r2, n_four);
+      window_pair(p, n, c1, tinv[n], tr4[n], site_at(ia), fj, acc, n_r2, n_four);
     }
     // warp totals, one atomic per statistic per warp
 #pragma unroll
