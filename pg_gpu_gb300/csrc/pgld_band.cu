@@ -502,7 +502,9 @@ static int binned_sums_range(pgld_context* h, const pgld_hap_panel* panel, const
   if (rc) return rc;
   i64* items = (i64*)ws;
   char* scratch = (char*)ws + ((((size_t)(nb + 1) * 8) + 255) & ~size_t(255));
-  rc = pgld::band_schedule(h, pos, n, max_dist, items, scratch, sb, st);
+  rc = pgld::band_schedule(h, pos, n, max_dist, items, scratch, sb, st, pgld::kTile,
+                           pgld::band_multi_applies(a, pgld::kModeBinned) ? pgld::band_multi_cols()
+                                                                         : pgld::kTile);
   if (rc) return rc;
   a.item_off = items;
   a.n_blocks = nb;

@@ -65,6 +65,7 @@ bool band_fast_applies(const BandArgs& a, int mode);
 int launch_band_fast(pgld_context* h, const BandArgs& a, int mode, cudaStream_t st);
 // binned sums of three or four populations in float32 (pgld_band_multi.cu)
 bool band_multi_applies(const BandArgs& a, int mode);
+int band_multi_cols();  // SNPs j of its tiles (their rows are kTile)
 int launch_band_multi(pgld_context* h, const BandArgs& a, cudaStream_t st);
 
 }  // namespace pgld

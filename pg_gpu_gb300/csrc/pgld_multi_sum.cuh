@@ -98,24 +98,24 @@ __device__ __forceinline__ void flush(float* acc, double* slots, const Places& p
   }
 }
 
-// The pairs of a 32 x 32 tile grouped by bin, in steps of 32 pairs of one bin
+// The pairs of a tile (32 to a row) grouped by bin, in steps of 32 pairs of one bin
 // (the last of a bin padded): a step's totals then go to one bin however the
 // tile's distances fall, so short distances with several bins across a row
 // cost no more than long ones.  The order is fixed (bin, then warp, then row,
 // then column): equal inputs give equal sums.
 constexpr int kGroupPairs = 1024;
-template <int WARPS>
+template <int WARPS, int PAIRS = kGroupPairs>
 struct Groups {
-  unsigned short list[kGroupPairs + 31 * kMaxBins];  // pair = 32 row + column; 0xffff: none
-  unsigned char step_bin[kGroupPairs / 32 + kMaxBins];
+  unsigned short list[PAIRS + 31 * kMaxBins];  // pair = 32 row + column; 0xffff: none
+  unsigned char step_bin[PAIRS / 32 + kMaxBins];
   unsigned short warp_cnt[WARPS][kMaxBins];
   int n_steps;
 };
 
 // bin[q]: bin (or -1) of the thread's pair (row0 + q, lane).  All WARPS warps
 // call it together (sync() meets them); fills g and adds the pairs per bin to bcnt.
-template <int WARPS, int ROWS, class Sync>
-__device__ __forceinline__ void group_pairs(Groups<WARPS>& g, const int (&bin)[ROWS], int row0,
+template <int WARPS, int ROWS, int PAIRS, class Sync>
+__device__ __forceinline__ void group_pairs(Groups<WARPS, PAIRS>& g, const int (&bin)[ROWS], int row0,
                                             int warp, int n_bins, unsigned long long* bcnt,
                                             Sync&& sync) {
   const int lane = threadIdx.x & 31;
@@ -179,22 +179,41 @@ __device__ __forceinline__ void group_pairs(Groups<WARPS>& g, const int (&bin)[R
 // features of the lane's pair of bin b (pair 0xffff: of nobody, whose quotients
 // are 0).  Up to three populations take one pass (G = 0); four take two, G = 0
 // with 66 statistics and G = 1 with 39, so that the sums stay in registers.
-template <int P, int G, class F, int WARPS, class Load>
-__device__ __forceinline__ void sum_steps(const Groups<WARPS>& g, int s0, int s1, double* slots,
+template <int P, int G, class F, int WARPS, int PAIRS, class Load>
+__device__ __forceinline__ void sum_steps(const Groups<WARPS, PAIRS>& g, int s0, int s1, double* slots,
                                           int n_stats, const Places& pl, Load&& load) {
   constexpr bool G0 = P < 4 || G == 0, G1 = P < 4 || G == 1;
   constexpr int N = (G0 ? group_size(P, 0) : 0) + (G1 ? group_size(P, 1) : 0);
   constexpr int K0 = G0 ? 0 : group_size(P, 0);
   const int lane = threadIdx.x & 31;
-  float acc[N];
+  // a lane's haplotype sums of pi2_iiii keep their rounding errors (TwoSum): with
+  // few haplotypes those sums add a few recurring values, whose roundings do not
+  // average out (30 haplotypes: 2e-9 of the statistic after eight steps)
+  constexpr bool kKeep = G0 && !F::geno;
+  constexpr int E = kKeep ? P : 1;
+  float acc[N], err[E];
   for (int s = s0; s < s1;) {
     const int b = g.step_bin[s];
 #pragma unroll
     for (int k = 0; k < N; ++k) acc[k] = 0.f;
+#pragma unroll
+    for (int k = 0; k < E; ++k) err[k] = 0.f;
     for (; s < s1 && g.step_bin[s] == b; ++s) {
       F f[P];
       load((int)g.list[32 * s + lane], b, f);
-      eval<P, G0, G1>(f, [&](int k, float v) { acc[k] += v; });
+      eval<P, G0, G1>(f, [&](int k, float v) {
+        if (kKeep && k < 3 * P && k % 3 == 2) {
+          const float t = __fadd_rn(acc[k], v), z = __fsub_rn(t, acc[k]);
+          err[k / 3] += __fadd_rn(__fsub_rn(acc[k], __fsub_rn(t, z)), __fsub_rn(v, z));
+          acc[k] = t;
+        } else {
+          acc[k] += v;
+        }
+      });
+    }
+    if (kKeep) {
+#pragma unroll
+      for (int k = 0; k < E; ++k) acc[3 * k + 2] += err[k];
     }
     flush<N, K0>(acc, slots + b * n_stats, pl);
   }
