@@ -486,10 +486,10 @@ def run_gpu(args, pool, cores):
                 "d2h_bytes_per_step": int(d2h),
                 "api": "HaplotypeMatrix(host int8).compute_ld_statistics_gpu_two_pops(raw=True)"},
         # per step: one pack per population, then the binned call: tile counts,
-        # 3 scan launches and the band kernel; tc: also the integer-position
+        # 2 scan launches and the band kernel; tc: also the integer-position
         # copy and the operand expansion -- one launch for both populations in
         # the combined 64 x 128 layout, one per population in the 64 x 64 one
-        "gpu_launches": args.steps * (cfg["pops"] + 5 + (
+        "gpu_launches": args.steps * (cfg["pops"] + 4 + (
             0 if args.form != "tc" else
             1 + (1 if (cfg["pops"] == 2 and (tuned is None or tuned["choice"][0] != 1))
                  else cfg["pops"]))),
