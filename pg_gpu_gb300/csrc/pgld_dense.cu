@@ -24,9 +24,10 @@ constexpr int kT = 32;         // SNPs per tile side
 constexpr int kThreads = 256;  // warp w: rows w + 8 q of the tile, lane: column
 constexpr int kKW = 32;        // words of a plane staged per chunk
 constexpr int kPad = 33;
+constexpr int kPadRows = 36;   // 16-byte aligned rows
 
 struct __align__(16) Smem {
-  uint32_t ci[kKW][kPad], vi[kKW][kPad], cj[kKW][kPad], vj[kKW][kPad];
+  uint32_t ci[kKW][kPadRows], vi[kKW][kPadRows], cj[kKW][kPad], vj[kKW][kPad];
   double tr[kT][kT + 1];   // mirrored tile
   double bins[kMaxBins + 1];
   int thr[kMaxBins + 1];
@@ -37,9 +38,11 @@ struct __align__(16) Smem {
 // upper-triangle tile t -> (bi, bj), bj >= bi, of nb blocks (row bi owns
 // tiles bi .. nb - 1, starting at bi nb - bi (bi - 1) / 2)
 __device__ __forceinline__ void tri_decode(i64 t, i64 nb, i64& bi, i64& bj) {
-  // largest bi with start(bi) <= t, from the quadratic, then corrected
-  const double b = (double)(2 * nb + 1);
-  i64 r = (i64)floor((b - sqrt(b * b - 8.0 * (double)t)) / 2.0);
+  // largest bi with start(bi) <= t, from the quadratic, then corrected (in
+  // float32: a float64 root by every thread of a block takes 5,000 cycles)
+  const i64 b = 2 * nb + 1;
+  const float disc = (float)(b * b - 8 * t);
+  i64 r = (i64)(0.5f * ((float)b - sqrtf(disc > 0.f ? disc : 0.f)));
   r = max((i64)0, min(r, nb - 1));
   auto start = [&](i64 x) { return x * nb - x * (x - 1) / 2; };
   while (r > 0 && start(r) > t) --r;
@@ -48,23 +51,31 @@ __device__ __forceinline__ void tri_decode(i64 t, i64 nb, i64& bi, i64& bj) {
   bj = r + (t - start(r));
 }
 
-// stage carrier and valid (carrier | reference) words of 32 SNPs, transposed
-__device__ __forceinline__ void stage(uint32_t (*c)[kPad], uint32_t (*v)[kPad],
-                                      const uint32_t* __restrict__ planes, int W, i64 s0, i64 n,
-                                      int w0) {
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-#pragma unroll
-  for (int q = 0; q < kT / 8; ++q) {
-    const int sl = wid * (kT / 8) + q;
-    const i64 s = s0 + sl;
-    const int w = w0 + lane;
+// carrier and valid (carrier | reference) words [w0, w0 + 32) of the tile's rows
+// and columns, transposed; L = 1 << lsh lanes (at least the words there are) to a
+// SNP.  Row r is kept at 4 (r % 8) + r / 8: the four rows of a warp are one 16-byte
+// load
+__device__ __forceinline__ void stage(Smem& sm, const uint32_t* __restrict__ planes, int W, i64 i0,
+                                      i64 j0, i64 n, int w0, int lsh) {
+  const int w = threadIdx.x & ((1 << lsh) - 1);
+  for (int x = threadIdx.x; x < (2 * kT) << lsh; x += kThreads) {
+    const int row = x >> lsh, r = row & (kT - 1);
+    const bool col = row >= kT;
+    const i64 s = (col ? j0 : i0) + r;
     uint32_t cc = 0, zz = 0;
-    if (s < n && w < W) {
-      cc = __ldg(planes + s * 2 * W + w);
-      zz = __ldg(planes + s * 2 * W + W + w);
+    if (s < n && w0 + w < W) {
+      const uint32_t* p = planes + s * 2 * W + w0 + w;
+      cc = __ldg(p);
+      zz = __ldg(p + W);
     }
-    c[lane][sl] = cc;
-    v[lane][sl] = cc | zz;
+    if (col) {
+      sm.cj[w][r] = cc;
+      sm.vj[w][r] = cc | zz;
+    } else {
+      const int k = 4 * (r & 7) + (r >> 3);
+      sm.ci[w][k] = cc;
+      sm.vi[w][k] = cc | zz;
+    }
   }
 }
 
@@ -78,20 +89,20 @@ __device__ __forceinline__ void tile_counts(Smem& sm, const uint32_t* planes, in
   for (int q = 0; q < 4; ++q) cc[q] = cv[q] = vc[q] = vv[q] = 0;
   for (int w0 = 0; w0 < W; w0 += kKW) {
     __syncthreads();
-    stage(sm.ci, sm.vi, planes, W, i0, n, w0);
-    stage(sm.cj, sm.vj, planes, W, j0, n, w0);
+    stage(sm, planes, W, i0, j0, n, w0, W <= 8 ? 3 : W <= 16 ? 4 : 5);
     __syncthreads();
     const int nw = min(kKW, W - w0);
     for (int w = 0; w < nw; ++w) {
       const uint32_t cj = sm.cj[w][lane], vj = sm.vj[w][lane];
+      const uint4 c4 = *reinterpret_cast<const uint4*>(&sm.ci[w][4 * wid]);
+      const uint4 v4 = *reinterpret_cast<const uint4*>(&sm.vi[w][4 * wid]);
+      const uint32_t ci[4] = {c4.x, c4.y, c4.z, c4.w}, vi[4] = {v4.x, v4.y, v4.z, v4.w};
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
-        const int r = wid + 8 * q;
-        const uint32_t ci = sm.ci[w][r], vi = sm.vi[w][r];
-        cc[q] += __popc(ci & cj);
-        cv[q] += __popc(ci & vj);
-        vc[q] += __popc(vi & cj);
-        vv[q] += __popc(vi & vj);
+        cc[q] += __popc(ci[q] & cj);
+        cv[q] += __popc(ci[q] & vj);
+        vc[q] += __popc(vi[q] & cj);
+        vv[q] += __popc(vi[q] & vj);
       }
     }
   }
@@ -201,9 +212,11 @@ __device__ __forceinline__ int bin_index(const int* thr, int n_bins, int d) {
 // are written grouped by bin at cursor[b] (advanced atomically per tile).
 // The float64 pipe (two operations per SM and clock) would bound it: integer
 // positions are compared as integers, counting asks only whether the
-// denominator is positive, and the quotient is an integer division.  300
-// haplotypes x 5,001 SNPs: 0.50 ms for each of the two passes when both divided
-// and searched the bins in float64, 0.31 ms now.
+// denominator is positive, the quotient is an integer division, and a warp's pairs
+// of a bin take their places with one shared-memory addition.  300 haplotypes x
+// 5,001 SNPs, both passes: 1.0 ms when they divided and searched the bins in
+// float64, 0.62 with a float64 root per thread to find a tile, an addition per
+// pair and 32 lanes to a staged SNP, 0.42 now.
 __global__ void __launch_bounds__(kThreads) pairs_by_bin_kernel(
     const uint32_t* __restrict__ planes, int W, const double* __restrict__ values, i64 n,
     const double* __restrict__ pos, const int* __restrict__ ipos, const int* __restrict__ ipos_bad,
@@ -235,9 +248,11 @@ __global__ void __launch_bounds__(kThreads) pairs_by_bin_kernel(
     __syncthreads();
     int bin[4], slot[4];
     double val[4];
+    const i64 j = j0 + lane;
+    const int pj = use_int && j < n ? ipos[j] : 0;
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
-      const i64 i = i0 + wid + 8 * q, j = j0 + lane;
+      const i64 i = i0 + wid + 8 * q;
       bin[q] = -1;
       val[q] = 0.0;
       if (i < j && j < n) {
@@ -251,19 +266,25 @@ __global__ void __launch_bounds__(kThreads) pairs_by_bin_kernel(
           // (n11 n00 - n10 n01)^2 over pA (n - pA) pB (n - pB) of the pair's
           // valid haplotypes as exact integers, divided once; NaN where the
           // denominator is 0
-          const long long a = n11[q], pa = cv[q], pb = vc[q], nn = nv[q];
-          const long long b = pa - a, c = pb - a, d = nn - pa - pb + a;
-          const long long x = a * d - b * c;
-          const long long den = pa * (nn - pa) * pb * (nn - pb);
-          defined = den > 0;
-          if (out && defined) v = quotient(x * x, den);
+          const int a = n11[q], pa = cv[q], pb = vc[q], nn = nv[q];
+          defined = pa > 0 && pa < nn && pb > 0 && pb < nn;
+          if (out && defined) {
+            const int b = pa - a, c = pb - a, d = nn - pa - pb + a;
+            const long long x = (long long)a * d - (long long)b * c;
+            v = quotient(x * x, ((long long)pa * (nn - pa)) * ((long long)pb * (nn - pb)));
+          }
         }
         val[q] = v;
         if (defined)
-          bin[q] = use_int ? bin_index(sm.thr, n_bins, ipos[j] - ipos[i])
+          bin[q] = use_int ? bin_index(sm.thr, n_bins, pj - ipos[i])
                            : bin_index(sm.bins, n_bins, pos[j] - pos[i]);
       }
-      slot[q] = bin[q] >= 0 ? atomicAdd(&sm.bin_cnt[bin[q]], 1) : 0;
+      // the warp's pairs of a bin take their places with one addition
+      const unsigned same = __match_any_sync(0xffffffffu, bin[q]);
+      const int first = __ffs(same) - 1;
+      int at = 0;
+      if (lane == first && bin[q] >= 0) at = atomicAdd(&sm.bin_cnt[bin[q]], __popc(same));
+      slot[q] = __shfl_sync(0xffffffffu, at, first) + __popc(same & ((1u << lane) - 1u));
     }
     __syncthreads();
     for (int x = threadIdx.x; x < n_bins; x += kThreads) {
@@ -486,7 +507,7 @@ __device__ __forceinline__ i64 tri_row(i64 i, i64 n) { return i * (2 * n - i - 1
 // joint counts of every pair (HaplotypeMatrix.tally_gpu_haplotypes): a warp's
 // stores are 32 consecutive pairs of a row.  2,000 SNPs x 200 haplotypes (2.0
 // million pairs, 32 MB): 279 us with a lane group per pair that searched the
-// triangle for its SNPs, 26 us here.
+// triangle for its SNPs, 22 us here.
 template <bool VALID>
 __global__ void __launch_bounds__(kThreads) tally_kernel(const uint32_t* __restrict__ planes,
                                                          const uint32_t* __restrict__ valid, int W,
