@@ -103,13 +103,13 @@ struct PackArgs {
   const int32_t* before;  // kept sites before each site, [n_snp + 1] (NULL: all kept)
   uint32_t *planes, *valid, *ext;
   int32_t* flags;
-  int words;              // words per block (a power of two, at most kWarps)
+  int words_log2;         // words per block (at most kWarps)
 };
 
 // A warp turns 32 rows x 128 sites into one word per site and plane: a row's
 // comparison bytes move to the row's bit (a high multiply, beside the
 // comparisons on the other pipe) in a register per plane and eight rows, byte
-// transposes then give the words.  The block's `words` words of a site are
+// transposes then give the words.  The block's words of a site are
 // stored together (32-byte segments at eight words), through shared memory.
 // Values above the planes' show in the words themselves: valid, but in no plane.
 template <class S, bool ALIGNED>
@@ -117,9 +117,9 @@ __global__ void __launch_bounds__(kThreads) pack_kernel(PackArgs a) {
   constexpr int kPitch = kWarps + 1;
   __shared__ uint32_t out[S::N][kWarpSites * kPitch];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int chunks = kWarps / a.words;          // 128-site chunks per block
-  const int word = blockIdx.y * a.words + warp % a.words;
-  const i64 s0 = ((i64)blockIdx.x * chunks + warp / a.words) * kWarpSites + 4 * lane;
+  const int words = 1 << a.words_log2, chunks = kWarps >> a.words_log2;  // 128-site chunks per block
+  const int word = blockIdx.y * words + (warp & (words - 1));
+  const i64 s0 = ((i64)blockIdx.x * chunks + (warp >> a.words_log2)) * kWarpSites + 4 * lane;
   const int live = min(32, a.n_rows - 32 * word);  // rows of the word (none for a padding word)
   uint32_t acc[S::N][4];
 #pragma unroll
@@ -164,12 +164,12 @@ __global__ void __launch_bounds__(kThreads) pack_kernel(PackArgs a) {
   for (int p = 0; p < S::N; ++p) {
     const uint32_t l0 = __byte_perm(acc[p][0], acc[p][1], 0x5140), l1 = __byte_perm(acc[p][0], acc[p][1], 0x7362);
     const uint32_t h0 = __byte_perm(acc[p][2], acc[p][3], 0x5140), h1 = __byte_perm(acc[p][2], acc[p][3], 0x7362);
-    uint32_t* o = out[p] + 4 * lane * kPitch + warp;
+    uint32_t* o = out[p] + lane * kPitch + warp;  // site 4 lane + k at 32 k + lane
     const uint32_t w[4] = {__byte_perm(l0, h0, 0x5410), __byte_perm(l0, h0, 0x7632),
                            __byte_perm(l1, h1, 0x5410), __byte_perm(l1, h1, 0x7632)};
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-      o[k * kPitch] = w[k];
+      o[32 * k * kPitch] = w[k];
       if (p == 0) above[k] = ~w[k];
       else if (p < S::kMain) above[k] &= ~w[k];
       else if (p == S::kValid) above[k] &= w[k];
@@ -188,9 +188,9 @@ __global__ void __launch_bounds__(kThreads) pack_kernel(PackArgs a) {
   __syncthreads();
   // consecutive threads: the words of a site, then the next site of the block
   const i64 b0 = (i64)blockIdx.x * chunks * kWarpSites;
-  for (int t = threadIdx.x; t < chunks * kWarpSites * a.words; t += kThreads) {
-    const int w = t % a.words, at = t / a.words;
-    const int W0 = blockIdx.y * a.words + w;
+  for (int t = threadIdx.x; t < (chunks * kWarpSites) << a.words_log2; t += kThreads) {
+    const int w = t & (words - 1), at = t >> a.words_log2;
+    const int W0 = blockIdx.y * words + w;
     const i64 s = b0 + at;
     if (W0 >= a.W || s >= a.n_snp) continue;
     i64 d = s;
@@ -198,7 +198,8 @@ __global__ void __launch_bounds__(kThreads) pack_kernel(PackArgs a) {
       d = a.before[s];
       if (a.before[s + 1] == d) continue;
     }
-    const int from = (at % kWarpSites) * kPitch + (at / kWarpSites) * a.words + w;
+    const int site = at & (kWarpSites - 1);
+    const int from = (32 * (site & 3) + (site >> 2)) * kPitch + ((at / kWarpSites) << a.words_log2) + w;
 #pragma unroll
     for (int p = 0; p < S::kMain; ++p) a.planes[d * S::kMain * a.W + p * a.W + W0] = out[p][from];
     if (a.valid) a.valid[d * a.W + W0] = out[S::kValid][from];
@@ -209,11 +210,14 @@ __global__ void __launch_bounds__(kThreads) pack_kernel(PackArgs a) {
 
 template <class S>
 int launch_pack(pgld_context* h, PackArgs a, cudaStream_t st) {
-  a.words = 1;
-  while (a.words < a.W && a.words < kWarps) a.words <<= 1;
-  const i64 per_block = (i64)(kWarps / a.words) * kWarpSites;
+  int words = 1;
+  while (words < a.W && words < kWarps) {
+    words <<= 1;
+    ++a.words_log2;
+  }
+  const i64 per_block = (i64)(kWarps / words) * kWarpSites;
   const dim3 grid((unsigned)((a.n_snp + per_block - 1) / per_block),
-                  (unsigned)((a.W + a.words - 1) / a.words));
+                  (unsigned)((a.W + words - 1) / words));
   if ((((uintptr_t)a.x | (uintptr_t)a.ld) & 3) == 0)
     pack_kernel<S, true><<<grid, kThreads, 0, st>>>(a);
   else
