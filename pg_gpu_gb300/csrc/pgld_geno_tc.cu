@@ -583,7 +583,8 @@ static unsigned pack_gtc_blocks(const pgld_context* h, long long n_blocks) {
 // groups, 3.6 with three (sixteen warps in two groups: 5.1, registers and totals
 // of four steps); three populations of 200, 20,000 SNPs 1.78 and 1.41 ms with one
 // group of eight warps and two of four; one population of 200, 60,000 SNPs: 1.5 ms
-// with distances and bins in 64 bits and a butterfly per total, 0.86 here.
+// with distances and bins in 64 bits, a butterfly per total and an addition to the
+// slots each, 0.83 here.
 // ---------------------------------------------------------------------------
 struct BParams {
   int kchunks;
@@ -807,6 +808,12 @@ __global__ void __launch_bounds__(Binned<P>::kThreads, 1)
     const bool use_int = a.bcoord == nullptr && *a.ipos_bad == 0;
     const int maxd_int = a.max_dist >= 2147483647.0 ? 2147483647 : (int)floor(a.max_dist);
     long long lo = 0;
+    // one population: a lane's running total (its row and statistic of eight) and,
+    // in lanes 0-7, its row's pairs, added to the slots when the bin changes: the
+    // rows of a tile mostly share a bin, and eight float64 additions to one slot
+    // retry one another
+    double v_run = 0.0;
+    int v_bin = -1, n_bin = -1, n_run = 0;
     // the tile is ready on the group's own barrier, whose phases the group alone
     // follows (a stage's would pass through other groups' tiles)
     for (int t = grp, u = 0;; t += G, ++u) {
@@ -990,7 +997,12 @@ __global__ void __launch_bounds__(Binned<P>::kThreads, 1)
             }
             if (lane == k) {
               slot = bb;
-              atomicAdd(&bcnt[bb], (unsigned long long)__popc(same));
+              if (bb != n_bin) {
+                if (n_bin >= 0) atomicAdd(&bcnt[n_bin], (unsigned long long)n_run);
+                n_bin = bb;
+                n_run = 0;
+              }
+              n_run += __popc(same);
             }
             pending[k] &= ~same;
             more |= pending[k];
@@ -999,9 +1011,24 @@ __global__ void __launch_bounds__(Binned<P>::kThreads, 1)
           multi::halve_plain<24>(v);
           const int at = multi::halved<24>(0);
           const int bb = __shfl_sync(0xffffffffu, slot, at < 0 ? 0 : at / 3);
-          if (at >= 0 && bb >= 0) atomicAdd(&acc[bb * 3 + at % 3], (double)v[0]);
+          if (at >= 0 && bb >= 0) {
+            if (bb != v_bin) {
+              if (v_bin >= 0) atomicAdd(&acc[v_bin * 3 + at % 3], v_run);
+              v_bin = bb;
+              v_run = 0.0;
+            }
+            v_run += (double)v[0];
+          }
         } while (more);
       }
+      if (n_run >= 1 << 30) {
+        atomicAdd(&bcnt[n_bin], (unsigned long long)n_run);
+        n_run = 0;
+      }
+    }
+    if (P == 1) {
+      if (v_bin >= 0) atomicAdd(&acc[v_bin * 3 + multi::halved<24>(0) % 3], v_run);
+      if (n_bin >= 0 && n_run) atomicAdd(&bcnt[n_bin], (unsigned long long)n_run);
     }
   }
 

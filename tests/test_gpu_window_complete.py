@@ -38,3 +38,19 @@ def test_complete_lists_match_general_kernel(columns, H, absent):
         np.testing.assert_allclose(here[:, k], ref[:, k], rtol=1e-12, atol=1e-12 * np.abs(ref[:, k]).max())
     checked = [0, 1, 2] if "r2" in columns else [0, 2]
     assert np.array_equal(n[:, checked], m[:, checked])
+
+
+# lists shorter than the operand's boxes, down to one SNP
+@pytest.mark.parametrize("M", [1, 2, 5, 127, 130])
+def test_short_lists(M):
+    rng = np.random.default_rng(M)
+    x = (rng.random((50, M + 1)) < 0.4).astype(np.int8)
+    x[:, M] = -1
+    pk = _ops.pack(torch.as_tensor(x, device="cuda"))
+    b, e = np.array([0, 0], np.int64), np.array([M, M // 2], np.int64)
+    got = []
+    for n in (M, M + 1):
+        s, c = _ops.window_sums(pk, np.arange(n, dtype=np.int32), b, e, form="tc", columns=("sigma_d2",))
+        got.append((s.cpu().numpy()[:, 1], c.cpu().numpy()[:, [0, 2]]))
+    np.testing.assert_allclose(got[0][0], got[1][0], rtol=1e-12, atol=1e-12 * np.abs(got[1][0]).max())
+    assert np.array_equal(got[0][1], got[1][1])
