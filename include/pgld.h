@@ -564,7 +564,8 @@ int pgld_vcf_pack_gt(const char* text, int64_t len, int32_t n_samples, int64_t n
  * at most 2,016 haplotypes).  Automatic: layout 2 for the binned
  * two-population sums and the window sums, layout 1 for the per-pair
  * outputs.  And a cap on the pipeline stages of the tensor-core kernels
- * (0: as many as shared memory holds).  No counterpart in the
+ * (0: as many as shared memory holds, three for the binned sums of layout 2).
+ * No counterpart in the
  * reference, whose chunk sizes come from free device memory
  * (ld_pipeline.py:16-49, _memutil.py:6-52). */
 int pgld_set_tc_config(pgld_handle h, int32_t layout, int32_t max_stages);

@@ -1174,7 +1174,11 @@ int pgld_tc_wide_binned(pgld_context* h, const pgld_hap_panel* panel, pgld::Band
   int max_smem = 0;
   cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, h->device);
   int stages = (int)std::min<long long>(8, ((long long)max_smem - (long long)fixed) / kStage);
-  if (h->tc_stages_cap > 0) stages = std::min(stages, h->tc_stages_cap);
+  // three stages unless the caller chose: the epilogue bounds the kernel, and a
+  // fourth stage's copies run further ahead of it for nothing (two populations
+  // of 50, 200, 700 and 1,000: 3.19 / 3.18, 3.22 / 3.21, 3.43 / 3.36 and 12.16 /
+  // 11.87 ms with four / three; two: 3.23, 3.32, 3.69 and 13.7)
+  stages = std::min(stages, h->tc_stages_cap > 0 ? h->tc_stages_cap : 3);
   if (stages < 2) return pgld_fail(h, PGLD_ERR_TOO_LARGE, "tensor-core form: shared memory");
   prm.stages = stages;
   const size_t smem = (size_t)stages * kStage + fixed;
