@@ -20,7 +20,7 @@ def _torch():
 # --------------------------------------------------------------------------
 class PackFlags:
     """The flag pairs (missing, other) that packing launches write, read back
-    together on first use."""
+    together on first use (again after a pair was handed to another launch)."""
 
     def __init__(self, count, device):
         self.device_flags = _torch().zeros(2 * count, dtype=_torch().int32, device=device)
@@ -28,6 +28,7 @@ class PackFlags:
 
     def pair(self, k):
         """The k-th launch's device pair."""
+        self._host = None  # a copy from before this launch is stale
         return self.device_flags[2 * k:2 * k + 2]
 
     def read(self, k):
@@ -198,7 +199,8 @@ def pack(hap, rows=None, kept=None, flags=None, k=0):
     so only the packed planes are written to device memory (the call then
     returns once the kernel is done with the host matrix).  kept: the result
     of kept_sites, to pack those sites only.  flags: a PackFlags shared by
-    several calls, of which this one writes pair k."""
+    several calls, of which this one writes pair k; the caller then reads the
+    flags after the last call, which also waits for the host matrix."""
     torch = _torch()
     if not _host_readable(hap):
         hap = L.as_device(hap, np.int8)
@@ -216,7 +218,8 @@ def pack(hap, rows=None, kept=None, flags=None, k=0):
     before, n_out = (None, n_snp) if kept is None else (kept[0], kept[1].numel())
     planes = torch.empty((n_out, 2 * W), dtype=torch.int32, device=dev)
     valid = torch.empty((n_out, W), dtype=torch.int32, device=dev)
-    if flags is None:
+    own = flags is None
+    if own:
         flags, k = PackFlags(1, dev), 0
     if n_rows == 0:
         planes.zero_()
@@ -228,9 +231,20 @@ def pack(hap, rows=None, kept=None, flags=None, k=0):
                                                   L.ptr(planes), L.ptr(valid),
                                                   L.ptr(flags.pair(k)), L.stream_ptr()), h)
     pk = PackedPop.pending(planes, valid, W, n_rows, n_out, flags, k)
-    if not hap.is_cuda:
+    if own and not hap.is_cuda:
         pk._resolve()  # the host matrix is read in place: finish before returning
     return pk
+
+
+def pack_all(hap, row_lists, kept=None):
+    """pack of several populations of one matrix, their flags read together."""
+    on_device = isinstance(hap, _torch().Tensor) and hap.is_cuda
+    flags = PackFlags(len(row_lists), hap.device if on_device else "cuda")
+    try:
+        return [pack(hap, rows, kept, flags, k) for k, rows in enumerate(row_lists)]
+    finally:
+        if row_lists and _host_readable(hap):
+            flags.read(0)  # the host matrix is read in place: finish before returning
 
 
 def panel(pops):

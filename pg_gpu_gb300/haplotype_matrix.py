@@ -442,10 +442,9 @@ class HaplotypeMatrix:
             self.transfer_to_gpu()
             src = self._haplotypes
         new = [p for p in dict.fromkeys(pops) if p not in self._packed]
-        flags = _ops.PackFlags(len(new), "cuda" if not src.is_cuda else src.device) if new else None
-        for k, p in enumerate(new):
-            r = self._pop_rows(p) if rows is None else rows[pops.index(p)]
-            self._packed[p] = _ops.pack(src, r, flags=flags, k=k)
+        if new:
+            of = self._pop_rows if rows is None else dict(zip(pops, rows)).__getitem__
+            self._packed.update(zip(new, _ops.pack_all(src, [of(p) for p in new])))
         return [self._packed[p] for p in pops]
 
     # ------------------------------------------------------------ LD methods
@@ -494,8 +493,7 @@ class HaplotypeMatrix:
         rows = [self._pop_rows(p) for p in pops]
         if None not in rows:
             rows = _ops.device_rows(rows, src.shape[0])
-        flags = _ops.PackFlags(len(pops), kept[1].device)
-        packs = [_ops.pack(src, r, kept, flags, k) for k, r in enumerate(rows)]
+        packs = _ops.pack_all(src, rows, kept)
         pos = _ops.positions_f64(self._positions).index_select(0, kept[1])
         sums, cnt = _ops.binned_sums(packs, pos, bins)
         return (bins, *_ops.host_sums(sums, cnt))
