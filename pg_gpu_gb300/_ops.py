@@ -146,9 +146,12 @@ KEEP_BIALLELIC, KEEP_SEGREGATING, KEEP_DIPLOID = range(3)
 
 def site_counts(x, rows=None, sums=True, flags=False):
     """Per-site counts of an int8 matrix (device, or a pinned host tensor read
-    in place) over `rows` (None: all): int32 (sum of the values above 0, number
-    of values >= 0, presence bits of 0 / 1 / above 1), None where not asked."""
+    in place; others are copied first, as by pack) over `rows` (None: all): int32
+    (sum of the values above 0, number of values >= 0, presence bits of 0 / 1 /
+    above 1), None where not asked."""
     torch = _torch()
+    if not _host_readable(x):
+        x = L.as_device(x, np.int8)
     dev = x.device if x.is_cuda else torch.device("cuda", torch.cuda.current_device())
     n_total, n = x.shape
     rows_t = None if rows is None else _check_rows(rows, n_total)

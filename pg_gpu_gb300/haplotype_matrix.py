@@ -479,14 +479,22 @@ class HaplotypeMatrix:
         sums, cnt = _ops.binned_sums(packs, _ops.positions_f64(self._positions), bins)
         return (bins, *_ops.host_sums(sums, cnt))
 
+    def _int8_source(self):
+        """The matrix as site_counts and pack read it (int8 rows, one site after
+        another), or None: other types are filtered as they are."""
+        if self._device == "CPU" and self._pinned is not None:
+            return self._pinned
+        h = self._haplotypes
+        if self._device == "GPU":
+            return L.as_device(h) if _is_torch(h) and h.is_cuda and str(h.dtype) == "torch.int8" else None
+        return L.as_device(h) if h.dtype == np.int8 else None
+
     def _binned_biallelic(self, bins, pops):
         """_binned of apply_biallelic_filter(): the sites are chosen and the
         populations packed from the matrix itself, without the gathered copy."""
-        src = self._pinned if self._device == "CPU" else self._haplotypes
+        src = self._int8_source()
         if src is None:
-            if self._haplotypes.dtype != np.int8:
-                return self.apply_biallelic_filter()._binned(bins, pops)
-            src = L.as_device(self._haplotypes, np.int8)
+            return self.apply_biallelic_filter()._binned(bins, pops)
         kept = _ops.kept_sites(_ops.KEEP_BIALLELIC, _ops.site_counts(src, sums=False, flags=True))
         if kept[1].numel() == 0:
             raise ValueError("genotypes cannot be empty")
