@@ -481,13 +481,16 @@ class HaplotypeMatrix:
 
     def _int8_source(self):
         """The matrix as site_counts and pack read it (int8 rows, one site after
-        another), or None: other types are filtered as they are."""
+        another), or None: other types are filtered as they are, and host arrays
+        that run backwards or overlap are gathered first."""
         if self._device == "CPU" and self._pinned is not None:
-            return self._pinned
+            h = self._pinned
+            return h if h.stride(0) >= h.shape[1] else None
         h = self._haplotypes
         if self._device == "GPU":
             return L.as_device(h) if _is_torch(h) and h.is_cuda and str(h.dtype) == "torch.int8" else None
-        return L.as_device(h) if h.dtype == np.int8 else None
+        ok = isinstance(h, np.ndarray) and h.dtype == np.int8 and min(h.strides) >= 0
+        return L.as_device(h) if ok else None
 
     def _binned_biallelic(self, bins, pops):
         """_binned of apply_biallelic_filter(): the sites are chosen and the
@@ -501,8 +504,10 @@ class HaplotypeMatrix:
         rows = [self._pop_rows(p) for p in pops]
         if None not in rows:
             rows = _ops.device_rows(rows, src.shape[0])
+        pos = self._positions
+        pos = _ops.positions_f64(pos if _is_torch(pos) else np.ascontiguousarray(pos))
         packs = _ops.pack_all(src, rows, kept)
-        pos = _ops.positions_f64(self._positions).index_select(0, kept[1])
+        pos = pos.index_select(0, kept[1])
         sums, cnt = _ops.binned_sums(packs, pos, bins)
         return (bins, *_ops.host_sums(sums, cnt))
 

@@ -65,11 +65,20 @@ def test_device_matrix_as_held(form):
     same(held(t, pos), hap, pos)
 
 
-@pytest.mark.parametrize("form", ["int8", "fortran", "int16", "pinned"])
+@pytest.mark.parametrize("form", ["int8", "backwards", "fortran", "int16", "pinned", "overlap"])
 def test_host_matrix(form):
     hap, pos = panel()
+    if form == "backwards":
+        x = hap[:, ::-1].copy()[:, ::-1]
+        p = pos[::-1].copy()[::-1]
+        return same(HaplotypeMatrix(x, p), hap, pos)
     if form == "pinned":
         return same(HaplotypeMatrix(torch.as_tensor(hap).pin_memory(), pos), hap, pos)
+    if form == "overlap":
+        # windows of one pinned row: row r starts at site r
+        row = torch.as_tensor(hap.reshape(-1)[:M + H]).pin_memory()
+        x = row.as_strided((H, M), (1, 1))
+        return same(HaplotypeMatrix(x, pos), x.numpy(), pos)
     x = np.asfortranarray(hap) if form == "fortran" else hap.astype(form)
     same(HaplotypeMatrix(x, pos), hap, pos)
 
