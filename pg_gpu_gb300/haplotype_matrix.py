@@ -349,6 +349,9 @@ class HaplotypeMatrix:
                          else positions_idx)
         if self._device == "GPU":
             import torch
+            # (index_select faults on the device instead of raising)
+            if idx.size and not 0 <= idx.min() <= idx.max() < min(self.num_variants, len(self._positions)):
+                raise IndexError("variant index out of range")
             ti = torch.as_tensor(idx, device=self._haplotypes.device, dtype=torch.int64)
             hap = self._haplotypes.index_select(1, ti)
             pos = self._positions.index_select(0, ti)
@@ -506,6 +509,9 @@ class HaplotypeMatrix:
             rows = _ops.device_rows(rows, src.shape[0])
         pos = self._positions
         pos = _ops.positions_f64(pos if _is_torch(pos) else np.ascontiguousarray(pos))
+        # (a gather past the end would fault on the device)
+        if pos.numel() < src.shape[1] and int(kept[1][-1]) >= pos.numel():
+            raise IndexError("a site has no position")
         packs = _ops.pack_all(src, rows, kept)
         pos = pos.index_select(0, kept[1])
         sums, cnt = _ops.binned_sums(packs, pos, bins)

@@ -90,3 +90,19 @@ def test_site_counts_of_strided_and_wider_tensors():
     for t in (d.repeat_interleave(2, 1)[:, ::2], d.t().contiguous().t(), d.to(torch.int32)):
         for a, b in zip(_ops.site_counts(t, flags=True), ref):
             assert torch.equal(a.cpu(), b)
+
+
+# checked on the host: a gather past the end would fault on the device
+@pytest.mark.parametrize("device", ["cpu", "cuda"])
+def test_positions_that_end_early(device):
+    hap, pos = panel()
+    hap[:, -2] = 0
+    hap[:, -1] = 0
+    x = hap if device == "cpu" else torch.as_tensor(hap, device=device)
+    same(HaplotypeMatrix(x, pos[:-1]), hap[:, :-1], pos[:-1])  # the sites without one are dropped
+    hm = HaplotypeMatrix(x, pos[:M // 2])
+    with pytest.raises(IndexError):
+        hm.compute_ld_statistics_gpu_single_pop(BINS, raw=True)
+    if device == "cuda":
+        with pytest.raises(IndexError):
+            hm.get_subset([M - 1])
