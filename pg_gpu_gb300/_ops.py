@@ -98,9 +98,9 @@ class Rows:
 
 
 def device_rows(row_lists, n_total):
-    """Rows of several populations' host index lists, checked against n_total
-    and uploaded together."""
-    host = [np.asarray(r).astype(np.int32, copy=False).reshape(-1) for r in row_lists]
+    """Rows of several populations' index lists, checked against n_total (as they
+    are: a cast first would wrap) and uploaded together."""
+    host = [np.asarray(r).reshape(-1) for r in row_lists]
     whole = _check_rows(np.concatenate(host), n_total)
     ends = np.cumsum([r.size for r in host])
     return [Rows(whole[e - r.size:e]) for e, r in zip(ends, host)]
