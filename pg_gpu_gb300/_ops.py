@@ -97,10 +97,15 @@ class Rows:
         self.tensor = tensor
 
 
+def host_rows(rows):
+    """Row indices that may be a tensor (on the device, too), on the host."""
+    return rows.tolist() if isinstance(rows, _torch().Tensor) else rows
+
+
 def device_rows(row_lists, n_total):
     """Rows of several populations' index lists, checked against n_total (as they
     are: a cast first would wrap) and uploaded together."""
-    host = [np.asarray(r).reshape(-1) for r in row_lists]
+    host = [np.asarray(host_rows(r)).reshape(-1) for r in row_lists]
     whole = _check_rows(np.concatenate(host), n_total)
     ends = np.cumsum([r.size for r in host])
     return [Rows(whole[e - r.size:e]) for e, r in zip(ends, host)]

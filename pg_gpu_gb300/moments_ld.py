@@ -171,7 +171,7 @@ def _compute_ld_sums(mat, pops, bins, gen_dists, max_bp, use_genotypes=False, po
     if use_genotypes:
         # variants polymorphic across the union of the populations (moments_ld.py:256-280)
         g = L.as_device(mat.genotypes, np.int8)
-        rows = sorted(set(i for p in pops for i in mat.sample_sets[p]))
+        rows = sorted(set(i for p in pops for i in _ops.host_rows(mat.sample_sets[p])))
         kept = _ops.kept_sites(_ops.KEEP_DIPLOID, _ops.site_counts(g, rows))
         pos_d = L.as_device(mat.positions, np.float64).index_select(0, kept[1])
         bc = (None if gen_dists is None else

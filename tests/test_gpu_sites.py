@@ -109,3 +109,21 @@ def test_heterozygosity(P, M, ploidy):
             want.append((2 * ri * alt[i] / (m[i] * (m[i] - 1))).sum() if i == j else
                         ((ri * alt[j] + alt[i] * rj) / (m[i] * m[j])).sum())
     np.testing.assert_allclose(got, want, rtol=1e-12)
+
+
+# a GenotypeMatrix does not ask for lists: rows as device tensors, arrays and lists
+@pytest.mark.parametrize("form", ["device", "host", "array"])
+def test_genotype_sample_sets_of_other_kinds(form):
+    from pg_gpu_gb300 import moments_ld
+    from pg_gpu_gb300.genotype_matrix import GenotypeMatrix
+    rng = np.random.default_rng(3)
+    g = torch.as_tensor(rng.binomial(2, rng.beta(0.4, 0.4, 300), (30, 300)).astype(np.int8), device="cuda")
+    pos = np.sort(rng.choice(30_000, 300, replace=False))
+    lists = {"pop0": list(range(14)), "pop1": list(range(10, 30))}
+    to = {"device": lambda r: torch.tensor(r, device="cuda"), "host": torch.tensor, "array": np.array}[form]
+    got, want = (moments_ld.compute_ld_statistics(
+        genotype_matrix=GenotypeMatrix(g, pos, sample_sets=sets), use_genotypes=True,
+        bp_bins=[0, 5000, 20_000], report=False)
+        for sets in ({k: to(r) for k, r in lists.items()}, lists))
+    for a, b in zip(got["sums"], want["sums"]):
+        np.testing.assert_allclose(a, b, rtol=1e-12)
