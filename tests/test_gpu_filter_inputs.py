@@ -106,3 +106,14 @@ def test_positions_that_end_early(device):
     if device == "cuda":
         with pytest.raises(IndexError):
             hm.get_subset([M - 1])
+
+
+def test_host_array_set_on_a_device_matrix():
+    hap, pos = panel()
+    sets = {"a": list(range(20)), "b": list(range(20, H))}
+    ref = HaplotypeMatrix(torch.as_tensor(hap, device="cuda"), pos, sample_sets=sets)
+    hm = HaplotypeMatrix(torch.zeros_like(ref.haplotypes), pos, sample_sets=sets)
+    hm.haplotypes = hap
+    got, want = ([(p.planes, p.valid) for p in m.packed_all(["a", "b"])] for m in (hm, ref))
+    for a, b in zip(got, want):
+        assert all(torch.equal(x, y) for x, y in zip(a, b))
