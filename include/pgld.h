@@ -415,9 +415,15 @@ int pgld_geno_stats(pgld_handle h, const pgld_pair_counts* counts, int64_t n_pai
 /* Rogers-Huff r of every SNP pair i < j (condensed upper triangle, float64) of
  * one population of n_rows individuals with dosages 0 / 1 / 2 and none missing;
  * NaN where a SNP has no variance.  Replaces rogers_huff_r's tiles
- * (ld_statistics.py:410-521). */
+ * (ld_statistics.py:410-521).  Synchronises: the sites' sums lie in the handle's
+ * workspace. */
 int pgld_geno_rogers_huff(pgld_handle h, const uint32_t* planes, int32_t n_words, int32_t n_rows,
                           int64_t n_snp, double* out, void* stream);
+/* The same, asynchronous, with the caller's device buffer for the sites' sums
+ * (two int32 per SNP, 8-byte aligned). */
+int pgld_geno_rogers_huff_sites(pgld_handle h, const uint32_t* planes, int32_t n_words,
+                                int32_t n_rows, int64_t n_snp, int32_t* sites, double* out,
+                                void* stream);
 
 /* Per-pair outputs over the distance band of one population, in the
  * reference's pair order: counts [n_pairs][9] int32 (nullable), n_valid

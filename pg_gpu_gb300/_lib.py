@@ -99,6 +99,7 @@ _SIGS = {
     "pgld_geno_band_pairs_at": ([_P, ctypes.POINTER(GenoPanel), _P, _D, _P, _P, _P, _P, _I32, _I64,
                                  _I32, _P], ctypes.c_int),
     "pgld_geno_rogers_huff": ([_P, _P, _I32, _I32, _I64, _P, _P], ctypes.c_int),
+    "pgld_geno_rogers_huff_sites": ([_P, _P, _I32, _I32, _I64, _P, _P, _P], ctypes.c_int),
     "pgld_hap_band_pairs": ([_P, ctypes.POINTER(HapPanel), _P, _D, _P, _P, _P, _I64, _I32, _P],
                             ctypes.c_int),
     "pgld_hap_binned_sums": ([_P, ctypes.POINTER(HapPanel), _P, _D, _P, _P, _I32, _P, _P, _I32,

@@ -733,8 +733,9 @@ def rogers_huff_all(pk):
     out = torch.empty(m * (m - 1) // 2, dtype=torch.float64, device=pk.planes.device)
     if out.numel():
         h = L.handle()
-        L.check(L.lib().pgld_geno_rogers_huff(h, L.ptr(pk.planes), pk.n_words, pk.n_rows, m,
-                                              L.ptr(out), L.stream_ptr()), h)
+        sites = torch.empty((m, 2), dtype=torch.int32, device=out.device)
+        L.check(L.lib().pgld_geno_rogers_huff_sites(h, L.ptr(pk.planes), pk.n_words, pk.n_rows, m,
+                                                    L.ptr(sites), L.ptr(out), L.stream_ptr()), h)
     return out
 
 

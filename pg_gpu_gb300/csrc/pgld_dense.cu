@@ -671,27 +671,41 @@ int pgld_tally_tiles(pgld_context* h, const uint32_t* planes, const uint32_t* va
   return PGLD_OK;
 }
 
-extern "C" int pgld_geno_rogers_huff(pgld_handle h, const uint32_t* planes, int32_t n_words,
-                                     int32_t n_rows, int64_t n_snp, double* out, void* stream) {
+extern "C" int pgld_geno_rogers_huff_sites(pgld_handle h, const uint32_t* planes, int32_t n_words,
+                                           int32_t n_rows, int64_t n_snp, int32_t* sites, double* out,
+                                           void* stream) {
   using namespace pgld::dense;
   PGLD_REQUIRE(h, h != nullptr, "pgld_geno_rogers_huff: NULL handle");
   PGLD_REQUIRE(h, n_words >= 1 && n_rows >= 0 && n_rows <= 8192 && n_rows <= 32 * (int64_t)n_words && n_snp >= 0,
                "pgld_geno_rogers_huff: sizes");
   if (n_snp < 2) return PGLD_OK;
-  PGLD_REQUIRE(h, planes && out, "pgld_geno_rogers_huff: NULL buffer");
+  PGLD_REQUIRE(h, planes && sites && out, "pgld_geno_rogers_huff: NULL buffer");
+  PGLD_REQUIRE(h, ((uintptr_t)sites & 7) == 0, "pgld_geno_rogers_huff: sites must be 8-byte aligned");
   PGLD_CHECK_CUDA(h, cudaSetDevice(h->device));
   cudaStream_t st = (cudaStream_t)stream;
-  void* ws = nullptr;
-  int rc = pgld_workspace(h, (size_t)n_snp * sizeof(int2), &ws);
-  if (rc) return rc;
+  int2* site = reinterpret_cast<int2*>(sites);
   const unsigned sb = (unsigned)std::max<i64>(1, std::min<i64>((n_snp + 255) / 256, h->n_sm * 8LL));
-  dosage_site_kernel<<<sb, 256, 0, st>>>(planes, n_words, n_snp, n_rows, (int2*)ws);
+  dosage_site_kernel<<<sb, 256, 0, st>>>(planes, n_words, n_snp, n_rows, site);
   const i64 nb = (n_snp + kT - 1) / kT;
   const int grid = dense_grid(h, (const void*)rogers_huff_kernel, 0, nb * (nb + 1) / 2);
   pgld_time_begin(h, st);
-  rogers_huff_kernel<<<grid, kThreads, 0, st>>>(planes, n_words, n_snp, n_rows, (const int2*)ws, out);
+  rogers_huff_kernel<<<grid, kThreads, 0, st>>>(planes, n_words, n_snp, n_rows, site, out);
   pgld_time_end(h, st);
   PGLD_CHECK_CUDA(h, cudaGetLastError());
+  return PGLD_OK;
+}
+
+extern "C" int pgld_geno_rogers_huff(pgld_handle h, const uint32_t* planes, int32_t n_words,
+                                     int32_t n_rows, int64_t n_snp, double* out, void* stream) {
+  PGLD_REQUIRE(h, h != nullptr && n_snp >= 0, "pgld_geno_rogers_huff: sizes");
+  PGLD_CHECK_CUDA(h, cudaSetDevice(h->device));
+  void* ws = nullptr;
+  int rc = pgld_workspace(h, (size_t)n_snp * 8, &ws);
+  if (rc) return rc;
+  rc = pgld_geno_rogers_huff_sites(h, planes, n_words, n_rows, n_snp, (int32_t*)ws, out, stream);
+  if (rc) return rc;
+  // the handle's workspace holds the sites: a call on another stream may take it next
+  PGLD_CHECK_CUDA(h, cudaStreamSynchronize((cudaStream_t)stream));
   return PGLD_OK;
 }
 

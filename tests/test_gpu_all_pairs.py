@@ -81,3 +81,33 @@ def test_single_terms_and_tables(n, pad):
         more = spec_terms(P) + [(S, L.DD_II, (0,), 1.0)]
         want = np_(_ops.stats(views[:P], nv[:P], more, S + 1))[:, :S]
         np.testing.assert_allclose(got, want, rtol=1e-14, atol=1e-15 * np.abs(want).max())
+
+
+def test_rogers_huff_on_two_streams():
+    """Calls on two streams of one handle: each has its own table of sites."""
+    rng = np.random.default_rng(12)
+    m, n = 9000, 400
+    packs = [_ops.pack_geno(torch.as_tensor(
+        rng.binomial(2, rng.beta(0.3 + k, 0.5, m), (n, m)).astype(np.int8), device="cuda")) for k in range(2)]
+    want = [_ops.rogers_huff_all(pk) for pk in packs]
+    streams = [torch.cuda.Stream() for _ in packs]
+    torch.cuda.synchronize()
+    got = []
+    for _ in range(3):
+        for pk, s in zip(packs, streams):
+            with torch.cuda.stream(s):
+                got.append(_ops.rogers_huff_all(pk))
+    torch.cuda.synchronize()
+    for k, r in enumerate(got):
+        assert torch.equal(torch.nan_to_num(r, nan=9.0), torch.nan_to_num(want[k % 2], nan=9.0))
+
+
+def test_rogers_huff_entry_with_its_own_sites():
+    from pg_gpu_gb300 import _lib as L
+    rng = np.random.default_rng(4)
+    pk = _ops.pack_geno(torch.as_tensor(rng.integers(0, 3, (50, 70)).astype(np.int8), device="cuda"))
+    out = torch.empty(70 * 69 // 2, dtype=torch.float64, device="cuda")
+    h = L.handle()
+    L.check(L.lib().pgld_geno_rogers_huff(h, L.ptr(pk.planes), pk.n_words, pk.n_rows, 70, L.ptr(out),
+                                          L.stream_ptr()), h)
+    assert torch.equal(out, _ops.rogers_huff_all(pk))
