@@ -108,9 +108,9 @@ def rogers_huff_r(matrix):
     import torch
     g = dosage(matrix)
     pk = _ops.pack_geno(g)
-    if not pk.has_other:
+    if not (pk.has_other or pk.has_missing):
         return _ops.rogers_huff_all(pk)
-    # dosages above 2 fold into the counts' classes
+    # dosages above 2 (or past 127, which wrap below 0) fold into the counts' classes
     m = g.shape[1]
     ii, jj = torch.triu_indices(m, m, offset=1, device=g.device)
     return rh_pairs(g, ii.to(torch.int32), jj.to(torch.int32))

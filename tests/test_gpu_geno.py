@@ -370,3 +370,18 @@ def test_full_size_geno_band():
     assert np.array_equal(np.isnan(got), np.isnan(ref))
     m = ~np.isnan(ref) & (np.abs(ref) > 1e-30)
     assert (np.abs(got[m] - ref[m]) / np.abs(ref[m])).max() <= 1e-6
+
+
+def test_rogers_huff_of_codes_whose_sum_wraps():
+    """Two codes of 64 and more add up to a negative dosage: such individuals are
+    left out of the pairs, as missing ones are."""
+    from pg_gpu_gb300.haplotype_matrix import HaplotypeMatrix
+    rng = np.random.default_rng(9)
+    hap = rng.integers(0, 2, (40, 50)).astype(np.int8)
+    hap[0:2, 3] = 100
+    hap[6:8, 8:11] = 64
+    r = np_(ld_statistics.rogers_huff_r(HaplotypeMatrix(hap, np.arange(50))))
+    g = hap[0::2] + hap[1::2]
+    assert g.min() < 0 and not ((g > 2).any())
+    ii, jj = np.triu_indices(50, 1)
+    np.testing.assert_allclose(r, O.rogers_huff_r_pairs(g, ii, jj), rtol=1e-12, atol=1e-13)
