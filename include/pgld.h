@@ -141,6 +141,12 @@ int pgld_keep_sites(pgld_handle h, int32_t rule, const int32_t* sum, const int32
 int pgld_heterozygosity(pgld_handle h, int32_t n_pops, const int32_t* const* sum,
                         const int32_t* const* valid, const int32_t* n_rows, int32_t ploidy,
                         int64_t n_snp, double* out, void* stream);
+/* The same in n_parts partial sums, out [n_parts][n_pops (n_pops + 1) / 2], which
+ * depend on n_snp and n_parts alone: added in a fixed order they repeat to the
+ * last bit, where the sums above are added in the order that blocks end in. */
+int pgld_heterozygosity_parts(pgld_handle h, int32_t n_pops, const int32_t* const* sum,
+                              const int32_t* const* valid, const int32_t* n_rows, int32_t ploidy,
+                              int64_t n_snp, int32_t n_parts, double* out, void* stream);
 
 /* Joint counts [n11, n10, n01, n00] of listed SNP pairs for one
  * population; counts row stride counts_ld (int32 elements, >= 4).

@@ -84,6 +84,8 @@ _SIGS = {
                         ctypes.c_int),
     "pgld_heterozygosity": ([_P, _I32, ctypes.POINTER(_P), ctypes.POINTER(_P),
                              ctypes.POINTER(_I32), _I32, _I64, _P, _P], ctypes.c_int),
+    "pgld_heterozygosity_parts": ([_P, _I32, ctypes.POINTER(_P), ctypes.POINTER(_P),
+                                   ctypes.POINTER(_I32), _I32, _I64, _I32, _P, _P], ctypes.c_int),
     "pgld_hap_counts_pairs": ([_P, _P, _P, _I32, _I64, _P, _P, _I64, _P, _I64, _P, _P],
                               ctypes.c_int),
     "pgld_hap_tally": ([_P, _P, _P, _I32, _I64, _P, _P, _P], ctypes.c_int),

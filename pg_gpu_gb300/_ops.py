@@ -187,16 +187,18 @@ def kept_sites(rule, counts):
 
 def heterozygosity(sums, valids, n_rows, ploidy):
     """float64 H_ij (i <= j) on the host from per-population site sums (and
-    valid counts, or None where every row counts)."""
+    valid counts, or None where every row counts); equal inputs give equal bits."""
     torch = _torch()
     P = len(sums)
-    out = torch.empty(P * (P + 1) // 2, dtype=torch.float64, device=sums[0].device)
+    n = sums[0].numel()
+    parts = min(max(1, -(-n // 256)), 256)
+    out = torch.empty((parts, P * (P + 1) // 2), dtype=torch.float64, device=sums[0].device)
     ptrs = [(ctypes.c_void_p * P)(*(t.data_ptr() if t is not None else None for t in ts))
             for ts in (sums, valids)]
     h = L.handle()
-    L.check(L.lib().pgld_heterozygosity(h, P, *ptrs, (ctypes.c_int32 * P)(*n_rows), ploidy,
-                                        sums[0].numel(), L.ptr(out), L.stream_ptr()), h)
-    return out.cpu().numpy()
+    L.check(L.lib().pgld_heterozygosity_parts(h, P, *ptrs, (ctypes.c_int32 * P)(*n_rows), ploidy, n,
+                                              parts, L.ptr(out), L.stream_ptr()), h)
+    return out.cpu().numpy().sum(0)
 
 
 def pack(hap, rows=None, kept=None, flags=None, k=0):

@@ -383,6 +383,9 @@ struct HetArgs {
   double per;  // allele copies per row
 };
 
+// PARTS: block b's sums to out[b][], for the caller to add in a fixed order (equal
+// inputs then give equal bits); else added to out[] in whatever order the blocks end
+template <bool PARTS>
 __global__ void __launch_bounds__(256) het_kernel(HetArgs a, i64 n, double* __restrict__ out) {
   __shared__ double sh[8];
   double tot[10] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
@@ -418,7 +421,8 @@ __global__ void __launch_bounds__(256) het_kernel(HetArgs a, i64 n, double* __re
       __syncthreads();
       if (threadIdx.x == 0) {
         for (int w = 1; w < 8; ++w) v += sh[w];
-        atomicAdd(out + o, v);
+        if (PARTS) out[(size_t)blockIdx.x * (a.n_pops * (a.n_pops + 1) / 2) + o] = v;
+        else atomicAdd(out + o, v);
       }
       ++o;
     }
@@ -549,9 +553,10 @@ extern "C" int pgld_keep_sites(pgld_handle h, int32_t rule, const int32_t* sum, 
   return PGLD_OK;
 }
 
-extern "C" int pgld_heterozygosity(pgld_handle h, int32_t n_pops, const int32_t* const* sum,
-                                   const int32_t* const* valid, const int32_t* n_rows,
-                                   int32_t ploidy, int64_t n_snp, double* out, void* stream) {
+// parts > 0: the sums of that many blocks; 0: their total
+static int heterozygosity(pgld_handle h, int32_t n_pops, const int32_t* const* sum,
+                          const int32_t* const* valid, const int32_t* n_rows, int32_t ploidy,
+                          int64_t n_snp, int32_t parts, double* out, void* stream) {
   using namespace pgld::sites;
   PGLD_REQUIRE(h, h != nullptr, "pgld_heterozygosity: NULL handle");
   PGLD_REQUIRE(h, n_pops >= 1 && n_pops <= PGLD_MAX_POPS && n_snp >= 0 && ploidy >= 1,
@@ -568,10 +573,28 @@ extern "C" int pgld_heterozygosity(pgld_handle h, int32_t n_pops, const int32_t*
   }
   PGLD_CHECK_CUDA(h, cudaSetDevice(h->device));
   cudaStream_t st = (cudaStream_t)stream;
-  PGLD_CHECK_CUDA(h, cudaMemsetAsync(out, 0, (size_t)n_pops * (n_pops + 1) / 2 * 8, st));
-  if (n_snp == 0) return PGLD_OK;
-  const unsigned blocks = (unsigned)std::min<i64>((n_snp + 255) / 256, (i64)h->n_sm * 4);
-  het_kernel<<<blocks, 256, 0, st>>>(a, n_snp, out);
+  if (parts > 0) {
+    het_kernel<true><<<(unsigned)parts, 256, 0, st>>>(a, n_snp, out);
+  } else {
+    PGLD_CHECK_CUDA(h, cudaMemsetAsync(out, 0, (size_t)n_pops * (n_pops + 1) / 2 * 8, st));
+    if (n_snp == 0) return PGLD_OK;
+    const unsigned blocks = (unsigned)std::min<i64>((n_snp + 255) / 256, (i64)h->n_sm * 4);
+    het_kernel<false><<<blocks, 256, 0, st>>>(a, n_snp, out);
+  }
   PGLD_CHECK_CUDA(h, cudaGetLastError());
   return PGLD_OK;
+}
+
+extern "C" int pgld_heterozygosity(pgld_handle h, int32_t n_pops, const int32_t* const* sum,
+                                   const int32_t* const* valid, const int32_t* n_rows,
+                                   int32_t ploidy, int64_t n_snp, double* out, void* stream) {
+  return heterozygosity(h, n_pops, sum, valid, n_rows, ploidy, n_snp, 0, out, stream);
+}
+
+extern "C" int pgld_heterozygosity_parts(pgld_handle h, int32_t n_pops, const int32_t* const* sum,
+                                         const int32_t* const* valid, const int32_t* n_rows,
+                                         int32_t ploidy, int64_t n_snp, int32_t n_parts, double* out,
+                                         void* stream) {
+  PGLD_REQUIRE(h, n_parts >= 1 && n_parts <= 1 << 20, "pgld_heterozygosity_parts: n_parts");
+  return heterozygosity(h, n_pops, sum, valid, n_rows, ploidy, n_snp, n_parts, out, stream);
 }

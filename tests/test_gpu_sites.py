@@ -127,3 +127,14 @@ def test_genotype_sample_sets_of_other_kinds(form):
         for sets in ({k: to(r) for k, r in lists.items()}, lists))
     for a, b in zip(got["sums"], want["sums"]):
         np.testing.assert_allclose(a, b, rtol=1e-12)
+
+
+@pytest.mark.parametrize("M", [0, 1, 257, 100_001])
+def test_heterozygosity_repeats_to_the_last_bit(M):
+    rng = np.random.default_rng(M)
+    n = [30, 41, 7]
+    s = [torch.as_tensor(rng.integers(0, k + 1, M).astype(np.int32), device="cuda") for k in n]
+    first = _ops.heterozygosity(s, [None] * 3, n, 1)
+    assert first.shape == (6,) and (M > 0 or not first.any())
+    for _ in range(30):
+        assert np.array_equal(_ops.heterozygosity(s, [None] * 3, n, 1), first)
