@@ -1214,11 +1214,12 @@ int pgld_tc_pack_rows(pgld_context* h, const uint32_t* planes, int W, long long 
 int pgld_site_freqs(pgld_context* h, const uint32_t* planes, const uint32_t* valid, int W,
                     long long n_snp, float4* site, cudaStream_t st);
 
-// shared memory, stages and the register check of a one-population launch
+// shared memory, stages and the register check of a one-population launch; first:
+// a launch made ready before, in the same timed interval
 template <int MODE, int COLS = pgld::win::kAllColumns>
 static int wide_one_pop_launch(pgld_context* h, pgld::tcw::Params& prm, const CUtensorMap& map_a,
                                const CUtensorMap& map_b, cudaStream_t st, const char* what,
-                               bool timed = true) {
+                               const std::function<int()>& first = nullptr) {
   using namespace pgld::tcw;
   if (h->test_fault == PGLD_TEST_FAULT_NO_COPIES) {
     prm.no_copies = 1;
@@ -1247,9 +1248,11 @@ static int wide_one_pop_launch(pgld_context* h, pgld::tcw::Params& prm, const CU
 #endif
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return pgld_cuda_fail(h, e, "band_wide smem attribute");
-  if (timed) pgld_time_begin(h, st);
-  kern<<<(unsigned)h->n_sm, kThreads, smem, st>>>(map_a, map_b, prm);
-  if (timed) pgld_time_end(h, st);
+  pgld_time_begin(h, st);
+  const int rc = first ? first() : PGLD_OK;
+  if (!rc) kern<<<(unsigned)h->n_sm, kThreads, smem, st>>>(map_a, map_b, prm);
+  pgld_time_end(h, st);
+  if (rc) return rc;
   e = cudaGetLastError();
   if (e != cudaSuccess) return pgld_cuda_fail(h, e, what);
   return PGLD_OK;
@@ -1415,20 +1418,16 @@ int pgld_tc_wide_windows(pgld_context* h, const pgld_hap_panel* panel, const int
   prm.wcnt = counts;
   prm.state = state;
   // one timed interval: of the two kernels one has the windows
-  pgld_time_begin(h, st);
+  std::function<int()> complete;
   if (state) {
     rc = pgld_window_complete_sums(h, state, W, n_idx, op, list_site, wb, we, n_win, tiles, sums,
-                                   counts, columns, st);
+                                   counts, columns, st, &complete);
     if (rc) return rc;
   }
   const char* what = "band_wide_kernel (windows)";
-  if (sigma)
-    rc = wide_one_pop_launch<pgld::kModeWindows, 2>(h, prm, map_a, map_b, st, what, false);
-  else if (columns == 32)
-    rc = wide_one_pop_launch<pgld::kModeWindows, 32>(h, prm, map_a, map_b, st, what, false);
-  else
-    rc = wide_one_pop_launch<pgld::kModeWindows, pgld::win::kAllColumns>(h, prm, map_a, map_b, st, what,
-                                                                         false);
-  pgld_time_end(h, st);
-  return rc;
+  if (sigma) return wide_one_pop_launch<pgld::kModeWindows, 2>(h, prm, map_a, map_b, st, what, complete);
+  if (columns == 32)
+    return wide_one_pop_launch<pgld::kModeWindows, 32>(h, prm, map_a, map_b, st, what, complete);
+  return wide_one_pop_launch<pgld::kModeWindows, pgld::win::kAllColumns>(h, prm, map_a, map_b, st, what,
+                                                                         complete);
 }

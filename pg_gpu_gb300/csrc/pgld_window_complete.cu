@@ -558,14 +558,16 @@ __global__ void __launch_bounds__(kThreads, 1)
 }
 
 template <int COLS>
-static int launch(pgld_context* h, const Params& prm, const CUtensorMap& map_a,
-                  const CUtensorMap& map_b, size_t smem, cudaStream_t st) {
+static int prepare(pgld_context* h, const Params& prm, const CUtensorMap& map_a,
+                  const CUtensorMap& map_b, size_t smem, cudaStream_t st, std::function<int()>* out) {
   auto kern = window_complete_kernel<COLS>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return pgld_cuda_fail(h, e, "window_complete smem attribute");
-  kern<<<(unsigned)h->n_sm, kThreads, smem, st>>>(map_a, map_b, prm);
-  e = cudaGetLastError();
-  if (e != cudaSuccess) return pgld_cuda_fail(h, e, "window_complete_kernel");
+  *out = [=]() -> int {
+    kern<<<(unsigned)h->n_sm, kThreads, smem, st>>>(map_a, map_b, prm);
+    const cudaError_t l = cudaGetLastError();
+    return l != cudaSuccess ? pgld_cuda_fail(h, l, "window_complete_kernel") : PGLD_OK;
+  };
   return PGLD_OK;
 }
 
@@ -592,11 +594,13 @@ int pgld_window_complete_pack(pgld_context* h, const uint32_t* planes, int W, lo
 }
 
 // The windows' sums where state says the list is complete (columns: 2, 32 or all).
-// The caller times it together with the general kernel.
+// Makes the launch ready: the caller issues it just before the general kernel, in
+// one timed interval.
 int pgld_window_complete_sums(pgld_context* h, const State* state, int W, long long n_idx,
                               const unsigned char* op, const float2* site, const long long* wb,
                               const long long* we, int n_win, const long long* tile_off, double* sums,
-                              unsigned long long* counts, int columns, cudaStream_t st) {
+                              unsigned long long* counts, int columns, cudaStream_t st,
+                              std::function<int()>* launch) {
   CUtensorMap map_a, map_b;
   int rc = pgld::tchost::make_map(h, &map_a, op, n_idx, 32 * W, 128);
   if (rc) return rc;
@@ -627,7 +631,7 @@ int pgld_window_complete_sums(pgld_context* h, const State* state, int W, long l
   if (stages < 2) return pgld_fail(h, PGLD_ERR_TOO_LARGE, "complete windows: shared memory");
   prm.stages = stages;
   const size_t smem = (size_t)stages * kStage + fixed;
-  if (columns == 2) return launch<2>(h, prm, map_a, map_b, smem, st);
-  if (columns == 32) return launch<32>(h, prm, map_a, map_b, smem, st);
-  return launch<pgld::win::kAllColumns>(h, prm, map_a, map_b, smem, st);
+  if (columns == 2) return prepare<2>(h, prm, map_a, map_b, smem, st, launch);
+  if (columns == 32) return prepare<32>(h, prm, map_a, map_b, smem, st, launch);
+  return prepare<pgld::win::kAllColumns>(h, prm, map_a, map_b, smem, st, launch);
 }

@@ -3,6 +3,8 @@
 #pragma once
 #include <stdint.h>
 
+#include <functional>
+
 namespace pgld {
 namespace wcomp {
 
@@ -46,4 +48,4 @@ int pgld_window_complete_sums(pgld_context* h, const pgld::wcomp::State* state, 
                               long long n_idx, const unsigned char* op, const float2* site,
                               const long long* wb, const long long* we, int n_win,
                               const long long* tile_off, double* sums, unsigned long long* counts,
-                              int columns, cudaStream_t st);
+                              int columns, cudaStream_t st, std::function<int()>* launch);
