@@ -135,7 +135,8 @@ __global__ void __launch_bounds__(256) pack_complete_kernel(
   const long long step = (long long)gridDim.x * 8;
   constexpr int kRows = 4;  // list positions in flight per warp
   for (long long r0 = (long long)blockIdx.x * 8 + (threadIdx.x >> 5); r0 < n_idx; r0 += kRows * step) {
-    if (!*complete) return;
+    // one decision for the warp: another warp may clear the flag while this one reads it
+    if (!__any_sync(0xffffffffu, *complete)) return;
     long long s[kRows];
     uint32_t c[kRows][WL], z[kRows][WL];
 #pragma unroll
