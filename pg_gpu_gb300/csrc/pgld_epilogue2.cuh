@@ -111,27 +111,16 @@ PGLD_HD V pi2_num(const Pop& p) {
   const V w = vfma(vsub(vs(2.0f), p.ns), p.t, vadd(p.x, p.m1));
   return dot2(p.a, pn, p.x, w);
 }
-// fast::Draws of two pairs
-struct Draws {
-  V X1, X2, X3, X4, T1, T2;
-};
-PGLD_HD Draws draws(const Pop& p) {
-  Draws d;
-  const V nx = vneg(p.x);
-  d.X1 = vfma(p.c1, p.m1, nx);
-  d.X2 = vfma(p.c2, p.m1, p.x);
-  d.X3 = vfma(p.c3, p.m1, p.x);
-  d.X4 = vfma(p.c4, p.m1, nx);
-  d.T1 = vfma(p.pA, d.X4, vneg(vmul(p.c2, p.qA)));
-  d.T2 = vfma(p.pA, d.X3, vneg(vmul(p.c1, p.qA)));
-  return d;
+// fast::pi2_pairs with nm = 1 - n, and the negative of fast::triple_num2 with
+// nmix = -mixB: operands negated where they are formed, not in packed
+// instructions of their own (13.31 -> 13.25 ms for two populations of 1,000, a
+// chromosome arm)
+PGLD_HD V pi2_pairs(const Pop& p, V hA, V hB, V nm) {
+  return vfma(hA, hB, vfma(p.a, vfma(p.s, vs(-2.0f), nm), vmul(p.b, vfma(p.t, vs(-2.0f), nm))));
 }
-PGLD_HD V pi2_draws(const Pop& p, const Draws& d) {
-  return vfma(d.T1, p.pB, vneg(vfma(p.c1, d.X4, vmul(p.c3, d.X2))));
-}
-PGLD_HD V triple_num2(const Draws& t, const Pop& s) { return vfma(s.pB, t.T1, vmul(s.qB, t.T2)); }
-PGLD_HD V ijij_num4(const Draws& i, const Draws& j) {
-  return vfma(i.X1, j.X4, vfma(i.X2, j.X3, vfma(i.X3, j.X2, vmul(i.X4, j.X1))));
+PGLD_HD V triple_neg2(const Pop& t, V hA, V nmix, const Pop& s) {
+  const V yb = vfma(t.pA, t.c4, vmul(t.c2, t.qA)), yB = vfma(t.pA, t.c3, vmul(t.c1, t.qA));
+  return vfma(hA, nmix, vfma(yb, s.pB, vmul(yB, s.qB)));
 }
 
 // the reciprocal factors of the valid n of two lanes: 1/n, 1/(n(n-1)),
@@ -148,8 +137,8 @@ PGLD_HD void recip_entry4(int n, float4* e) {
 }
 // statistics 11 (pi2_0_0_1_1) and 12 (pi2_0_1_0_1) leave stats2_to with the
 // scale r22; their values are the num * r22 products (or sums of them) times
-// these exact powers of two
-constexpr float kPost11 = 0.5f, kPost12 = 0.25f;
+// these exact powers of two.  10 and 13 (pi2_i_i_i_j) leave it negative
+constexpr float kPost11 = 0.5f, kPost12 = 0.0625f;
 PGLD_HD R2 recip(const float4* T4, int n0, int n1) {
   const float4 a = T4[n0], b = T4[n1];
   return {make_float2(a.x, b.x), make_float2(a.y, b.y), make_float2(a.z, b.z),
@@ -175,12 +164,14 @@ PGLD_HD void stats2_to(const Pop& p, const Pop& q, const float4* T4, Sink&& sink
   sink(8, dz_num(q, wq), rq.r4);
   sink(5, vmul(p.x, wq), r22);
   sink(6, vmul(q.x, wp), r22);
-  const V uAp = vmul(p.pA, p.qA), uAq = vmul(q.pA, q.qA);
-  sink(11, vfma(uAp, vmul(q.pB, q.qB), vmul(uAq, vmul(p.pB, p.qB))), r22);  // x kPost11
-  const Draws dp = draws(p), dq = draws(q);
-  sink(9, pi2_draws(p, dp), rp.r4);
-  sink(14, pi2_draws(q, dq), rq.r4);
-  sink(12, ijij_num4(dp, dq), r22);                                          // x kPost12
+  // -2 mixB and -(n n' - dA dA' - dB dB')
+  const V nmp = vfma(p.ns, vs(-1.0f), vs(1.0f)), nmq = vfma(q.ns, vs(-1.0f), vs(1.0f));
+  const V nmix2 = vfma(p.dB, q.dB, vmul(p.ns, vmul(q.ns, vs(-1.0f)))), nmix = vmul(nmix2, vs(0.5f));
+  sink(12, dot2(vmul(nmp, q.m1), vfma(p.dA, q.dA, nmix2), wp, wq), r22);  // x kPost12
+  const V uAp = vmul(p.pA, p.qA), uAq = vmul(q.pA, q.qA), uBp = vmul(p.pB, p.qB), uBq = vmul(q.pB, q.qB);
+  sink(11, vfma(uAp, uBq, vmul(uAq, uBp)), r22);                          // x kPost11
+  sink(9, pi2_pairs(p, uAp, uBp, nmp), rp.r4);
+  sink(14, pi2_pairs(q, uAq, uBq, nmq), rq.r4);
   const V dc = vfma(p.dA, q.dB, vmul(p.dB, q.dA));
 #if PGLD_F2_SSCALE
   const V h31p = vmul_s(rp.r3h, rq.inv);
@@ -188,17 +179,17 @@ PGLD_HD void stats2_to(const Pop& p, const Pop& q, const float4* T4, Sink&& sink
   const V h31p = vmul(rp.r3h, rq.inv);
 #endif
   sink(4, vmul(p.x, dc), h31p);
-  sink(10, triple_num2(dp, q), h31p);
+  sink(10, triple_neg2(p, uAp, nmix, q), h31p);  // negative
 #if PGLD_F2_SSCALE
   const V h31q = vmul_s(rq.r3h, rp.inv);
 #else
   const V h31q = vmul(rq.r3h, rp.inv);
 #endif
   sink(7, vmul(q.x, dc), h31q);
-  sink(13, triple_num2(dq, p), h31q);
+  sink(13, triple_neg2(q, uAq, nmix, p), h31q);  // negative
 }
 
-// the sink's products, statistics 11 and 12 still without their post factors
+// the sink's products, statistics 10 - 13 still without their post factors
 PGLD_HD void stats2_raw(const Pop& p, const Pop& q, const float4* T4, V o[15]) {
   stats2_to(p, q, T4, [&](int k, V num, V sc) { o[k] = vmul(num, sc); });
 }
@@ -206,10 +197,12 @@ PGLD_HD void stats2(const Pop& p, const Pop& q, const float4* T4, V o[15]) {
   stats2_raw(p, q, T4, o);
   o[11] = vmul(o[11], vs(kPost11));
   o[12] = vmul(o[12], vs(kPost12));
+  o[10] = vsub(vs(0.f), o[10]);
+  o[13] = vsub(vs(0.f), o[13]);
 }
-// the post factor of statistic k of the two-population list (scaling by a
-// power of two commutes with every rounding of a sum of the sink's products)
-PGLD_HD constexpr double post2(int k) { return k == 11 ? kPost11 : k == 12 ? kPost12 : 1.0; }
+// the post factor of statistic k of the two-population list (scaling by a power
+// of two and the sign commute with every rounding of a sum of the sink's products)
+PGLD_HD constexpr double post2(int k) { return k == 11 ? kPost11 : k == 12 ? kPost12 : k == 10 || k == 13 ? -1.0 : 1.0; }
 
 // a / b with b > 0: the CUDA fast division (within 2 ulp for b below 2^126)
 PGLD_HD float fdiv(float a, float b) {

@@ -14,13 +14,18 @@
 // one class round apart (21 for three populations, 53 for four) instead of one
 // division per term (63 and 315 terms).
 //
-// Features per population are exact float32 integers, or one rounding of an
-// exact integer, for sample sizes up to kMaxN.  Products of draws from one
-// population are taken over distinct individuals as whole features: for two
-// draws X_pq = pA pB - c1 and its three siblings, for three T_q = pA X_PQ' -
-// c2 qA and T_Q.  The numerators of the mixed statistics are then sums of
-// non-negative products of features: no cancellation, a few float32 roundings
-// each, where the expanded polynomials needed 64-bit integers.
+// Features per population are exact float32 integers for sample sizes up to
+// kMaxN.  The numerators of mixed pi2 statistics are counts of draws: the product
+// of two exact features, one per SNP, less the choices that take a haplotype (an
+// individual) twice, a sum of non-negative products that is smaller by a factor
+// n.  They are exact where they are small or 0 and otherwise round once in
+// effect, like the 64-bit integers of the term table on their way to float32;
+// pi2_ijij is a two-product sum by Kahan's algorithm, and DD of one population
+// keeps its rounding error.  Against 64 bits the values of every statistic are no
+// further off than the table's: root mean square 0.51 - 0.83 units of 2^-24 of the
+// statistic where the table has 0.59 - 0.87 (three and four haplotype populations of
+// 30 - 400), 0.46 - 0.81 and 0.55 - 0.86 (two to four genotype populations of 30 -
+// 500), the largest ones 4.2 and 4.6 units of the terms' absolute sum.
 //
 // A quotient is num * (r + rl): r the approximate reciprocal of the
 // denominator den (the exact integer in float32: a product of two exact
@@ -84,13 +89,18 @@ PGLD_HD Den make_den(float den) {
   return d;
 }
 PGLD_HD float quot(float num, Den d) { return fmaf(num, d.r, fast::fmul(num, d.rl)); }
+// of a numerator and the rest that its rounding dropped
+PGLD_HD float quot(float num, float rest, Den d) {
+  return fmaf(num, d.r, fmaf(rest, d.r, fast::fmul(num, d.rl)));
+}
 
 struct Size {
-  float n, m2, k, m2b;  // n, n (n - 1), n - 2, (n - 2)(n - 3)
+  float n, m, m2, k, m2b;  // n, n - 1, n (n - 1), n - 2, (n - 2)(n - 3)
 };
 PGLD_HD Size make_size(float n) {
   Size s;
   s.n = n;
+  s.m = n - 1.0f;
   s.m2 = n * (n - 1.0f);
   s.k = n - 2.0f;
   s.m2b = s.k * (n - 3.0f);
@@ -112,11 +122,11 @@ PGLD_HD float four_four(float a, float b) {
 // ---- haplotypes ------------------------------------------------------------
 struct Hap {
   Size z;
+  float c1, c2, c3, c4;
   float x, w, dA, dB;         // c1c4 - c2c3, dA dB + e, qA - pA, qB - pB
   float pA, qA, pB, qB, hA, hB;  // hA = pA qA, hB = pB qB
-  float X1, X2, X3, X4;       // pA pB - c1, pA qB - c2, qA pB - c3, qA qB - c4
-  float T1, T2;               // distinct draws (A, a, b) and (A, a, B)
-  float dd, dz, pi;           // numerators over d4
+  float yb, yB;               // pA c4 + c2 qA, pA c3 + c1 qA: draws (A, a), one of them also b / B
+  float dd, ddr, dz, pi;      // numerators over d4, ddr the rest of dd
   static constexpr bool geno = false;
 };
 
@@ -124,6 +134,7 @@ PGLD_HD Hap make_hap(float c1, float c2, float c3, float c4) {
   const fast::Pop p = fast::make(c1, c2, c3, c4);
   Hap h;
   h.z = make_size(p.ns);
+  h.c1 = c1; h.c2 = c2; h.c3 = c3; h.c4 = c4;
   h.x = p.x;
   h.dA = p.dA;
   h.dB = p.dB;
@@ -131,36 +142,36 @@ PGLD_HD Hap make_hap(float c1, float c2, float c3, float c4) {
   h.pA = p.pA; h.qA = p.qA; h.pB = p.pB; h.qB = p.qB;
   h.hA = p.pA * p.qA;
   h.hB = p.pB * p.qB;
-  h.X1 = p.pA * p.pB - c1;
-  h.X2 = p.pA * p.qB - c2;
-  h.X3 = p.qA * p.pB - c3;
-  h.X4 = p.qA * p.qB - c4;
-  h.T1 = fmaf(p.pA, h.X4, -(c2 * p.qA));
-  h.T2 = fmaf(p.pA, h.X3, -(c1 * p.qA));
-  h.dd = fast::dd_num(p);
+  h.yb = p.pA * c4 + c2 * p.qA;
+  h.yB = p.pA * c3 + c1 * p.qA;
+  const fast::X2 d = fast::dd_split(p);
+  h.dd = d.s;
+  h.ddr = d.e;
   h.dz = fast::dz_num(p);
-  h.pi = fast::pi2_num(p);
+  h.pi = fast::pi2_pairs(p, h.hA, h.hB);
   return h;
 }
 
-PGLD_HD float ijij(const Hap& i, const Hap& j) {
-  return fmaf(i.X1, j.X4, fmaf(i.X2, j.X3, fmaf(i.X3, j.X2, fast::fmul(i.X4, j.X1))));
-}
 PGLD_HD float dz31(const Hap& t, const Hap& s) { return t.x * (t.dA * s.dB + t.dB * s.dA); }
+// heterozygosity of one draw each from a and b at the first / second SNP
+PGLD_HD float mixA(const Hap& a, const Hap& b) { return a.pA * b.qA + a.qA * b.pA; }
+PGLD_HD float mixB(const Hap& a, const Hap& b) { return a.pB * b.qB + a.qB * b.pB; }
+// sixteen times the draws: Y Y' + m m' (n n' - dA dA' - dB dB')
+PGLD_HD float ijij(const Hap& i, const Hap& j) {
+  const float g = i.z.n * j.z.n - i.dA * j.dA - i.dB * j.dB;
+  return fast::dot2(i.z.m * j.z.m, g, i.w, j.w);
+}
 // the four terms of pi2_ttts are equal
 PGLD_HD float triple(const Hap& t, const Hap& s, Den d, bool) {
-  return quot(fmaf(s.pB, t.T1, fast::fmul(s.qB, t.T2)), d);
+  return quot(fmaf(t.hA, mixB(t, s), -fmaf(t.yb, s.pB, fast::fmul(t.yB, s.qB))), d);
 }
 PGLD_HD float dz211(const Hap& s, const Hap& a, const Hap& b) {
   return s.x * (a.dA * b.dB + b.dA * a.dB);
 }
-// heterozygosity of one draw each from a and b at the first / second SNP
-PGLD_HD float mixA(const Hap& a, const Hap& b) { return a.pA * b.qA + a.qA * b.pA; }
-PGLD_HD float mixB(const Hap& a, const Hap& b) { return a.pB * b.qB + a.qB * b.pB; }
 // s and a at the first SNP, s and b at the second
 PGLD_HD float shared(const Hap& s, const Hap& a, const Hap& b) {
-  return fmaf(a.qA, fmaf(s.X1, b.qB, fast::fmul(s.X2, b.pB)),
-              fast::fmul(a.pA, fmaf(s.X3, b.qB, fast::fmul(s.X4, b.pB))));
+  const float y1 = s.c1 * b.qB + s.c2 * b.pB, y2 = s.c3 * b.qB + s.c4 * b.pB;
+  return fmaf(mixA(s, a), mixB(s, b), -fmaf(a.qA, y1, fast::fmul(a.pA, y2)));
 }
 
 // ---- genotypes -------------------------------------------------------------
@@ -171,8 +182,8 @@ struct Geno {
   float m1, m3;
   float y, w;               // n m4 - m1 m3 = D16 / 4, m1 m3 - m4
   float P2, R2, Q2, S2, hA, hB;
-  float X1, X2, X3, X4;     // distinct draws (1 +- c_I), (1 +- c_J): ++, +-, -+, --
-  float TA1, TA2, TB1, TB2; // distinct draws (1+c)(1-c) at I and 1 +- c at J; exchanged
+  float J1, J2, J3, J4;     // a quarter of sum (1 +- c_I)(1 +- c_J): ++, +-, -+, --
+  float EA1, EA2, EB1, EB2; // half the draws hA one of which has also 1 +- c_J; exchanged
   float u, v;               // n m7 - m1 m6, n m5 - m3 m2: a third draw's corrections
   float dd, dz, pi;         // numerators over 4, 2 and 16 d4
   static constexpr bool geno = true;
@@ -208,14 +219,13 @@ PGLD_HD Geno make_geno(const gmom::Mom& o) {
   g.P2 = n + m3; g.R2 = n - m3; g.Q2 = n + m1; g.S2 = n - m1;
   g.hA = g.P2 * g.R2 - (n - m6);
   g.hB = g.Q2 * g.S2 - (n - m2);
-  const float g3 = (n - 1.0f) * m3, g1 = (n - 1.0f) * m1;
-  const float s1 = g.z.m2 + g.w, s2 = g.z.m2 - g.w, t1 = g3 + g1, t2 = g3 - g1;
-  g.X1 = s1 + t1; g.X2 = s2 + t2; g.X3 = s2 - t2; g.X4 = s1 - t1;
-  const float eA = 2.0f * (g1 - m3 * m4 + m7), eB = 2.0f * (g3 - m1 * m4 + m5);
-  g.TA1 = fmaf(g.hA, g.z.k + m1, -eA);
-  g.TA2 = fmaf(g.hA, g.z.k - m1, eA);
-  g.TB1 = fmaf(g.hB, g.z.k + m3, -eB);
-  g.TB2 = fmaf(g.hB, g.z.k - m3, eB);
+  const float s1 = 0.25f * (n + m4), s2 = 0.25f * (n - m4), t1 = 0.25f * (m3 + m1), t2 = 0.25f * (m3 - m1);
+  g.J1 = s1 + t1; g.J2 = s2 + t2; g.J3 = s2 - t2; g.J4 = s1 - t1;
+  const float eA = g.z.m * m1 - m3 * m4 + m7, eB = g.z.m * m3 - m1 * m4 + m5;
+  g.EA1 = g.hA + eA;
+  g.EA2 = g.hA - eA;
+  g.EB1 = g.hB + eB;
+  g.EB2 = g.hB - eB;
   g.u = n * m7 - m1 * m6;
   g.v = n * m5 - m3 * m2;
   // one population: the polynomials cancel heavily, so in 64-bit integers
@@ -226,8 +236,12 @@ PGLD_HD Geno make_geno(const gmom::Mom& o) {
   return g;
 }
 
+PGLD_HD float mixA(const Geno& a, const Geno& b) { return a.z.n * b.z.n - a.m3 * b.m3; }
+PGLD_HD float mixB(const Geno& a, const Geno& b) { return a.z.n * b.z.n - a.m1 * b.m1; }
+// a quarter of the draws: w w' + m m' (n n' - m3 m3' - m1 m1')
 PGLD_HD float ijij(const Geno& i, const Geno& j) {
-  return fmaf(i.X1, j.X4, fmaf(i.X2, j.X3, fmaf(i.X3, j.X2, fast::fmul(i.X4, j.X1))));
+  const float g = i.z.n * j.z.n - i.m3 * j.m3 - i.m1 * j.m1;
+  return fast::dot2(i.z.m * j.z.m, g, i.w, j.w);
 }
 // y (m3 m1' + m1 m3') - (u m1' + v m3'): the two corrections are summed exactly
 // (TwoProduct, TwoSum; Ogita, Rump and Oishi, "Accurate sum and dot product",
@@ -240,20 +254,20 @@ PGLD_HD float dz31(const Geno& t, const Geno& s) {
                              fast::fadd(pe, qe));
   return fast::fsub(fmaf(t.y, t.m3 * s.m1 + t.m1 * s.m3, -h), l);
 }
-// t twice at the first SNP, and twice at the second
+// half the draws with t twice at the first SNP, and twice at the second
 PGLD_HD float triple(const Geno& t, const Geno& s, Den d, bool first) {
-  const float a = quot(fmaf(t.TA1, s.S2, fast::fmul(t.TA2, s.Q2)), d);
-  const float b = quot(fmaf(t.TB1, s.R2, fast::fmul(t.TB2, s.P2)), d);
+  const float a = quot(fmaf(t.hA, mixB(t, s), -fmaf(t.EA1, s.S2, fast::fmul(t.EA2, s.Q2))), d);
+  const float b = quot(fmaf(t.hB, mixA(t, s), -fmaf(t.EB1, s.R2, fast::fmul(t.EB2, s.P2))), d);
   return first ? two_two(a, b) : two_two(b, a);
 }
 PGLD_HD float dz211(const Geno& s, const Geno& a, const Geno& b) {
   return s.y * (a.m3 * b.m1 + b.m3 * a.m1);
 }
-PGLD_HD float mixA(const Geno& a, const Geno& b) { return a.z.n * b.z.n - a.m3 * b.m3; }
-PGLD_HD float mixB(const Geno& a, const Geno& b) { return a.z.n * b.z.n - a.m1 * b.m1; }
+// a quarter of the draws
 PGLD_HD float shared(const Geno& s, const Geno& a, const Geno& b) {
-  return fmaf(a.R2, fmaf(s.X1, b.S2, fast::fmul(s.X2, b.Q2)),
-              fast::fmul(a.P2, fmaf(s.X3, b.S2, fast::fmul(s.X4, b.Q2))));
+  return fmaf(mixA(s, a), mixB(s, b),
+              -fmaf(a.R2, fmaf(s.J1, b.S2, fast::fmul(s.J2, b.Q2)),
+                    fast::fmul(a.P2, fmaf(s.J3, b.S2, fast::fmul(s.J4, b.Q2)))));
 }
 
 // denominator M a b of a class
@@ -262,6 +276,8 @@ PGLD_HD Den class_den(float a, float b) {
   return make_den(F::geno ? a * b : round_den<M>(a, b));
 }
 
+PGLD_HD float dd_quot(const Hap& h, Den d) { return quot(h.dd, h.ddr, d); }
+PGLD_HD float dd_quot(const Geno& g, Den d) { return quot(g.dd, d); }
 // D of one population (x of the haplotype, y of the genotype features)
 PGLD_HD float dval(const Hap& h) { return h.x; }
 PGLD_HD float dval(const Geno& g) { return g.y; }
@@ -276,7 +292,7 @@ PGLD_HD void eval(const F (&f)[P], Sink&& sink) {
 #pragma unroll
     for (int i = 0; i < P; ++i) {
       const Den d = class_den<F, 1>(f[i].z.m2, f[i].z.m2b);
-      sink(k++, quot(f[i].dd, d));
+      sink(k++, dd_quot(f[i], d));
       sink(k++, quot(f[i].dz, d));
       sink(k++, quot(f[i].pi, d));
     }
@@ -385,13 +401,13 @@ inline std::vector<Place> order(int P, bool geno) {
       o.push_back({dz(i, j, j), geno ? 0.5f : 1.0f});
       o.push_back({dz(j, i, i), geno ? 0.5f : 1.0f});
       o.push_back({pi2(i, i, j, j), geno ? 1.0f / 32 : 0.5f});
-      o.push_back({pi2(i, j, i, j), geno ? 1.0f / 64 : 0.25f});
+      o.push_back({pi2(i, j, i, j), 1.0f / 16});
     }
   for (int i = 0; i < P; ++i)
     for (int j = 0; j < P; ++j)
       if (j != i) {
         o.push_back({dz(i, i, j), geno ? 0.25f : 0.5f});
-        o.push_back({pi2(i, i, i, j), geno ? 1.0f / 64 : 0.5f});
+        o.push_back({pi2(i, i, i, j), geno ? 1.0f / 32 : 0.5f});
       }
   for (int s = 0; s < P; ++s)
     for (int a = 0; a < P; ++a)
@@ -399,7 +415,7 @@ inline std::vector<Place> order(int P, bool geno) {
         if (a != s && b != s) {
           o.push_back({dz(s, a, b), geno ? 0.25f : 0.5f});
           o.push_back({pi2(s, s, a, b), geno ? 1.0f / 32 : 0.25f});
-          o.push_back({pi2(s, a, s, b), geno ? 1.0f / 128 : 0.125f});
+          o.push_back({pi2(s, a, s, b), geno ? 1.0f / 32 : 0.125f});
         }
   if (P == 4)
     for (int b = 1; b < 4; ++b) {
