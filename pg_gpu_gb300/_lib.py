@@ -18,6 +18,7 @@ LIB_PATH = os.path.join(HERE, "libpgld.so")
 MAX_POPS = 4
 F64, F32 = 0, 1
 FORM_PLAIN, FORM_TC = 0, 1
+ERR_TOO_LARGE, ERR_NO_MEMORY = -3, -6
 
 # enum pgld_kind
 DD_II, DD_IJ, DZ_III, DZ_IIJ, DZ_IJI, DZ_IJJ, DZ_IJK = range(7)

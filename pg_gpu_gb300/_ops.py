@@ -795,15 +795,19 @@ def geno_binned_sums(pops, pos_d, bins, max_dist=None, bin_coord=None, form="aut
     """(sums (n_bins, n_stats) float64, pair counts (n_bins,) int64), genotype statistics.
 
     form: "tc" (moments from tcgen05 MMAs), "plain" (AND + popcount) or
-    "auto" (tensor cores whenever they apply)."""
+    "auto" (tensor cores whenever they apply; for several populations the
+    popcount form where their operands, 96 bytes per SNP and 32 individuals of
+    every population, do not fit beside what the device holds)."""
+    retry = False
     if form == "auto":
         # two populations of 500 individuals x 100,000 SNPs to 100 kb: 94 ms
-        # in the popcount form, 9 ms here.  Above 2,048 individuals the
+        # in the popcount form, 4.7 ms here.  Above 2,048 individuals the
         # statistics of several populations go through the exact per-pair term
         # table, which dominates either form (the popcount one is slightly
         # faster then)
         small = len(pops) == 1 or max(pk.n_words for pk in pops) <= 64
         form = "tc" if small and geno_tc_applies(pops) else "plain"
+        retry = form == "tc" and len(pops) > 1
     if form not in ("tc", "plain"):
         raise ValueError("form must be 'tc', 'plain' or 'auto'")
     torch = _torch()
@@ -820,10 +824,16 @@ def geno_binned_sums(pops, pos_d, bins, max_dist=None, bin_coord=None, form="aut
     md = float(bins_np[-1]) if max_dist is None else float(max_dist)
     bc = None if bin_coord is None else L.as_device(bin_coord, np.float64)
     h = L.handle()
-    L.check(L.lib().pgld_geno_binned_sums_form(h, ctypes.byref(geno_panel(pops)), L.ptr(pos_d), md,
-                                               L.ptr(bc), L.ptr(bins_d), n_bins, L.ptr(sums),
-                                               L.ptr(cnt), 1 if form == "tc" else 0,
-                                               L.stream_ptr()), h)
+
+    def run(tc):
+        return L.lib().pgld_geno_binned_sums_form(
+            h, ctypes.byref(geno_panel(pops)), L.ptr(pos_d), md, L.ptr(bc), L.ptr(bins_d), n_bins,
+            L.ptr(sums), L.ptr(cnt), L.FORM_TC if tc else L.FORM_PLAIN, L.stream_ptr())
+
+    rc = run(form == "tc")
+    if rc in (L.ERR_NO_MEMORY, L.ERR_TOO_LARGE) and retry:
+        rc = run(False)
+    L.check(rc, h)
     return sums, cnt
 
 
