@@ -160,16 +160,16 @@ def tc_mma_peak(gpu_index, launch_ms=20.0, sustained_s=3.0):
     return _PEAK
 
 
-def tc_roofline(pairs_per_s, ops_per_pair, basis, gpu_index=0, sm_mhz=None):
+def tc_roofline(pairs_per_s, ops_per_pair, basis, gpu_index=0, sm_mhz=None, bound="tensor"):
     """Tensor-pipe roofline of a tensor-core workload: ops_per_pair int8-
-    equivalent operations per pair (the algorithmic contraction) per second,
-    against the measured E4M3 tcgen05 burst rate of this GPU; basis names the
-    timed region.  frac_clock_normalised divides each rate by the median SM
+    equivalent operations per pair (those that the kernel's contraction executes)
+    per second, against the measured E4M3 tcgen05 burst rate of this GPU; basis
+    names the timed region, bound what limits the kernel.  frac_clock_normalised divides each rate by the median SM
     clock it ran at."""
     pk = tc_mma_peak(gpu_index)
     peak = pk["burst"]
     achieved = pairs_per_s * ops_per_pair / 1e12
-    out = {"bound": "tensor", "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
+    out = {"bound": bound, "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
            "frac": achieved / peak, "traffic": None, "ops_per_pair": ops_per_pair,
            "peak_source": "measured on this GPU: tcgen05 kind::f8f6f4 M128 N128 K32 from "
                           "shared memory on every SM (pgld_tc_mma_rate), burst of ten ~20 ms "
@@ -621,8 +621,12 @@ def run_windows(args):
         "config": {"workload": "windows512", "haplotypes": 400, "windows": int(len(sizes)),
                    "n_snp": int(sizes.sum()), "pairs": n_pairs, "form": "tc"},
         "kernel_ms": k_ms,
-        "roofline": tc_roofline(n_pairs / (k_ms / 1e3), 8 * 400,
-                                "window kernel launches, CUDA events on the call's stream"),
+        # without missing data a pair's statistics follow from n11 alone: one
+        # operand row per SNP, 2 H operations a pair instead of 8 H, and the
+        # epilogue's float32 instructions are the limit
+        "roofline": tc_roofline(n_pairs / (k_ms / 1e3), (8 if pk.has_missing else 2) * 400,
+                                "window kernel launches, CUDA events on the call's stream",
+                                bound="tensor" if pk.has_missing else "float32 pipe"),
         "plain_one_launch": {"ms_per_step": t_plain, "value": n_pairs / (t_plain / 1e3)},
         "plain_per_window_launches": {"ms_per_step": t_per, "value": n_pairs / (t_per / 1e3),
                                       "ratio_tc_one_launch_over_this": t_per / t_one}}),
