@@ -690,22 +690,24 @@ __global__ void __launch_bounds__(256) table_kernel(StatsArgs a, i64 n_pairs, bo
       put_nd(2, pgld::pi2_iiii(p));
     } else {
       const pgld::PopC q = load_pop(a, 1, k, wide);
-      auto dz_mixed = [](const pgld::PopC& t, const pgld::PopC& u) {
-        const pgld::ND x = pgld::dz_iij(t, u), y = pgld::dz_iji(t, u);
-        return pgld::ND{x.num + y.num, 2 * x.den};
+      // the mean of two quotients of one denominator, halved last: twice the
+      // denominator would pass 2^63 from 46,341 haplotypes on
+      auto put_mean = [&](int s, const pgld::ND& x, const pgld::ND& y) {
+        put(s, x.num + y.num, x.den);
+        o[s] *= 0.5;
       };
       put_nd(0, pgld::dd_ii(p));
       put_nd(1, pgld::dd_ij(p, q));
       put_nd(2, pgld::dd_ii(q));
       put_nd(3, pgld::dz_iii(p));
-      put_nd(4, dz_mixed(p, q));
+      put_mean(4, pgld::dz_iij(p, q), pgld::dz_iji(p, q));
       put_nd(5, pgld::dz_ijj(p, q));
       put_nd(6, pgld::dz_ijj(q, p));
-      put_nd(7, dz_mixed(q, p));
+      put_mean(7, pgld::dz_iij(q, p), pgld::dz_iji(q, p));
       put_nd(8, pgld::dz_iii(q));
       put_nd(9, pgld::pi2_iiii(p));
       put_nd(10, pgld::pi2_triple(p, q));
-      put_nd(11, pgld::pi2_iikk_sym(p, q));
+      put_mean(11, pgld::pi2_iikk(p, q), pgld::pi2_iikk(q, p));
       put_nd(12, pgld::pi2_ijij(p, q));
       put_nd(13, pgld::pi2_triple(q, p));
       put_nd(14, pgld::pi2_iiii(q));

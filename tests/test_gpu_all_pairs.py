@@ -111,3 +111,23 @@ def test_rogers_huff_entry_with_its_own_sites():
     L.check(L.lib().pgld_geno_rogers_huff(h, L.ptr(pk.planes), pk.n_words, pk.n_rows, 70, L.ptr(out),
                                           L.stream_ptr()), h)
     assert torch.equal(out, _ops.rogers_huff_all(pk))
+
+
+# where the largest denominators of a table come near 2^63: the table's kernel and
+# the general one see the same integers
+@pytest.mark.parametrize("n", [38_000, 46_300, 46_400, 50_000, 55_000])
+def test_table_at_the_largest_sample_sizes(n):
+    from pg_gpu_gb300.ld_pipeline import spec_terms
+    rng = np.random.default_rng(n)
+    c = [torch.as_tensor(rng.multinomial(n, rng.dirichlet(np.full(4, 0.7), 500)).astype(np.int32),
+                         device="cuda") for _ in range(2)]
+    got = np_(_ops.stats(c, [None, None], spec_terms(2), 15))
+    want = np_(_ops.stats(c, [None, None], spec_terms(2) + [(15, 0, (0,), 1.0)], 16))[:, :15]
+    assert np.all(np.abs(got - want) <= 1e-14 * np.abs(want) + 1e-15 * np.abs(want).max(0))
+    x = [v.cpu().numpy().astype(object) for v in c]
+    (a1, a2, a3, a4), (b1, b2, b3, b4) = (tuple(v.T) for v in x)
+    # Dz_0_0_1 against exact integers
+    D, dA, dB = a1 * a4 - a2 * a3, a3 + a4 - a1 - a2, a2 + a4 - a1 - a3
+    num = D * (dA * (b2 + b4 - b1 - b3) + dB * (b3 + b4 - b1 - b2))
+    exact = np.array([float(v) for v in num]) / float(2 * n * n * (n - 1) * (n - 2))
+    np.testing.assert_allclose(got[:, 4], exact, rtol=1e-14)
