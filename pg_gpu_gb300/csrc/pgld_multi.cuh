@@ -156,14 +156,15 @@ PGLD_HD float dz31(const Hap& t, const Hap& s) { return t.x * (t.dA * s.dB + t.d
 // heterozygosity of one draw each from a and b at the first / second SNP
 PGLD_HD float mixA(const Hap& a, const Hap& b) { return a.pA * b.qA + a.qA * b.pA; }
 PGLD_HD float mixB(const Hap& a, const Hap& b) { return a.pB * b.qB + a.qB * b.pB; }
+// twice mixB, from what ijij needs of the pair
+PGLD_HD float mix2(const Hap& a, const Hap& b) { return a.z.n * b.z.n - a.dB * b.dB; }
 // sixteen times the draws: Y Y' + m m' (n n' - dA dA' - dB dB')
 PGLD_HD float ijij(const Hap& i, const Hap& j) {
-  const float g = i.z.n * j.z.n - i.dA * j.dA - i.dB * j.dB;
-  return fast::dot2(i.z.m * j.z.m, g, i.w, j.w);
+  return fast::dot2(i.z.m * j.z.m, mix2(i, j) - i.dA * j.dA, i.w, j.w);
 }
 // the four terms of pi2_ttts are equal
 PGLD_HD float triple(const Hap& t, const Hap& s, Den d, bool) {
-  return quot(fmaf(t.hA, mixB(t, s), -fmaf(t.yb, s.pB, fast::fmul(t.yB, s.qB))), d);
+  return quot(fmaf(t.hA, 0.5f * mix2(t, s), -fmaf(t.yb, s.pB, fast::fmul(t.yB, s.qB))), d);
 }
 PGLD_HD float dz211(const Hap& s, const Hap& a, const Hap& b) {
   return s.x * (a.dA * b.dB + b.dA * a.dB);
