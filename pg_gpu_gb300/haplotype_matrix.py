@@ -338,6 +338,7 @@ class HaplotypeMatrix:
             self._haplotypes = self._haplotypes.cpu().numpy()
             self._positions = self._positions.cpu().numpy()
             self._device = "CPU"
+            self._pinned = None  # the device matrix may have been changed since
             self._packed = {}
 
     def _pos_np(self):

@@ -117,3 +117,16 @@ def test_host_array_set_on_a_device_matrix():
     got, want = ([(p.planes, p.valid) for p in m.packed_all(["a", "b"])] for m in (hm, ref))
     for a, b in zip(got, want):
         assert all(torch.equal(x, y) for x, y in zip(a, b))
+
+
+@pytest.mark.parametrize("ac", [True, False])
+def test_pinned_matrix_changed_on_the_device(ac):
+    hap, pos = panel()
+    hm = HaplotypeMatrix(torch.as_tensor(hap).pin_memory(), pos)
+    hm.transfer_to_gpu()
+    hm.haplotypes[:, 5::9] = 0
+    changed = hm.haplotypes.cpu().numpy()
+    hm.transfer_to_cpu()
+    got = hm.compute_ld_statistics_gpu_single_pop(BINS, raw=True, ac_filter=ac)
+    ref = HaplotypeMatrix(torch.as_tensor(changed, device="cuda"), pos)
+    assert got == ref.compute_ld_statistics_gpu_single_pop(BINS, raw=True, ac_filter=ac)
