@@ -123,6 +123,10 @@ def compute_ld_statistics(vcf_file=None, rec_map_file=None, pop_file=None, pops=
             lists, n = [mat.sample_sets[p] for p in pops], mat.genotypes.shape[0]
         else:
             lists, n = [mat._pop_rows(p) for p in pops], mat.haplotypes.shape[0]
+        # no mean of no rows (an empty list, as from a population file that names
+        # none of the samples)
+        if any(isinstance(r, list) and not r for r in lists):
+            raise IndexError("a population has no rows")
         rows = _ops.device_rows(lists, n)
     ld_sums = _compute_ld_sums(mat, pops, bins, gen, max_bp, use_genotypes, rows)
     het = _compute_heterozygosity(mat, pops, use_genotypes, rows)

@@ -138,3 +138,15 @@ def test_heterozygosity_repeats_to_the_last_bit(M):
     assert first.shape == (6,) and (M > 0 or not first.any())
     for _ in range(30):
         assert np.array_equal(_ops.heterozygosity(s, [None] * 3, n, 1), first)
+
+
+@pytest.mark.parametrize("geno", [False, True])
+def test_moments_of_an_empty_population_are_refused(geno):
+    from pg_gpu_gb300 import moments_ld
+    from pg_gpu_gb300.genotype_matrix import GenotypeMatrix
+    from pg_gpu_gb300.haplotype_matrix import HaplotypeMatrix
+    x = torch.as_tensor(np.random.default_rng(2).integers(0, 2, (12, 40)).astype(np.int8), device="cuda")
+    m = (GenotypeMatrix if geno else HaplotypeMatrix)(x, np.arange(40), sample_sets={"a": [0, 1, 2, 3], "b": []})
+    with pytest.raises(IndexError):
+        moments_ld.compute_ld_statistics(pops=["a", "b"], bp_bins=[0, 10, 20], report=False, use_genotypes=geno,
+                                         **{"genotype_matrix" if geno else "haplotype_matrix": m})
