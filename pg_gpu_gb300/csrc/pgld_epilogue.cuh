@@ -193,13 +193,14 @@ PGLD_HD float pi2_num(const Pop& p) {
 // rounds once in effect.  Root mean square error of the numerators in units of
 // 2^-24 (60,000 pairs, 200 - 2,000 haplotypes): 0.40 - 0.45, where the expanded
 // polynomials by Kahan's algorithm have 0.40 - 0.49 (and take 63 operations for
-// two populations, these 33), and products of draws over distinct haplotypes
+// two populations, these 35), and products of draws over distinct haplotypes
 // from one population, with two to four roundings (30 operations), 0.43 - 0.62.
 // hA = pA qA and hB = pB qB; yb, yB = the draws (A, a) of which one is also b / B;
 // mixB = the draws (b, B) of one haplotype from each population
+// (the choices that take one twice: a (n - 1 + 2 s) + b (n - 1 + 2 t) = (a + b) (2 n -
+// 1) + x e, at least half the first product)
 PGLD_HD float pi2_pairs(const Pop& p, float hA, float hB) {
-  const float m = p.ns - 1.0f;
-  return fmaf(hA, hB, -fmaf(p.a, fmaf(p.s, 2.0f, m), fmul(p.b, fmaf(p.t, 2.0f, m))));
+  return fmaf(hA, hB, fmaf(p.a + p.b, fmaf(p.ns, -2.0f, 1.0f), fmul(p.x, -p.e)));
 }
 // pi2(t,t,t,s) times 2
 PGLD_HD float triple_num2(const Pop& t, float hA, float mixB, const Pop& s) {

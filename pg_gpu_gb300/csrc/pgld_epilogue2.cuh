@@ -111,15 +111,14 @@ PGLD_HD V pi2_num(const Pop& p) {
   const V w = vfma(vsub(vs(2.0f), p.ns), p.t, vadd(p.x, p.m1));
   return dot2(p.a, pn, p.x, w);
 }
-// fast::pi2_pairs with nm = 1 - n, and the negative of fast::triple_num2 with
-// nmix = -mixB: operands negated where they are formed, not in packed
-// instructions of their own (13.31 -> 13.25 ms for two populations of 1,000, a
-// chromosome arm)
-PGLD_HD V pi2_pairs(const Pop& p, V hA, V hB, V nm) {
-  return vfma(hA, hB, vfma(p.a, vfma(p.s, vs(-2.0f), nm), vmul(p.b, vfma(p.t, vs(-2.0f), nm))));
+// fast::pi2_pairs, and the negative of fast::triple_num2 with nmix = -mixB: operands
+// are negated where they are formed, since a packed negation is an instruction of
+// its own (13.31 -> 13.25 ms for two populations of 1,000, a chromosome arm)
+PGLD_HD V pi2_pairs(const Pop& p, V hA, V hB) {
+  const V k = vfma(p.ns, vs(-2.0f), vs(1.0f)), ne = vmul(p.e, vs(-1.0f));
+  return vfma(hA, hB, vfma(vadd(p.a, p.b), k, vmul(p.x, ne)));
 }
-PGLD_HD V triple_neg2(const Pop& t, V hA, V nmix, const Pop& s) {
-  const V yb = vfma(t.pA, t.c4, vmul(t.c2, t.qA)), yB = vfma(t.pA, t.c3, vmul(t.c1, t.qA));
+PGLD_HD V triple_neg2(V hA, V yb, V yB, V nmix, const Pop& s) {
   return vfma(hA, nmix, vfma(yb, s.pB, vmul(yB, s.qB)));
 }
 
@@ -156,37 +155,47 @@ PGLD_HD void stats2_to(const Pop& p, const Pop& q, const float4* T4, Sink&& sink
 #else
   const V r22 = vmul(rp.r2, rq.r2);
 #endif
-  const V wp = vfma(p.dA, p.dB, p.e), wq = vfma(q.dA, q.dB, q.e);
-  sink(0, dd_num(p), rp.r4);
+  // what needs one population first: its counts and most of its features are then
+  // done with, and the registers hold (the binned kernel spills 100 bytes more
+  // where the statistics of a kind stand together)
+  struct Own {
+    V w, hA, hB, yb, yB;
+  };
+  auto own = [&](const Pop& t, V r4, int k) -> Own {
+    Own o;
+    o.w = vfma(t.dA, t.dB, t.e);
+    o.hA = vmul(t.pA, t.qA);
+    o.hB = vmul(t.pB, t.qB);
+    o.yb = vfma(t.pA, t.c4, vmul(t.c2, t.qA));
+    o.yB = vfma(t.pA, t.c3, vmul(t.c1, t.qA));
+    sink(k ? 2 : 0, dd_num(t), r4);
+    sink(k ? 8 : 3, dz_num(t, o.w), r4);
+    sink(k ? 14 : 9, pi2_pairs(t, o.hA, o.hB), r4);
+    return o;
+  };
+  const Own op = own(p, rp.r4, 0), oq = own(q, rq.r4, 1);
   sink(1, vmul(p.x, q.x), r22);
-  sink(2, dd_num(q), rq.r4);
-  sink(3, dz_num(p, wp), rp.r4);
-  sink(8, dz_num(q, wq), rq.r4);
-  sink(5, vmul(p.x, wq), r22);
-  sink(6, vmul(q.x, wp), r22);
-  // -2 mixB and -(n n' - dA dA' - dB dB')
-  const V nmp = vfma(p.ns, vs(-1.0f), vs(1.0f)), nmq = vfma(q.ns, vs(-1.0f), vs(1.0f));
-  const V nmix2 = vfma(p.dB, q.dB, vmul(p.ns, vmul(q.ns, vs(-1.0f)))), nmix = vmul(nmix2, vs(0.5f));
-  sink(12, dot2(vmul(nmp, q.m1), vfma(p.dA, q.dA, nmix2), wp, wq), r22);  // x kPost12
-  const V uAp = vmul(p.pA, p.qA), uAq = vmul(q.pA, q.qA), uBp = vmul(p.pB, p.qB), uBq = vmul(q.pB, q.qB);
-  sink(11, vfma(uAp, uBq, vmul(uAq, uBp)), r22);                          // x kPost11
-  sink(9, pi2_pairs(p, uAp, uBp, nmp), rp.r4);
-  sink(14, pi2_pairs(q, uAq, uBq, nmq), rq.r4);
+  sink(5, vmul(p.x, oq.w), r22);
+  sink(6, vmul(q.x, op.w), r22);
+  sink(11, vfma(op.hA, oq.hB, vmul(oq.hA, op.hB)), r22);  // x kPost11
   const V dc = vfma(p.dA, q.dB, vmul(p.dB, q.dA));
+  // -2 mixB and -(n n' - dA dA' - dB dB')
+  const V nmix2 = vfma(p.dB, q.dB, vmul(p.ns, vmul(q.ns, vs(-1.0f)))), nmix = vmul(nmix2, vs(0.5f));
+  sink(12, dot2(vmul(vfma(p.ns, vs(-1.0f), vs(1.0f)), q.m1), vfma(p.dA, q.dA, nmix2), op.w, oq.w), r22);  // x kPost12
 #if PGLD_F2_SSCALE
   const V h31p = vmul_s(rp.r3h, rq.inv);
 #else
   const V h31p = vmul(rp.r3h, rq.inv);
 #endif
   sink(4, vmul(p.x, dc), h31p);
-  sink(10, triple_neg2(p, uAp, nmix, q), h31p);  // negative
+  sink(10, triple_neg2(op.hA, op.yb, op.yB, nmix, q), h31p);  // negative
 #if PGLD_F2_SSCALE
   const V h31q = vmul_s(rq.r3h, rp.inv);
 #else
   const V h31q = vmul(rq.r3h, rp.inv);
 #endif
   sink(7, vmul(q.x, dc), h31q);
-  sink(13, triple_neg2(q, uAq, nmix, p), h31q);  // negative
+  sink(13, triple_neg2(oq.hA, oq.yb, oq.yB, nmix, p), h31q);  // negative
 }
 
 // the sink's products, statistics 10 - 13 still without their post factors
