@@ -145,6 +145,12 @@ def _host_readable(hap):
             and hap.dim() == 2 and hap.stride(1) == 1 and hap.is_pinned())
 
 
+def is_device_int8(x):
+    """Whether x is an int8 matrix on the device (of any strides)."""
+    torch = _torch()
+    return isinstance(x, torch.Tensor) and x.is_cuda and x.dtype == torch.int8 and x.dim() == 2
+
+
 # rules of kept_sites (pgld_keep_sites)
 KEEP_BIALLELIC, KEEP_SEGREGATING, KEEP_DIPLOID = range(3)
 
@@ -155,7 +161,9 @@ def site_counts(x, rows=None, sums=True, flags=False):
     (sum of the values above 0, number of values >= 0, presence bits of 0 / 1 /
     above 1), None where not asked."""
     torch = _torch()
-    if not _host_readable(x):
+    if is_device_int8(x):
+        x = x.contiguous()
+    elif not _host_readable(x):
         x = L.as_device(x, np.int8)
     dev = x.device if x.is_cuda else torch.device("cuda", torch.cuda.current_device())
     n_total, n = x.shape

@@ -492,7 +492,7 @@ class HaplotypeMatrix:
             return h if h.stride(0) >= h.shape[1] else None
         h = self._haplotypes
         if self._device == "GPU":
-            return L.as_device(h) if _is_torch(h) and h.is_cuda and str(h.dtype) == "torch.int8" else None
+            return h.contiguous() if _ops.is_device_int8(h) else None
         ok = isinstance(h, np.ndarray) and h.dtype == np.int8 and min(h.strides) >= 0
         return L.as_device(h) if ok else None
 
