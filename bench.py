@@ -164,8 +164,8 @@ def tc_roofline(pairs_per_s, ops_per_pair, basis, gpu_index=0, sm_mhz=None, boun
     """Tensor-pipe roofline of a tensor-core workload: ops_per_pair int8-
     equivalent operations per pair (those that the kernel's contraction executes)
     per second, against the measured E4M3 tcgen05 burst rate of this GPU; basis
-    names the timed region, bound what limits the kernel.  frac_clock_normalised divides each rate by the median SM
-    clock it ran at."""
+    names the timed region, bound what limits the kernel.  frac_clock_normalised
+    divides each rate by the median SM clock it ran at."""
     pk = tc_mma_peak(gpu_index)
     peak = pk["burst"]
     achieved = pairs_per_s * ops_per_pair / 1e12

@@ -197,8 +197,8 @@ PGLD_HD float pi2_num(const Pop& p) {
 // from one population, with two to four roundings (30 operations), 0.43 - 0.62.
 // hA = pA qA and hB = pB qB; yb, yB = the draws (A, a) of which one is also b / B;
 // mixB = the draws (b, B) of one haplotype from each population
-// (the choices that take one twice: a (n - 1 + 2 s) + b (n - 1 + 2 t) = (a + b) (2 n -
-// 1) + x e, at least half the first product)
+// the choices that take one twice: a (n - 1 + 2 s) + b (n - 1 + 2 t) = (a + b) (2 n -
+// 1) + x e, where x e takes at most half of the first product back
 PGLD_HD float pi2_pairs(const Pop& p, float hA, float hB) {
   return fmaf(hA, hB, fmaf(p.a + p.b, fmaf(p.ns, -2.0f, 1.0f), fmul(p.x, -p.e)));
 }
